@@ -1,0 +1,74 @@
+"""GPU: rows whose column span lies in a shared-memory bitmap — sizes at the
+edges of its words, units, tiles and register-held products, both phases."""
+import numpy as np
+import pytest
+
+import oracle
+from helpers import TOL32, TOL64, check_product, check_sum
+from trident_b200 import ops
+from trident_b200._lib import TSPG_F_ACC_FUSE
+from trident_b200.csr import HostCSR
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(lens, n, rng, dup=False, sort=True):
+    rp = np.zeros(len(lens) + 1, np.int64)
+    rp[1:] = np.cumsum(lens)
+    cols = [rng.choice(n, size=k, replace=dup) for k in lens]
+    cols = np.concatenate([np.sort(c) if sort else c for c in cols]).astype(np.int32)
+    return HostCSR(len(lens), n, rp, cols, rng.uniform(-1, 1, cols.size))
+
+
+def _pair(n, dup, seed):
+    """A rows of 1 ... 1100 entries (staging rounds of 128 / 256 / 512) over B
+    rows of 0, 1, 31 ... 33, 127 ... 129 and 400 entries; the first and last
+    columns are hit."""
+    rng = np.random.default_rng(seed)
+    blens = np.minimum(rng.choice([0, 1, 1, 2, 5, 31, 32, 33, 127, 128, 129, 400], size=1200), n)
+    blens[:3] = [1, 2, 1]
+    B = _rows(blens, n, rng, dup=dup, sort=not dup)
+    B.col[0], B.col[-1] = n - 1, 0
+    alens = [0, 1, 2, 3, 7, 15, 16, 17, 31, 32, 33, 64, 127, 128, 129, 255, 256, 257, 511, 513, 1100] * 3
+    return _rows(alens, 1200, rng), B
+
+
+@pytest.mark.parametrize("dup", [False, True])
+@pytest.mark.parametrize("n", [700, 1023, 1024, 1025, 4097, 33000, 150000])
+def test_span_rows_match_the_oracle(ctx, n, dup):
+    A, B = _pair(n, dup, seed=n)
+    dA, dB = A.to_device(rowptr_bits=32), B.to_device(rowptr_bits=32)
+    check_product(ops.spgemm(ctx, dA, dB), A, B, tol=TOL64)
+    plan = ops.Plan(ctx, dA, dB)  # new values of the same pattern
+    A2 = HostCSR(A.nrows, A.ncols, A.rowptr, A.col, A.val[::-1].copy())
+    check_product(plan.numeric(A2.to_device(rowptr_bits=32), dB), A2, B)
+    plan.close()
+
+
+@pytest.mark.parametrize("n", [1025, 33000])
+def test_span_rows_fp32_wide_offsets(ctx, n):
+    A, B = _pair(n, False, seed=5 * n)
+    A, B = (HostCSR(M.nrows, M.ncols, M.rowptr, M.col, M.val.astype(np.float32).astype(np.float64))
+            for M in (A, B))
+    check_product(ops.spgemm(ctx, A.to_device(rowptr_bits=64, val_bits=32), B.to_device(rowptr_bits=64, val_bits=32)),
+                  A, B, tol=TOL32)
+
+
+def test_span_rows_with_an_addend(ctx):
+    A, B = _pair(4097, False, seed=11)
+    E = _rows(np.tile([0, 300, 1500], 21), 4097, np.random.default_rng(3))
+    C = ops.sp_mma(ctx, A.to_device(), B.to_device(), E.to_device(), flags=TSPG_F_ACC_FUSE)
+    rp, cj, cx, _ = oracle.spgemm(A, B)
+    check_sum(C, HostCSR(A.nrows, B.ncols, rp, cj, cx), E)
+
+
+def test_dense_rows_two_ctas_per_sm():
+    # more DENSE rows than 16 per SM, their outputs on both sides of the slots
+    # that fit shared memory
+    c = ops.Context(0)
+    c.set_tuning({"num_lim": [256, 1024, 2048, 2048]})
+    rng = np.random.default_rng(7)
+    B = _rows(np.full(600, 900), 60000, rng)
+    A = _rows(rng.choice([5, 40], size=2600), 600, rng)
+    check_product(ops.spgemm(c, A.to_device(rowptr_bits=64), B.to_device(rowptr_bits=64)), A, B)
+    c.close()

@@ -18,7 +18,7 @@
 #include <new>
 #include <vector>
 
-#include "spgemm_cluster.cuh"
+#include "spgemm_span.cuh"
 
 namespace tspg {
 
@@ -217,16 +217,7 @@ template <typename PT, typename VT>
 static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
   tspg_ctx *ctx = b->ctx;
   const int nprod = (int)b->A.size();
-  TSPG_CUDA(ctx, cudaFuncSetAttribute(k_phase<PT, VT, false>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kDynSmem));
-  TSPG_CUDA(ctx, cudaFuncSetAttribute(k_phase<PT, VT, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kDynSmem));
-  TSPG_CUDA(ctx, cudaFuncSetAttribute(k_dense_rank<PT, VT>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kDynSmem));
-  TSPG_CUDA(ctx, cudaFuncSetAttribute(k_groups<PT, VT, false>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupDynSmem));
-  TSPG_CUDA(ctx, cudaFuncSetAttribute(k_groups<PT, VT, true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupDynSmem));
+  TSPG_TRY((set_smem_attr<PT, VT>(ctx->device)));
   // the cluster form must be launchable before it is captured (k_phase leaves
   // its rows alone)
   if (ctx->tune.cluster && cluster_slots<PT, VT>(ctx->device, ctx->tune.cluster) <= 0)
@@ -326,8 +317,12 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
   const int64_t nb = (R + kScanTile - 1) / kScanTile;
   int64_t *errw = ctx->d_words + kErrWord;
 
+  int64_t ncols = 0;
+  for (int p = 0; p < nprod; ++p) ncols = std::max(ncols, b->B[p].ncols);
+
   // ---- graph 1: symbolic
   if (rebuild) {
+    int row_kernels = 0;
     cudaGraph_t g;
     TSPG_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(b->sched, 0, 2 * sizeof(Sched), s);
@@ -348,8 +343,15 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
       PhaseArgs pa{b->d_base, b->sched, b->list, b->rowf, b->rowc, b->cp, nullptr, 0, errw,
                    ctx->d_prof};
       phase_mark(ctx, 0, 0, s);
-      k_phase<PT, VT, false><<<ctx->num_sms, kSymThreads, kDynSmem, s>>>(prods, pa);
-      k_groups<PT, VT, false><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
+      const int64_t before = ctx->launches;
+      const int st = launch_symbolic_rows<PT, VT>(ctx, s, prods, pa, ncols);
+      row_kernels = int(ctx->launches - before);
+      ctx->launches = before;  // counted at each replay
+      if (st != TSPG_OK) {
+        cudaStreamEndCapture(s, &g);
+        if (g) cudaGraphDestroy(g);
+        return st;
+      }
       phase_mark(ctx, 0, 1, s);
       k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(b->rowc, R, b->partial);
       k_scan_partials<<<1, 1024, 0, s>>>(b->partial, nb);
@@ -357,7 +359,7 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
                                                          b->sched + 1, b->rowf);
     }
     k_gather_offsets<<<(nprod + 256) / 256, 256, 0, s>>>(b->cp, b->d_base, nprod, b->offs);
-    b->g1_kernels = 2 + (!(flags & TSPG_F_B_SORTED) && b->RB > 0) + (R > 0 ? 8 : 0);
+    b->g1_kernels = 2 + (!(flags & TSPG_F_B_SORTED) && b->RB > 0) + (R > 0 ? 6 + row_kernels : 0);
     cudaMemcpyAsync(b->h_offs, b->offs, sizeof(int64_t) * (nprod + 1), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(b->h_offs + nprod + 1, &b->sched[0].max_a_row, sizeof(int64_t),
                     cudaMemcpyDeviceToHost, s);
@@ -414,6 +416,7 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
     b->g2 = nullptr;
     cudaGraph_t g;
     TSPG_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    int row_kernels = 0;
     k_set_batch_out<PT, VT><<<(nprod + 255) / 256, 256, 0, s>>>(prods, b->d_base, b->cp, nprod,
                                                                 b->Cj, (VT *)b->Cx, b->Cp);
     if (R > 0) {
@@ -423,14 +426,19 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
       PhaseArgs pa{b->d_base, b->sched + 1, b->list, b->rowf, b->rowc, b->cp,
                    b->curbuf, b->cur_stride, errw, ctx->d_prof ? ctx->d_prof + kProfPerPhase : nullptr};
       phase_mark(ctx, 1, 0, s);
-      launch_dense_cluster<PT, VT>(ctx, s, prods, pa);  // launchable: checked above
-      k_dense_rank<PT, VT><<<ctx->num_sms, kRankThreads, kDynSmem, s>>>(prods, pa);
-      k_phase<PT, VT, true><<<ctx->num_sms, kThreads, kDynSmem, s>>>(prods, pa);
-      k_groups<PT, VT, true><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
+      const int64_t before = ctx->launches;
+      const int st = launch_numeric_rows<PT, VT>(ctx, s, prods, pa, ncols, 0);
+      row_kernels = int(ctx->launches - before);
+      ctx->launches = before;  // counted at each replay
+      if (st != TSPG_OK) {
+        cudaStreamEndCapture(s, &g);
+        if (g) cudaGraphDestroy(g);
+        return st;
+      }
       phase_mark(ctx, 1, 1, s);
     }
     k_zero_rowptr<PT, VT><<<(nprod + 31) / 32, 32, 0, s>>>(prods, nprod);
-    b->g2_kernels = 2 + (R > 0 ? 5 + (ctx->tune.cluster ? 1 : 0) : 0);
+    b->g2_kernels = 2 + (R > 0 ? 2 + row_kernels : 0);
     cudaError_t e = cudaStreamEndCapture(s, &g);
     if (e != cudaSuccess) {
       ctx->last_cuda = (int)e;

@@ -11,46 +11,7 @@
 #include <algorithm>
 #include <new>
 
-#include "spgemm_cluster.cuh"
-
-namespace tspg {
-
-// The dynamic shared-memory limit is a per-device attribute of a kernel: it
-// is raised once per device (the caller has made ctx->device current), so a
-// process that drives several GPUs sets it on each of them.
-template <typename PT, typename VT>
-static int set_smem_attr(int device) {
-  constexpr int kMaxDev = 64;
-  static bool done[kMaxDev] = {};  // per device and instantiation; benign if raced
-  const bool cached = device >= 0 && device < kMaxDev;
-  if (!cached || !done[device]) {
-    cudaError_t e1 = cudaFuncSetAttribute(k_phase<PT, VT, false>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kDynSmem);
-    cudaError_t e2 = cudaFuncSetAttribute(k_phase<PT, VT, true>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kDynSmem);
-    cudaError_t e3 = cudaFuncSetAttribute(k_groups<PT, VT, false>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kGroupDynSmem);
-    cudaError_t e4 = cudaFuncSetAttribute(k_groups<PT, VT, true>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kGroupDynSmem);
-    cudaError_t e5 = cudaFuncSetAttribute(k_onepass<PT, VT>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kGroupDynSmem);
-    cudaError_t e6 = cudaFuncSetAttribute(k_dense_rank<PT, VT>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          kDynSmem);
-    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess ||
-        e5 != cudaSuccess || e6 != cudaSuccess)
-      return TSPG_ECUDA;
-    if (cached) done[device] = true;
-  }
-  return TSPG_OK;
-}
-
-}  // namespace tspg
+#include "spgemm_span.cuh"
 
 using namespace tspg;
 
@@ -63,6 +24,7 @@ struct tspg_plan {
   int64_t c_nnz = 0;
   int64_t mults = 0;
   int64_t max_a_row = 0;
+  int64_t dense_rows = 0;  // numeric DENSE rows
   void *prods = nullptr;
   int64_t *base = nullptr;
   int64_t *rowf = nullptr;
@@ -208,8 +170,7 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
     pa.ox = P->ox;
     pa.defer = P->defer;
     phase_mark(ctx, 0, 0, s);
-    k_phase<PT, VT, false><<<ctx->num_sms, kSymThreads, kDynSmem, s>>>(prods, pa);
-    k_groups<PT, VT, false><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
+    TSPG_TRY((launch_symbolic_rows<PT, VT>(ctx, s, prods, pa, n)));
     if (onepass) {
       k_onepass<PT, VT><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
       // the rows sent back (too many columns for their 64-slot attempt and
@@ -231,11 +192,13 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
                                                           P->nb, P->cp, P->sched + 1, P->rowf);
   }
   TSPG_CUDA(ctx, cudaGetLastError());
-  ctx->launches += 2 + (!(flags & TSPG_F_B_SORTED) && B->nnz > 0 && B->nrows > 0) + (m > 0 ? 8 : 0) +
+  ctx->launches += 2 + (!(flags & TSPG_F_B_SORTED) && B->nnz > 0 && B->nrows > 0) + (m > 0 ? 6 : 0) +
                    extra;
   int64_t *h = ctx->h_words;
   TSPG_CUDA(ctx, cudaMemcpyAsync(h, P->cp + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   TSPG_CUDA(ctx, cudaMemcpyAsync(h + 1, &P->sched[0].total, 4 * sizeof(int64_t),
+                                 cudaMemcpyDeviceToHost, s));
+  TSPG_CUDA(ctx, cudaMemcpyAsync(h + 6, &P->sched[1].cnt, 3 * sizeof(int64_t),
                                  cudaMemcpyDeviceToHost, s));
   TSPG_CUDA(ctx, cudaMemcpyAsync(h + 5, ctx->d_words + kErrWord, sizeof(int64_t),
                                  cudaMemcpyDeviceToHost, s));
@@ -243,6 +206,7 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
   P->c_nnz = h[0];
   P->mults = h[1];
   P->max_a_row = h[3];
+  P->dense_rows = h[6] + h[7] + h[8];
   if (h[5] != 0) {
     cudaMemsetAsync(ctx->d_words + kErrWord, 0, sizeof(int64_t), s);
     return TSPG_ECUDA;
@@ -274,15 +238,12 @@ static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P,
                P->curbuf, P->cur_stride, ctx->d_words + kErrWord,
                ctx->d_prof ? ctx->d_prof + kProfPerPhase : nullptr};
   phase_mark(ctx, 1, 0, s);
-  TSPG_CUDA(ctx, launch_dense_cluster<PT, VT>(ctx, s, prods, pa));
-  k_dense_rank<PT, VT><<<ctx->num_sms, kRankThreads, kDynSmem, s>>>(prods, pa);
-  k_phase<PT, VT, true><<<ctx->num_sms, kThreads, kDynSmem, s>>>(prods, pa);
-  k_groups<PT, VT, true><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
+  TSPG_TRY((launch_numeric_rows<PT, VT>(ctx, s, prods, pa, P->n, P->dense_rows)));
   if (P->onepass)
     k_onepass_copy<PT, VT><<<grid_for(m * 32, 256, ctx->num_sms * 16), 256, 0, s>>>(
         prods, P->rowf, P->rowc, P->cp, P->oj, (const VT *)P->ox, m);
   phase_mark(ctx, 1, 1, s);
-  ctx->launches += 6 + (P->onepass ? 1 : 0);
+  ctx->launches += 3 + (P->onepass ? 1 : 0);
   TSPG_CUDA(ctx, cudaGetLastError());
   return TSPG_OK;
 }

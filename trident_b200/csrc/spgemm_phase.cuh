@@ -320,6 +320,7 @@ struct PhaseArgs {
   int32_t *oj = nullptr;     // one-pass rows: scratch columns and values
   void *ox = nullptr;
   uint64_t *defer = nullptr;  // one-pass rows sent back to the two-pass path
+  uint32_t skip = 0;          // classes k_groups leaves to k_span (bit per class)
 };
 
 // Optional per-class accounting (SM cycles spent in each row class), and
@@ -1796,20 +1797,22 @@ __global__ void __launch_bounds__(NUM ? kThreads : kSymThreads, 1)
   gm.stage = nullptr;
   // numeric: when k_dense_rank did every DENSE row, start past them
   const int64_t first = NUM && A.S->rank_left == 0 ? s_items[CLS_DENSE2 + 1] : 0;
+  // ... and end before the G1024 rows when k_span did those
+  const int64_t last = s_items[NUM && (A.skip >> CLS_G1024 & 1u) ? CLS_G1024 : kCtaClasses];
   // stage 1: CTA-level rows, heaviest class first
   while (true) {
     if (tid == 0) sh.slot[15] = atomicAdd(&A.S->work, 1ull);
     __syncthreads();
     const int64_t item = first + (int64_t)sh.slot[15];
     __syncthreads();
-    if (item >= s_items[kCtaClasses]) break;
+    if (item >= last) break;
     // numeric: the heavy DENSE0 / DENSE1 rows (heaviest first) are interleaved
     // with the lighter CTA rows, one in every K items, so fewer heavy rows are
     // in flight at once and their output segments (the targets of the global
     // reductions) stay in L2; symbolic: heaviest first
     int64_t pos = item;
     if (NUM && first == 0) {
-      const int64_t H = s_items[2], L = s_items[kCtaClasses] - H;
+      const int64_t H = s_items[2], L = last - H;
       int64_t K = H > 0 ? min(int64_t(kHeavyPeriod), 1 + L / H) : 1;
       // (past the interleaved stretch the light rows follow in order: pos = item)
       if (K > 1 && item < K * H) pos = item % K == 0 ? item / K : H + (item - item / K - 1);
@@ -1846,54 +1849,6 @@ __global__ void __launch_bounds__(NUM ? kThreads : kSymThreads, 1)
   }
 }
 
-// The numeric DENSE rows of the rank form (at most kRankMaxCols columns, not
-// taken by the column-window rule), persistent, before k_phase: 24 warps per
-// SM, where k_phase's 16 warps keep the 128 registers of the hash rows'
-// radix sort.  Heavy rows (DENSE0 / DENSE1) are spread over the DENSE2 rows
-// as in k_phase, so few of their reduction targets are live at once.
-template <typename PT, typename VT>
-__global__ void __launch_bounds__(kRankThreads, 1)
-    k_dense_rank(const ProdDev<PT, VT> *prods, PhaseArgs A) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ PhaseShared sh;
-  __shared__ unsigned long long s_item;
-  const int tid = threadIdx.x;
-  const int64_t H = A.S->cnt[CLS_DENSE0] + A.S->cnt[CLS_DENSE1];
-  const int64_t L = A.S->cnt[CLS_DENSE2];
-  const int64_t c01 = A.S->cnt[CLS_DENSE0];
-  const int64_t K = H > 0 ? min(int64_t(kHeavyPeriod), 1 + L / H) : 1;
-  GroupMem gm;
-  gm.cnt = nullptr;
-  gm.tmp = sh.scan;
-  gm.itmp = sh.itmp;
-  gm.lst = sh.lst;
-  gm.nl = sh.nl + 47;
-  gm.cap = 1024;
-  gm.stage = nullptr;
-  while (true) {
-    if (tid == 0) s_item = atomicAdd(&A.S->work3, 1ull);
-    __syncthreads();
-    const int64_t item = (int64_t)s_item;
-    __syncthreads();
-    if (item >= H + L) break;
-    int64_t pos = item;
-    if (K > 1 && item < K * H) pos = item % K == 0 ? item / K : H + (item - item / K - 1);
-    // the DENSE classes' lists are contiguous: DENSE0, DENSE1, DENSE2
-    const int c = pos < c01 ? CLS_DENSE0 : pos < H ? CLS_DENSE1 : CLS_DENSE2;
-    const int64_t idx = A.S->off[CLS_DENSE0] + pos;
-    const long long t0 = clock64();
-    const RowRef rr = decode_row(A, idx);
-    const ProdDev<PT, VT> &P = prods[rr.p];
-    if (P.n <= kRankMaxCols && !win_row(P, A.rowf[rr.g], int64_t(A.rowc[rr.g]), A.S->tune)) {
-      num_dense_rank_row<kRankThreads, PT, VT>(prods, A, idx, smem, gm);
-      prof_add(A, c, t0, tid == 0);
-    } else if (tid == 0) {
-      A.S->rank_left = 1;  // read by k_phase, which runs after this kernel
-    }
-    __syncthreads();
-  }
-}
-
 // The group classes (G256, G128, G32 rows), persistent: the CTA splits into
 // 256-thread groups, then 128-thread groups, then warps; each fetches its
 // rows on its own, and no CTA-wide barrier follows the set-up.
@@ -1907,9 +1862,9 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     sh.cnt[threadIdx.x] = A.S->cnt[threadIdx.x];
   }
   __syncthreads();
-  group_rows<256, NUM, PT, VT>(prods, A, CLS_G256, smem, sh);
-  group_rows<128, NUM, PT, VT>(prods, A, CLS_G128, smem, sh);
-  group_rows<32, NUM, PT, VT>(prods, A, CLS_G32, smem, sh);
+  if (!(A.skip >> CLS_G256 & 1u)) group_rows<256, NUM, PT, VT>(prods, A, CLS_G256, smem, sh);
+  if (!(A.skip >> CLS_G128 & 1u)) group_rows<128, NUM, PT, VT>(prods, A, CLS_G128, smem, sh);
+  if (!(A.skip >> CLS_G32 & 1u)) group_rows<32, NUM, PT, VT>(prods, A, CLS_G32, smem, sh);
 }
 
 // One-pass warp rows of a plain product (the symbolic record's CLS_ONEPASS
