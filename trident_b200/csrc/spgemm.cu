@@ -24,7 +24,7 @@ struct tspg_plan {
   int64_t c_nnz = 0;
   int64_t mults = 0;
   int64_t max_a_row = 0;
-  int64_t dense_rows = 0;  // numeric DENSE rows
+  int64_t ncnt[NCLS] = {};  // numeric rows per class
   void *prods = nullptr;
   int64_t *base = nullptr;
   int64_t *rowf = nullptr;
@@ -198,7 +198,7 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
   TSPG_CUDA(ctx, cudaMemcpyAsync(h, P->cp + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   TSPG_CUDA(ctx, cudaMemcpyAsync(h + 1, &P->sched[0].total, 4 * sizeof(int64_t),
                                  cudaMemcpyDeviceToHost, s));
-  TSPG_CUDA(ctx, cudaMemcpyAsync(h + 6, &P->sched[1].cnt, 3 * sizeof(int64_t),
+  TSPG_CUDA(ctx, cudaMemcpyAsync(h + 6, &P->sched[1].cnt, NCLS * sizeof(int64_t),
                                  cudaMemcpyDeviceToHost, s));
   TSPG_CUDA(ctx, cudaMemcpyAsync(h + 5, ctx->d_words + kErrWord, sizeof(int64_t),
                                  cudaMemcpyDeviceToHost, s));
@@ -206,7 +206,7 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
   P->c_nnz = h[0];
   P->mults = h[1];
   P->max_a_row = h[3];
-  P->dense_rows = h[6] + h[7] + h[8];
+  for (int c = 0; c < NCLS; ++c) P->ncnt[c] = h[6 + c];
   if (h[5] != 0) {
     cudaMemsetAsync(ctx->d_words + kErrWord, 0, sizeof(int64_t), s);
     return TSPG_ECUDA;
@@ -238,7 +238,7 @@ static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P,
                P->curbuf, P->cur_stride, ctx->d_words + kErrWord,
                ctx->d_prof ? ctx->d_prof + kProfPerPhase : nullptr};
   phase_mark(ctx, 1, 0, s);
-  TSPG_TRY((launch_numeric_rows<PT, VT>(ctx, s, prods, pa, P->n, P->dense_rows)));
+  TSPG_TRY((launch_numeric_rows<PT, VT>(ctx, s, prods, pa, P->n, P->ncnt)));
   if (P->onepass)
     k_onepass_copy<PT, VT><<<grid_for(m * 32, 256, ctx->num_sms * 16), 256, 0, s>>>(
         prods, P->rowf, P->rowc, P->cp, P->oj, (const VT *)P->ox, m);

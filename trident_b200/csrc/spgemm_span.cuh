@@ -560,35 +560,69 @@ inline int launch_symbolic_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT,
   return TSPG_OK;
 }
 
+// One numeric class of `rows` rows (-1: not known) with at most `cap` outputs
+// each, as span rows of NT threads; a class too small to give every SM its
+// CTAs takes wider ones, so that its last row ends sooner.
+template <int NT, typename PT, typename VT>
+inline cudaError_t launch_span_class(tspg_ctx *ctx, cudaStream_t s,
+                                     const ProdDev<PT, VT> *prods, const PhaseArgs &pa,
+                                     int64_t ncols, uint32_t cap, int cls, int64_t rows) {
+  if constexpr (NT < 512) {
+    if (rows >= 0 && rows <= int64_t(ctx->num_sms) * (512 / NT))
+      return launch_span_class<2 * NT, PT, VT>(ctx, s, prods, pa, ncols, cap, cls, rows);
+  }
+  return launch_span<NT, true, PT, VT>(ctx, s, prods, pa,
+                                       span_layout<NT, true, PT, VT>(ncols, cap), cls, cls + 1);
+}
+
 // The persistent kernels of a numeric phase whose products have at most
-// `ncols` columns and `dense_rows` DENSE rows (0: not known).
+// `ncols` columns; cnt: rows per class when the host knows them (else null),
+// so that no kernel is launched for an empty class.
 template <typename PT, typename VT>
 inline int launch_numeric_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, VT> *prods,
-                               PhaseArgs pa, int64_t ncols, int64_t dense_rows) {
+                               PhaseArgs pa, int64_t ncols, const int64_t *cnt) {
   TSPG_CUDA(ctx, launch_dense_cluster<PT, VT>(ctx, s, prods, pa));
-  const SpanLay L1 = span_layout<128, true, PT, VT>(ncols, uint32_t(ctx->tune.num[1]));
-  const SpanLay L2 = span_layout<256, true, PT, VT>(ncols, uint32_t(ctx->tune.num[2]));
-  const SpanLay L3 = span_layout<512, true, PT, VT>(ncols, uint32_t(ctx->tune.num[3]));
+  const Tune &tn = ctx->tune;
+  auto rows = [&](int c) { return cnt ? cnt[c] : int64_t(-1); };
+  const int64_t dense = cnt ? cnt[CLS_DENSE0] + cnt[CLS_DENSE1] + cnt[CLS_DENSE2] : -1;
   const uint32_t nb = uint32_t((ncols + 1023) >> 10);
-  if (nb * 196u <= kRank2Smem && dense_rows >= int64_t(kRank2Rows) * ctx->num_sms)
-    k_dense_rank<512, 2, PT, VT><<<ctx->num_sms * 2, 512, kRank2Smem, s>>>(prods, pa, kRank2Smem);
-  else
-    k_dense_rank<kRankThreads, 1, PT, VT><<<ctx->num_sms, kRankThreads, kDynSmem, s>>>(prods, pa, kDynSmem);
-  if (span_ctas<512>(L3) >= 1) {
+  if (dense != 0) {
+    if (nb * 196u <= kRank2Smem && dense >= int64_t(kRank2Rows) * ctx->num_sms)
+      k_dense_rank<512, 2, PT, VT><<<ctx->num_sms * 2, 512, kRank2Smem, s>>>(prods, pa, kRank2Smem);
+    else
+      k_dense_rank<kRankThreads, 1, PT, VT><<<ctx->num_sms, kRankThreads, kDynSmem, s>>>(prods, pa,
+                                                                                         kDynSmem);
+    ctx->launches += 1;
+  }
+  if (span_ctas<512>(span_layout<512, true, PT, VT>(ncols, uint32_t(tn.num[3]))) >= 1) {
     pa.skip |= 1u << CLS_G1024;
-    TSPG_CUDA(ctx, (launch_span<512, true, PT, VT>(ctx, s, prods, pa, L3, CLS_G1024, CLS_G1024 + 1)));
+    if (rows(CLS_G1024))
+      TSPG_CUDA(ctx, (launch_span_class<512>(ctx, s, prods, pa, ncols, uint32_t(tn.num[3]),
+                                             CLS_G1024, rows(CLS_G1024))));
   }
-  if (span_ctas<256>(L2) >= 2) {
+  if (span_ctas<256>(span_layout<256, true, PT, VT>(ncols, uint32_t(tn.num[2]))) >= 2) {
     pa.skip |= 1u << CLS_G256;
-    TSPG_CUDA(ctx, (launch_span<256, true, PT, VT>(ctx, s, prods, pa, L2, CLS_G256, CLS_G256 + 1)));
+    if (rows(CLS_G256))
+      TSPG_CUDA(ctx, (launch_span_class<256>(ctx, s, prods, pa, ncols, uint32_t(tn.num[2]),
+                                             CLS_G256, rows(CLS_G256))));
   }
-  if (span_ctas<128>(L1) >= 2) {
+  if (span_ctas<128>(span_layout<128, true, PT, VT>(ncols, uint32_t(tn.num[1]))) >= 2) {
     pa.skip |= 1u << CLS_G128;
-    TSPG_CUDA(ctx, (launch_span<128, true, PT, VT>(ctx, s, prods, pa, L1, CLS_G128, CLS_G128 + 1)));
+    if (rows(CLS_G128))
+      TSPG_CUDA(ctx, (launch_span_class<128>(ctx, s, prods, pa, ncols, uint32_t(tn.num[1]),
+                                             CLS_G128, rows(CLS_G128))));
   }
-  k_phase<PT, VT, true><<<ctx->num_sms, kThreads, kDynSmem, s>>>(prods, pa);
-  k_groups<PT, VT, true><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
-  ctx->launches += 3;
+  // k_phase: DENSE rows that are neither rank nor span rows, G1024 hash rows
+  const bool left = ncols > kRankMaxCols || tn.win != 0;
+  if ((left && dense != 0) || (!(pa.skip >> CLS_G1024 & 1u) && rows(CLS_G1024))) {
+    k_phase<PT, VT, true><<<ctx->num_sms, kThreads, kDynSmem, s>>>(prods, pa);
+    ctx->launches += 1;
+  }
+  if (rows(CLS_G32) || (!(pa.skip >> CLS_G256 & 1u) && rows(CLS_G256)) ||
+      (!(pa.skip >> CLS_G128 & 1u) && rows(CLS_G128))) {
+    k_groups<PT, VT, true><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
+    ctx->launches += 1;
+  }
   TSPG_CUDA(ctx, cudaGetLastError());
   return TSPG_OK;
 }
