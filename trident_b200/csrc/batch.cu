@@ -326,17 +326,18 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
     cudaGraph_t g;
     TSPG_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(b->sched, 0, 2 * sizeof(Sched), s);
-    k_set_tune<<<1, 32, 0, s>>>(b->sched, 2, ctx->tune);
-    cudaMemsetAsync(b->rowc, 0, sizeof(int32_t) * (R > 0 ? R : 1), s);
+    const Tune tune = span_tune(ctx->tune, ncols);
+    const bool check = !(flags & TSPG_F_B_SORTED) && b->RB > 0 && needs_sorted(tune, ncols);
+    k_set_tune<<<1, 32, 0, s>>>(b->sched, 2, tune);
     cudaMemsetAsync(b->cp, 0, sizeof(int64_t), s);
-    if (!(flags & TSPG_F_B_SORTED) && b->RB > 0)
+    if (check)
       k_check_sorted_batch<PT, VT><<<(unsigned)std::min<int64_t>((b->RB * 32 + 255) / 256,
                                                                  int64_t(ctx->num_sms) * 16),
                                      256, 0, s>>>(prods, b->d_bbase, nprod, b->RB);
     if (R > 0) {
       k_row_mults<PT, VT><<<(unsigned)std::min<int64_t>((R * 32 + 255) / 256,
                                                         int64_t(ctx->num_sms) * 16),
-                            256, 0, s>>>(prods, b->d_base, nprod, R, b->rowf, b->sched);
+                            256, 0, s>>>(prods, b->d_base, nprod, R, b->rowf, b->sched, b->rowc);
       k_sched_offsets<<<1, 32, 0, s>>>(b->sched);
       k_scatter<PT, VT, 0><<<(unsigned)((R + 255) / 256), 256, 0, s>>>(
           prods, b->d_base, nprod, R, b->rowf, b->rowc, b->cp, b->sched, b->list);
@@ -353,13 +354,13 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
         return st;
       }
       phase_mark(ctx, 0, 1, s);
-      k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(b->rowc, R, b->partial);
-      k_scan_partials<<<1, 1024, 0, s>>>(b->partial, nb);
-      k_scan_final<<<(unsigned)nb, kScanThreads, 0, s>>>(b->rowc, R, b->partial, nb, b->cp,
-                                                         b->sched + 1, b->rowf);
+      const int64_t scans = ctx->launches;
+      launch_scan(ctx, s, b->rowc, R, b->partial, b->cp, b->sched + 1, b->rowf);
+      row_kernels += int(ctx->launches - scans);
+      ctx->launches = scans;
     }
     k_gather_offsets<<<(nprod + 256) / 256, 256, 0, s>>>(b->cp, b->d_base, nprod, b->offs);
-    b->g1_kernels = 2 + (!(flags & TSPG_F_B_SORTED) && b->RB > 0) + (R > 0 ? 6 + row_kernels : 0);
+    b->g1_kernels = 2 + check + (R > 0 ? 3 + row_kernels : 0);
     cudaMemcpyAsync(b->h_offs, b->offs, sizeof(int64_t) * (nprod + 1), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(b->h_offs + nprod + 1, &b->sched[0].max_a_row, sizeof(int64_t),
                     cudaMemcpyDeviceToHost, s);
@@ -427,7 +428,7 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
                    b->curbuf, b->cur_stride, errw, ctx->d_prof ? ctx->d_prof + kProfPerPhase : nullptr};
       phase_mark(ctx, 1, 0, s);
       const int64_t before = ctx->launches;
-      const int st = launch_numeric_rows<PT, VT>(ctx, s, prods, pa, ncols, nullptr);
+      const int st = launch_numeric_rows<PT, VT>(ctx, s, prods, pa, ncols, nullptr, false);
       row_kernels = int(ctx->launches - before);
       ctx->launches = before;  // counted at each replay
       if (st != TSPG_OK) {

@@ -1,15 +1,22 @@
 // spgemm.cu — host side of the two-phase SpGEMM (C = A·B, C = C_in + A·B).
 //
 // Call sequence of one product on the caller's stream:
-//   k_set_prod, [k_check_sorted_rows], k_row_mults, k_sched_offsets,
-//   k_scatter<sym>, k_phase + k_groups <symbolic>, k_scan_reduce / k_scan_partials /
-//   k_scan_final, one 2-word device->host read + stream sync (nnz(C), longest
-//   A row), then k_set_out, k_sched_offsets, k_scatter<num>, k_phase + k_groups <numeric>.
+//   k_setup, [k_check_sorted_rows: column-window rows only], k_row_mults,
+//   k_scatter<sym>, k_span / k_phase + k_groups <symbolic>, the scan, whose
+//   last block leaves nnz(C), the longest A row and the class counts in mapped
+//   host memory, one stream sync, then k_scatter<num>, which takes the output
+//   arrays, k_dense_rank, k_span / k_phase + k_groups <numeric>.
+// Products of kFuseRows rows or more spend a small launch of their own on the
+// list offsets and the host's words instead of a last block.  1024 uniform
+// rows of 17 entries: 24 launches, 3 copies and 8 allocations, 171 us -> 10
+// launches and one allocation, 99 us.
 // KokkosSparse::spgemm (include/KokkosWrap.hpp:375) and the cuSPARSE paths
 // (include/cusparse_helpers.cuh:908-1344) do the same job with library-owned
 // allocation and ~10 stream syncs per call.
 #include <algorithm>
+#include <initializer_list>
 #include <new>
+#include <utility>
 
 #include "spgemm_span.cuh"
 
@@ -57,6 +64,18 @@ struct tspg_plan {
     *p = (T *)q;
     return TSPG_OK;
   }
+  // n arrays out of one block (each on a 256-byte boundary)
+  int get_all(std::initializer_list<std::pair<void **, size_t>> parts) {
+    size_t total = 0;
+    for (auto &p : parts) total += (p.second + 255) & ~size_t(255);
+    char *q = nullptr;
+    TSPG_TRY(get(&q, total));
+    for (auto &p : parts) {
+      *p.first = q;
+      q += (p.second + 255) & ~size_t(255);
+    }
+    return TSPG_OK;
+  }
   ~tspg_plan() {
     for (int i = nblocks - 1; i >= 0; --i) ws_free(ctx, blocks[i], stream);
   }
@@ -72,6 +91,7 @@ constexpr int kFlagOnePass = 1 << 30;
 // host round trip before the symbolic launch), with a scratch of at most
 // this many entries.
 constexpr int64_t kOnePassMinRows = 1 << 16;
+static_assert(kOnePassMinRows >= kFuseRows, "the one-pass branch sets the list offsets itself");
 constexpr int64_t kOnePassMaxEntries = int64_t(1) << 30;
 
 static inline unsigned grid_for(int64_t work, int per_block, int cap) {
@@ -86,27 +106,23 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
                          const tspg_csr *B, int flags, tspg_plan *P) {
   TSPG_TRY(set_smem_attr<PT, VT>(ctx->device));
   const int64_t m = A->nrows, n = B->ncols, k = A->ncols;
+  const Tune tune = span_tune(ctx->tune, n);
   P->m = m;
   P->n = n;
   P->k = k;
   P->a_nnz = A->nnz;
   P->b_nnz = B->nnz;
   P->nb = (m + kScanTile - 1) / kScanTile;
-  ProdDev<PT, VT> *prods;
-  TSPG_TRY(P->get(&prods, 1));
-  P->prods = prods;
-  TSPG_TRY(P->get(&P->base, 2));
-  TSPG_TRY(P->get(&P->rowf, m));
-  TSPG_TRY(P->get(&P->rowc, m));
-  TSPG_TRY(P->get(&P->cp, m + 1));
-  TSPG_TRY(P->get(&P->list, m));
-  TSPG_TRY(P->get(&P->sched, 3));
-  TSPG_TRY(P->get(&P->partial, P->nb + 1));
+  TSPG_TRY(P->get_all({{&P->prods, sizeof(ProdDev<PT, VT>)},
+                       {(void **)&P->base, 2 * sizeof(int64_t)},
+                       {(void **)&P->sched, 3 * sizeof(Sched)},
+                       {(void **)&P->rowf, m * sizeof(int64_t)},
+                       {(void **)&P->rowc, m * sizeof(int32_t)},
+                       {(void **)&P->cp, (m + 1) * sizeof(int64_t)},
+                       {(void **)&P->list, m * sizeof(uint64_t)},
+                       {(void **)&P->partial, (P->nb + 1) * sizeof(int64_t)}}));
+  ProdDev<PT, VT> *prods = (ProdDev<PT, VT> *)P->prods;
   bool onepass = (flags & kFlagOnePass) && !(P->E.col && P->E.nnz > 0) && m >= kOnePassMinRows;
-  TSPG_CUDA(ctx, cudaMemsetAsync(P->sched, 0, 3 * sizeof(Sched), s));
-  k_set_tune<<<1, 32, 0, s>>>(P->sched, 3, ctx->tune, onepass ? 1 : 0);
-  TSPG_CUDA(ctx, cudaMemsetAsync(P->rowc, 0, (m > 0 ? m : 1) * sizeof(int32_t), s));
-  TSPG_CUDA(ctx, cudaMemsetAsync(P->cp, 0, sizeof(int64_t), s));
 
   ProdDev<PT, VT> v{};
   v.Ap = (const PT *)A->rowptr;
@@ -125,89 +141,86 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
     v.Ex = (const VT *)P->E.val;
     v.ep_bits = P->E.rowptr_bits;
   }
-  k_set_prod<PT, VT><<<1, 1, 0, s>>>(prods, v, P->base, m);
-  if (!(flags & TSPG_F_B_SORTED) && B->nnz > 0 && B->nrows > 0) {
+  k_setup<PT, VT><<<1, 128, 0, s>>>(prods, v, P->base, P->sched, 3, tune, onepass ? 1 : 0);
+  ctx->launches += 1;
+  // sorted B rows only matter to the column-window rows
+  if (!(flags & TSPG_F_B_SORTED) && B->nnz > 0 && B->nrows > 0 && needs_sorted(tune, n)) {
     k_check_sorted_rows<PT><<<grid_for(B->nrows * 32, 256, ctx->num_sms * 16), 256,
                               0, s>>>(v.Bp, v.Bj, B->nrows, &prods->b_sorted);
+    ctx->launches += 1;
   }
-  int extra = 0;
-  if (m > 0) {
-    k_row_mults<PT, VT><<<grid_for(m * 32, 256, ctx->num_sms * 16), 256, 0, s>>>(
-        prods, P->base, 1, m, P->rowf, P->sched, onepass ? P->rowc : nullptr);
-    if (onepass) {
-      // the one-pass rows' scratch offsets: a scan of their output bounds
-      k_scan_reduce<<<(unsigned)P->nb, kScanThreads, 0, s>>>(P->rowc, m, P->partial);
-      k_scan_partials<<<1, 1024, 0, s>>>(P->partial, P->nb);
-      k_scan_final<<<(unsigned)P->nb, kScanThreads, 0, s>>>(P->rowc, m, P->partial, P->nb,
-                                                            P->cp, P->sched + 1, nullptr);
-      extra += 3;
-      int64_t *h = ctx->h_words;
-      TSPG_CUDA(ctx, cudaMemcpyAsync(h, P->cp + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-      TSPG_CUDA(ctx, cudaMemcpyAsync(h + 1, &P->sched[0].cnt[CLS_ONEPASS], sizeof(int64_t),
-                                     cudaMemcpyDeviceToHost, s));
-      TSPG_CUDA(ctx, cudaStreamSynchronize(s));
-      const int64_t tot = h[0], rows = h[1];
-      // one pass when most rows take it (R-MAT 20: a tenth of the rows, and
-      // those with more than 32 outputs need their second attempt: +0.9 ms
-      // of symbolic phase; Galerkin A·P: every row, -0.9 ms per call)
-      if (tot > 0 && 2 * rows >= m && tot <= kOnePassMaxEntries &&
-          P->get(&P->oj, size_t(tot)) == TSPG_OK && P->get((VT **)&P->ox, size_t(tot)) == TSPG_OK &&
-          P->get(&P->defer, size_t(rows)) == TSPG_OK) {
-        P->onepass = tot;
-      } else {  // every row two-pass: the one-pass rows back to their classes
-        onepass = false;
-        k_fold_onepass<<<1, 32, 0, s>>>(P->sched);
-        TSPG_CUDA(ctx, cudaMemsetAsync(P->rowc, 0, m * sizeof(int32_t), s));
-        extra += 1;
-      }
-    }
-    k_sched_offsets<<<1, 32, 0, s>>>(P->sched);
-    k_scatter<PT, VT, 0><<<grid_for(m, 256, INT32_MAX), 256, 0, s>>>(
-        prods, P->base, 1, m, P->rowf, P->rowc, P->cp, P->sched, P->list);
-    PhaseArgs pa{P->base, P->sched, P->list, P->rowf, P->rowc, P->cp,
-                 nullptr, 0, ctx->d_words + kErrWord, ctx->d_prof};
-    pa.oj = P->oj;
-    pa.ox = P->ox;
-    pa.defer = P->defer;
-    phase_mark(ctx, 0, 0, s);
-    TSPG_TRY((launch_symbolic_rows<PT, VT>(ctx, s, prods, pa, n)));
-    if (onepass) {
-      k_onepass<PT, VT><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
-      // the rows sent back (too many columns for their 64-slot attempt and
-      // too large for a warp's full table): their symbolic count, as
-      // 256-thread rows of their own record
-      Sched *D = P->sched + 2;
-      k_defer_setup<<<1, 32, 0, s>>>(P->sched, D);
-      k_sched_offsets<<<1, 32, 0, s>>>(D);
-      PhaseArgs pd = pa;
-      pd.S = D;
-      pd.list = P->defer;
-      k_groups<PT, VT, false><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pd);
-      extra += 4;
-    }
-    phase_mark(ctx, 0, 1, s);
-    k_scan_reduce<<<(unsigned)P->nb, kScanThreads, 0, s>>>(P->rowc, m, P->partial);
-    k_scan_partials<<<1, 1024, 0, s>>>(P->partial, P->nb);
-    k_scan_final<<<(unsigned)P->nb, kScanThreads, 0, s>>>(P->rowc, m, P->partial,
-                                                          P->nb, P->cp, P->sched + 1, P->rowf);
-  }
-  TSPG_CUDA(ctx, cudaGetLastError());
-  ctx->launches += 2 + (!(flags & TSPG_F_B_SORTED) && B->nnz > 0 && B->nrows > 0) + (m > 0 ? 6 : 0) +
-                   extra;
   int64_t *h = ctx->h_words;
-  TSPG_CUDA(ctx, cudaMemcpyAsync(h, P->cp + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-  TSPG_CUDA(ctx, cudaMemcpyAsync(h + 1, &P->sched[0].total, 4 * sizeof(int64_t),
-                                 cudaMemcpyDeviceToHost, s));
-  TSPG_CUDA(ctx, cudaMemcpyAsync(h + 6, &P->sched[1].cnt, NCLS * sizeof(int64_t),
-                                 cudaMemcpyDeviceToHost, s));
-  TSPG_CUDA(ctx, cudaMemcpyAsync(h + 5, ctx->d_words + kErrWord, sizeof(int64_t),
-                                 cudaMemcpyDeviceToHost, s));
+  if (m == 0) {
+    TSPG_CUDA(ctx, cudaGetLastError());
+    return TSPG_OK;  // nothing to count: c_nnz, mults and max_a_row stay 0
+  }
+  k_row_mults<PT, VT><<<grid_for(m * 32, 256, ctx->num_sms * 16), 256, 0, s>>>(
+      prods, P->base, 1, m, P->rowf, P->sched, P->rowc, m < kFuseRows);
+  ctx->launches += 1;
+  if (onepass) {
+    // the one-pass rows' scratch offsets: a scan of their output bounds
+    launch_scan(ctx, s, P->rowc, m, P->partial, P->cp, P->sched + 1, nullptr);
+    TSPG_CUDA(ctx, cudaGetLastError());
+    TSPG_CUDA(ctx, cudaMemcpyAsync(h + HW_TOTAL, P->cp + m, sizeof(int64_t),
+                                   cudaMemcpyDeviceToHost, s));
+    TSPG_CUDA(ctx, cudaMemcpyAsync(h + HW_ONEPASS, &P->sched[0].cnt[CLS_ONEPASS], sizeof(int64_t),
+                                   cudaMemcpyDeviceToHost, s));
+    TSPG_CUDA(ctx, cudaStreamSynchronize(s));
+    const int64_t tot = h[HW_TOTAL], rows = h[HW_ONEPASS];
+    // one pass when most rows take it (R-MAT 20: a tenth of the rows, and
+    // those with more than 32 outputs need their second attempt: +0.9 ms
+    // of symbolic phase; Galerkin A·P: every row, -0.9 ms per call)
+    if (tot > 0 && 2 * rows >= m && tot <= kOnePassMaxEntries &&
+        P->get(&P->oj, size_t(tot)) == TSPG_OK && P->get((VT **)&P->ox, size_t(tot)) == TSPG_OK &&
+        P->get(&P->defer, size_t(rows)) == TSPG_OK) {
+      P->onepass = tot;
+    } else {  // every row two-pass: the one-pass rows back to their classes
+      onepass = false;
+      k_fold_onepass<<<1, 32, 0, s>>>(P->sched);
+      ctx->launches += 1;
+    }
+  }
+  if (m >= kFuseRows) {
+    k_sched_offsets<<<1, 32, 0, s>>>(P->sched);
+    ctx->launches += 1;
+  }
+  k_scatter<PT, VT, 0><<<grid_for(m, 256, INT32_MAX), 256, 0, s>>>(
+      prods, P->base, 1, m, P->rowf, P->rowc, P->cp, P->sched, P->list);
+  ctx->launches += 1;
+  PhaseArgs pa{P->base, P->sched, P->list, P->rowf, P->rowc, P->cp,
+               nullptr, 0, ctx->d_words + kErrWord, ctx->d_prof};
+  pa.oj = P->oj;
+  pa.ox = P->ox;
+  pa.defer = P->defer;
+  phase_mark(ctx, 0, 0, s);
+  TSPG_TRY((launch_symbolic_rows<PT, VT>(ctx, s, prods, pa, n)));
+  if (onepass) {
+    k_onepass<PT, VT><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
+    // the rows sent back (too many columns for their 64-slot attempt and
+    // too large for a warp's full table): their symbolic count, as
+    // 256-thread rows of their own record
+    Sched *D = P->sched + 2;
+    k_defer_setup<<<1, 32, 0, s>>>(P->sched, D);
+    k_sched_offsets<<<1, 32, 0, s>>>(D);
+    PhaseArgs pd = pa;
+    pd.S = D;
+    pd.list = P->defer;
+    k_groups<PT, VT, false><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pd);
+    ctx->launches += 4;
+  }
+  phase_mark(ctx, 0, 1, s);
+  HostWords sh;
+  sh.words = h;
+  sh.sym = P->sched;
+  sh.err = ctx->d_words + kErrWord;
+  launch_scan(ctx, s, P->rowc, m, P->partial, P->cp, P->sched + 1, P->rowf, sh);
+  TSPG_CUDA(ctx, cudaGetLastError());
   TSPG_CUDA(ctx, cudaStreamSynchronize(s));
-  P->c_nnz = h[0];
-  P->mults = h[1];
-  P->max_a_row = h[3];
-  for (int c = 0; c < NCLS; ++c) P->ncnt[c] = h[6 + c];
-  if (h[5] != 0) {
+  P->c_nnz = h[HW_TOTAL];
+  P->mults = h[HW_MULTS];
+  P->max_a_row = h[HW_MAX_A];
+  for (int c = 0; c < NCLS; ++c) P->ncnt[c] = h[HW_CNT + c];
+  if (h[HW_ERR] != 0) {
     cudaMemsetAsync(ctx->d_words + kErrWord, 0, sizeof(int64_t), s);
     return TSPG_ECUDA;
   }
@@ -219,9 +232,9 @@ static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P,
                         tspg_csr_out *C) {
   const int64_t m = P->m;
   ProdDev<PT, VT> *prods = (ProdDev<PT, VT> *)P->prods;
-  k_set_out<PT, VT><<<1, 1, 0, s>>>(prods, C->col, (VT *)C->val, C->rowptr,
-                                    C->rowptr_bits);
   if (m == 0) {
+    k_set_out<PT, VT><<<1, 1, 0, s>>>(prods, C->col, (VT *)C->val, C->rowptr,
+                                      C->rowptr_bits);
     k_zero_rowptr<PT, VT><<<1, 32, 0, s>>>(prods, 1);
     ctx->launches += 2;
     TSPG_CUDA(ctx, cudaGetLastError());
@@ -231,19 +244,29 @@ static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P,
     P->cur_stride = P->max_a_row;
     TSPG_TRY(P->get(&P->curbuf, 2 * size_t(ctx->num_sms) * P->cur_stride));
   }
-  k_sched_offsets<<<1, 32, 0, s>>>(P->sched + 1);
+  OutArgs out;
+  out.Cj = C->col;
+  out.Cx = C->val;
+  out.Cp = C->rowptr;
+  out.cp_bits = C->rowptr_bits;
+  out.set = 1;
+  out.finish = m < kFuseRows;
+  if (m >= kFuseRows) {
+    k_sched_offsets<<<1, 32, 0, s>>>(P->sched + 1);
+    ctx->launches += 1;
+  }
   k_scatter<PT, VT, 1><<<grid_for(m, 256, INT32_MAX), 256, 0, s>>>(
-      prods, P->base, 1, m, P->rowf, P->rowc, P->cp, P->sched + 1, P->list);
+      prods, P->base, 1, m, P->rowf, P->rowc, P->cp, P->sched + 1, P->list, out);
   PhaseArgs pa{P->base, P->sched + 1, P->list, P->rowf, P->rowc, P->cp,
                P->curbuf, P->cur_stride, ctx->d_words + kErrWord,
                ctx->d_prof ? ctx->d_prof + kProfPerPhase : nullptr};
   phase_mark(ctx, 1, 0, s);
-  TSPG_TRY((launch_numeric_rows<PT, VT>(ctx, s, prods, pa, P->n, P->ncnt)));
+  TSPG_TRY((launch_numeric_rows<PT, VT>(ctx, s, prods, pa, P->n, P->ncnt, m < kFuseRows)));
   if (P->onepass)
     k_onepass_copy<PT, VT><<<grid_for(m * 32, 256, ctx->num_sms * 16), 256, 0, s>>>(
         prods, P->rowf, P->rowc, P->cp, P->oj, (const VT *)P->ox, m);
   phase_mark(ctx, 1, 1, s);
-  ctx->launches += 3 + (P->onepass ? 1 : 0);
+  ctx->launches += 1 + (P->onepass ? 1 : 0);
   TSPG_CUDA(ctx, cudaGetLastError());
   return TSPG_OK;
 }
@@ -458,19 +481,17 @@ extern "C" int tspg_spgemm_count(tspg_ctx *ctx, void *stream,
     TSPG_TRY(sc.get(&base, 2));
     TSPG_TRY(sc.get(&rowf, m));
     TSPG_TRY(sc.get(&sched, 1));
-    TSPG_CUDA(ctx, cudaMemsetAsync(sched, 0, sizeof(Sched), s));
-    k_set_tune<<<1, 32, 0, s>>>(sched, 1, ctx->tune);
     ProdDev<PT, VT> v{};
     v.Ap = (const PT *)A->rowptr;
     v.Aj = A->col;
     v.Bp = (const PT *)B->rowptr;
     v.m = m;
     v.n = B->ncols;
-    k_set_prod<PT, VT><<<1, 1, 0, s>>>(prods, v, base, m);
+    k_setup<PT, VT><<<1, 128, 0, s>>>(prods, v, base, sched, 1, ctx->tune, 0);
     if (m > 0)
       k_row_mults<PT, VT><<<grid_for(m * 32, 256, ctx->num_sms * 16), 256, 0, s>>>(
           prods, base, 1, m, rowf, sched);
-    ctx->launches += 2 + (m > 0);
+    ctx->launches += 1 + (m > 0);
     TSPG_CUDA(ctx, cudaGetLastError());
     int64_t *h = ctx->h_words;
     TSPG_CUDA(ctx, cudaMemcpyAsync(h, &sched->total, 2 * sizeof(int64_t),

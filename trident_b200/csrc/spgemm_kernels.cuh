@@ -180,7 +180,7 @@ struct Sched {
   int64_t nonempty;
   unsigned long long work2;  // row counter of the cluster kernel (column-window rows)
   int32_t onepass;  // symbolic record of a plain product: one-pass rows on
-  int32_t pad32;
+  uint32_t ticket;  // blocks done, of the kernel whose last block finishes a step
   int64_t cand[NCLS];           // one-pass candidates by the class they left
   unsigned long long ndefer;    // one-pass rows sent back to the two-pass path
   unsigned long long work3;     // row counter of the rank-form DENSE kernel
@@ -230,12 +230,58 @@ static __global__ void k_set_tune(Sched *S, int n, Tune t, int onepass = 0) {
   }
 }
 
+// Everything a single product's symbolic phase starts from, in one launch of
+// one block (two memsets and two kernels before): the Sched records zeroed,
+// their row binning, the product's descriptor and row base.
 template <typename PT, typename VT>
-__global__ void k_set_prod(ProdDev<PT, VT> *dst, ProdDev<PT, VT> v,
-                           int64_t *base, int64_t m) {
-  *dst = v;
-  base[0] = 0;
-  base[1] = m;
+__global__ void __launch_bounds__(128) k_setup(ProdDev<PT, VT> *dst, ProdDev<PT, VT> v,
+                                               int64_t *base, Sched *S, int n, Tune t,
+                                               int onepass) {
+  uint64_t *w = (uint64_t *)S;
+  static_assert(sizeof(Sched) % 8 == 0, "Sched is zeroed by words");
+  for (int i = threadIdx.x; i < int(n * sizeof(Sched) / 8); i += blockDim.x) w[i] = 0;
+  __syncthreads();
+  if (threadIdx.x < n) {
+    S[threadIdx.x].tune = t;
+    S[threadIdx.x].onepass = threadIdx.x == 0 ? onepass : 0;
+  }
+  if (threadIdx.x == 0) {
+    *dst = v;
+    base[0] = 0;
+    base[1] = v.m;
+  }
+}
+
+// True in every thread of the grid's last block to get here (the others'
+// writes are then visible to it).  The ticket is left at zero.
+__device__ __forceinline__ bool last_block(uint32_t *ticket) {
+  __shared__ uint32_t s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (s_last) {
+      *ticket = 0;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  return s_last != 0;
+}
+
+// Class offsets into the row list; resets the work counters.
+__device__ __forceinline__ void sched_offsets(Sched *S) {
+  int64_t o = 0;
+  for (int c = 0; c < NCLS; ++c) {
+    S->off[c] = o;
+    S->cur[c] = o;
+    S->next[c] = 0;
+    o += *(volatile int64_t *)&S->cnt[c];
+  }
+  S->work = 0;
+  S->work2 = 0;
+  S->work3 = 0;
+  S->rank_left = 0;
 }
 
 // int32 row offsets widened to int64 (operands of mixed offset widths).
@@ -296,7 +342,8 @@ constexpr int kThreadRowMax = 64;
 constexpr int kHintEntries = 8;
 
 // Products per row (rowf), the symbolic class counts, the product total, the
-// sum of min(products, ncols) and the longest A row.  A warp takes 32 rows at
+// sum of min(products, ncols) and the longest A row; with `finish` the last
+// block turns the class counts into list offsets.  A warp takes 32 rows at
 // a time: lane i walks row i's A entries itself (4 entries per step, so the
 // loads of 32 rows are in flight together) when the row has at most
 // kThreadRowMax entries, and the whole warp walks each longer row; class
@@ -307,7 +354,7 @@ constexpr int kHintEntries = 8;
 template <typename PT, typename VT>
 __global__ void __launch_bounds__(256) k_row_mults(
     const ProdDev<PT, VT> *prods, const int64_t *base, int nprod, int64_t R,
-    int64_t *rowf, Sched *S, int32_t *obound = nullptr) {
+    int64_t *rowf, Sched *S, int32_t *rowc = nullptr, int finish = 0) {
   __shared__ unsigned long long s_cnt[NCLS], s_cand[NCLS];
   __shared__ unsigned long long s_tot, s_up, s_ne;
   __shared__ long long s_maxa;
@@ -406,7 +453,9 @@ __global__ void __launch_bounds__(256) k_row_mults(
         left = c;
         c = CLS_ONEPASS;
       }
-      if (obound) obound[g] = one ? int32_t(onepass_bound(f, n, S->tune)) : 0;
+      // zero, or a one-pass row's scratch bound, until the symbolic kernels
+      // write the counts of the rows that have products
+      if (rowc) rowc[g] = one ? int32_t(onepass_bound(f, n, S->tune)) : 0;
       if (c >= 0) ne += 1;
       tot += f;
       up += f < n ? f : n;
@@ -451,6 +500,7 @@ __global__ void __launch_bounds__(256) k_row_mults(
     atomicAdd((unsigned long long *)&S->nonempty, s_ne);
     atomicMax((long long *)&S->max_a_row, s_maxa);
   }
+  if (finish && last_block(&S->ticket) && threadIdx.x == 0) sched_offsets(S);
 }
 
 // The one-pass rows of a symbolic record go back to the classes they left
@@ -469,31 +519,29 @@ static __global__ void k_defer_setup(const Sched *S, Sched *D) {
   if (threadIdx.x == 0 && blockIdx.x == 0) D->cnt[CLS_G256] = int64_t(S->ndefer);
 }
 
-// Class offsets into the row list; resets the work counters.
 static __global__ void k_sched_offsets(Sched *S) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    int64_t o = 0;
-    for (int c = 0; c < NCLS; ++c) {
-      S->off[c] = o;
-      S->cur[c] = o;
-      S->next[c] = 0;
-      o += S->cnt[c];
-    }
-    S->work = 0;
-    S->work2 = 0;
-    S->work3 = 0;
-    S->rank_left = 0;
-  }
+  if (threadIdx.x == 0 && blockIdx.x == 0) sched_offsets(S);
 }
+
+// The output arrays of a single product (set: they go into its descriptor).
+struct OutArgs {
+  int32_t *Cj = nullptr;
+  void *Cx = nullptr;
+  void *Cp = nullptr;
+  int32_t cp_bits = 0;
+  int16_t set = 0;
+  int16_t finish = 0;
+};
 
 // Scatter rows into the class lists.  mode 0: symbolic (class from rowf);
 // mode 1: numeric (class from rowc) which also writes the output row offsets
-// of each product and the largest A row among DENSE rows.
+// of each product, and whose last block (out.finish) makes the record ready
+// for the numeric kernels and for another numeric run of a plan.
 template <typename PT, typename VT, int MODE>
 __global__ void __launch_bounds__(256) k_scatter(
     ProdDev<PT, VT> *prods, const int64_t *base, int nprod, int64_t R,
     const int64_t *rowf, const int32_t *rowc, const int64_t *cp, Sched *S,
-    uint64_t *list) {
+    uint64_t *list, OutArgs out = OutArgs()) {
   __shared__ unsigned long long s_cnt[NCLS], s_base[NCLS];
   if (threadIdx.x < NCLS) s_cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -510,18 +558,22 @@ __global__ void __launch_bounds__(256) k_scatter(
     } else {
       c = num_class(rowc[g], rowf[g], S->tune);
       const int64_t off = cp[g] - cp[base[p]];
-      if (prods[p].cp_bits == 32)
-        ((int32_t *)prods[p].Cp)[r] = (int32_t)off;
-      else
-        ((int64_t *)prods[p].Cp)[r] = off;
+      void *const Cp = out.set ? out.Cp : prods[p].Cp;
+      const bool narrow = (out.set ? out.cp_bits : prods[p].cp_bits) == 32;
+      if (narrow) ((int32_t *)Cp)[r] = (int32_t)off;
+      else ((int64_t *)Cp)[r] = off;
       if (r == prods[p].m - 1) {
         const int64_t end = cp[g + 1] - cp[base[p]];
-        if (prods[p].cp_bits == 32)
-          ((int32_t *)prods[p].Cp)[r + 1] = (int32_t)end;
-        else
-          ((int64_t *)prods[p].Cp)[r + 1] = end;
+        if (narrow) ((int32_t *)Cp)[r + 1] = (int32_t)end;
+        else ((int64_t *)Cp)[r + 1] = end;
       }
     }
+  }
+  if (MODE == 1 && out.set && blockIdx.x == 0 && threadIdx.x == 0) {
+    prods[0].Cj = out.Cj;
+    prods[0].Cx = (VT *)out.Cx;
+    prods[0].Cp = out.Cp;
+    prods[0].cp_bits = out.cp_bits;
   }
   // each class present in the warp takes its slots with one shared atomic
   const int lane = threadIdx.x & 31;
@@ -545,6 +597,7 @@ __global__ void __launch_bounds__(256) k_scatter(
   }
   __syncthreads();
   if (c >= 0) list[s_base[c] + my] = (uint64_t(p) << 40) | uint64_t(r);
+  if (MODE == 1 && out.finish && last_block(&S->ticket) && threadIdx.x == 0) sched_offsets(S);
 }
 
 // Products whose A has zero rows still need rowptr[0] = 0.
@@ -565,7 +618,7 @@ constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
 static __global__ void __launch_bounds__(kScanThreads)
-    k_scan_reduce(const int32_t *in, int64_t R, int64_t *partial) {
+    k_scan_reduce(const int32_t *in, int64_t R, int64_t *partial, uint32_t *ticket = nullptr) {
   __shared__ int64_t tmp[kScanThreads / 32 + 1];
   const int64_t t0 = int64_t(blockIdx.x) * kScanTile;
   int64_t s = 0;
@@ -580,6 +633,20 @@ static __global__ void __launch_bounds__(kScanThreads)
     int64_t v = threadIdx.x < kScanThreads / 32 ? tmp[threadIdx.x] : 0;
     v = warp_sum(v);
     if (threadIdx.x == 0) partial[blockIdx.x] = v;
+  }
+  // the last block scans the partials in place (partial[nb] = total)
+  if (ticket && last_block(ticket)) {
+    const int64_t nb = gridDim.x;
+    int64_t carry = 0;
+    for (int64_t b0 = 0; b0 < nb; b0 += kScanThreads) {
+      const int64_t j = b0 + threadIdx.x;
+      const int64_t v = j < nb ? *(volatile int64_t *)(partial + j) : 0;
+      int64_t tot;
+      const int64_t ex = group_excl_scan<kScanThreads, int64_t>(v, tmp, 0, &tot);
+      if (j < nb) partial[j] = carry + ex;
+      carry += tot;
+    }
+    if (threadIdx.x == 0) partial[nb] = carry;
   }
 }
 
@@ -603,10 +670,40 @@ static __global__ void __launch_bounds__(1024) k_scan_partials(int64_t *partial,
   if (threadIdx.x == 0) partial[nb] = carry;
 }
 
-// Also counts the numeric classes of the rows into *Snum.
+// What the symbolic phase of a single product leaves for the host, written
+// from the device into mapped pinned memory (a stream sync then suffices; a
+// device->host copy took 2.6 us each): nnz(C), the record's sums, the error
+// word and the numeric class counts.
+enum { HW_TOTAL = 0, HW_MULTS, HW_MAX_A, HW_ERR, HW_ONEPASS, HW_CNT };
+struct HostWords {
+  int64_t *words = nullptr;      // null: nothing is left
+  const Sched *sym = nullptr;    // the symbolic record
+  const int64_t *err = nullptr;  // the device error word
+};
+
+// One thread: the numeric record's list offsets and the host's words.
+__device__ __forceinline__ void finish_symbolic(Sched *Snum, int64_t total, const HostWords &host) {
+  sched_offsets(Snum);
+  volatile int64_t *w = host.words;
+  w[HW_TOTAL] = total;
+  w[HW_MULTS] = host.sym->total;
+  w[HW_MAX_A] = host.sym->max_a_row;
+  w[HW_ERR] = *host.err;
+  for (int c = 0; c < NCLS; ++c) w[HW_CNT + c] = *(volatile int64_t *)&Snum->cnt[c];
+  __threadfence_system();
+}
+
+static __global__ void k_finish_symbolic(Sched *Snum, const int64_t *total, HostWords host) {
+  if (threadIdx.x == 0) finish_symbolic(Snum, *total, host);
+}
+
+// Final pass of the scan; partial == null: the one block has everything.
+// Also counts the numeric classes of the rows into *Snum (rowf given); with
+// host.words the last block finishes the symbolic phase.
 static __global__ void __launch_bounds__(kScanThreads)
     k_scan_final(const int32_t *in, int64_t R, const int64_t *partial,
-                 int64_t nb, int64_t *out, Sched *Snum, const int64_t *rowf) {
+                 int64_t nb, int64_t *out, Sched *Snum, const int64_t *rowf,
+                 HostWords host = HostWords()) {
   __shared__ int64_t tmp[kScanThreads / 32 + 1];
   __shared__ unsigned long long s_cnt[NCLS];
   if (threadIdx.x < NCLS) s_cnt[threadIdx.x] = 0;
@@ -638,16 +735,46 @@ static __global__ void __launch_bounds__(kScanThreads)
   }
   int64_t tot;
   int64_t ex = group_excl_scan<kScanThreads, int64_t>(s, tmp, 0, &tot);
-  ex += partial[blockIdx.x];
+  if (partial) ex += partial[blockIdx.x];
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     if (j0 + i < R) out[j0 + i] = ex;
     ex += v[i];
   }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[R] = partial[nb];
+  const int64_t total = partial ? partial[nb] : tot;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[R] = total;
   __syncthreads();
   if (threadIdx.x < NCLS && s_cnt[threadIdx.x])
     atomicAdd((unsigned long long *)&Snum->cnt[threadIdx.x], s_cnt[threadIdx.x]);
+  if (host.words && last_block(&Snum->ticket) && threadIdx.x == 0)
+    finish_symbolic(Snum, total, host);
+}
+
+// Rows from which a step's last block no longer does what a small launch of
+// its own can: every block then pays a fence and a ticket (2.1M rows: count
+// pass +14 us, final scan +6 us, against 2-3 us a launch).
+constexpr int64_t kFuseRows = 1 << 16;
+
+// Exclusive scan of in[0, R) into out[0, R] (R > 0): one launch up to
+// kScanTile rows, two below kFuseRows, else three.  S: a zeroed record (its
+// ticket is used).
+static inline void launch_scan(tspg_ctx *ctx, cudaStream_t s, const int32_t *in, int64_t R,
+                               int64_t *partial, int64_t *out, Sched *S, const int64_t *rowf,
+                               HostWords host = HostWords()) {
+  const int64_t nb = (R + kScanTile - 1) / kScanTile;
+  const bool fuse = R < kFuseRows;
+  if (nb > 1) {
+    k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(in, R, partial, fuse ? &S->ticket : nullptr);
+    if (!fuse) k_scan_partials<<<1, 1024, 0, s>>>(partial, nb);
+    ctx->launches += fuse ? 1 : 2;
+  }
+  k_scan_final<<<(unsigned)nb, kScanThreads, 0, s>>>(in, R, nb > 1 ? partial : nullptr, nb, out, S,
+                                                     rowf, fuse ? host : HostWords());
+  ctx->launches += 1;
+  if (host.words && !fuse) {
+    k_finish_symbolic<<<1, 32, 0, s>>>(S, out + R, host);
+    ctx->launches += 1;
+  }
 }
 
 }  // namespace tspg

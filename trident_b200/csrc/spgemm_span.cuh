@@ -527,6 +527,23 @@ inline cudaError_t launch_span(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, 
   return cudaGetLastError();
 }
 
+// Sorted B rows only matter to rows swept in column windows: wider than the
+// rank form's bitmap, or taken by the window form of the tuning.
+inline bool needs_sorted(const Tune &t, int64_t ncols) { return ncols > kRankMaxCols || t.win != 0; }
+
+// The row binning of a run: while the bitmap of 128-thread span rows stays
+// small (8 CTAs per SM), numeric rows of more than kSpanWarpRow outputs leave
+// the warps for them.  Uniform rows of order 1024 with ~250 outputs: numeric
+// 49 -> 15 us; Poisson(15) of order 100k 0.55 -> 0.48 ms, of order 200k (5
+// CTAs per SM) 1.16 -> 1.23 ms.
+constexpr int64_t kSpanWarpCols = 131072;
+constexpr int32_t kSpanWarpRow = 128;
+inline Tune span_tune(Tune t, int64_t ncols) {
+  if (ncols <= kSpanWarpCols && t.num[0] > kSpanWarpRow && t.num[1] >= t.num[0])
+    t.num[0] = kSpanWarpRow;
+  return t;
+}
+
 // A class takes the span form when at least two of its CTAs fit an SM: with
 // one, too few rows are in flight (numeric, R-MAT of order 800k: 9.44 ms as
 // span rows at one CTA per SM, 8.77 ms as hash rows; symbolic at two: 2.38
@@ -576,17 +593,20 @@ inline cudaError_t launch_span_class(tspg_ctx *ctx, cudaStream_t s,
 }
 
 // The persistent kernels of a numeric phase whose products have at most
-// `ncols` columns; cnt: rows per class when the host knows them (else null),
-// so that no kernel is launched for an empty class.
+// `ncols` columns; cnt: rows per class when the host knows them (else null).
+// skip_empty: no kernel is launched for an empty class (small products, where
+// a launch counts).
 template <typename PT, typename VT>
 inline int launch_numeric_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, VT> *prods,
-                               PhaseArgs pa, int64_t ncols, const int64_t *cnt) {
+                               PhaseArgs pa, int64_t ncols, const int64_t *cnt,
+                               bool skip_empty) {
   TSPG_CUDA(ctx, launch_dense_cluster<PT, VT>(ctx, s, prods, pa));
   const Tune &tn = ctx->tune;
   auto rows = [&](int c) { return cnt ? cnt[c] : int64_t(-1); };
+  auto some = [&](int c) { return !skip_empty || rows(c) != 0; };
   const int64_t dense = cnt ? cnt[CLS_DENSE0] + cnt[CLS_DENSE1] + cnt[CLS_DENSE2] : -1;
   const uint32_t nb = uint32_t((ncols + 1023) >> 10);
-  if (dense != 0) {
+  if (!skip_empty || dense != 0) {
     if (nb * 196u <= kRank2Smem && dense >= int64_t(kRank2Rows) * ctx->num_sms)
       k_dense_rank<512, 2, PT, VT><<<ctx->num_sms * 2, 512, kRank2Smem, s>>>(prods, pa, kRank2Smem);
     else
@@ -596,30 +616,31 @@ inline int launch_numeric_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, 
   }
   if (span_ctas<512>(span_layout<512, true, PT, VT>(ncols, uint32_t(tn.num[3]))) >= 1) {
     pa.skip |= 1u << CLS_G1024;
-    if (rows(CLS_G1024))
+    if (some(CLS_G1024))
       TSPG_CUDA(ctx, (launch_span_class<512>(ctx, s, prods, pa, ncols, uint32_t(tn.num[3]),
                                              CLS_G1024, rows(CLS_G1024))));
   }
   if (span_ctas<256>(span_layout<256, true, PT, VT>(ncols, uint32_t(tn.num[2]))) >= 2) {
     pa.skip |= 1u << CLS_G256;
-    if (rows(CLS_G256))
+    if (some(CLS_G256))
       TSPG_CUDA(ctx, (launch_span_class<256>(ctx, s, prods, pa, ncols, uint32_t(tn.num[2]),
                                              CLS_G256, rows(CLS_G256))));
   }
   if (span_ctas<128>(span_layout<128, true, PT, VT>(ncols, uint32_t(tn.num[1]))) >= 2) {
     pa.skip |= 1u << CLS_G128;
-    if (rows(CLS_G128))
+    if (some(CLS_G128))
       TSPG_CUDA(ctx, (launch_span_class<128>(ctx, s, prods, pa, ncols, uint32_t(tn.num[1]),
                                              CLS_G128, rows(CLS_G128))));
   }
   // k_phase: DENSE rows that are neither rank nor span rows, G1024 hash rows
   const bool left = ncols > kRankMaxCols || tn.win != 0;
-  if ((left && dense != 0) || (!(pa.skip >> CLS_G1024 & 1u) && rows(CLS_G1024))) {
+  if ((left && (!skip_empty || dense != 0)) ||
+      (!(pa.skip >> CLS_G1024 & 1u) && some(CLS_G1024))) {
     k_phase<PT, VT, true><<<ctx->num_sms, kThreads, kDynSmem, s>>>(prods, pa);
     ctx->launches += 1;
   }
-  if (rows(CLS_G32) || (!(pa.skip >> CLS_G256 & 1u) && rows(CLS_G256)) ||
-      (!(pa.skip >> CLS_G128 & 1u) && rows(CLS_G128))) {
+  if (some(CLS_G32) || (!(pa.skip >> CLS_G256 & 1u) && some(CLS_G256)) ||
+      (!(pa.skip >> CLS_G128 & 1u) && some(CLS_G128))) {
     k_groups<PT, VT, true><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
     ctx->launches += 1;
   }
