@@ -265,7 +265,10 @@ int tspg_spgemm_acc(tspg_ctx *ctx, void *stream, const tspg_csr *A,
  * LocalMatrix::csc_to_csr (include/KokkosWrap.hpp:442-531): a CSC tile
  * passed as the CSR of its transpose comes back as the CSR of the tile.
  * T->nrows = M->ncols, T->ncols = M->nrows; output capacity / allocator as
- * for SpGEMM.  Synchronises `stream` once. */
+ * for SpGEMM.  Entries that share a row and a column keep their order.
+ * Stream-ordered; synchronises `stream` only when the context's budget refuses
+ * the workspace of the counting-sort passes (12 + 4 + val_bits / 8 bytes per
+ * entry) and the segment sort takes their place. */
 int tspg_transpose(tspg_ctx *ctx, void *stream, const tspg_csr *M,
                    tspg_csr_out *T);
 

@@ -310,4 +310,54 @@ __device__ __forceinline__ void red_add(float *p, float v) {
   asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
 }
 
+// The last of the rows [0, m) of offsets rp (less base) that starts at or
+// before entry e: a warp-wide 32-way search.  m >= 1, rp[0] = base, e >= 0.
+template <typename PT>
+__device__ __forceinline__ int64_t first_row(const PT *__restrict__ rp, int64_t m, int64_t base,
+                                             int64_t e, int lane) {
+  int64_t lo = 0, hi = m;
+  while (hi - lo > 1) {
+    const int64_t step = (hi - lo + 31) / 32, i = lo + lane * step;
+    const unsigned b = __ballot_sync(0xffffffffu, i < hi && int64_t(__ldg(rp + i)) - base <= e);
+    lo += int64_t(31 - __clz(b)) * step;
+    hi = lo + step < hi ? lo + step : hi;
+  }
+  return lo;
+}
+
+// Rows of a window of 32 consecutive entries, one per lane (e ascending over
+// the lanes), r being the last row that starts at or before the window.  Lanes
+// search the next 32 row starts by shuffles; past those (runs of empty rows)
+// the next ones, then the offsets themselves.  r becomes lane 31's row.
+template <typename PT>
+__device__ __forceinline__ int64_t window_row(const PT *__restrict__ rp, int64_t m, int64_t base,
+                                              int64_t &r, int64_t e, int lane) {
+  constexpr unsigned FULL = 0xffffffffu;
+  int64_t mine = r;
+  bool open = true;  // this lane's row may lie past the starts seen so far
+  for (int t = 0; t < 4; ++t) {
+    const int64_t nx = r + 1 + lane < m ? int64_t(__ldg(rp + r + 1 + lane)) - base : INT64_MAX;
+    int j = 0;
+#pragma unroll
+    for (int st = 16; st > 0; st >>= 1)
+      if (__shfl_sync(FULL, nx, j + st - 1) <= e) j += st;
+    if (__shfl_sync(FULL, nx, 31) <= e) j = 32;
+    if (open) mine = r + j;
+    open = open && j == 32;
+    if (!__any_sync(FULL, open)) break;
+    r += 32;
+  }
+  if (open) {
+    int64_t a = mine, z = m;
+    while (z - a > 1) {
+      const int64_t mid = (a + z) >> 1;
+      if (int64_t(__ldg(rp + mid)) - base <= e) a = mid; else z = mid;
+    }
+    mine = a;
+  }
+  __syncwarp();
+  r = __shfl_sync(FULL, mine, 31);
+  return mine;
+}
+
 }  // namespace tspg
