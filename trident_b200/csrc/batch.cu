@@ -335,9 +335,10 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
                                                                  int64_t(ctx->num_sms) * 16),
                                      256, 0, s>>>(prods, b->d_bbase, nprod, b->RB);
     if (R > 0) {
-      k_row_mults<PT, VT><<<(unsigned)std::min<int64_t>((R * 32 + 255) / 256,
-                                                        int64_t(ctx->num_sms) * 16),
-                            256, 0, s>>>(prods, b->d_base, nprod, R, b->rowf, b->sched, b->rowc);
+      const int64_t counts = ctx->launches;
+      launch_row_mults<PT, VT>(ctx, s, prods, b->d_base, nprod, R, b->rowf, b->sched, b->rowc, 0,
+                               R < kFuseRows ? nullptr : b->list);
+      ctx->launches = counts;
       k_sched_offsets<<<1, 32, 0, s>>>(b->sched);
       k_scatter<PT, VT, 0><<<(unsigned)((R + 255) / 256), 256, 0, s>>>(
           prods, b->d_base, nprod, R, b->rowf, b->rowc, b->cp, b->sched, b->list);
@@ -360,7 +361,7 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
       ctx->launches = scans;
     }
     k_gather_offsets<<<(nprod + 256) / 256, 256, 0, s>>>(b->cp, b->d_base, nprod, b->offs);
-    b->g1_kernels = 2 + check + (R > 0 ? 3 + row_kernels : 0);
+    b->g1_kernels = 2 + check + (R > 0 ? 3 + (R >= kFuseRows) + row_kernels : 0);
     cudaMemcpyAsync(b->h_offs, b->offs, sizeof(int64_t) * (nprod + 1), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(b->h_offs + nprod + 1, &b->sched[0].max_a_row, sizeof(int64_t),
                     cudaMemcpyDeviceToHost, s);

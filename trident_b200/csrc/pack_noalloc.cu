@@ -101,14 +101,14 @@ int pack_noalloc_impl(cudaStream_t s, const tspg_csr *M, int64_t len,
     k_scan_final<<<(unsigned)nb, kScanThreads, 0, s>>>(cnt, len, partial, nb, newp, unused,
                                                        nullptr);
   }
-  const int64_t work = (M->nnz + kPackItems - 1) / kPackItems;
+  const int64_t work = (M->nnz + kPackRun - 1) / kPackRun * 32;
   const int64_t w = work > len + 1 ? work : len + 1;
   const unsigned grid = (unsigned)std::min<int64_t>((w + 255) / 256, int64_t(num_sms) * 32);
   if (M->val_bits == 64)
-    k_pack_copy<PT, 8><<<grid, 256, 0, s>>>(ptr, len, M->col, M->val, mask, newp,
+    k_pack_copy<PT, 8><<<grid, 256, 0, s>>>(ptr, len, M->col, M->val, newp,
                                             (char *)out_buf, kept_dev);
   else
-    k_pack_copy<PT, 4><<<grid, 256, 0, s>>>(ptr, len, M->col, M->val, mask, newp,
+    k_pack_copy<PT, 4><<<grid, 256, 0, s>>>(ptr, len, M->col, M->val, newp,
                                             (char *)out_buf, kept_dev);
   if (cudaGetLastError() != cudaSuccess) return TSPG_ECUDA;
   return TSPG_OK;

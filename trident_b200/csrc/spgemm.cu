@@ -154,9 +154,9 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
     TSPG_CUDA(ctx, cudaGetLastError());
     return TSPG_OK;  // nothing to count: c_nnz, mults and max_a_row stay 0
   }
-  k_row_mults<PT, VT><<<grid_for(m * 32, 256, ctx->num_sms * 16), 256, 0, s>>>(
-      prods, P->base, 1, m, P->rowf, P->sched, P->rowc, m < kFuseRows);
-  ctx->launches += 1;
+  const bool fuse = m < kFuseRows;
+  launch_row_mults<PT, VT>(ctx, s, prods, P->base, 1, m, P->rowf, P->sched, P->rowc, fuse,
+                           fuse ? nullptr : P->list);
   if (onepass) {
     // the one-pass rows' scratch offsets: a scan of their output bounds
     launch_scan(ctx, s, P->rowc, m, P->partial, P->cp, P->sched + 1, nullptr);
@@ -489,9 +489,8 @@ extern "C" int tspg_spgemm_count(tspg_ctx *ctx, void *stream,
     v.n = B->ncols;
     k_setup<PT, VT><<<1, 128, 0, s>>>(prods, v, base, sched, 1, ctx->tune, 0);
     if (m > 0)
-      k_row_mults<PT, VT><<<grid_for(m * 32, 256, ctx->num_sms * 16), 256, 0, s>>>(
-          prods, base, 1, m, rowf, sched);
-    ctx->launches += 1 + (m > 0);
+      launch_row_mults<PT, VT>(ctx, s, prods, base, 1, m, rowf, sched, nullptr, 0, nullptr);
+    ctx->launches += 1;
     TSPG_CUDA(ctx, cudaGetLastError());
     int64_t *h = ctx->h_words;
     TSPG_CUDA(ctx, cudaMemcpyAsync(h, &sched->total, 2 * sizeof(int64_t),
@@ -505,35 +504,75 @@ extern "C" int tspg_spgemm_count(tspg_ctx *ctx, void *stream,
 
 namespace tspg {
 
-// Flop count of A·B fused with the SUMMA stage mask: one warp per row of A;
-// entry (i, k) adds nnz(B row k) to the row's products and, when that row of B
-// is non-empty, sets bit k of the word mask.  Bit k ends up set exactly when
-// column k of A holds an entry and row k of B is non-empty, i.e. the AND of
-// the column mask of A and the row mask of B.
+// Flop count of A·B fused with the SUMMA stage mask, over A's entries in runs
+// of kMaskRun per warp (balanced however they cluster in rows; a warp per row
+// waited on the hub rows of an R-MAT tile: 126 -> 20 us for 0.7M entries).
+// Entry (i, k) adds nnz(B row k) to row i's products — summed over the lanes of
+// the row, one reduction per row and window — and, when that row of B is
+// non-empty, sets bit k of the word mask.  Bit k ends up set exactly when
+// column k of A holds an entry and row k of B is non-empty, i.e. the AND of the
+// column mask of A and the row mask of B.
+constexpr int kMaskRun = 128;
 template <typename APT, typename BPT>
-__global__ void k_count_mask(const APT *Ap, const int32_t *Aj, const BPT *Bp, int64_t m,
-                             int64_t n, uint32_t *mask, unsigned long long *tot) {
+__global__ void __launch_bounds__(256)
+    k_count_mask(const APT *__restrict__ Ap, const int32_t *__restrict__ Aj,
+                 const BPT *__restrict__ Bp, int64_t m, uint32_t *mask,
+                 unsigned long long *rowf) {
+  constexpr int U = kMaskRun / 32;
   const int lane = threadIdx.x & 31;
-  const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  unsigned long long wm = 0, wu = 0;
-  for (int64_t r = warp; r < m; r += nwarps) {
-    const int64_t a0 = int64_t(Ap[r]), a1 = int64_t(Ap[r + 1]);
-    int64_t sum = 0;
-    for (int64_t q = a0 + lane; q < a1; q += 32) {
-      const int32_t k = __ldg(Aj + q);
-      const int64_t len = int64_t(Bp[k + 1]) - int64_t(Bp[k]);
-      sum += len;
-      if (len > 0) {
-        const uint32_t bit = 1u << (k & 31);
-        if (!(*(volatile uint32_t *)(mask + (k >> 5)) & bit)) atomicOr(mask + (k >> 5), bit);
-      }
-    }
-    sum = warp_sum(sum);
-    wm += (unsigned long long)sum;
-    wu += (unsigned long long)(sum < n ? sum : n);
+  const int64_t e0 = ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kMaskRun;
+  const int64_t base = int64_t(Ap[0]), count = int64_t(Ap[m]) - base;
+  if (e0 >= count) return;
+  int32_t k[U];
+  int64_t len[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int64_t e = e0 + u * 32 + lane;
+    k[u] = e < count ? __ldg(Aj + base + e) : -1;
   }
-  if (lane == 0 && (wm | wu)) {
+#pragma unroll
+  for (int u = 0; u < U; ++u) len[u] = k[u] >= 0 ? int64_t(__ldg(Bp + k[u] + 1)) - int64_t(__ldg(Bp + k[u])) : 0;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (len[u] > 0) {
+      const uint32_t bit = 1u << (k[u] & 31);
+      if (!(*(volatile uint32_t *)(mask + (k[u] >> 5)) & bit)) atomicOr(mask + (k[u] >> 5), bit);
+    }
+  }
+  int64_t r = first_row(Ap, m, base, e0, lane);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (e0 + u * 32 < count) {  // uniform
+      const int64_t row = window_row(Ap, m, base, r, e0 + u * 32 + lane, lane);
+      // inclusive sums inside runs of one row; the run's last lane adds it
+      const int64_t prev = __shfl_up_sync(0xffffffffu, row, 1);
+      const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != row);
+      const int head = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+      int64_t sum = len[u];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int64_t x = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane - o >= head) sum += x;
+      }
+      const bool last = lane == 31 || ((heads >> (lane + 1)) & 1u);
+      if (last && sum > 0) atomicAdd(rowf + row, (unsigned long long)sum);
+    }
+  }
+}
+
+// Totals of the row products: mults and sum of min(products, n).
+__global__ void __launch_bounds__(256)
+    k_count_totals(const unsigned long long *rowf, int64_t m, int64_t n, unsigned long long *tot) {
+  unsigned long long wm = 0, wu = 0;
+  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+  for (int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < m; r += stride) {
+    const unsigned long long f = rowf[r];
+    wm += f;
+    wu += f < (unsigned long long)n ? f : (unsigned long long)n;
+  }
+  wm = warp_sum(wm);
+  wu = warp_sum(wu);
+  if ((threadIdx.x & 31) == 0 && (wm | wu)) {
     atomicAdd(tot, wm);
     atomicAdd(tot + 1, wu);
   }
@@ -547,9 +586,13 @@ __global__ void k_mask_bytes(const uint32_t *w, int64_t nbytes, uint8_t *out) {
 
 template <typename APT, typename BPT>
 static void launch_count_mask(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A, const tspg_csr *B,
-                              uint32_t *words, unsigned long long *tot) {
-  k_count_mask<APT, BPT><<<grid_for(A->nrows * 32, 256, ctx->num_sms * 16), 256, 0, s>>>(
-      (const APT *)A->rowptr, A->col, (const BPT *)B->rowptr, A->nrows, B->ncols, words, tot);
+                              uint32_t *words, unsigned long long *rowf, unsigned long long *tot) {
+  if (A->nnz > 0)
+    k_count_mask<APT, BPT><<<unsigned((A->nnz + 8 * kMaskRun - 1) / (8 * kMaskRun)), 256, 0, s>>>(
+        (const APT *)A->rowptr, A->col, (const BPT *)B->rowptr, A->nrows, words, rowf);
+  k_count_totals<<<grid_for(A->nrows, 256, ctx->num_sms * 4), 256, 0, s>>>(rowf, A->nrows, B->ncols,
+                                                                          tot);
+  ctx->launches += 1 + (A->nnz > 0);
 }
 
 }  // namespace tspg
@@ -564,18 +607,16 @@ extern "C" int tspg_spgemm_count_mask(tspg_ctx *ctx, void *stream, const tspg_cs
   cudaStream_t s = (cudaStream_t)stream;
   TSPG_CUDA(ctx, cudaSetDevice(ctx->device));
   Scratch sc(ctx, s);
-  uint32_t *words;
-  unsigned long long *tot;
-  TSPG_TRY(sc.get(&words, (kdim + 31) / 32));
-  TSPG_TRY(sc.get(&tot, 2));
-  TSPG_CUDA(ctx, cudaMemsetAsync(words, 0, sizeof(uint32_t) * ((kdim + 31) / 32 > 0 ? (kdim + 31) / 32 : 1), s));
-  TSPG_CUDA(ctx, cudaMemsetAsync(tot, 0, 2 * sizeof(unsigned long long), s));
+  uint32_t *words;  // the mask words, then (8-byte aligned) two totals and the row products
+  const int64_t nw = ((kdim + 31) / 32 + 1) & ~int64_t(1);
+  TSPG_TRY(sc.get(&words, nw + 2 * (A->nrows + 2)));
+  unsigned long long *tot = (unsigned long long *)(words + nw), *rowf = tot + 2;
+  TSPG_CUDA(ctx, cudaMemsetAsync(words, 0, sizeof(uint32_t) * (nw + 2 * (A->nrows + 2)), s));
   if (A->nrows > 0) {
-    if (A->rowptr_bits == 32 && B->rowptr_bits == 32) launch_count_mask<int32_t, int32_t>(ctx, s, A, B, words, tot);
-    else if (A->rowptr_bits == 32) launch_count_mask<int32_t, int64_t>(ctx, s, A, B, words, tot);
-    else if (B->rowptr_bits == 32) launch_count_mask<int64_t, int32_t>(ctx, s, A, B, words, tot);
-    else launch_count_mask<int64_t, int64_t>(ctx, s, A, B, words, tot);
-    ctx->launches += 1;
+    if (A->rowptr_bits == 32 && B->rowptr_bits == 32) launch_count_mask<int32_t, int32_t>(ctx, s, A, B, words, rowf, tot);
+    else if (A->rowptr_bits == 32) launch_count_mask<int32_t, int64_t>(ctx, s, A, B, words, rowf, tot);
+    else if (B->rowptr_bits == 32) launch_count_mask<int64_t, int32_t>(ctx, s, A, B, words, rowf, tot);
+    else launch_count_mask<int64_t, int64_t>(ctx, s, A, B, words, rowf, tot);
   }
   if (nbytes > 0) {
     k_mask_bytes<<<(unsigned)((nbytes + 255) / 256), 256, 0, s>>>(words, nbytes, mask);

@@ -186,6 +186,7 @@ struct Sched {
   unsigned long long work3;     // row counter of the rank-form DENSE kernel
   int32_t rank_left;            // DENSE rows that kernel left to k_phase (0 / 1)
   int32_t pad32b;
+  unsigned long long nlong;     // A rows left to k_row_mults_long
 };
 
 __device__ __forceinline__ int find_prod(const int64_t *base, int nprod,
@@ -338,6 +339,10 @@ __global__ void k_check_sorted_rows(const PT *Bp, const int32_t *Bj,
 // reduction), block-aggregated class counts.
 // Rows of at most this many A entries are walked by one lane in k_row_mults.
 constexpr int kThreadRowMax = 64;
+// ... and rows of more than this many are listed for k_row_mults_long (a CTA
+// per row took 0.42 ms on the 119-entry rows of the Galerkin R·AP, a warp per
+// row 0.1 ms).
+constexpr int kLongRow = 256;
 // A entries a one-pass candidate looks at for repeated columns.
 constexpr int kHintEntries = 8;
 
@@ -351,10 +356,15 @@ constexpr int kHintEntries = 8;
 // would otherwise all hit one counter).  One warp per row, as first built,
 // took 0.8 ms on the 2.1M rows of the Galerkin A·P (27 entries each): four
 // dependent loads per row, one row per warp at a time.
+//
+// longs: the rows of more than kLongRow entries are listed there instead
+// (k_row_mults_long): R-MAT's hub rows are neighbours, and the warp that held
+// 32 of them was the pass (order 2^18, 16 draws a row: 0.58 ms).  Without a
+// list the warp keeps 8 loads per lane in flight on such a row.
 template <typename PT, typename VT>
 __global__ void __launch_bounds__(256) k_row_mults(
     const ProdDev<PT, VT> *prods, const int64_t *base, int nprod, int64_t R,
-    int64_t *rowf, Sched *S, int32_t *rowc = nullptr, int finish = 0) {
+    int64_t *rowf, Sched *S, int32_t *rowc = nullptr, int finish = 0, uint64_t *longs = nullptr) {
   __shared__ unsigned long long s_cnt[NCLS], s_cand[NCLS];
   __shared__ unsigned long long s_tot, s_up, s_ne;
   __shared__ long long s_maxa;
@@ -395,16 +405,27 @@ __global__ void __launch_bounds__(256) k_row_mults(
       for (int u = 0; u < 4; ++u)
         if (k[u] >= 0) f += int64_t(__ldg(Bp + k[u] + 1)) - int64_t(__ldg(Bp + k[u]));
     }
-    for (unsigned lr = __ballot_sync(0xffffffffu, !mine); lr; lr &= lr - 1) {
+    const bool listed = longs && len > kLongRow;
+    if (const unsigned lm = __ballot_sync(0xffffffffu, listed)) {
+      unsigned long long at = 0;
+      if (lane == 0) at = atomicAdd(&S->nlong, (unsigned long long)__popc(lm));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (listed) longs[at + __popc(lm & ((1u << lane) - 1u))] = (uint64_t(p) << 40) | uint64_t(r);
+    }
+    for (unsigned lr = __ballot_sync(0xffffffffu, !mine && !listed); lr; lr &= lr - 1) {
       const int j = __ffs(lr) - 1;
       const int pj = __shfl_sync(0xffffffffu, p, j);
       const int64_t b0 = __shfl_sync(0xffffffffu, a0, j), b1 = __shfl_sync(0xffffffffu, a1, j);
       const int32_t *Ajj = prods[pj].Aj;
       const PT *Bpj = prods[pj].Bp;
       int64_t sum = 0;
-      for (int64_t q = b0 + lane; q < b1; q += 32) {
-        const int64_t k = __ldg(Ajj + q);
-        sum += int64_t(__ldg(Bpj + k + 1)) - int64_t(__ldg(Bpj + k));
+      for (int64_t q = b0; q < b1; q += 32 * 8) {
+        int32_t k[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) k[u] = q + u * 32 + lane < b1 ? __ldg(Ajj + q + u * 32 + lane) : -1;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (k[u] >= 0) sum += int64_t(__ldg(Bpj + k[u] + 1)) - int64_t(__ldg(Bpj + k[u]));
       }
       sum = warp_sum(sum);
       if (lane == j) f = sum;
@@ -417,7 +438,7 @@ __global__ void __launch_bounds__(256) k_row_mults(
     int same = 0, seen = 0;
     {
       const int64_t fe = f < (valid ? prods[p].n : 0) ? f : (valid ? prods[p].n : 0);
-      const bool need = S->onepass && valid && fe > 0 && fe <= S->tune.sym[2] &&
+      const bool need = S->onepass && valid && !listed && fe > 0 && fe <= S->tune.sym[2] &&
                         int64_t(S->tune.load) * fe > 2 * kCappedCols;
       if (__any_sync(0xffffffffu, need)) {
         const int32_t *Bj = valid ? prods[p].Bj : nullptr;
@@ -433,7 +454,7 @@ __global__ void __launch_bounds__(256) k_row_mults(
       }
     }
     int c = -1, left = -1;
-    if (valid) {
+    if (valid && !listed) {
       if (prods[p].Ej) {  // the addend's entries count as products of the row
         int64_t e0, e1;
         addend_row(prods[p], r, e0, e1);
@@ -501,6 +522,107 @@ __global__ void __launch_bounds__(256) k_row_mults(
     atomicMax((long long *)&S->max_a_row, s_maxa);
   }
   if (finish && last_block(&S->ticket) && threadIdx.x == 0) sched_offsets(S);
+}
+
+// The rows k_row_mults listed (more than kLongRow A entries), a CTA each,
+// with the same results per row.
+template <typename PT, typename VT>
+__global__ void __launch_bounds__(256) k_row_mults_long(
+    const ProdDev<PT, VT> *prods, const int64_t *base, int64_t *rowf, Sched *S, int32_t *rowc,
+    const uint64_t *longs) {
+  __shared__ int64_t part[8];
+  __shared__ unsigned long long s_cnt[NCLS], s_cand[NCLS];
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid < NCLS) s_cnt[tid] = s_cand[tid] = 0;
+  const int64_t n = int64_t(S->nlong);
+  unsigned long long tot = 0, up = 0, ne = 0;  // thread 0's
+  long long maxa = 0;
+  for (int64_t i = blockIdx.x; i < n; i += gridDim.x) {
+    const int p = int(longs[i] >> 40);
+    const int64_t r = int64_t(longs[i] & ((uint64_t(1) << 40) - 1));
+    const ProdDev<PT, VT> &P = prods[p];
+    const int32_t *__restrict__ Aj = P.Aj;
+    const PT *__restrict__ Bp = P.Bp;
+    const int64_t a0 = int64_t(P.Ap[r]), a1 = int64_t(P.Ap[r + 1]);
+    int64_t sum = 0;
+    for (int64_t q = a0 + tid; q < a1; q += 256 * 4) {
+      int32_t k[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) k[u] = q + u * 256 < a1 ? __ldg(Aj + q + u * 256) : -1;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (k[u] >= 0) sum += int64_t(__ldg(Bp + k[u] + 1)) - int64_t(__ldg(Bp + k[u]));
+    }
+    sum = warp_sum(sum);
+    if (lane == 0) part[tid >> 5] = sum;
+    __syncthreads();
+    if (tid == 0) {
+      int64_t f = 0;
+      for (int w = 0; w < 8; ++w) f += part[w];
+      const int64_t g = base[p] + r;
+      bool repeats = false;  // as in k_row_mults: kHintEntries (< kLongRow) entries
+      if (S->onepass && onepass_row(f, P.n, S->tune) && !onepass_full(f, P.n, S->tune)) {
+        int same = 0, prev = -2;
+        for (int t = 0; t < kHintEntries; ++t) {
+          const int64_t k = __ldg(Aj + a0 + t);
+          const int64_t q0 = int64_t(__ldg(Bp + k)), q1 = int64_t(__ldg(Bp + k + 1));
+          const int first = q1 > q0 ? __ldg(P.Bj + q0) : -1;
+          same += first >= 0 && first == prev;
+          prev = first;
+        }
+        repeats = 4 * same >= kHintEntries - 1;
+      }
+      if (P.Ej) {
+        int64_t e0, e1;
+        addend_row(P, r, e0, e1);
+        f += e1 - e0;
+      }
+      rowf[g] = f;
+      int c = sym_class(f, P.n, S->tune);
+      const bool one = S->onepass && onepass_row(f, P.n, S->tune) &&
+                       (onepass_full(f, P.n, S->tune) || repeats);
+      if (one) {
+        ++s_cand[c];
+        c = CLS_ONEPASS;
+      }
+      if (rowc) rowc[g] = one ? int32_t(onepass_bound(f, P.n, S->tune)) : 0;
+      if (c >= 0) {
+        ++s_cnt[c];
+        ++ne;
+      }
+      tot += (unsigned long long)f;
+      up += (unsigned long long)(f < P.n ? f : P.n);
+      if (a1 - a0 > maxa) maxa = a1 - a0;
+    }
+    __syncthreads();
+  }
+  if (tid == 0 && maxa > 0) {
+    for (int c = 0; c < NCLS; ++c) {
+      if (s_cnt[c]) atomicAdd((unsigned long long *)&S->cnt[c], s_cnt[c]);
+      if (s_cand[c]) atomicAdd((unsigned long long *)&S->cand[c], s_cand[c]);
+    }
+    atomicAdd((unsigned long long *)&S->total, tot);
+    atomicAdd((unsigned long long *)&S->upper, up);
+    atomicAdd((unsigned long long *)&S->nonempty, ne);
+    atomicMax((long long *)&S->max_a_row, maxa);
+  }
+}
+
+// The count pass of R rows: rowf, the record's class counts and sums.  longs
+// (R entries): the list of long rows of products of kFuseRows rows or more,
+// whose count takes a launch of its own.
+template <typename PT, typename VT>
+static inline void launch_row_mults(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, VT> *prods,
+                                    const int64_t *base, int nprod, int64_t R, int64_t *rowf,
+                                    Sched *S, int32_t *rowc, int finish, uint64_t *longs) {
+  const unsigned g = unsigned((R * 32 + 255) / 256 < int64_t(ctx->num_sms) * 16
+                                  ? (R * 32 + 255) / 256 : int64_t(ctx->num_sms) * 16);
+  k_row_mults<PT, VT><<<g, 256, 0, s>>>(prods, base, nprod, R, rowf, S, rowc, finish, longs);
+  ctx->launches += 1;
+  if (longs) {
+    k_row_mults_long<PT, VT><<<ctx->num_sms * 8, 256, 0, s>>>(prods, base, rowf, S, rowc, longs);
+    ctx->launches += 1;
+  }
 }
 
 // The one-pass rows of a symbolic record go back to the classes they left
