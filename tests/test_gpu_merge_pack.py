@@ -231,3 +231,27 @@ def test_packed_tile_multiplies_like_masked_tile(ctx):
     buf, kept = ops.compress(ctx, dB, rowmask)
     Bp = ops.unpack(buf, 256, 200, kept)
     check_product(ops.spgemm(ctx, A.to_device(), Bp), A, B)
+
+
+def _sorted_rows(lens, n, seed):
+    rng = np.random.default_rng(seed)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    col = [np.sort(rng.choice(n, size=k, replace=False)) for k in lens]
+    col = np.concatenate(col).astype(np.int32) if len(col) else np.zeros(0, np.int32)
+    return HostCSR(len(lens), n, rp, col, rng.uniform(-1, 1, col.size))
+
+
+@pytest.mark.parametrize("la,lb,n", [
+    ([2047], [1], 5000), ([2048], [2048], 2048), ([2049, 0, 0], [0, 0, 2047], 4096), ([1024] * 5, [1024] * 5, 1024),
+    ([0] * 5000 + [3, 0, 2], [0] * 4999 + [5, 0, 1, 0], 40), ([7, 0, 1] * 3000, [8, 1, 0] * 3000, 9),
+    ([30000, 5, 0, 30000], [29999, 0, 5, 1], 40000), ([0, 0], [0, 0], 3), ([1] * 4096, [1] * 4096, 1)])
+def test_spadd_tile_edges(ctx, la, lb, n):
+    # merged tiles of 2048 entries: rows and equal pairs cut by a tile's edge,
+    # more than 1024 rows in a tile, runs of empty rows, one operand empty
+    A, B = _sorted_rows(la, n, 1), _sorted_rows(lb, n, 2)
+    Z = _sorted_rows([0] * len(la), n, 3)
+    check_sum(ops.spadd(ctx, A.to_device(), B.to_device(), rowptr_bits=32), A, B)
+    check_sum(ops.spadd(ctx, B.to_device(rowptr_bits=64), A.to_device(rowptr_bits=32)), B, A)
+    check_sum(ops.spadd(ctx, A.to_device(), Z.to_device()), A, Z)
+    check_sum(ops.spadd(ctx, Z.to_device(), A.to_device()), Z, A)
+    check_sum(ops.spadd(ctx, A.to_device(), A.to_device()), A, A)

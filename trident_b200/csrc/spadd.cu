@@ -3,246 +3,306 @@
 // Replaces cusparse_spgeam (include/cusparse_helpers.cuh:799-905: csrgeam2
 // bufferSize + Nnz + compute, five stream syncs, the nnz through the host) and
 // LocalMatrix::spadd (include/KokkosWrap.hpp:394-439: KK spadd symbolic +
-// numeric).  Rows are sorted and duplicate-free, so every entry finds its
-// output slot from its rank in the other row.  Rows with up to kMergeHeavy
-// entries in A and B together: one warp per row, merging 32-column chunks of
-// both rows in registers (merge_row_warp; per-entry binary searches of the
-// other row, as first built, took twice as long).  Longer rows (the hub rows of
-// partial C tiles reach 10^5 entries, and one warp per such row left the merge
-// waiting on a handful of warps) are listed and merged by a whole CTA: its
-// warps take the ranges between merge-path cuts of the row.
+// numeric).  Rows are sorted and duplicate-free, so both operands are sequences
+// sorted by (row, column) and the union is one merge of the two.  It is cut
+// into tiles of kMergeTile merged entries, whatever the rows' lengths: one
+// thread per cut finds its row in the sum of the row offsets, then its place
+// inside the row (merge path); a CTA merges a tile, each thread 7 entries,
+// first counting, then writing.
+//
+// What bounds it: the serial merges and the two searches before them (about 30
+// warp instructions per 32 entries and pass); the operands cross memory twice.
+// R-MAT of order 2^18, 64 draws a row, A + B: 0.83 -> 0.43 ms against one warp
+// per row merging 32-column chunks ranked by shuffles (about 400 instructions
+// per 32 entries, hub rows in a kernel of their own); 0.49 ms with a tile's
+// loads in loops of unknown length instead of all in flight.
 #include "internal.cuh"
 #include "spgemm_kernels.cuh"
 
 namespace tspg {
 
-constexpr int64_t kMergeHeavy = 4096;  // rows above this go to the CTA merge
-constexpr int kMergeThreads = 512;
+constexpr int kMergeThreads = 256;
+constexpr int kMergePer = 7;  // merged entries per thread: odd, so that threads stepping through
+                               // shared memory in step hit different banks
+constexpr int kMergeTile = kMergeThreads * kMergePer;
+constexpr int kMergeRows = 1024;                      // row ends kept in shared memory
 
-// Chunked warp merge of one light row.  Each iteration loads the next 32
-// columns of A and of B (coalesced).  Every entry up to lim, the smaller of
-// the two chunk maxima, is final this iteration (entries past a full chunk are
-// larger than its maximum); its output position is its index in its chunk
-// plus its rank in the other chunk (a 5-step search over the other chunk's
-// registers by shuffles) minus the columns of both rows below it.  A column in
-// both rows leaves once, from A, with the two values added.  At least 32
-// entries leave per iteration and no global load depends on another.
-// WRITE = false returns the size of the union only; WRITE = true writes no
-// position at or past cap (the row's size from the count pass), so rows that
-// break the sorted / duplicate-free contract cannot write outside their row.
-template <bool WRITE, typename VT>
-__device__ __forceinline__ int64_t merge_row_warp(const int32_t *__restrict__ Aj,
-                                                  const VT *__restrict__ Ax, int64_t a0,
-                                                  int64_t a1, const int32_t *__restrict__ Bj,
-                                                  const VT *__restrict__ Bx, int64_t b0,
-                                                  int64_t b1, int32_t *__restrict__ cj,
-                                                  VT *__restrict__ cx, int64_t cap, int lane) {
-  constexpr unsigned FULL = 0xffffffffu;
-  const unsigned below = (1u << lane) - 1u;
-  int64_t pa = a0, pb = b0, out = 0;
-  while (pa < a1 || pb < b1) {
-    const bool va = pa + lane < a1, vb = pb + lane < b1;
-    const int32_t ai = va ? __ldg(Aj + pa + lane) : INT32_MAX;  // no column is INT32_MAX
-    const int32_t bi = vb ? __ldg(Bj + pb + lane) : INT32_MAX;
-    VT av = VT(0), bv = VT(0);
-    if constexpr (WRITE) {
-      if (va) av = __ldg(Ax + pa + lane);
-      if (vb) bv = __ldg(Bx + pb + lane);
-    }
-    const int32_t lastA = __shfl_sync(FULL, ai, 31), lastB = __shfl_sync(FULL, bi, 31);
-    const int32_t lim = min(pa + 32 <= a1 ? lastA : INT32_MAX, pb + 32 <= b1 ? lastB : INT32_MAX);
-    int ra = 0, rb = 0;  // entries of the other chunk below this lane's entry
-#pragma unroll
-    for (int st = 16; st > 0; st >>= 1) {
-      if (__shfl_sync(FULL, bi, ra + st - 1) < ai) ra += st;
-      if (__shfl_sync(FULL, ai, rb + st - 1) < bi) rb += st;
-    }
-    if (ra == 31 && lastB < ai) ra = 32;
-    if (rb == 31 && lastA < bi) rb = 32;
-    const int32_t bat = __shfl_sync(FULL, bi, ra & 31), aat = __shfl_sync(FULL, ai, rb & 31);
-    const bool ca = va && ai <= lim, cb = vb && bi <= lim;
-    const bool dupa = ca && ra < 32 && bat == ai, dupb = cb && rb < 32 && aat == bi;
-    const unsigned dm = __ballot_sync(FULL, dupa);
-    const int na = __popc(__ballot_sync(FULL, ca)), nb = __popc(__ballot_sync(FULL, cb));
-    if constexpr (WRITE) {
-      const VT bvat = __shfl_sync(FULL, bv, ra & 31);
-      if (ca) {
-        const int64_t pos = out + lane + ra - __popc(dm & below);
-        if (pos < cap) {
-          cj[pos] = ai;
-          cx[pos] = dupa ? av + bvat : av;
-        }
-      }
-      if (cb && !dupb) {
-        const unsigned mk = rb >= 32 ? FULL : ((1u << rb) - 1u);
-        const int64_t pos = out + lane + rb - __popc(dm & mk);
-        if (pos < cap) {
-          cj[pos] = bi;
-          cx[pos] = bv;
-        }
-      }
-    }
-    out += na + nb - __popc(dm);
-    pa += na;
-    pb += nb;
-  }
-  return out;
-}
+// A cut of the merged sequence before entry d: the row whose entries it falls
+// into (the last one starting at or before d), the first row starting at or
+// after d, and the entries of A and B (from their first) before it.
+struct MergeCut {
+  int64_t row, first, i, j;
+};
 
 template <typename PTA, typename PTB>
-__global__ void __launch_bounds__(256)
-    k_spadd_count(int64_t m, const PTA *Ap, const int32_t *Aj, const PTB *Bp,
-                  const int32_t *Bj, int32_t *rowc, int64_t *heavy, int64_t *nheavy) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t r = warp; r < m; r += nwarps) {
-    const int64_t a0 = Ap[r], a1 = Ap[r + 1], b0 = Bp[r], b1 = Bp[r + 1];
-    if ((a1 - a0) + (b1 - b0) > kMergeHeavy) {
-      if (lane == 0) heavy[atomicAdd((unsigned long long *)nheavy, 1ull)] = r;
-      continue;
-    }
-    const int64_t n = merge_row_warp<false, double>(Aj, nullptr, a0, a1, Bj, nullptr, b0, b1,
-                                                    nullptr, nullptr, 0, lane);
-    if (lane == 0) rowc[r] = int32_t(n);
-  }
-}
-
-template <typename PTA, typename PTB, typename VT>
-__global__ void __launch_bounds__(256)
-    k_spadd_fill(int64_t m, const PTA *Ap, const int32_t *Aj, const VT *Ax,
-                 const PTB *Bp, const int32_t *Bj, const VT *Bx,
-                 const int64_t *cp, void *Cp, int cp_bits, int32_t *Cj, VT *Cx) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t r = warp; r < m; r += nwarps) {
-    const int64_t a0 = Ap[r], a1 = Ap[r + 1], b0 = Bp[r], b1 = Bp[r + 1];
-    const int64_t o = cp[r];
-    if (lane == 0) {
-      if (cp_bits == 32) ((int32_t *)Cp)[r] = int32_t(o);
-      else ((int64_t *)Cp)[r] = o;
-      if (r == m - 1) {
-        if (cp_bits == 32) ((int32_t *)Cp)[m] = int32_t(cp[m]);
-        else ((int64_t *)Cp)[m] = cp[m];
-      }
-    }
-    if ((a1 - a0) + (b1 - b0) > kMergeHeavy) continue;  // merged by k_spadd_heavy
-    merge_row_warp<true, VT>(Aj, Ax, a0, a1, Bj, Bx, b0, b1, Cj + o, Cx + o, cp[r + 1] - o, lane);
-  }
-}
-
-// Heavy rows: one CTA of kMergeWarps warps per row.  The merged sequence is
-// cut at kMergeWarps + 1 diagonals (merge path: the A entries among the first
-// d merged entries, A before B on equal columns); a column present in both
-// rows whose A entry falls before a cut and B entry after it moves whole to
-// the earlier range, so every range merges on its own.  Each warp merges its
-// range with merge_row_warp.  The count pass keeps the cuts and the per-warp
-// counts (meta: kMergeWarps counts, then kMergeWarps + 1 pairs of cuts per
-// listed row) for the fill pass.
-constexpr int kMergeWarps = kMergeThreads / 32;
-constexpr int kHeavyMeta = kMergeWarps + 2 * (kMergeWarps + 1);
-
-__device__ __forceinline__ void merge_cut(const int32_t *__restrict__ aj, int64_t la,
-                                          const int32_t *__restrict__ bj, int64_t lb, int64_t d,
-                                          int64_t &i, int64_t &j) {
-  int64_t lo = d > lb ? d - lb : 0, hi = d < la ? d : la;
+__global__ void __launch_bounds__(128)
+    k_merge_cuts(int64_t m, const PTA *__restrict__ Ap, const int32_t *__restrict__ Aj,
+                 const PTB *__restrict__ Bp, const int32_t *__restrict__ Bj, int64_t ntiles,
+                 MergeCut *cuts) {
+  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t > ntiles) return;
+  const int64_t ab = int64_t(Ap[0]), bb = int64_t(Bp[0]);
+  auto start = [&](int64_t r) { return int64_t(__ldg(Ap + r)) - ab + int64_t(__ldg(Bp + r)) - bb; };
+  const int64_t total = start(m);
+  const int64_t d = t * kMergeTile < total ? t * kMergeTile : total;
+  int64_t lo = 0, hi = m;  // the last row in [0, m] with start <= d
   while (lo < hi) {
     const int64_t mid = (lo + hi + 1) >> 1;
-    if (__ldg(aj + mid - 1) <= __ldg(bj + d - mid)) lo = mid; else hi = mid - 1;
+    if (start(mid) <= d) lo = mid; else hi = mid - 1;
   }
-  i = lo;
-  j = d - lo;
-  // the B entry that follows an equal A entry: the diagonal after d takes it
-  // first (A is strictly increasing), so the next cut's j stays >= this one
-  if (i > 0 && j < lb && __ldg(aj + i - 1) == __ldg(bj + j)) ++j;
+  MergeCut c;
+  c.row = lo;
+  if (start(lo) < d) {
+    c.first = lo + 1;
+  } else {
+    int64_t a = 0, z = lo;  // the first row with start >= d
+    while (a < z) {
+      const int64_t mid = (a + z) >> 1;
+      if (start(mid) < d) a = mid + 1; else z = mid;
+    }
+    c.first = a;
+  }
+  c.i = int64_t(__ldg(Ap + lo)) - ab;
+  c.j = int64_t(__ldg(Bp + lo)) - bb;
+  if (lo < m) {
+    // A before B on equal columns: among the row's first q merged entries are
+    // x of A, the least x with A[x] > B[q - 1 - x]
+    const int64_t la = int64_t(__ldg(Ap + lo + 1)) - ab - c.i, lb = int64_t(__ldg(Bp + lo + 1)) - bb - c.j;
+    const int64_t q = d - c.i - c.j;
+    const int32_t *aj = Aj + ab + c.i, *bj = Bj + bb + c.j;
+    int64_t x = q > lb ? q - lb : 0, y = q < la ? q : la;
+    while (x < y) {
+      const int64_t mid = (x + y) >> 1;
+      if (__ldg(aj + mid) <= __ldg(bj + q - 1 - mid)) x = mid + 1; else y = mid;
+    }
+    c.i += x;
+    c.j += q - x;
+  }
+  cuts[t] = c;
 }
 
+// One tile: WRITE = false leaves its number of output entries in rowc[tile];
+// WRITE = true writes them from off[tile] on, and the offsets of the rows that
+// start in the tile.  A column in both rows leaves with A's entry (the two
+// values added); B's entry of the pair is a "dup" and leaves nothing, so entry
+// x of the tile goes to slot x - (dups before x).
 template <bool WRITE, typename PTA, typename PTB, typename VT>
 __global__ void __launch_bounds__(kMergeThreads)
-    k_spadd_heavy(const int64_t *heavy, const int64_t *nheavy, const PTA *Ap,
-                  const int32_t *Aj, const VT *Ax, const PTB *Bp, const int32_t *Bj,
-                  const VT *Bx, int32_t *rowc, const int64_t *cp, int64_t *meta, int32_t *Cj,
-                  VT *Cx) {
-  __shared__ int64_t cnt[kMergeWarps];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t nh = *nheavy;
-  for (int64_t h = blockIdx.x; h < nh; h += gridDim.x) {
-    const int64_t r = heavy[h];
-    const int64_t a0 = Ap[r], a1 = Ap[r + 1], b0 = Bp[r], b1 = Bp[r + 1];
-    const int64_t la = a1 - a0, lb = b1 - b0;
-    int64_t *mt = meta + h * kHeavyMeta;
-    int64_t *cuts = mt + kMergeWarps;  // (i, j) per diagonal
-    if constexpr (!WRITE) {
-      if (threadIdx.x <= kMergeWarps) {
-        int64_t i, j;
-        merge_cut(Aj + a0, la, Bj + b0, lb, (la + lb) * threadIdx.x / kMergeWarps, i, j);
-        cuts[2 * threadIdx.x] = i;
-        cuts[2 * threadIdx.x + 1] = j;
+    k_merge_tiles(int64_t m, const PTA *__restrict__ Ap, const int32_t *__restrict__ Aj,
+                  const VT *__restrict__ Ax, const PTB *__restrict__ Bp,
+                  const int32_t *__restrict__ Bj, const VT *__restrict__ Bx, int64_t ntiles,
+                  const MergeCut *__restrict__ cuts, int32_t *tilec, const int64_t *off, void *Cp,
+                  int cp_bits, int32_t *Cj, VT *Cx) {
+  __shared__ VT sv[WRITE ? kMergeTile + 2 : 1];       // A's values, then B's, one more of B
+  __shared__ int32_t sc[kMergeTile + 2];              // one column of A before, A's, B's, one of B
+  __shared__ uint16_t sea[kMergeRows], seb[kMergeRows];  // row ends in the tile
+  __shared__ uint16_t sdup[kMergeThreads + 1];        // dups before a thread's entries
+  __shared__ uint8_t sbit[kMergeThreads + 1];         // a thread's dups, bit per entry
+  __shared__ int wsum[kMergeThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int64_t ab = int64_t(Ap[0]), bb = int64_t(Bp[0]);
+  const MergeCut c0 = cuts[blockIdx.x], c1 = cuts[blockIdx.x + 1];
+  const int nA = int(c1.i - c0.i), nB = int(c1.j - c0.j), n = nA + nB;
+  const int32_t *__restrict__ aj = Aj + ab + c0.i;
+  const int32_t *__restrict__ bj = Bj + bb + c0.j;
+  const int64_t rl = c1.row < m ? c1.row : m - 1;  // the last row with entries here, or one after
+  const int64_t R = rl - c0.row + 1;
+  const bool small = R <= kMergeRows;
+  int32_t *sa = sc + 1, *sb = sc + 1 + nA;
+  {  // all of a thread's loads in flight
+    const VT *__restrict__ ax = Ax + ab + c0.i, *__restrict__ bx = Bx + bb + c0.j;
+    int32_t lc[kMergePer];
+    VT lv[kMergePer];
+#pragma unroll
+    for (int t = 0; t < kMergePer; ++t) {
+      const int x = tid + t * kMergeThreads;
+      if (x < n) {
+        lc[t] = x < nA ? __ldg(aj + x) : __ldg(bj + (x - nA));
+        if (WRITE) lv[t] = x < nA ? __ldg(ax + x) : __ldg(bx + (x - nA));
       }
-      __syncthreads();  // the cuts are read back through L1-bypassing loads below
-      const int64_t i0 = __ldcg(cuts + 2 * w), j0 = __ldcg(cuts + 2 * w + 1);
-      const int64_t i1 = __ldcg(cuts + 2 * w + 2), j1 = __ldcg(cuts + 2 * w + 3);
-      const int64_t n = merge_row_warp<false, VT>(Aj + a0, nullptr, i0, i1, Bj + b0, nullptr, j0,
-                                                  j1, nullptr, nullptr, 0, lane);
-      if (lane == 0) {
-        mt[w] = n;
-        cnt[w] = n;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        int64_t t = 0;
-        for (int k = 0; k < kMergeWarps; ++k) t += cnt[k];
-        rowc[r] = int32_t(t);
-      }
-    } else {
-      const int64_t i0 = cuts[2 * w], j0 = cuts[2 * w + 1];
-      const int64_t i1 = cuts[2 * w + 2], j1 = cuts[2 * w + 3];
-      int64_t off = cp[r];
-      for (int k = 0; k < w; ++k) off += mt[k];
-      merge_row_warp<true, VT>(Aj + a0, Ax + a0, i0, i1, Bj + b0, Bx + b0, j0, j1, Cj + off,
-                               Cx + off, mt[w], lane);
     }
-    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kMergePer; ++t) {
+      const int x = tid + t * kMergeThreads;
+      if (x < n) {
+        sa[x] = lc[t];
+        if (WRITE) sv[x] = lv[t];
+      }
+    }
+  }
+  if (tid == 0) {
+    // the pair cut by the tile's edge: A's entry before the tile (same row as
+    // its first), B's entry after it (same row as its last)
+    const int64_t a0 = int64_t(Ap[c0.row]) - ab;
+    sc[0] = c0.row < m && c0.i > a0 ? __ldg(aj - 1) : -1;
+    int32_t after = -1;
+    if (c1.row < m && int64_t(Ap[c1.row]) - ab + int64_t(Bp[c1.row]) - bb < c1.i + c1.j &&
+        c1.j < int64_t(Bp[c1.row + 1]) - bb) {
+      after = __ldg(bj + nB);
+      if (WRITE) sv[n] = __ldg(Bx + bb + c0.j + nB);
+    }
+    sb[nB] = after;
+  }
+  // ends of row c0.row + k, clipped to the tile
+  auto end_a = [&](int64_t k) {
+    const int64_t e = int64_t(__ldg(Ap + c0.row + k + 1)) - ab - c0.i;
+    return int(e < nA ? e : nA);
+  };
+  auto end_b = [&](int64_t k) {
+    const int64_t e = int64_t(__ldg(Bp + c0.row + k + 1)) - bb - c0.j;
+    return int(e < nB ? e : nB);
+  };
+  if (small)
+    for (int k = tid; k < int(R); k += kMergeThreads) {
+      sea[k] = uint16_t(end_a(k));
+      seb[k] = uint16_t(end_b(k));
+    }
+  __syncthreads();
+  auto ea = [&](int64_t k) { return small ? int(sea[k]) : end_a(k); };
+  auto eb = [&](int64_t k) { return small ? int(seb[k]) : end_b(k); };
+  const int x0 = tid * kMergePer;
+  int32_t col[kMergePer];
+  VT val[kMergePer];
+  unsigned dups = 0;
+  if (x0 < n) {
+    int64_t lo = 0, hi = R - 1;  // the first row that ends past x0
+    while (lo < hi) {
+      const int64_t mid = (lo + hi) >> 1;
+      if (ea(mid) + eb(mid) > x0) hi = mid; else lo = mid + 1;
+    }
+    int64_t k = lo;
+    int as = k > 0 ? ea(k - 1) : 0, bs = k > 0 ? eb(k - 1) : 0, ae = ea(k), be = eb(k);
+    // the row's merge path at x0
+    const int q = x0 - as - bs, la = ae - as, lb = be - bs;
+    int x = q > lb ? q - lb : 0, y = q < la ? q : la;
+    while (x < y) {
+      const int mid = (x + y) >> 1;
+      if (sa[as + mid] <= sb[bs + q - 1 - mid]) x = mid + 1; else y = mid;
+    }
+    int i = as + x, j = bs + q - x;
+    // columns at the cursors (INT32_MAX past the row's end) and of the A entry
+    // before i (-1 when that is not in this row)
+    int32_t ca = i < ae ? sa[i] : INT32_MAX, cb = j < be ? sb[j] : INT32_MAX;
+    int32_t pa = i > as ? sa[i - 1] : k == 0 && i == 0 ? sc[0] : -1;
+#pragma unroll
+    for (int t = 0; t < kMergePer; ++t) {
+      if (x0 + t < n) {
+        while (i == ae && j == be) {  // the next row with entries
+          ++k;
+          ae = ea(k);
+          be = eb(k);
+          ca = i < ae ? sa[i] : INT32_MAX;
+          cb = j < be ? sb[j] : INT32_MAX;
+          pa = -1;
+        }
+        if (ca <= cb) {  // (an exhausted A row has ca = INT32_MAX > any column)
+          col[t] = ca;
+          if (WRITE) {
+            // B's entry of the pair, possibly the one after the tile
+            const bool pair = cb == ca || (j == nB && i == nA - 1 && sb[nB] == ca);
+            val[t] = sv[i];
+            if (pair) val[t] += sv[nA + j];
+          }
+          pa = ca;
+          ++i;
+          ca = i < ae ? sa[i] : INT32_MAX;
+        } else {
+          col[t] = cb;
+          if (cb == pa) dups |= 1u << t;
+          if (WRITE) val[t] = sv[nA + j];
+          ++j;
+          cb = j < be ? sb[j] : INT32_MAX;
+        }
+      }
+    }
+  }
+  // dups before this thread's entries
+  const int mine = __popc(dups);
+  const int inc = warp_scan_incl(mine);
+  if (lane == 31) wsum[w] = inc;
+  __syncthreads();
+  int before = inc - mine, all = 0;
+#pragma unroll
+  for (int v = 0; v < kMergeThreads / 32; ++v) {
+    const int c = wsum[v];
+    if (v < w) before += c;
+    all += c;
+  }
+  if (!WRITE) {
+    if (tid == 0) tilec[blockIdx.x] = n - all;
+    return;
+  }
+  // the inputs are dead: their space takes the output in order
+  int pos = x0 - before;
+#pragma unroll
+  for (int t = 0; t < kMergePer; ++t) {
+    if (x0 + t < n && !((dups >> t) & 1u)) {
+      sc[pos] = col[t];
+      sv[pos] = val[t];
+      ++pos;
+    }
+  }
+  sdup[tid] = uint16_t(before);
+  sbit[tid] = uint8_t(dups);
+  if (tid == 0) {
+    sdup[kMergeThreads] = uint16_t(all);
+    sbit[kMergeThreads] = 0;
+  }
+  __syncthreads();
+  const int64_t o = off[blockIdx.x];
+#pragma unroll
+  for (int t = 0; t < kMergePer; ++t) {
+    const int x = tid + t * kMergeThreads;
+    if (x < n - all) {
+      Cj[o + x] = sc[x];
+      Cx[o + x] = sv[x];
+    }
+  }
+  // rows that start in this tile (the last tile: up to row m)
+  const int64_t last = blockIdx.x == ntiles - 1 ? m + 1 : c1.first;
+  for (int64_t r = c0.first + tid; r < last; r += kMergeThreads) {
+    const int x = int(int64_t(Ap[r]) - ab - c0.i + int64_t(Bp[r]) - bb - c0.j);
+    const int64_t at = o + x - sdup[x / kMergePer] -
+                       __popc(sbit[x / kMergePer] & ((1u << (x % kMergePer)) - 1u));
+    if (cp_bits == 32) ((int32_t *)Cp)[r] = int32_t(at);
+    else ((int64_t *)Cp)[r] = at;
   }
 }
 
 template <typename PTA, typename PTB, typename VT>
 static int spadd_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
                       const tspg_csr *B, tspg_csr_out *C) {
-  const int64_t m = A->nrows;
-  Scratch sc(ctx, s);
-  int32_t *rowc;
-  int64_t *cp, *partial, *heavy, *meta;
-  const int64_t nb = (m + kScanTile - 1) / kScanTile;
-  Sched *dummy;
-  TSPG_TRY(sc.get(&rowc, m));
-  TSPG_TRY(sc.get(&cp, m + 1));
-  TSPG_TRY(sc.get(&partial, nb + 1));
-  TSPG_TRY(sc.get(&dummy, 1));
-  // heavy[0] = count of listed rows, heavy[1..] = the rows
-  const int64_t max_heavy = (A->nnz + B->nnz) / (kMergeHeavy + 1) + 1;
-  TSPG_TRY(sc.get(&heavy, max_heavy + 1));
-  TSPG_TRY(sc.get(&meta, max_heavy * kHeavyMeta));
-  TSPG_CUDA(ctx, cudaMemsetAsync(heavy, 0, sizeof(int64_t), s));
-  TSPG_CUDA(ctx, cudaMemsetAsync(cp, 0, sizeof(int64_t), s));
-  TSPG_CUDA(ctx, cudaMemsetAsync(dummy, 0, sizeof(Sched), s));
-  const unsigned grid = (unsigned)std::min<int64_t>((m * 32 + 255) / 256, int64_t(ctx->num_sms) * 16);
-  if (m > 0) {
-    k_spadd_count<PTA, PTB><<<grid, 256, 0, s>>>(m, (const PTA *)A->rowptr, A->col,
-                                                 (const PTB *)B->rowptr, B->col, rowc,
-                                                 heavy + 1, heavy);
-    k_spadd_heavy<false, PTA, PTB, VT><<<ctx->num_sms * 2, kMergeThreads, 0, s>>>(
-        heavy + 1, heavy, (const PTA *)A->rowptr, A->col, (const VT *)A->val,
-        (const PTB *)B->rowptr, B->col, (const VT *)B->val, rowc, nullptr, meta, nullptr, nullptr);
-    k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(rowc, m, partial);
-    k_scan_partials<<<1, 1024, 0, s>>>(partial, nb);
-    k_scan_final<<<(unsigned)nb, kScanThreads, 0, s>>>(rowc, m, partial, nb, cp, dummy, nullptr);
-    ctx->launches += 5;
+  const int64_t m = A->nrows, total = A->nnz + B->nnz;
+  if (m == 0 || total == 0) {
+    C->nnz = 0;
+    TSPG_CUDA(ctx, cudaMemsetAsync(C->rowptr, 0, size_t(m + 1) * (C->rowptr_bits / 8), s));
+    return TSPG_OK;
   }
+  const int64_t ntiles = (total + kMergeTile - 1) / kMergeTile;
+  const int64_t nb = (ntiles + kScanTile - 1) / kScanTile;
+  Scratch sc(ctx, s);
+  MergeCut *cuts;
+  int32_t *tilec;
+  int64_t *off, *partial;
+  Sched *rec;
+  TSPG_TRY(sc.get(&cuts, ntiles + 1));
+  TSPG_TRY(sc.get(&tilec, ntiles));
+  TSPG_TRY(sc.get(&off, ntiles + 1));
+  TSPG_TRY(sc.get(&partial, nb + 1));
+  TSPG_TRY(sc.get(&rec, 1));
+  TSPG_CUDA(ctx, cudaMemsetAsync(rec, 0, sizeof(Sched), s));
+  const PTA *Ap = (const PTA *)A->rowptr;
+  const PTB *Bp = (const PTB *)B->rowptr;
+  k_merge_cuts<PTA, PTB><<<unsigned((ntiles + 128) / 128), 128, 0, s>>>(m, Ap, A->col, Bp, B->col,
+                                                                       ntiles, cuts);
+  k_merge_tiles<false, PTA, PTB, VT><<<unsigned(ntiles), kMergeThreads, 0, s>>>(
+      m, Ap, A->col, nullptr, Bp, B->col, nullptr, ntiles, cuts, tilec, nullptr, nullptr, 0, nullptr,
+      nullptr);
+  ctx->launches += 2;
+  launch_scan(ctx, s, tilec, ntiles, partial, off, rec, nullptr);
   TSPG_CUDA(ctx, cudaGetLastError());
   int64_t *h = ctx->h_words;
-  TSPG_CUDA(ctx, cudaMemcpyAsync(h, cp + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  TSPG_CUDA(ctx, cudaMemcpyAsync(h, off + ntiles, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   TSPG_CUDA(ctx, cudaStreamSynchronize(s));
   const int64_t nnz = h[0];
   if (C->rowptr_bits == 32 && nnz > INT32_MAX) return TSPG_EOVERFLOW;
@@ -256,17 +316,10 @@ static int spadd_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
     C->val = cx;
     C->capacity = nnz;
   }
-  if (m == 0) {
-    TSPG_CUDA(ctx, cudaMemsetAsync(C->rowptr, 0, C->rowptr_bits / 8, s));
-    return TSPG_OK;
-  }
-  k_spadd_fill<PTA, PTB, VT><<<grid, 256, 0, s>>>(
-      m, (const PTA *)A->rowptr, A->col, (const VT *)A->val, (const PTB *)B->rowptr,
-      B->col, (const VT *)B->val, cp, C->rowptr, C->rowptr_bits, C->col, (VT *)C->val);
-  k_spadd_heavy<true, PTA, PTB, VT><<<ctx->num_sms * 2, kMergeThreads, 0, s>>>(
-      heavy + 1, heavy, (const PTA *)A->rowptr, A->col, (const VT *)A->val,
-      (const PTB *)B->rowptr, B->col, (const VT *)B->val, nullptr, cp, meta, C->col, (VT *)C->val);
-  ctx->launches += 2;
+  k_merge_tiles<true, PTA, PTB, VT><<<unsigned(ntiles), kMergeThreads, 0, s>>>(
+      m, Ap, A->col, (const VT *)A->val, Bp, B->col, (const VT *)B->val, ntiles, cuts, nullptr, off,
+      C->rowptr, C->rowptr_bits, C->col, (VT *)C->val);
+  ctx->launches += 1;
   TSPG_CUDA(ctx, cudaGetLastError());
   return TSPG_OK;
 }
