@@ -86,3 +86,23 @@ def test_mcl_iteration_and_empty(ctx):
     ops.mcl_inflate(ctx, Z, 2.0)
     ops.mcl_normalize(ctx, Z)
     assert ops.mcl_prune(ctx, Z, 0.5).nnz == 0
+
+
+@pytest.mark.parametrize("lens", [[1, 0, 255, 256, 257, 31], [2047, 2048, 2049, 0, 5000, 3], [0] * 3000 + [2048, 0, 0],
+                                  [9] * 700, [4096]])
+def test_row_and_tile_edges(ctx, lens):
+    # rows in a warp's registers (256), a CTA's (2048) and longer; prune tiles
+    # of 2048 entries with runs of empty rows at their edges
+    rng = np.random.default_rng(len(lens))
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    H = HostCSR(len(lens), 6000, rp, rng.integers(0, 6000, rp[-1]).astype(np.int32), rng.uniform(0.1, 1, rp[-1]))
+    for power in (2.0, 1.5, 1.0):
+        got = ops.mcl_inflate(ctx, H.to_device(), power).val.cpu().numpy()
+        want = oracle.mcl_inflate(H.rowptr, H.val, power)
+        assert np.all(np.abs(got - want) <= 1e-12 * np.abs(want))
+    for tol in (0.0, 0.3, 0.99, 2.0):
+        P = ops.mcl_prune(ctx, H.to_device(), tol).to_host()
+        prp, cj, cx = oracle.mcl_prune(H.rowptr, H.col, H.val, tol)
+        np.testing.assert_array_equal(P.rowptr, prp)
+        np.testing.assert_array_equal(P.col, cj)
+        np.testing.assert_array_equal(P.val, cx)

@@ -3,9 +3,9 @@
 // The reference's MCL driver (src/mcl.cu:56-149) copies its tile to the host
 // for each of prune, normalize and inflation, loops over the rows there and
 // copies the result back.  Here each is one or a few kernels on the caller's
-// stream: normalize and inflation rewrite the values in place (one warp per
-// row: its sum, then the scaled values), prune compacts the kept entries into
-// a new CSR (count pass, device scan, order-preserving fill).  The row sums
+// stream: normalize and inflation rewrite the values in place (a warp or a CTA
+// per row: its sum, then the scaled values), prune compacts the kept entries
+// into a new CSR (count pass, device scan, order-preserving fill).  The row sums
 // are over this tile's rows only: the reference then adds the partial sums of
 // the ranks of a process row (MPI_Allreduce on the row communicator), a step
 // that does not exist on one GPU.
@@ -14,93 +14,182 @@
 namespace tspg {
 
 // Rows scaled to sum 1 (entries of a row whose sum is <= 1e-20 become 0),
-// after raising every value to `power` when do_pow (inflation).
+// after raising every value to `power` when do_pow (inflation).  Rows of up to
+// 256 entries stay in a warp's registers, of up to 2048 in the CTA's: one read
+// and one write of the values.  Longer ones are powered and summed, then read
+// back.  The 8 rows of a CTA lie ngroups apart, so the neighbouring hub rows of
+// a graph go to different CTAs (a warp per row, hub rows of 25k entries: 0.61
+// ms for 46M entries).  power 2 is one multiplication (pow costs ~150
+// instructions an entry).
+template <typename VT>
+__device__ __forceinline__ VT mcl_pow(VT v, VT power, int do_pow) {
+  return do_pow == 2 ? v * v : do_pow ? VT(pow(v, power)) : v;
+}
+
 template <typename PT, typename VT>
-__global__ void k_mcl_rows(const PT *rp, const VT *val, int64_t m, VT power, int do_pow,
-                           VT *out) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t r = warp; r < m; r += nwarps) {
-    const int64_t a0 = int64_t(rp[r]), a1 = int64_t(rp[r + 1]);
-    VT sum = VT(0);
-    for (int64_t p = a0 + lane; p < a1; p += 32) {
-      VT v = val[p];
-      if (do_pow) {
-        v = pow(v, power);
-        out[p] = v;
+__global__ void __launch_bounds__(256)
+    k_mcl_rows(const PT *rp, const VT *val, int64_t m, int64_t ngroups, VT power, int do_pow,
+               VT *out) {
+  constexpr int U = 8;
+  __shared__ VT part[8];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  for (int64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
+    const int64_t r = w * ngroups + g;
+    const int64_t a0 = r < m ? int64_t(rp[r]) : 0, len = r < m ? int64_t(rp[r + 1]) - a0 : 0;
+    if (len > 0 && len <= 32 * U) {
+      VT v[U], sum = VT(0);
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = u * 32 + lane < len ? val[a0 + u * 32 + lane] : VT(0);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u * 32 + lane < len) {
+          v[u] = mcl_pow(v[u], power, do_pow);
+          sum += v[u];
+        }
+      sum = warp_sum(sum);
+      const bool keep = sum > VT(1e-20);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u * 32 + lane < len) out[a0 + u * 32 + lane] = keep ? v[u] / sum : VT(0);
+    }
+    // the longer ones of the 8 rows, a CTA each (uniform over the CTA)
+    if (!__syncthreads_or(len > 32 * U)) continue;
+    for (int q = 0; q < 8; ++q) {
+      const int64_t row = q * ngroups + g;
+      if (row >= m) break;
+      const int64_t b0 = int64_t(rp[row]), n = int64_t(rp[row + 1]) - b0;
+      if (n <= 32 * U) continue;
+      const bool held = n <= 256 * U;
+      VT v[U], sum = VT(0);
+      for (int64_t c = 0; c < n; c += 256 * U) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = c + u * 256 + tid < n ? val[b0 + c + u * 256 + tid] : VT(0);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (c + u * 256 + tid < n) {
+            v[u] = mcl_pow(v[u], power, do_pow);
+            sum += v[u];
+            if (!held && do_pow) out[b0 + c + u * 256 + tid] = v[u];
+          }
       }
-      sum += v;
-    }
-    sum = warp_sum(sum);
-    __syncwarp();  // the powered values written above are read back below
-    const bool keep = sum > VT(1e-20);
-    for (int64_t p = a0 + lane; p < a1; p += 32) {
-      const VT v = do_pow ? out[p] : val[p];
-      out[p] = keep ? v / sum : VT(0);
-    }
-  }
-}
-
-// Prune, pass 1: entries per row with |v| > tol.
-template <typename PT, typename VT>
-__global__ void k_prune_count(const PT *rp, const VT *val, int64_t m, VT tol, int32_t *cnt) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t r = warp; r < m; r += nwarps) {
-    const int64_t a0 = int64_t(rp[r]), a1 = int64_t(rp[r + 1]);
-    int c = 0;
-    for (int64_t p0 = a0; p0 < a1; p0 += 32) {
-      const int64_t p = p0 + lane;
-      c += __popc(__ballot_sync(0xffffffffu, p < a1 && fabs(val[p]) > tol));
-    }
-    if (lane == 0) cnt[r] = c;
-  }
-}
-
-// Prune, pass 2: the kept entries of every row, in their order, at the row's
-// new offset.
-template <typename PT, typename VT>
-__global__ void k_prune_fill(const PT *rp, const int32_t *col, const VT *val, int64_t m, VT tol,
-                             const int64_t *np, int32_t *ocol, VT *oval) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t r = warp; r < m; r += nwarps) {
-    const int64_t a0 = int64_t(rp[r]), a1 = int64_t(rp[r + 1]);
-    int64_t o = np[r];
-    for (int64_t p0 = a0; p0 < a1; p0 += 32) {
-      const int64_t p = p0 + lane;
-      const VT v = p < a1 ? val[p] : VT(0);
-      const bool k = p < a1 && fabs(v) > tol;
-      const unsigned b = __ballot_sync(0xffffffffu, k);
-      if (k) {
-        const int64_t q = o + __popc(b & ((1u << lane) - 1u));
-        ocol[q] = col[p];
-        oval[q] = v;
+      sum = warp_sum(sum);
+      if (lane == 0) part[w] = sum;
+      __syncthreads();
+      sum = VT(0);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum += part[k];
+      const bool keep = sum > VT(1e-20);
+      const VT *src = do_pow ? out : val;  // the thread's own writes, if powered
+      for (int64_t c = 0; c < n; c += 256 * U) {
+        if (!held) {
+#pragma unroll
+          for (int u = 0; u < U; ++u) v[u] = c + u * 256 + tid < n ? src[b0 + c + u * 256 + tid] : VT(0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (c + u * 256 + tid < n) out[b0 + c + u * 256 + tid] = keep ? v[u] / sum : VT(0);
       }
-      o += __popc(b);
+      __syncthreads();  // part is free again
     }
   }
 }
 
-__global__ void k_offsets32(const int64_t *src, int64_t n, int32_t *dst) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = int32_t(src[i]);
-}
-
-static unsigned warp_grid(tspg_ctx *ctx, int64_t rows) {
-  return (unsigned)std::max<int64_t>(1, std::min<int64_t>((rows * 32 + 255) / 256,
-                                                          int64_t(ctx->num_sms) * 16));
+// Prune: the entries with |v| > tol, in their order.  Tiles of kPruneTile
+// entries whatever the rows' lengths (a warp per row took 0.23 + 0.38 ms for
+// 46M entries in rows of up to 25k); warp w of a tile owns 256 consecutive
+// ones.  FILL = false leaves the tile's number of kept entries in tilec;
+// FILL = true writes them from off[tile] on, and the offsets of the rows that
+// start in the tile.
+constexpr int kPruneTile = 2048;
+template <bool FILL, typename PT, typename VT>
+__global__ void __launch_bounds__(256)
+    k_prune_tiles(const PT *__restrict__ rp, const int32_t *__restrict__ col,
+                  const VT *__restrict__ val, int64_t m, int64_t nnz, VT tol, int64_t ntiles,
+                  int32_t *tilec, const int64_t *off, void *np, int np_bits, int32_t *ocol,
+                  VT *oval) {
+  constexpr int U = 8;
+  __shared__ unsigned mask[64 + 1];
+  __shared__ int before[64 + 1];
+  __shared__ int64_t row0[2];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int64_t base = int64_t(rp[0]);
+  const int64_t span = int64_t(rp[m]) - base, total = span < nnz ? span : nnz;
+  const int64_t t = blockIdx.x, d0 = t * kPruneTile < total ? t * kPruneTile : total;
+  const int64_t d1 = d0 + kPruneTile < total ? d0 + kPruneTile : total;
+  VT v[U];
+  int32_t c[U];
+  unsigned b[U];
+  int kept = 0;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int64_t e = d0 + w * 256 + u * 32 + lane;
+    v[u] = e < d1 ? __ldg(val + base + e) : VT(0);
+    if (FILL) c[u] = e < d1 ? __ldg(col + base + e) : 0;
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int64_t e = d0 + w * 256 + u * 32 + lane;
+    b[u] = __ballot_sync(0xffffffffu, e < d1 && fabs(v[u]) > tol);
+    if (lane == 0) mask[w * U + u] = b[u];
+    kept += __popc(b[u]);
+  }
+  if (FILL && w < 2) {
+    // the first row that starts at or after d0 (w = 0), and the one that ends
+    // this tile's rows (the last tile: one past row m)
+    const int64_t d = w == 0 ? d0 : d1;
+    int64_t lo = 0, hi = m + 1;  // rows below lo start before d, row hi does not
+    while (hi > lo) {
+      const int64_t step = (hi - lo + 31) / 32, i = lo + lane * step;
+      const unsigned s = __ballot_sync(0xffffffffu, i < hi && int64_t(__ldg(rp + i)) - base < d);
+      const int n = __popc(s);
+      if (n == 0) break;
+      const int64_t at = lo + int64_t(n - 1) * step;
+      lo = at + 1;
+      hi = at + step < hi ? at + step : hi;
+    }
+    if (lane == 0) row0[w] = w == 1 && t == ntiles - 1 ? m + 1 : lo;
+  }
+  __syncthreads();
+  if (w == 0) {  // entries kept before each window of 32
+    const int a = __popc(mask[2 * lane]), z = __popc(mask[2 * lane + 1]);
+    const int inc = warp_scan_incl(a + z);
+    before[2 * lane] = inc - a - z;
+    before[2 * lane + 1] = inc - z;
+    if (lane == 31) {
+      before[64] = inc;
+      mask[64] = 0;
+    }
+  }
+  __syncthreads();
+  if (!FILL) {
+    if (tid == 0) tilec[t] = before[64];
+    return;
+  }
+  const int64_t o = off[t];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if ((b[u] >> lane) & 1u) {
+      const int64_t q = o + before[w * U + u] + __popc(b[u] & ((1u << lane) - 1u));
+      ocol[q] = c[u];
+      oval[q] = v[u];
+    }
+  }
+  for (int64_t r = row0[0] + tid; r < row0[1]; r += 256) {
+    const int x = int(int64_t(__ldg(rp + r)) - base - d0);
+    const int64_t q = o + before[x >> 5] + __popc(mask[x >> 5] & ((1u << (x & 31)) - 1u));
+    if (np_bits == 32) ((int32_t *)np)[r] = int32_t(q);
+    else ((int64_t *)np)[r] = q;
+  }
 }
 
 template <typename PT, typename VT>
 static int mcl_rows_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, double power,
                          int do_pow, void *val_out) {
   if (M->nrows > 0 && M->nnz > 0) {
-    k_mcl_rows<PT, VT><<<warp_grid(ctx, M->nrows), 256, 0, s>>>(
-        (const PT *)M->rowptr, (const VT *)M->val, M->nrows, VT(power), do_pow, (VT *)val_out);
+    const int64_t ngroups = (M->nrows + 7) / 8;
+    k_mcl_rows<PT, VT><<<unsigned(std::min<int64_t>(ngroups, int64_t(ctx->num_sms) * 8)), 256, 0, s>>>(
+        (const PT *)M->rowptr, (const VT *)M->val, M->nrows, ngroups, VT(power),
+        do_pow && power == 2.0 ? 2 : do_pow, (VT *)val_out);
     ctx->launches += 1;
   }
   TSPG_CUDA(ctx, cudaGetLastError());
@@ -110,26 +199,29 @@ static int mcl_rows_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, doubl
 template <typename PT, typename VT>
 static int prune_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, double tol,
                       tspg_csr_out *out) {
-  const int64_t m = M->nrows, nb = (m + kScanTile - 1) / kScanTile;
-  Scratch sc(ctx, s);
-  int32_t *cnt;
-  int64_t *np, *partial;
-  Sched *dummy;
-  TSPG_TRY(sc.get(&cnt, m));
-  TSPG_TRY(sc.get(&np, m + 1));
-  TSPG_TRY(sc.get(&partial, nb + 1));
-  TSPG_TRY(sc.get(&dummy, 1));
-  TSPG_CUDA(ctx, cudaMemsetAsync(np, 0, sizeof(int64_t) * (m + 1), s));
-  const unsigned g = warp_grid(ctx, m);
-  if (m > 0) {
-    k_prune_count<PT, VT><<<g, 256, 0, s>>>((const PT *)M->rowptr, (const VT *)M->val, m, VT(tol), cnt);
-    k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(cnt, m, partial);
-    k_scan_partials<<<1, 1024, 0, s>>>(partial, nb);
-    k_scan_final<<<(unsigned)nb, kScanThreads, 0, s>>>(cnt, m, partial, nb, np, dummy, nullptr);
-    ctx->launches += 4;
+  const int64_t m = M->nrows;
+  if (m == 0 || M->nnz == 0) {
+    out->nnz = 0;
+    TSPG_CUDA(ctx, cudaMemsetAsync(out->rowptr, 0, size_t(m + 1) * (out->rowptr_bits / 8), s));
+    return TSPG_OK;
   }
+  const int64_t ntiles = (M->nnz + kPruneTile - 1) / kPruneTile;
+  Scratch sc(ctx, s);
+  int32_t *tilec;
+  int64_t *off, *partial;
+  Sched *rec;
+  TSPG_TRY(sc.get(&tilec, ntiles));
+  TSPG_TRY(sc.get(&off, ntiles + 1));
+  TSPG_TRY(sc.get(&partial, (ntiles + kScanTile - 1) / kScanTile + 1));
+  TSPG_TRY(sc.get(&rec, 1));
+  TSPG_CUDA(ctx, cudaMemsetAsync(rec, 0, sizeof(Sched), s));
+  k_prune_tiles<false, PT, VT><<<unsigned(ntiles), 256, 0, s>>>(
+      (const PT *)M->rowptr, nullptr, (const VT *)M->val, m, M->nnz, VT(tol), ntiles, tilec, nullptr,
+      nullptr, 0, nullptr, nullptr);
+  ctx->launches += 1;
+  launch_scan(ctx, s, tilec, ntiles, partial, off, rec, nullptr);
   int64_t *h = ctx->h_words;
-  TSPG_CUDA(ctx, cudaMemcpyAsync(h, np + m, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  TSPG_CUDA(ctx, cudaMemcpyAsync(h, off + ntiles, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
   TSPG_CUDA(ctx, cudaStreamSynchronize(s));
   const int64_t nnz = h[0];
   out->nnz = nnz;
@@ -143,17 +235,10 @@ static int prune_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, double t
     out->val = cx;
     out->capacity = nnz;
   }
-  if (m > 0 && nnz > 0) {
-    k_prune_fill<PT, VT><<<g, 256, 0, s>>>((const PT *)M->rowptr, M->col, (const VT *)M->val, m,
-                                           VT(tol), np, out->col, (VT *)out->val);
-    ctx->launches += 1;
-  }
-  if (out->rowptr_bits == 64) {
-    TSPG_CUDA(ctx, cudaMemcpyAsync(out->rowptr, np, sizeof(int64_t) * (m + 1), cudaMemcpyDeviceToDevice, s));
-  } else {
-    k_offsets32<<<(unsigned)((m + 1 + 255) / 256), 256, 0, s>>>(np, m + 1, (int32_t *)out->rowptr);
-    ctx->launches += 1;
-  }
+  k_prune_tiles<true, PT, VT><<<unsigned(ntiles), 256, 0, s>>>(
+      (const PT *)M->rowptr, M->col, (const VT *)M->val, m, M->nnz, VT(tol), ntiles, nullptr, off,
+      out->rowptr, out->rowptr_bits, out->col, (VT *)out->val);
+  ctx->launches += 1;
   TSPG_CUDA(ctx, cudaGetLastError());
   return TSPG_OK;
 }
