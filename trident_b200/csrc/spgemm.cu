@@ -195,7 +195,7 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
   phase_mark(ctx, 0, 0, s);
   TSPG_TRY((launch_symbolic_rows<PT, VT>(ctx, s, prods, pa, n)));
   if (onepass) {
-    k_onepass<PT, VT><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
+    k_onepass<PT, VT><<<ctx->num_sms, kOnepassThreads, kOnepassSmem, s>>>(prods, pa);
     // the rows sent back (too many columns for their 64-slot attempt and
     // too large for a warp's full table): their symbolic count, as
     // 256-thread rows of their own record

@@ -1670,10 +1670,9 @@ __device__ __forceinline__ bool esc_fits(const RowMeta &m, int64_t fmax) {
 
 // Group-level rows of class `cls`: the group leader fetches one row index at a
 // time; the group exits when the class runs out.
-template <int G, bool NUM, typename PT, typename VT, bool ONEPASS = false>
+template <int G, bool NUM, typename PT, typename VT>
 __device__ void group_rows(const ProdDev<PT, VT> *prods, const PhaseArgs &A,
                            int cls, unsigned char *smem, PhaseShared &sh) {
-  static_assert(!ONEPASS || (G == 32 && NUM), "one-pass rows are warp rows");
   constexpr int NG = kGroupThreads / G;  // groups of this size per CTA
   // slices start on 16-byte boundaries (the tables are cleared with 16-byte stores)
   constexpr int SLICE = (NUM ? kTableSmem / NG : (kTableSmem * 2 / 3) / NG) & ~15;
@@ -1725,9 +1724,7 @@ __device__ void group_rows(const ProdDev<PT, VT> *prods, const PhaseArgs &A,
       for (int t = 0; i < e; ++i, ++t) {
         const long long t0 = clock64();
         const RowMeta m = shfl_meta(mine, t);
-        if constexpr (ONEPASS) {
-          num_hash_row<G, TMAXN, PT, VT, true>(prods, A, m, slice, gm, gid, lane);
-        } else if constexpr (NUM) {
+        if constexpr (NUM) {
           if (esc_fits(m, TMAXN / 2))
             num_esc_row<G, TMAXN, PT, VT>(prods, A, m, slice, gm, gid, lane);
           else
@@ -1867,23 +1864,199 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
   if (!(A.skip >> CLS_G32 & 1u)) group_rows<32, NUM, PT, VT>(prods, A, CLS_G32, smem, sh);
 }
 
-// One-pass warp rows of a plain product (the symbolic record's CLS_ONEPASS
-// list), after k_groups in the symbolic launch: each row is multiplied in
-// full (the numeric warp-row form, its table sized by the output bound) into
-// the scratch.  A warp row's symbolic pass (hash count) is then not needed:
-// Galerkin A·P (27-point 128^3, ~119 products and ~12 outputs per row)
-// paid 1.8 ms of symbolic and 3.5 ms of numeric launches for it.
+// One-pass rows of a plain product (the symbolic record's CLS_ONEPASS list),
+// after k_groups in the symbolic launch: each row is multiplied in full into
+// the scratch, so no symbolic pass counts it (Galerkin A·P paid 1.8 ms of
+// symbolic and 3.5 ms of numeric launches for it).
+constexpr int kOnepassThreads = 512;
+constexpr int kLaneSlots = kCappedCols;            // columns a lane's row may hold
+constexpr int kLaneLog = 5;
+static_assert(kLaneSlots == 1 << kLaneLog, "hash table per lane");
+constexpr int kOnepassSlice = kLaneSlots * 32 * 12;  // per warp: 32 x 32 columns and values
+constexpr int kOnepassSmem = (kOnepassThreads / 32) * kOnepassSlice;
+static_assert(kNumT32 * 12 <= kOnepassSlice, "the warp form's table");
+
+// 32 rows by one warp, a lane each: lane l walks row l's A entries in step
+// with the others (the next entry's B row bounds and the one after's column
+// in flight) and adds every product into its own kLaneSlots-slot hash table in
+// shared memory, [slot][lane]: no atomics, no bank conflicts.  The occupied
+// slots are sorted by insertion as they are gathered, and written to the
+// scratch.  A row with more than kLaneSlots columns goes back to the two-pass
+// path.  (A list searched from the last hit on instead of the table: 105-148
+// instructions a product, Galerkin A·P 3.0 ms.)
+//
+// Rows this short spend a warp's time on what surrounds the products (a warp
+// per row: ~1040 warp instructions for the 119 products of a Galerkin A·P
+// row); lanes of neighbouring rows also read neighbouring B rows, so their
+// loads coalesce.
 template <typename PT, typename VT>
-__global__ void __launch_bounds__(kGroupThreads, 1)
+__device__ void onepass_lanes(const ProdDev<PT, VT> &P, const PhaseArgs &A, const RowMeta &m,
+                              bool have, unsigned char *slice, int lane) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int U = 4;
+  int *keys = (int *)slice + lane;
+  VT *vals = (VT *)(slice + kLaneSlots * 32 * 4) + lane;
+  const int32_t *__restrict__ Aj = P.Aj;
+  const VT *__restrict__ Ax = P.Ax;
+  const PT *__restrict__ Bp = P.Bp;
+  const int32_t *__restrict__ Bj = P.Bj;
+  const VT *__restrict__ Bx = P.Bx;
+  const int64_t a0 = m.a0;
+  const int na = have ? int(m.a1 - a0) : 0;  // a one-pass row has < 2^31 products
+  const int steps = __reduce_max_sync(FULL, na);
+  int n = 0;
+  bool refused = false;
+#pragma unroll
+  for (int i = 0; i < kLaneSlots; ++i) keys[i * 32] = -1;
+  // entry t: value and B row; entry t + 1: column and value
+  VT av = VT(0), an = VT(0);
+  int64_t b0 = 0, b1 = 0;
+  int32_t kn = 0;
+  if (na > 0) {
+    const int64_t k = __ldg(Aj + a0);
+    av = __ldg(Ax + a0);
+    b0 = int64_t(__ldg(Bp + k));
+    b1 = int64_t(__ldg(Bp + k + 1));
+  }
+  if (na > 1) {
+    kn = __ldg(Aj + a0 + 1);
+    an = __ldg(Ax + a0 + 1);
+  }
+  for (int t = 0; t < steps; ++t) {
+    int64_t n0 = 0, n1 = 0;
+    if (t + 1 < na) {
+      n0 = int64_t(__ldg(Bp + kn));
+      n1 = int64_t(__ldg(Bp + int64_t(kn) + 1));
+    }
+    int32_t k2 = 0;
+    VT a2 = VT(0);
+    if (t + 2 < na) {
+      k2 = __ldg(Aj + a0 + t + 2);
+      a2 = __ldg(Ax + a0 + t + 2);
+    }
+    for (int64_t q = b0; __any_sync(FULL, q < b1); q += U) {
+      int32_t c[U];
+      VT x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        c[u] = q + u < b1 ? __ldg(Bj + q + u) : -1;
+        x[u] = q + u < b1 ? __ldg(Bx + q + u) : VT(0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (c[u] >= 0) {
+          const VT v = av * x[u];
+          uint32_t h = hash_slot(c[u], kLaneLog);
+          int k = keys[h * 32];
+          for (int it = 1; k != c[u] && k != -1 && it < kLaneSlots; ++it) {
+            h = (h + 1) & (kLaneSlots - 1);
+            k = keys[h * 32];
+          }
+          if (k == c[u]) {
+            vals[h * 32] += v;
+          } else if (k == -1) {
+            keys[h * 32] = c[u];
+            vals[h * 32] = v;
+            ++n;
+          } else {
+            refused = true;
+          }
+        }
+      }
+    }
+    av = an;
+    b0 = n0;
+    b1 = n1;
+    kn = k2;
+    an = a2;
+  }
+  // slot i's entry moves down into the sorted entries [0, n) gathered so far
+  n = 0;
+  for (int i = 0; i < kLaneSlots; ++i) {
+    const int k = keys[i * 32];
+    if (k != -1) {
+      const VT v = vals[i * 32];
+      int j = n++;
+      for (; j > 0; --j) {
+        const int kp = keys[(j - 1) * 32];
+        if (kp < k) break;
+        keys[j * 32] = kp;
+        vals[j * 32] = vals[(j - 1) * 32];
+      }
+      keys[j * 32] = k;
+      vals[j * 32] = v;
+    }
+  }
+  __syncwarp();
+  if (have && !refused) {
+    int32_t *const oj = A.oj + m.off;
+    VT *const ox = (VT *)A.ox + m.off;
+    for (int i = 0; i < n; ++i) {
+      oj[i] = keys[i * 32];
+      ox[i] = vals[i * 32];
+    }
+    A.rowc[m.g] = n;
+    A.rowf[m.g] = -1 - m.off;
+  }
+  const unsigned back = __ballot_sync(FULL, have && refused);
+  if (back) {
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(&A.S->ndefer, (unsigned long long)__popc(back));
+    at = __shfl_sync(FULL, at, 0);
+    if (have && refused)
+      A.defer[at + __popc(back & ((1u << lane) - 1u))] = (uint64_t(m.p) << 40) | uint64_t(m.r);
+  }
+  __syncwarp();
+}
+
+template <typename PT, typename VT>
+__global__ void __launch_bounds__(kOnepassThreads, 1)
     k_onepass(const ProdDev<PT, VT> *prods, PhaseArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ PhaseShared sh;
-  if (threadIdx.x < NCLS) {
-    sh.off[threadIdx.x] = A.S->off[threadIdx.x];
-    sh.cnt[threadIdx.x] = A.S->cnt[threadIdx.x];
+  __shared__ int lst[kOnepassThreads];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t count = A.S->cnt[CLS_ONEPASS], base = A.S->off[CLS_ONEPASS];
+  const int64_t warps = int64_t(gridDim.x) * (kOnepassThreads / 32);
+  unsigned char *slice = smem + w * kOnepassSlice;
+  GroupMem gm{};
+  gm.lst = lst + w * 32;
+  while (true) {
+    unsigned long long v = 0;
+    if (lane == 0) {
+      // 32 rows at a time; near the end as many as spread over the warps
+      const unsigned long long cur = *(volatile unsigned long long *)&A.S->next[CLS_ONEPASS];
+      const int64_t left = count - int64_t(cur);
+      const int64_t even = (left + warps - 1) / warps;
+      const unsigned long long take = even >= 32 ? 32 : even > 1 ? even : 1;
+      v = atomicAdd(&A.S->next[CLS_ONEPASS], take) | (take << 48);
+    }
+    v = __shfl_sync(0xffffffffu, v, 0);
+    const int64_t i = int64_t(v & ((1ull << 48) - 1));
+    if (i >= count) break;
+    const int rows = int(min(count - i, int64_t(v >> 48)));
+    const bool have = lane < rows;
+    const long long t0 = clock64();
+    RowMeta mine{};
+    if (have) {
+      mine = load_meta<false>(prods, A, base + i + lane);
+      mine.off = A.cp[mine.g];  // the row's scratch offset
+    }
+    // lanes in step take as long as the longest row (~40 instructions a
+    // product); a warp per row ~350 and 6 a product
+    const int f = int(mine.f);
+    const int fmax = __reduce_max_sync(0xffffffffu, f);
+    const int fsum = __reduce_add_sync(0xffffffffu, f);
+    if (40 * int64_t(fmax) <= 350 * int64_t(rows) + 6 * int64_t(fsum)) {
+      onepass_lanes<PT, VT>(prods[0], A, mine, have, slice, lane);
+    } else {
+      for (int t = 0; t < rows; ++t)
+        num_hash_row<32, kNumT32, PT, VT, true>(prods, A, shfl_meta(mine, t), slice, gm, w, lane);
+    }
+    if (A.prof && lane == 0) {
+      atomicAdd(A.prof + CLS_ONEPASS, (unsigned long long)(clock64() - t0));
+      atomicAdd(A.prof + NCLS + CLS_ONEPASS, (unsigned long long)rows);
+    }
   }
-  __syncthreads();
-  group_rows<32, true, PT, VT, true>(prods, A, CLS_ONEPASS, smem, sh);
 }
 
 // Numeric launch: the one-pass rows (rowf < 0) go from the scratch into C.  A

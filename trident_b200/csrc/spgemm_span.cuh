@@ -661,7 +661,7 @@ inline int set_smem_attr(int device) {
   };
   if (!raise(k_phase<PT, VT, false>, kDynSmem) || !raise(k_phase<PT, VT, true>, kDynSmem) ||
       !raise(k_groups<PT, VT, false>, kGroupDynSmem) ||
-      !raise(k_groups<PT, VT, true>, kGroupDynSmem) || !raise(k_onepass<PT, VT>, kGroupDynSmem) ||
+      !raise(k_groups<PT, VT, true>, kGroupDynSmem) || !raise(k_onepass<PT, VT>, kOnepassSmem) ||
       !raise(k_dense_rank<kRankThreads, 1, PT, VT>, kDynSmem) || !raise(k_dense_rank<512, 2, PT, VT>, kRank2Smem) ||
       !raise(k_span<128, false, PT, VT>, kSpanSmemMax) || !raise(k_span<256, false, PT, VT>, kSpanSmemMax) || !raise(k_span<512, false, PT, VT>, kSpanSmemMax) || !raise(k_span<128, true, PT, VT>, kSpanSmemMax) ||
       !raise(k_span<256, true, PT, VT>, kSpanSmemMax) ||
