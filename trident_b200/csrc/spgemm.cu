@@ -32,6 +32,7 @@ struct tspg_plan {
   int64_t mults = 0;
   int64_t max_a_row = 0;
   int64_t ncnt[NCLS] = {};  // numeric rows per class
+  bool strict_checked = false;  // ProdDev::b_strict is known
   void *prods = nullptr;
   int64_t *base = nullptr;
   int64_t *rowf = nullptr;
@@ -93,6 +94,9 @@ constexpr int kFlagOnePass = 1 << 30;
 constexpr int64_t kOnePassMinRows = 1 << 16;
 static_assert(kOnePassMinRows >= kFuseRows, "the one-pass branch sets the list offsets itself");
 constexpr int64_t kOnePassMaxEntries = int64_t(1) << 30;
+
+// Warp-class rows from which the check of B's rows for strict order pays.
+constexpr int64_t kStrictRows = 4096;
 
 static inline unsigned grid_for(int64_t work, int per_block, int cap) {
   int64_t g = (work + per_block - 1) / per_block;
@@ -228,10 +232,20 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
 }
 
 template <typename PT, typename VT>
-static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P,
+static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P, const tspg_csr *B,
                         tspg_csr_out *C) {
   const int64_t m = P->m;
   ProdDev<PT, VT> *prods = (ProdDev<PT, VT> *)P->prods;
+  // warp rows over long B rows add without atomics when no B row holds a
+  // column twice: worth a pass over B's columns where they are many (the
+  // answer belongs to the pattern, which a plan keeps)
+  if (!P->strict_checked && !P->onepass && P->ncnt[CLS_G32] >= kStrictRows &&
+      B->nnz >= kSeqRow * B->nrows && P->mults >= 8 * B->nnz) {
+    k_check_strict<PT, VT><<<grid_for(B->nnz, 1024, ctx->num_sms * 8), 256, 0, s>>>(
+        (const PT *)B->rowptr, B->col, B->nrows, P->sched + 2, prods);
+    ctx->launches += 1;
+    P->strict_checked = true;
+  }
   if (m == 0) {
     k_set_out<PT, VT><<<1, 1, 0, s>>>(prods, C->col, (VT *)C->val, C->rowptr,
                                       C->rowptr_bits);
@@ -422,7 +436,7 @@ extern "C" int tspg_spgemm_numeric(tspg_ctx *ctx, void *stream,
     ProdDev<PT, VT> *prods = (ProdDev<PT, VT> *)plan->prods;
     k_set_operands<PT, VT><<<1, 1, 0, s>>>(prods, v);
     ctx->launches += 1;
-    return numeric_impl<PT, VT>(ctx, s, plan, C);
+    return numeric_impl<PT, VT>(ctx, s, plan, B, C);
   });
 }
 
@@ -442,7 +456,10 @@ extern "C" int tspg_spgemm(tspg_ctx *ctx, void *stream, const tspg_csr *A,
     st = dispatch(plan->pt_bits, plan->vt_bits, [&](auto pt, auto vt) {
       using PT = std::remove_pointer_t<decltype(pt)>;
       using VT = std::remove_pointer_t<decltype(vt)>;
-      return numeric_impl<PT, VT>(ctx, (cudaStream_t)stream, plan, C);
+      // B with the offsets the symbolic phase used (widened when mixed)
+      tspg_csr b = *B;
+      if (plan->wide_b) b.rowptr = plan->wide_b;
+      return numeric_impl<PT, VT>(ctx, (cudaStream_t)stream, plan, &b, C);
     });
   }
   tspg_plan_destroy(plan);

@@ -145,6 +145,7 @@ struct ProdDev {
   void *Cp;       // output rowptr (product-local), cp_bits wide
   int32_t cp_bits;
   int32_t b_sorted;
+  int32_t b_strict;  // B's rows were found strictly increasing (k_check_strict)
   // optional addend of C = E + A·B (tspg_spgemm_acc): E's row r joins row r's
   // products as entries with coefficient 1; Ej == nullptr when there is none
   const void *Ep;
@@ -295,13 +296,14 @@ static __global__ void k_widen(const int32_t *src, int64_t n, int64_t *dst) {
 // symbolic pass is kept.
 template <typename PT, typename VT>
 __global__ void k_set_operands(ProdDev<PT, VT> *dst, ProdDev<PT, VT> v) {
-  const int32_t sorted = dst->b_sorted;
+  const int32_t sorted = dst->b_sorted, strict = dst->b_strict;
   const void *ep = dst->Ep;  // the addend stays the symbolic call's
   const int32_t *ej = dst->Ej;
   const VT *ex = dst->Ex;
   const int32_t eb = dst->ep_bits;
   *dst = v;
   dst->b_sorted = sorted;
+  dst->b_strict = strict;
   dst->Ep = ep;
   dst->Ej = ej;
   dst->Ex = ex;
@@ -332,6 +334,34 @@ __global__ void k_check_sorted_rows(const PT *Bp, const int32_t *Bj,
       if (Bj[q] >= Bj[q + 1]) bad = true;
   }
   if (__any_sync(0xffffffffu, bad) && lane == 0) *flag = 0;
+}
+
+// Are all of B's rows strictly increasing?  One streaming pass: the places
+// where a column is not above the one before it, less those between two rows,
+// are none.  rec: a zeroed record (its total and ticket are used).
+template <typename PT, typename VT>
+__global__ void __launch_bounds__(256)
+    k_check_strict(const PT *__restrict__ Bp, const int32_t *__restrict__ Bj, int64_t nb, Sched *rec,
+                   ProdDev<PT, VT> *prod) {
+  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t first = int64_t(Bp[0]), end = int64_t(Bp[nb]);
+  int64_t n = 0;
+  for (int64_t q = first + t; q + 1 < end; q += stride * 4) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t p = q + u * stride;
+      if (p + 1 < end) n += __ldg(Bj + p) >= __ldg(Bj + p + 1);
+    }
+  }
+  for (int64_t r = t; r < nb; r += stride) {
+    const int64_t b0 = int64_t(__ldg(Bp + r)), b1 = int64_t(__ldg(Bp + r + 1));
+    if (b1 > b0 && b1 < end) n -= __ldg(Bj + b1 - 1) >= __ldg(Bj + b1);
+  }
+  n = warp_sum(n);
+  if ((threadIdx.x & 31) == 0 && n != 0) atomicAdd((unsigned long long *)&rec->total, (unsigned long long)n);
+  if (last_block(&rec->ticket) && threadIdx.x == 0)
+    prod->b_strict = *(volatile int64_t *)&rec->total == 0;
 }
 
 // ---------------------------------------------------------------------------

@@ -110,51 +110,95 @@ __device__ __forceinline__ void for_products_balanced(
   }
 }
 
+// Position of the i-th set bit of m (i < popc(m)).
+__device__ __forceinline__ int nth_bit(unsigned m, int i) {
+  int at = 0;
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) {
+    const int c = __popc((m >> at) & ((1u << w) - 1u));
+    if (i >= c) {
+      i -= c;
+      at += w;
+    }
+  }
+  return at;
+}
+
 // One chunk of at most 32 A entries of a warp row: lane j holds entry j's
-// value a and B row bounds [b0, b0 + len) (len = 0 past the chunk's nc
-// entries); fn(col, a*b) for every product.  A warp scan numbers the chunk's
-// products and lanes take products lane, lane + 32, ... (U per step, loads in
-// flight), each finding its entry by a 5-step shuffle search.  (Lane j
-// walking entry j's B row itself, with no search, measured slower on the
-// Galerkin A·P rows, 27 entries x ~4.5: symbolic 2.35 vs 1.81 ms, numeric
-// 5.35 vs 3.72 ms — each load touches 32 B rows instead of a few, and lanes
-// whose B rows list the same columns hit them in the same step.)
+// value a and B row bounds [b0, b0 + len) (len = 0 past the chunk's entries);
+// fn(p, col, a*b) for every product, p its number in the chunk; returns their
+// number.  A warp scan numbers the products and lanes take products lane,
+// lane + 32, ... (U per step, loads in flight).  Entries without products are
+// squeezed out, so inside a window of 32 products every entry start is a bit of
+// its own in a warp-uniform mask and a lane's entry is a popcount away.  (A
+// 5-step shuffle search per product, 64-bit with int64 offsets, took two to
+// three times the instructions; lane j walking entry j's B row itself, with no
+// search, measured slower on the Galerkin A·P rows, 27 entries x ~4.5:
+// symbolic 2.35 vs 1.81 ms, numeric 5.35 vs 3.72 ms — each load touches 32 B
+// rows instead of a few.)
 template <bool NUM, typename IX, typename VT, typename F>
-__device__ __forceinline__ void warp_chunk(const int32_t *__restrict__ Bj,
-                                           const VT *__restrict__ Bx, IX b0, IX len, VT a,
-                                           int nc, int lane, F &&fn) {
+__device__ __forceinline__ uint32_t warp_chunk(const int32_t *__restrict__ Bj,
+                                               const VT *__restrict__ Bx, IX b0, IX len, VT a,
+                                               int lane, F &&fn) {
   constexpr int U = 4;
-  const IX inc = warp_scan_incl(len);
-  const IX tot = __shfl_sync(0xffffffffu, inc, 31);
-  const IX pre = inc - len;
-  // the step loop is uniform across the warp (the search shuffles)
-  for (IX pb = 0; pb < tot; pb += IX(32) * U) {
+  constexpr unsigned FULL = 0xffffffffu;
+  if (__any_sync(FULL, len > (IX(1) << 26))) {  // product numbers past 32 bits
+    uint32_t tot = 0;
+    for (int j = 0; j < 32; ++j) {
+      const IX n = __shfl_sync(FULL, len, j), q = __shfl_sync(FULL, b0, j);
+      const VT aj = __shfl_sync(FULL, a, j);
+      for (IX p = lane; p < n; p += 32) {
+        VT v = VT(0);
+        if constexpr (NUM) v = aj * __ldg(Bx + q + p);
+        fn(tot + uint32_t(p), __ldg(Bj + q + p), v);
+      }
+      tot += uint32_t(n);
+    }
+    return tot;
+  }
+  uint32_t n = uint32_t(len);
+  const unsigned nz = __ballot_sync(FULL, n > 0);
+  const int ne = __popc(nz);
+  if (nz & (nz + 1u)) {  // a gap: lane i takes the i-th entry that has products
+    const int src = lane < ne ? nth_bit(nz, lane) : 0;
+    n = __shfl_sync(FULL, n, src);
+    b0 = __shfl_sync(FULL, b0, src);
+    if constexpr (NUM) a = __shfl_sync(FULL, a, src);
+    if (lane >= ne) n = 0;
+  }
+  const uint32_t inc = warp_scan_incl(n);
+  const uint32_t tot = __shfl_sync(FULL, inc, 31);
+  const uint32_t pre = lane < ne ? inc - n : 0xffffffffu;
+  const IX bq = b0 - IX(inc - n);  // position of product p = bq + p
+  const unsigned le = 0xffffffffu >> (31 - lane);
+  int cur = -1;  // the last entry that started before the window
+  // the step loop is uniform across the warp
+  for (uint32_t pb = 0; pb < tot; pb += 32 * U) {
     int32_t cc[U];
     VT xv[U], av[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const IX p = pb + IX(u) * 32 + lane;
-      int j = 0;
-#pragma unroll
-      for (int st = 16; st > 0; st >>= 1) {
-        const IX v = __shfl_sync(0xffffffffu, pre, (j + st) & 31);
-        if (j + st < nc && v <= p) j += st;
-      }
-      const IX pj = __shfl_sync(0xffffffffu, pre, j);
-      const IX bj = __shfl_sync(0xffffffffu, b0, j);
-      if constexpr (NUM) av[u] = __shfl_sync(0xffffffffu, a, j);
-      const IX q = bj + (p - pj);
+      const uint32_t pw = pb + u * 32, p = pw + lane;
+      const uint32_t d = pre - pw;
+      const unsigned m = __reduce_or_sync(FULL, d < 32u ? 1u << d : 0u);
+      const int j = cur + __popc(m & le);
+      cur += __popc(m);
+      const IX q = __shfl_sync(FULL, bq, j) + IX(p);
       cc[u] = p < tot ? __ldg(Bj + q) : -1;
-      if constexpr (NUM) xv[u] = p < tot ? __ldg(Bx + q) : VT(0);
+      if constexpr (NUM) {
+        av[u] = __shfl_sync(FULL, a, j);
+        xv[u] = p < tot ? __ldg(Bx + q) : VT(0);
+      }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (cc[u] >= 0) {
-        if constexpr (NUM) fn(cc[u], av[u] * xv[u]);
-        else fn(cc[u], VT(0));
+        if constexpr (NUM) fn(pb + u * 32 + lane, cc[u], av[u] * xv[u]);
+        else fn(pb + u * 32 + lane, cc[u], VT(0));
       }
     }
   }
+  return tot;
 }
 
 // Flat product loop for group rows.  A entries are taken G at a time: lane j
@@ -188,7 +232,8 @@ __device__ __forceinline__ void for_products_flat(
       len = IX(__ldg(Bp + k + 1)) - b0;
     }
     if constexpr (G == 32) {
-      warp_chunk<NUM, IX, VT>(Bj, Bx, b0, len, a, nc, lane, fn);
+      warp_chunk<NUM, IX, VT>(Bj, Bx, b0, len, a, lane,
+                              [&](uint32_t, int32_t c, VT v) { fn(c, v); });
       continue;  // no staging to guard
     } else {
       IX tot;
@@ -223,6 +268,72 @@ __device__ __forceinline__ void for_products_flat(
         }
       }
       group_sync<G>(gid);  // the next chunk reuses the staging
+    }
+  }
+}
+
+// The products of a warp row, one B row at a time: lane l takes the row's
+// entries l, l + 32, ... and the warp stays in step between B rows.  While B's
+// rows hold no column twice, no two lanes of a step meet in one column, so
+// fn may update a table of the warp without atomics.  Four B rows' loads are in
+// flight.
+template <bool NUM, typename PT, typename VT, typename F>
+__device__ __forceinline__ void for_products_rows(
+    const int32_t *__restrict__ Aj, const VT *__restrict__ Ax, const PT *__restrict__ Bp,
+    const int32_t *__restrict__ Bj, const VT *__restrict__ Bx, int64_t a0, int64_t a1, int lane,
+    F &&fn) {
+  using IX = std::conditional_t<sizeof(PT) == 4, uint32_t, int64_t>;
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int U = 4;
+  for (int64_t c0 = a0; c0 < a1; c0 += 32) {
+    const int nc = int(min(int64_t(32), a1 - c0));
+    IX b0 = 0, len = 0;
+    VT a = VT(0);
+    if (lane < nc) {
+      const int64_t k = __ldg(Aj + c0 + lane);
+      if constexpr (NUM) a = __ldg(Ax + c0 + lane);
+      b0 = IX(__ldg(Bp + k));
+      len = IX(__ldg(Bp + k + 1)) - b0;
+    }
+    for (int j0 = 0; j0 < nc; j0 += U) {
+      int32_t c[U];
+      VT v[U];
+      IX q[U], n[U];
+      bool more = false;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int j = (j0 + u) & 31;  // past nc: len 0
+        q[u] = __shfl_sync(FULL, b0, j);
+        n[u] = j0 + u < nc ? __shfl_sync(FULL, len, j) : IX(0);
+        c[u] = IX(lane) < n[u] ? __ldg(Bj + q[u] + lane) : -1;
+        if constexpr (NUM) {
+          const VT aj = __shfl_sync(FULL, a, j);
+          v[u] = IX(lane) < n[u] ? aj * __ldg(Bx + q[u] + lane) : VT(0);
+        } else {
+          v[u] = VT(0);
+        }
+        more |= n[u] > IX(32);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (c[u] >= 0) fn(c[u], v[u]);
+        __syncwarp();
+      }
+      if (more) {  // uniform
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          VT aj = VT(0);
+          if constexpr (NUM) aj = __shfl_sync(FULL, a, (j0 + u) & 31);
+          for (IX p = 32; p < n[u]; p += 32) {
+            if (p + lane < n[u]) {
+              VT x = VT(0);
+              if constexpr (NUM) x = aj * __ldg(Bx + q[u] + p + lane);
+              fn(__ldg(Bj + q[u] + p + lane), x);
+            }
+            __syncwarp();
+          }
+        }
+      }
     }
   }
 }
@@ -919,20 +1030,25 @@ __device__ void num_esc_row(const ProdDev<PT, VT> *prods, const PhaseArgs &A, co
       b0 = int64_t(__ldg(P.Bp + k));
       len = int64_t(__ldg(P.Bp + k + 1)) - b0;
     }
-    int64_t tot, pre;
     if constexpr (G == 32) {
-      const int64_t inc = warp_scan_incl(len);
-      tot = __shfl_sync(0xffffffffu, inc, 31);
-      pre = inc - len;
-    } else {
-      pre = group_excl_scan<G, int64_t>(len, gm.tmp, gid, &tot);
-      if (lane < nc) {
-        spre[lane] = pre;
-        sb0[lane] = b0;
-        sa[lane] = a;
-      }
-      group_sync<G>(gid);
+      fb += int(warp_chunk<true, int64_t, VT>(P.Bj, P.Bx, b0, len, a, lane,
+                                              [&](uint32_t p, int32_t col, VT v) {
+                                                const uint32_t at = uint32_t(fb) + p;
+                                                if (at < uint32_t(FMAX)) {
+                                                  keys[at] = col;
+                                                  vals[at] = v;
+                                                }
+                                              }));
+      continue;
     }
+    int64_t tot;
+    const int64_t pre = group_excl_scan<G, int64_t>(len, gm.tmp, gid, &tot);
+    if (lane < nc) {
+      spre[lane] = pre;
+      sb0[lane] = b0;
+      sa[lane] = a;
+    }
+    group_sync<G>(gid);
     for (int64_t pb = 0; pb < tot; pb += int64_t(G) * U) {
       int32_t cc[U];
       VT xv[U], av[U];
@@ -941,24 +1057,10 @@ __device__ void num_esc_row(const ProdDev<PT, VT> *prods, const PhaseArgs &A, co
       for (int u = 0; u < U; ++u) {
         const int64_t p = pb + int64_t(u) * G + lane;
         int j = 0;
-        int64_t pj, bj;
-        if constexpr (G == 32) {
-#pragma unroll
-          for (int st = 16; st > 0; st >>= 1) {
-            const int64_t v = __shfl_sync(0xffffffffu, pre, (j + st) & 31);
-            if (j + st < nc && v <= p) j += st;
-          }
-          pj = __shfl_sync(0xffffffffu, pre, j);
-          bj = __shfl_sync(0xffffffffu, b0, j);
-          av[u] = __shfl_sync(0xffffffffu, a, j);
-        } else {
-          for (int st = G / 2; st > 0; st >>= 1)
-            if (j + st < nc && spre[j + st] <= p) j += st;
-          pj = spre[j];
-          bj = sb0[j];
-          av[u] = sa[j];
-        }
-        const int64_t q = bj + (p - pj);
+        for (int st = G / 2; st > 0; st >>= 1)
+          if (j + st < nc && spre[j + st] <= p) j += st;
+        av[u] = sa[j];
+        const int64_t q = sb0[j] + (p - spre[j]);
         at[u] = p < tot ? fb + p : -1;
         cc[u] = p < tot ? __ldg(P.Bj + q) : 0;
         xv[u] = p < tot ? __ldg(P.Bx + q) : VT(0);
@@ -1074,6 +1176,135 @@ __device__ void num_esc_row(const ProdDev<PT, VT> *prods, const PhaseArgs &A, co
   if (lane == 0 && running != c) set_error(A.err, 108);
   group_sync<G>(gid);
   prof_sub_g(A, 13, tp, lane == 0);
+}
+
+// Column bitmap with a uint16 counter per 128 columns (span rows): o is a
+// column less the bitmap's first.  span_mark sets the column's bit and, the
+// first time, counts it in its unit (true then); once the counters hold the
+// units' rank bases, span_rank is the column's rank.
+__device__ __forceinline__ bool span_mark(uint32_t *bm, uint32_t *uc, uint32_t o) {
+  uint32_t *x = bm + (o >> 5);
+  const uint32_t bit = 1u << (o & 31);
+  if (*(volatile uint32_t *)x & bit) return false;
+  if (atomicOr(x, bit) & bit) return false;
+  atomicAdd(uc + (o >> 8), 1u << ((o >> 3) & 16));
+  return true;
+}
+__device__ __forceinline__ int span_rank(const uint32_t *bm, const uint32_t *uc, uint32_t o) {
+  const uint4 x = ((const uint4 *)bm)[o >> 7];
+  const uint32_t below = (1u << (o & 31)) - 1u;
+  const int wi = (o >> 5) & 3;
+  int r = ((const uint16_t *)uc)[o >> 7];
+  r += __popc(wi > 0 ? x.x : x.x & below);
+  r += __popc(wi > 1 ? x.y : wi == 1 ? x.y & below : 0u);
+  r += __popc(wi > 2 ? x.z : wi == 2 ? x.z & below : 0u);
+  r += __popc(wi == 3 ? x.w & below : 0u);
+  return r;
+}
+
+// Warp rows in span form: the columns between the row's first and last lie in
+// a bitmap in the warp's slice, their outputs behind it in rank order; no
+// probing, no sort.  The row's span comes from the ends of its B rows, so it
+// wants them known to be strictly increasing (b_strict), or a matrix no wider
+// than the bitmap.  With b_strict and B rows of kSeqRow entries or more on
+// average the row is walked B row by B row and added up without atomics: lanes
+// of a flat step meet in the columns that neighbouring B rows share, and an
+// FP64 shared atomic is a compare-and-swap loop.
+constexpr int kSpanWarpBits = 32768;
+constexpr int64_t kSpanWarpMin = 64;  // products; shorter rows sort in registers
+constexpr int64_t kSeqRow = 16;  // half of a warp's lanes busy in a B row
+constexpr int kSpanWarpBytes = kSpanWarpBits / 8 + kSpanWarpBits / 64 + int(kNumLim32) * 12;
+static_assert(kSpanWarpBytes <= kTableSmem / (kGroupThreads / 32), "warp slice");
+
+// False (nothing done) when the row's span does not fit.
+template <typename PT, typename VT>
+__device__ bool num_span_warp_row(const ProdDev<PT, VT> *prods, const PhaseArgs &A,
+                                  const RowMeta &m, unsigned char *slice, int lane) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const ProdDev<PT, VT> &P = prods[m.p];
+  const int64_t na = m.a1 - m.a0;
+  uint32_t base = 0, width = uint32_t(P.n);
+  if (P.n > kSpanWarpBits) {
+    int mn = INT32_MAX, mx = -1;
+    for (int64_t c0 = m.a0 + lane; c0 < m.a1; c0 += 32) {
+      const int64_t k = __ldg(P.Aj + c0);
+      const int64_t b0 = int64_t(__ldg(P.Bp + k)), b1 = int64_t(__ldg(P.Bp + k + 1));
+      if (b1 > b0) {
+        mn = min(mn, __ldg(P.Bj + b0));
+        mx = max(mx, __ldg(P.Bj + b1 - 1));
+      }
+    }
+    mn = __reduce_min_sync(FULL, mn);
+    mx = __reduce_max_sync(FULL, mx);
+    if (mx < mn || mx - mn >= kSpanWarpBits) return false;
+    base = uint32_t(mn);
+    width = uint32_t(mx - mn) + 1u;
+  }
+  long long tp = clock64();
+  uint32_t *bm = (uint32_t *)slice, *uc = bm + kSpanWarpBits / 32;
+  VT *vals = (VT *)(uc + kSpanWarpBits / 256);
+  int32_t *keys = (int32_t *)(vals + kNumLim32);
+  const int units = int((width + 127) >> 7), nu8 = (units + 7) >> 3;
+  for (int i = lane; i < nu8 * 8; i += 32) ((uint4 *)bm)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = lane; i < nu8; i += 32) ((uint4 *)uc)[i] = make_uint4(0, 0, 0, 0);
+  for (int64_t e = lane; e < m.c; e += 32) vals[e] = VT(0);
+  __syncwarp();
+  prof_sub_g(A, 9, tp, lane == 0);
+  const bool seq = P.b_strict && m.f >= kSeqRow * na;
+  auto mark = [&](int32_t col, VT) { span_mark(bm, uc, uint32_t(col) - base); };
+  if (seq) for_products_rows<false, PT, VT>(P.Aj, P.Ax, P.Bp, P.Bj, P.Bx, m.a0, m.a1, lane, mark);
+  else
+    for_products_flat<32, false, PT, VT>(P.Aj, P.Ax, P.Bp, P.Bj, P.Bx, m.a0, m.a1, lane, 0, nullptr,
+                                         nullptr, mark);
+  __syncwarp();
+  prof_sub_g(A, 10, tp, lane == 0);
+  int total;
+  {  // unit counts to unit bases: lane l owns units 8l ... 8l + 7
+    uint4 x = lane < nu8 ? ((uint4 *)uc)[lane] : make_uint4(0, 0, 0, 0);
+    uint32_t *h = (uint32_t *)&x;
+    const uint32_t y = x.x + x.y + x.z + x.w;
+    const int s = int((y & 0xffffu) + (y >> 16)), inc = warp_scan_incl(s);
+    total = __shfl_sync(FULL, inc, 31);
+    uint32_t run = uint32_t(inc - s);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t lo = h[k] & 0xffffu, hi = h[k] >> 16;
+      h[k] = run | ((run + lo) << 16);
+      run += lo + hi;
+    }
+    if (lane < nu8) ((uint4 *)uc)[lane] = x;
+  }
+  __syncwarp();
+  prof_sub_g(A, 11, tp, lane == 0);
+  if (total != m.c) {  // uniform; only if the pattern changed
+    if (lane == 0) set_error(A.err, 111);
+    __syncwarp();
+    return true;
+  }
+  if (seq) {
+    for_products_rows<true, PT, VT>(P.Aj, P.Ax, P.Bp, P.Bj, P.Bx, m.a0, m.a1, lane,
+                                    [&](int32_t col, VT v) {
+                                      const int r = span_rank(bm, uc, uint32_t(col) - base);
+                                      keys[r] = col;
+                                      vals[r] += v;
+                                    });
+  } else {
+    for_products_flat<32, true, PT, VT>(P.Aj, P.Ax, P.Bp, P.Bj, P.Bx, m.a0, m.a1, lane, 0, nullptr,
+                                        nullptr, [&](int32_t col, VT v) {
+                                          const int r = span_rank(bm, uc, uint32_t(col) - base);
+                                          keys[r] = col;
+                                          atomicAdd(vals + r, v);
+                                        });
+  }
+  __syncwarp();
+  prof_sub_g(A, 12, tp, lane == 0);
+  for (int64_t e = lane; e < m.c; e += 32) {
+    P.Cj[m.off + e] = keys[e];
+    P.Cx[m.off + e] = vals[e];
+  }
+  __syncwarp();
+  prof_sub_g(A, 13, tp, lane == 0);
+  return true;
 }
 
 // DENSE numeric row, whole-row form (ncols <= kRankMaxCols).  Pass 1 sets the
@@ -1725,7 +1956,10 @@ __device__ void group_rows(const ProdDev<PT, VT> *prods, const PhaseArgs &A,
         const long long t0 = clock64();
         const RowMeta m = shfl_meta(mine, t);
         if constexpr (NUM) {
-          if (esc_fits(m, TMAXN / 2))
+          const ProdDev<PT, VT> &P = prods[m.p];
+          const bool span = !P.Ej && m.f > kSpanWarpMin && (P.b_strict || P.n <= kSpanWarpBits);
+          if (span && num_span_warp_row<PT, VT>(prods, A, m, slice, lane)) {
+          } else if (esc_fits(m, TMAXN / 2))
             num_esc_row<G, TMAXN, PT, VT>(prods, A, m, slice, gm, gid, lane);
           else
             num_hash_row<G, TMAXN, PT, VT>(prods, A, m, slice, gm, gid, lane);

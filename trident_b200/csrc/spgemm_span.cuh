@@ -224,25 +224,15 @@ __device__ __forceinline__ void span_row(const ProdDev<PT, VT> &P, const PhaseAr
   int cnt = 0;
   // true when the product set its column's bit
   auto mark = [&](int32_t col) {
+    if constexpr (NUM) return span_mark(bm, uc, uint32_t(col));
     uint32_t *x = bm + (col >> 5);
     const uint32_t bit = 1u << (col & 31);
     if (*(volatile uint32_t *)x & bit) return false;
     if (atomicOr(x, bit) & bit) return false;
-    if constexpr (NUM) atomicAdd(uc + (col >> 8), 1u << ((col >> 3) & 16));
-    else ++cnt;
+    ++cnt;
     return true;
   };
-  auto rank_of = [&](int32_t col) {
-    const uint4 x = ((const uint4 *)smem)[col >> 7];
-    const uint32_t below = (1u << (col & 31)) - 1u;
-    const int wi = (col >> 5) & 3;
-    int r = ((const uint16_t *)uc)[col >> 7];
-    r += __popc(wi > 0 ? x.x : x.x & below);
-    r += __popc(wi > 1 ? x.y : wi == 1 ? x.y & below : 0u);
-    r += __popc(wi > 2 ? x.z : wi == 2 ? x.z & below : 0u);
-    r += __popc(wi == 3 ? x.w & below : 0u);
-    return r;
-  };
+  auto rank_of = [&](int32_t col) { return span_rank(bm, uc, uint32_t(col)); };
   int ne = 0;
   uint32_t tot = 0;
   int32_t cc[TILES][4];
