@@ -72,3 +72,46 @@ def test_dense_rows_two_ctas_per_sm():
     A = _rows(rng.choice([5, 40], size=2600), 600, rng)
     check_product(ops.spgemm(c, A.to_device(rowptr_bits=64), B.to_device(rowptr_bits=64)), A, B)
     c.close()
+
+
+@pytest.mark.parametrize("val_bits", [64, 32])
+def test_kept_bitmaps(val_bits):
+    # a one-shot product of 65,536 rows or more keeps the bitmaps of its heavy
+    # DENSE rows for the numeric phase: 1,500 of them (f ~36,000, c ~27,000)
+    # among rows of 3 products and rows on both sides of the register-held ones
+    c = ops.Context(0)
+    c.set_tuning({"sym_lim": [512, 2048, 4096, 4096], "num_lim": [256, 1024, 2048, 2048]})
+    rng = np.random.default_rng(9)
+    B = _rows(np.concatenate([np.full(600, 900), np.full(100, 3)]), 60000, rng)
+    lens = np.ones(66000, np.int64)
+    heavy = rng.choice(66000, size=1800, replace=False)
+    lens[heavy] = np.where(np.arange(1800) < 1500, 40, 9)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    col = np.concatenate([np.sort(rng.choice(600, size=k, replace=False)) if k > 1 else [600 + i % 100]
+                          for i, k in enumerate(lens)]).astype(np.int32)
+    A = HostCSR(66000, 700, rp, col, rng.uniform(-1, 1, col.size))
+    if val_bits == 32:
+        A, B = (HostCSR(M.nrows, M.ncols, M.rowptr, M.col, M.val.astype(np.float32).astype(np.float64))
+                for M in (A, B))
+    dA, dB = (M.to_device(rowptr_bits=64, val_bits=val_bits) for M in (A, B))
+    check_product(ops.spgemm(c, dA, dB), A, B, tol=TOL64 if val_bits == 64 else TOL32)
+    c.close()
+
+
+def test_overlapped_kernels_of_a_large_batch_and_product(ctx):
+    # rows of every class in one product, launched to overlap, several times
+    rng = np.random.default_rng(21)
+    B = _rows(rng.choice([1, 8, 60, 400], size=3000), 30000, rng)
+    A = _rows(rng.choice([1, 3, 10, 40, 150], size=4000), 3000, rng)
+    dA, dB = A.to_device(), B.to_device()
+    for _ in range(5):
+        C = ops.spgemm(ctx, dA, dB)
+    check_product(C, A, B)
+    b = ops.Batch(ctx)
+    for _ in range(2):
+        b.add(dA, dB)
+    for _ in range(3):
+        b.run()
+    for i in range(2):
+        check_product(b.result(i), A, B)
+    b.close()

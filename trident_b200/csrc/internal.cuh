@@ -360,4 +360,35 @@ __device__ __forceinline__ int64_t window_row(const PT *__restrict__ rp, int64_t
   return mine;
 }
 
+// Kernels of one phase that work on different rows overlap: each is launched
+// with programmatic stream serialization (overlap = true), so that it may start
+// once the one before it has started on all its CTAs, and fills what that one
+// leaves idle — above all while its last rows run.  phase_begin lets the next
+// kernel start; phase_end, by one CTA before it exits, keeps a kernel from
+// completing before the one it overlaps, so whatever follows in the stream
+// still waits for all of them.  A kernel launched without the attribute starts
+// after everything before it, and both are then no-ops for it.
+__device__ __forceinline__ void phase_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void phase_end() {
+  if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... Q>
+inline cudaError_t launch_phase(bool overlap, unsigned grid, unsigned block, size_t smem,
+                                cudaStream_t s, void (*k)(P...), Q... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+
 }  // namespace tspg

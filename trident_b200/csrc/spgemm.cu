@@ -50,6 +50,9 @@ struct tspg_plan {
   int32_t *oj = nullptr;
   void *ox = nullptr;
   uint64_t *defer = nullptr;
+  uint32_t *bits = nullptr;  // DENSE rows' bitmaps for the numeric phase (one-shot products)
+  int32_t *slot = nullptr;
+  int64_t nslots = 0, slot_words = 0;
   void *blocks[16];
   int nblocks = 0;
 
@@ -95,6 +98,16 @@ constexpr int64_t kOnePassMinRows = 1 << 16;
 static_assert(kOnePassMinRows >= kFuseRows, "the one-pass branch sets the list offsets itself");
 constexpr int64_t kOnePassMaxEntries = int64_t(1) << 30;
 
+// One-shot products keep the column bitmaps of their heaviest DENSE rows from
+// the symbolic to the numeric phase, which then walks those rows' products once
+// instead of twice — while B's columns and values fit the L2 beside the outputs
+// (beyond it the first walk is what brings B in: on R-MAT scale 20 keeping 4 GB
+// of bitmaps made the numeric phase 4 % slower), in at most 4 GB of workspace,
+// and for enough rows.
+constexpr int64_t kKeepBytes = int64_t(4) << 30;
+constexpr int64_t kKeepNnz = int64_t(6) << 20;
+constexpr int64_t kKeepRows = 1024;
+
 // Warp-class rows from which the check of B's rows for strict order pays.
 constexpr int64_t kStrictRows = 4096;
 
@@ -110,7 +123,7 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
                          const tspg_csr *B, int flags, tspg_plan *P) {
   TSPG_TRY(set_smem_attr<PT, VT>(ctx->device));
   const int64_t m = A->nrows, n = B->ncols, k = A->ncols;
-  const Tune tune = span_tune(ctx->tune, n);
+  const Tune tune = span_tune<PT, VT>(ctx->tune, n);
   P->m = m;
   P->n = n;
   P->k = k;
@@ -167,10 +180,10 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
     TSPG_CUDA(ctx, cudaGetLastError());
     TSPG_CUDA(ctx, cudaMemcpyAsync(h + HW_TOTAL, P->cp + m, sizeof(int64_t),
                                    cudaMemcpyDeviceToHost, s));
-    TSPG_CUDA(ctx, cudaMemcpyAsync(h + HW_ONEPASS, &P->sched[0].cnt[CLS_ONEPASS], sizeof(int64_t),
+    TSPG_CUDA(ctx, cudaMemcpyAsync(h + HW_CNT, &P->sched[0].cnt, NCLS * sizeof(int64_t),
                                    cudaMemcpyDeviceToHost, s));
     TSPG_CUDA(ctx, cudaStreamSynchronize(s));
-    const int64_t tot = h[HW_TOTAL], rows = h[HW_ONEPASS];
+    const int64_t tot = h[HW_TOTAL], rows = h[HW_CNT + CLS_ONEPASS];
     // one pass when most rows take it (R-MAT 20: a tenth of the rows, and
     // those with more than 32 outputs need their second attempt: +0.9 ms
     // of symbolic phase; Galerkin A·P: every row, -0.9 ms per call)
@@ -182,6 +195,16 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
       onepass = false;
       k_fold_onepass<<<1, 32, 0, s>>>(P->sched);
       ctx->launches += 1;
+    }
+    // room for the bitmaps of the heaviest DENSE rows
+    const int64_t dense = h[HW_CNT] + h[HW_CNT + 1] + h[HW_CNT + 2];
+    const int64_t words = ((n + 1023) >> 10) * 32;
+    const int64_t slots = std::min(dense, kKeepBytes / (words * 4));
+    if (slots >= kKeepRows && B->nnz <= kKeepNnz && n <= kRankMaxCols &&
+        P->get(&P->slot, size_t(m)) == TSPG_OK && P->get(&P->bits, size_t(slots * words)) == TSPG_OK) {
+      TSPG_CUDA(ctx, cudaMemsetAsync(P->slot, 0xff, size_t(m) * sizeof(int32_t), s));
+      P->nslots = slots;
+      P->slot_words = words;
     }
   }
   if (m >= kFuseRows) {
@@ -196,8 +219,14 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
   pa.oj = P->oj;
   pa.ox = P->ox;
   pa.defer = P->defer;
+  if (P->nslots) {
+    pa.bits = P->bits;
+    pa.slot = P->slot;
+    pa.nslots = P->nslots;
+    pa.slot_words = P->slot_words;
+  }
   phase_mark(ctx, 0, 0, s);
-  TSPG_TRY((launch_symbolic_rows<PT, VT>(ctx, s, prods, pa, n)));
+  TSPG_TRY((launch_symbolic_rows<PT, VT>(ctx, s, prods, pa, n, true)));
   if (onepass) {
     k_onepass<PT, VT><<<ctx->num_sms, kOnepassThreads, kOnepassSmem, s>>>(prods, pa);
     // the rows sent back (too many columns for their 64-slot attempt and
@@ -274,8 +303,13 @@ static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P, const tspg_
   PhaseArgs pa{P->base, P->sched + 1, P->list, P->rowf, P->rowc, P->cp,
                P->curbuf, P->cur_stride, ctx->d_words + kErrWord,
                ctx->d_prof ? ctx->d_prof + kProfPerPhase : nullptr};
+  if (P->nslots) {
+    pa.bits = P->bits;
+    pa.slot = P->slot;
+    pa.slot_words = P->slot_words;
+  }
   phase_mark(ctx, 1, 0, s);
-  TSPG_TRY((launch_numeric_rows<PT, VT>(ctx, s, prods, pa, P->n, P->ncnt, m < kFuseRows)));
+  TSPG_TRY((launch_numeric_rows<PT, VT>(ctx, s, prods, pa, P->n, P->ncnt, m < kFuseRows, true)));
   if (P->onepass)
     k_onepass_copy<PT, VT><<<grid_for(m * 32, 256, ctx->num_sms * 16), 256, 0, s>>>(
         prods, P->rowf, P->rowc, P->cp, P->oj, (const VT *)P->ox, m);

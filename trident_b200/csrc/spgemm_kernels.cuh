@@ -826,7 +826,7 @@ static __global__ void __launch_bounds__(1024) k_scan_partials(int64_t *partial,
 // from the device into mapped pinned memory (a stream sync then suffices; a
 // device->host copy took 2.6 us each): nnz(C), the record's sums, the error
 // word and the numeric class counts.
-enum { HW_TOTAL = 0, HW_MULTS, HW_MAX_A, HW_ERR, HW_ONEPASS, HW_CNT };
+enum { HW_TOTAL = 0, HW_MULTS, HW_MAX_A, HW_ERR, HW_CNT };
 struct HostWords {
   int64_t *words = nullptr;      // null: nothing is left
   const Sched *sym = nullptr;    // the symbolic record

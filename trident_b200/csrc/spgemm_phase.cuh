@@ -432,6 +432,11 @@ struct PhaseArgs {
   void *ox = nullptr;
   uint64_t *defer = nullptr;  // one-pass rows sent back to the two-pass path
   uint32_t skip = 0;          // classes k_groups leaves to k_span (bit per class)
+  // column bitmaps of the first nslots DENSE symbolic rows, slot_words words
+  // each, for their numeric rank form; slot[g] = row g's, or -1
+  uint32_t *bits = nullptr;
+  int32_t *slot = nullptr;
+  int64_t nslots = 0, slot_words = 0;
 };
 
 // Optional per-class accounting (SM cycles spent in each row class), and
@@ -1339,17 +1344,24 @@ __device__ void num_dense_rank_row(const ProdDev<PT, VT> *prods, const PhaseArgs
   const VT *__restrict__ Bx = P.Bx;
   const int S1 = subgroup_width_avg(f, na, 32);
   long long tp = clock64();
-  for (int i = tid; i < nb * 32; i += NT) bm[i] = 0u;
-  __syncthreads();
-  auto mark = [&](int32_t col, VT) {
-    const uint32_t bit = 1u << (col & 31);
-    uint32_t &x = bmw(col >> 5);
-    if (!(*(volatile uint32_t *)&x & bit)) atomicOr(&x, bit);
-  };
-  for_products_balanced<NT, false, PT, VT>(Aj, Ax, Bp, Bj, Bx, a0, a1, f, S1, tid, 0,
-                                                 gm.lst, gm.nl, gm.cap, mark, gm.nl - 1);
-  for_addend<false>(P, rr.r, tid, NT, mark);
-  __syncthreads();
+  const int32_t slot = A.slot ? A.slot[rr.g] : -1;
+  if (slot >= 0) {  // the symbolic phase kept the row's bitmap
+    const uint32_t *__restrict__ kept = A.bits + slot * A.slot_words;
+    for (int i = tid; i < nb * 32; i += NT) bmw(i) = __ldcs(kept + i);
+    __syncthreads();
+  } else {
+    for (int i = tid; i < nb * 32; i += NT) bm[i] = 0u;
+    __syncthreads();
+    auto mark = [&](int32_t col, VT) {
+      const uint32_t bit = 1u << (col & 31);
+      uint32_t &x = bmw(col >> 5);
+      if (!(*(volatile uint32_t *)&x & bit)) atomicOr(&x, bit);
+    };
+    for_products_balanced<NT, false, PT, VT>(Aj, Ax, Bp, Bj, Bx, a0, a1, f, S1, tid, 0,
+                                                   gm.lst, gm.nl, gm.cap, mark, gm.nl - 1);
+    for_addend<false>(P, rr.r, tid, NT, mark);
+    __syncthreads();
+  }
   prof_sub(A, 0, tp);
   // Block scan: block b = words [32b, 32b + 32), lane l of a warp takes word
   // 32b + l (no bank conflicts).  wp[w] = rank of word w's first bit within
@@ -2088,6 +2100,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
     k_groups(const ProdDev<PT, VT> *prods, PhaseArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ PhaseShared sh;
+  phase_begin();
   if (threadIdx.x < NCLS) {
     sh.off[threadIdx.x] = A.S->off[threadIdx.x];
     sh.cnt[threadIdx.x] = A.S->cnt[threadIdx.x];
@@ -2096,6 +2109,7 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
   if (!(A.skip >> CLS_G256 & 1u)) group_rows<256, NUM, PT, VT>(prods, A, CLS_G256, smem, sh);
   if (!(A.skip >> CLS_G128 & 1u)) group_rows<128, NUM, PT, VT>(prods, A, CLS_G128, smem, sh);
   if (!(A.skip >> CLS_G32 & 1u)) group_rows<32, NUM, PT, VT>(prods, A, CLS_G32, smem, sh);
+  phase_end();
 }
 
 // One-pass rows of a plain product (the symbolic record's CLS_ONEPASS list),

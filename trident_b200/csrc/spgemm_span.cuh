@@ -192,11 +192,12 @@ __device__ __forceinline__ void span_tile(const uint32_t *pre, const IX *bq, con
 // Rows of at most TILES x 4 products per thread (and at most NT A entries)
 // keep their products in registers; longer ones walk them twice.  WIPE: the
 // bitmap may hold anything on entry (it is cleared here); otherwise it is
-// all zero on entry and on return.  Entered and left with the CTA in step.
+// all zero on entry and on return.  save (!NUM): where the bitmap of a row
+// that walks its products twice is kept for the numeric phase.  Entered and left with the CTA in step.
 template <int NT, bool NUM, int TILES, bool WIPE, typename PT, typename VT>
 __device__ __forceinline__ void span_row(const ProdDev<PT, VT> &P, const PhaseArgs &A,
                                          const RowMeta &m, unsigned char *smem, const SpanLay &L,
-                                         SpanShared<NT> &sh) {
+                                         SpanShared<NT> &sh, uint32_t *save = nullptr) {
   using IX = std::conditional_t<sizeof(PT) == 4, uint32_t, int64_t>;
   constexpr int NW = NT / 32, TP = 128;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -288,11 +289,17 @@ __device__ __forceinline__ void span_row(const ProdDev<PT, VT> &P, const PhaseAr
           for (int u = 0; u < 4; ++u)
             if (cc[t][u] >= 0) bm[cc[t][u] >> 5] = 0u;
       } else {
-        for (int i = tid; i < nu8 * 8; i += NT) ((uint4 *)smem)[i] = make_uint4(0, 0, 0, 0);
+        for (int i = tid; i < nu8 * 8; i += NT) {
+          if (save) ((uint4 *)save)[i] = ((uint4 *)smem)[i];
+          ((uint4 *)smem)[i] = make_uint4(0, 0, 0, 0);
+        }
       }
     }
     __syncthreads();
-    if (tid == 0) A.rowc[m.g] = sh.total;
+    if (tid == 0) {
+      A.rowc[m.g] = sh.total;
+      if (save && !reg) A.slot[m.g] = int32_t((save - A.bits) / A.slot_words);
+    }
     return;
   } else {
     __syncthreads();  // all bits and unit counts set
@@ -398,10 +405,14 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ SpanShared<NT> sh;
   const int tid = threadIdx.x;
+  phase_begin();
   int64_t count = 0;
   for (int c = c0; c < c1; ++c) count += A.S->cnt[c];
   const int64_t base = A.S->off[c0];
-  if (count == 0) return;
+  if (count == 0) {
+    phase_end();
+    return;
+  }
   for (int i = tid; i < L.nu8 * (NUM ? 9 : 8); i += NT)
     ((uint4 *)smem)[i] = make_uint4(0, 0, 0, 0);  // bitmap, then unit counters
   while (true) {
@@ -421,7 +432,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
     for (int t = 0; t < nrow; ++t) {
       const long long t0 = clock64();
       const RowMeta m = sh.meta[t];
-      span_row<NT, NUM, NUM ? 2 : 4, false, PT, VT>(prods[m.p], A, m, smem, L, sh);
+      uint32_t *save = nullptr;  // the first rows of the DENSE classes have slots
+      if (!NUM && c0 == 0 && A.bits && i0 + t < A.nslots) save = A.bits + (i0 + t) * A.slot_words;
+      span_row<NT, NUM, NUM ? 2 : 4, false, PT, VT>(prods[m.p], A, m, smem, L, sh, save);
       if (A.prof) {
         int c = c0;
         while (c + 1 < c1 && base + i0 + t >= A.S->off[c + 1]) ++c;
@@ -429,6 +442,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
       }
     }
   }
+  phase_end();
 }
 
 // The numeric DENSE rows of the rank form (at most kRankMaxCols columns, not
@@ -445,6 +459,7 @@ __global__ void __launch_bounds__(NT, CT)
   __shared__ SpanShared<NT> ss;
   __shared__ unsigned long long s_item;
   const int tid = threadIdx.x;
+  phase_begin();
   const int64_t H = A.S->cnt[CLS_DENSE0] + A.S->cnt[CLS_DENSE1];
   const int64_t L = A.S->cnt[CLS_DENSE2];
   const int64_t c01 = A.S->cnt[CLS_DENSE0];
@@ -488,15 +503,16 @@ __global__ void __launch_bounds__(NT, CT)
     }
     __syncthreads();
   }
+  phase_end();
 }
 
 // Two CTAs of k_dense_rank per SM when every rank row fits half of its shared
 // memory: one row's bitmap and emission passes run while another's value pass
 // waits on the L2's reductions (R-MAT of order 2^18, 16 draws a row: 27.7 ->
 // 23.9 ms).  Fewer rows than a few per SM end on the longest one, which the
-// 768-thread CTA finishes sooner (order 30k, 138 rows: 0.44 against 0.19 ms).
+// 768-thread CTA finishes sooner (order 30k, 138 rows: 0.44 against 0.20 ms).
 constexpr uint32_t kRank2Smem = 100 * 1024;
-constexpr int kRank2Rows = 16;  // DENSE rows per SM
+constexpr int kRank2Rows = 8;  // DENSE rows per SM
 constexpr uint32_t kSpanSmemMax = 220 * 1024;  // dynamic; the static part stays below 7 KiB
 
 // CTAs of k_span resident on one SM with this layout (64 registers a thread).
@@ -510,27 +526,38 @@ inline int span_ctas(const SpanLay &L) {
 
 template <int NT, bool NUM, typename PT, typename VT>
 inline cudaError_t launch_span(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, VT> *prods,
-                               const PhaseArgs &pa, const SpanLay &L, int c0, int c1) {
+                               const PhaseArgs &pa, const SpanLay &L, int c0, int c1,
+                               bool overlap) {
   const int ctas = span_ctas<NT>(L);
-  k_span<NT, NUM, PT, VT><<<ctx->num_sms * ctas, NT, L.bytes, s>>>(prods, pa, L, c0, c1);
   ctx->launches += 1;
-  return cudaGetLastError();
+  return launch_phase(overlap, ctx->num_sms * ctas, NT, L.bytes, s, k_span<NT, NUM, PT, VT>, prods,
+                      pa, L, c0, c1);
 }
 
 // Sorted B rows only matter to rows swept in column windows: wider than the
 // rank form's bitmap, or taken by the window form of the tuning.
 inline bool needs_sorted(const Tune &t, int64_t ncols) { return ncols > kRankMaxCols || t.win != 0; }
 
-// The row binning of a run: while the bitmap of 128-thread span rows stays
+// The row binning of a run.  While the bitmap of 128-thread span rows stays
 // small (8 CTAs per SM), numeric rows of more than kSpanWarpRow outputs leave
 // the warps for them.  Uniform rows of order 1024 with ~250 outputs: numeric
 // 49 -> 15 us; Poisson(15) of order 100k 0.55 -> 0.48 ms, of order 200k (5
-// CTAs per SM) 1.16 -> 1.23 ms.
+// CTAs per SM) 1.16 -> 1.23 ms.  And where 512-thread span rows with the full
+// bound's slots would have an SM to themselves, the bound drops to
+// kSpanHalfRow, at which two fit, the longer rows going to the DENSE kernel:
+// R-MAT of order 65k 1.39 -> 1.21 ms, 131k 2.05 -> 1.90 ms (a whole call); of
+// order 30k, where two fit anyway, 0.78 -> 0.83 ms.
 constexpr int64_t kSpanWarpCols = 131072;
 constexpr int32_t kSpanWarpRow = 128;
+constexpr int32_t kSpanHalfRow = 4096;
+template <typename PT, typename VT>
 inline Tune span_tune(Tune t, int64_t ncols) {
   if (ncols <= kSpanWarpCols && t.num[0] > kSpanWarpRow && t.num[1] >= t.num[0])
     t.num[0] = kSpanWarpRow;
+  if (t.num[3] > kSpanHalfRow && t.num[2] <= kSpanHalfRow && ncols <= kRankMaxCols &&
+      span_ctas<512>(span_layout<512, true, PT, VT>(ncols, uint32_t(t.num[3]))) < 2 &&
+      span_ctas<512>(span_layout<512, true, PT, VT>(ncols, uint32_t(kSpanHalfRow))) >= 2)
+    t.num[3] = kSpanHalfRow;
   return t;
 }
 
@@ -543,27 +570,30 @@ inline Tune span_tune(Tune t, int64_t ncols) {
 // The persistent kernels of a symbolic phase (one-pass rows aside).
 template <typename PT, typename VT>
 inline int launch_symbolic_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, VT> *prods,
-                                PhaseArgs pa, int64_t ncols) {
+                                PhaseArgs pa, int64_t ncols, bool may_overlap) {
   const SpanLay L1 = span_layout<128, false, PT, VT>(ncols, 0);
   const SpanLay L2 = span_layout<256, false, PT, VT>(ncols, 0);
   const SpanLay L3 = span_layout<512, false, PT, VT>(ncols, 0);
   if (span_ctas<512>(L3) >= 2) {
-    TSPG_CUDA(ctx, (launch_span<512, false, PT, VT>(ctx, s, prods, pa, L3, 0, CLS_G1024 + 1)));
+    TSPG_CUDA(ctx, (launch_span<512, false, PT, VT>(ctx, s, prods, pa, L3, 0, CLS_G1024 + 1, false)));
   } else {
     k_phase<PT, VT, false><<<ctx->num_sms, kSymThreads, kDynSmem, s>>>(prods, pa);
     ctx->launches += 1;
   }
+  const bool overlap = may_overlap && span_ctas<512>(L3) >= 2;  // k_phase lets nothing start early
   if (span_ctas<256>(L2) >= 2) {
-    TSPG_CUDA(ctx, (launch_span<256, false, PT, VT>(ctx, s, prods, pa, L2, CLS_G256, CLS_G256 + 1)));
+    TSPG_CUDA(ctx, (launch_span<256, false, PT, VT>(ctx, s, prods, pa, L2, CLS_G256, CLS_G256 + 1,
+                                                    overlap)));
     pa.skip |= 1u << CLS_G256;
   }
   if (span_ctas<128>(L1) >= 2) {
-    TSPG_CUDA(ctx, (launch_span<128, false, PT, VT>(ctx, s, prods, pa, L1, CLS_G128, CLS_G128 + 1)));
+    TSPG_CUDA(ctx, (launch_span<128, false, PT, VT>(ctx, s, prods, pa, L1, CLS_G128, CLS_G128 + 1,
+                                                    overlap)));
     pa.skip |= 1u << CLS_G128;
   }
-  k_groups<PT, VT, false><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
+  TSPG_CUDA(ctx, launch_phase(overlap, ctx->num_sms, kGroupThreads, kGroupDynSmem, s,
+                              k_groups<PT, VT, false>, prods, pa));
   ctx->launches += 1;
-  TSPG_CUDA(ctx, cudaGetLastError());
   return TSPG_OK;
 }
 
@@ -573,13 +603,15 @@ inline int launch_symbolic_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT,
 template <int NT, typename PT, typename VT>
 inline cudaError_t launch_span_class(tspg_ctx *ctx, cudaStream_t s,
                                      const ProdDev<PT, VT> *prods, const PhaseArgs &pa,
-                                     int64_t ncols, uint32_t cap, int cls, int64_t rows) {
+                                     int64_t ncols, uint32_t cap, int cls, int64_t rows,
+                                     bool overlap) {
   if constexpr (NT < 512) {
     if (rows >= 0 && rows <= int64_t(ctx->num_sms) * (512 / NT))
-      return launch_span_class<2 * NT, PT, VT>(ctx, s, prods, pa, ncols, cap, cls, rows);
+      return launch_span_class<2 * NT, PT, VT>(ctx, s, prods, pa, ncols, cap, cls, rows, overlap);
   }
   return launch_span<NT, true, PT, VT>(ctx, s, prods, pa,
-                                       span_layout<NT, true, PT, VT>(ncols, cap), cls, cls + 1);
+                                       span_layout<NT, true, PT, VT>(ncols, cap), cls, cls + 1,
+                                       overlap);
 }
 
 // The persistent kernels of a numeric phase whose products have at most
@@ -589,49 +621,61 @@ inline cudaError_t launch_span_class(tspg_ctx *ctx, cudaStream_t s,
 template <typename PT, typename VT>
 inline int launch_numeric_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, VT> *prods,
                                PhaseArgs pa, int64_t ncols, const int64_t *cnt,
-                               bool skip_empty) {
+                               bool skip_empty, bool may_overlap) {
   TSPG_CUDA(ctx, launch_dense_cluster<PT, VT>(ctx, s, prods, pa));
-  const Tune &tn = ctx->tune;
+  const Tune tn = span_tune<PT, VT>(ctx->tune, ncols);
   auto rows = [&](int c) { return cnt ? cnt[c] : int64_t(-1); };
   auto some = [&](int c) { return !skip_empty || rows(c) != 0; };
   const int64_t dense = cnt ? cnt[CLS_DENSE0] + cnt[CLS_DENSE1] + cnt[CLS_DENSE2] : -1;
   const uint32_t nb = uint32_t((ncols + 1023) >> 10);
+  bool overlap = false;  // the first kernel of the phase starts after the binning
   if (!skip_empty || dense != 0) {
     if (nb * 196u <= kRank2Smem && dense >= int64_t(kRank2Rows) * ctx->num_sms)
-      k_dense_rank<512, 2, PT, VT><<<ctx->num_sms * 2, 512, kRank2Smem, s>>>(prods, pa, kRank2Smem);
+      TSPG_CUDA(ctx, launch_phase(overlap, ctx->num_sms * 2, 512, kRank2Smem, s,
+                                  k_dense_rank<512, 2, PT, VT>, prods, pa, kRank2Smem));
     else
-      k_dense_rank<kRankThreads, 1, PT, VT><<<ctx->num_sms, kRankThreads, kDynSmem, s>>>(prods, pa,
-                                                                                         kDynSmem);
+      TSPG_CUDA(ctx, launch_phase(overlap, ctx->num_sms, kRankThreads, kDynSmem, s,
+                                  k_dense_rank<kRankThreads, 1, PT, VT>, prods, pa,
+                                  uint32_t(kDynSmem)));
     ctx->launches += 1;
+    overlap = may_overlap;
   }
   if (span_ctas<512>(span_layout<512, true, PT, VT>(ncols, uint32_t(tn.num[3]))) >= 1) {
     pa.skip |= 1u << CLS_G1024;
-    if (some(CLS_G1024))
+    if (some(CLS_G1024)) {
       TSPG_CUDA(ctx, (launch_span_class<512>(ctx, s, prods, pa, ncols, uint32_t(tn.num[3]),
-                                             CLS_G1024, rows(CLS_G1024))));
+                                             CLS_G1024, rows(CLS_G1024), overlap)));
+      overlap = may_overlap;
+    }
   }
   if (span_ctas<256>(span_layout<256, true, PT, VT>(ncols, uint32_t(tn.num[2]))) >= 2) {
     pa.skip |= 1u << CLS_G256;
-    if (some(CLS_G256))
+    if (some(CLS_G256)) {
       TSPG_CUDA(ctx, (launch_span_class<256>(ctx, s, prods, pa, ncols, uint32_t(tn.num[2]),
-                                             CLS_G256, rows(CLS_G256))));
+                                             CLS_G256, rows(CLS_G256), overlap)));
+      overlap = may_overlap;
+    }
   }
   if (span_ctas<128>(span_layout<128, true, PT, VT>(ncols, uint32_t(tn.num[1]))) >= 2) {
     pa.skip |= 1u << CLS_G128;
-    if (some(CLS_G128))
+    if (some(CLS_G128)) {
       TSPG_CUDA(ctx, (launch_span_class<128>(ctx, s, prods, pa, ncols, uint32_t(tn.num[1]),
-                                             CLS_G128, rows(CLS_G128))));
+                                             CLS_G128, rows(CLS_G128), overlap)));
+      overlap = may_overlap;
+    }
   }
   // k_phase: DENSE rows that are neither rank nor span rows, G1024 hash rows
   const bool left = ncols > kRankMaxCols || tn.win != 0;
   if ((left && (!skip_empty || dense != 0)) ||
       (!(pa.skip >> CLS_G1024 & 1u) && some(CLS_G1024))) {
-    k_phase<PT, VT, true><<<ctx->num_sms, kThreads, kDynSmem, s>>>(prods, pa);
+    k_phase<PT, VT, true><<<ctx->num_sms, kThreads, kDynSmem, s>>>(prods, pa);  // reads rank_left
     ctx->launches += 1;
+    overlap = false;
   }
   if (some(CLS_G32) || (!(pa.skip >> CLS_G256 & 1u) && some(CLS_G256)) ||
       (!(pa.skip >> CLS_G128 & 1u) && some(CLS_G128))) {
-    k_groups<PT, VT, true><<<ctx->num_sms, kGroupThreads, kGroupDynSmem, s>>>(prods, pa);
+    TSPG_CUDA(ctx, launch_phase(overlap, ctx->num_sms, kGroupThreads, kGroupDynSmem, s,
+                                k_groups<PT, VT, true>, prods, pa));
     ctx->launches += 1;
   }
   TSPG_CUDA(ctx, cudaGetLastError());
