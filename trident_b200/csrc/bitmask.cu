@@ -61,21 +61,18 @@ static int pack_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M,
   Scratch sc(ctx, s);
   int32_t *cnt;
   int64_t *newp, *partial;
-  Sched *dummy;
+  Sched *rec;
   const int64_t nb = (len + kScanTile - 1) / kScanTile;
-  TSPG_TRY(sc.get(&cnt, len));
-  TSPG_TRY(sc.get(&newp, len + 1));
-  TSPG_TRY(sc.get(&partial, nb + 1));
-  TSPG_TRY(sc.get(&dummy, 1));
-  TSPG_CUDA(ctx, cudaMemsetAsync(newp, 0, sizeof(int64_t), s));
-  TSPG_CUDA(ctx, cudaMemsetAsync(dummy, 0, sizeof(Sched), s));
+  TSPG_TRY(sc.get_all(part(&cnt, len), part(&newp, len + 1), part(&partial, nb + 1), part(&rec, 1)));
   const PT *ptr = (const PT *)M->rowptr;
   if (len > 0) {
-    k_pack_counts<PT><<<(unsigned)((len + 255) / 256), 256, 0, s>>>(ptr, len, mask, cnt);
-    k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(cnt, len, partial);
-    k_scan_partials<<<1, 1024, 0, s>>>(partial, nb);
-    k_scan_final<<<(unsigned)nb, kScanThreads, 0, s>>>(cnt, len, partial, nb, newp, dummy, nullptr);
-    ctx->launches += 4;
+    k_pack_counts<PT><<<(unsigned)((len + 255) / 256), 256, 0, s>>>(ptr, len, mask, cnt, &rec->ticket);
+    ctx->launches += 1;
+    launch_scan(ctx, s, cnt, len, partial, newp, rec, nullptr, HostWords(),
+                kept_host ? ctx->h_words : nullptr);
+  } else {
+    TSPG_CUDA(ctx, cudaMemsetAsync(newp, 0, sizeof(int64_t), s));
+    ctx->h_words[0] = 0;
   }
   ctx->launches += 1;
   const int64_t work = (M->nnz + kPackRun - 1) / kPackRun * 32;
@@ -89,8 +86,6 @@ static int pack_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M,
                                             (char *)out_buf, kept_dev);
   TSPG_CUDA(ctx, cudaGetLastError());
   if (kept_host) {
-    TSPG_CUDA(ctx, cudaMemcpyAsync(ctx->h_words, newp + len, sizeof(int64_t),
-                                   cudaMemcpyDeviceToHost, s));
     TSPG_CUDA(ctx, cudaStreamSynchronize(s));
     *kept_host = ctx->h_words[0];
   }

@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <mutex>
 #include <unordered_map>
+#include <utility>
 
 #include "tspg.h"
 
@@ -135,10 +136,23 @@ struct Scratch {
     *p = (T *)q;
     return TSPG_OK;
   }
+  // Several arrays out of one block, each on a 256-byte boundary.
+  template <typename... T>
+  int get_all(std::pair<T **, size_t>... part) {
+    auto room = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
+    char *q = nullptr;
+    TSPG_TRY(get(&q, (size_t(0) + ... + room(part.second * sizeof(T)))));
+    ((*part.first = (T *)q, q += room(part.second * sizeof(T))), ...);
+    return TSPG_OK;
+  }
   ~Scratch() {
     for (int i = n - 1; i >= 0; --i) ws_free(ctx, ptrs[i], s);
   }
 };
+template <typename T>
+inline std::pair<T **, size_t> part(T **p, int64_t count) {
+  return {p, size_t(count)};
+}
 
 inline int check_csr(const tspg_csr *M) {
   if (!M) return TSPG_EINVAL;

@@ -105,7 +105,7 @@ template <bool FILL, typename PT, typename VT>
 __global__ void __launch_bounds__(256)
     k_prune_tiles(const PT *__restrict__ rp, const int32_t *__restrict__ col,
                   const VT *__restrict__ val, int64_t m, int64_t nnz, VT tol, int64_t ntiles,
-                  int32_t *tilec, const int64_t *off, void *np, int np_bits, int32_t *ocol,
+                  int32_t *tilec, Sched *rec, const int64_t *off, void *np, int np_bits, int32_t *ocol,
                   VT *oval) {
   constexpr int U = 8;
   __shared__ unsigned mask[64 + 1];
@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   if (!FILL) {
     if (tid == 0) tilec[t] = before[64];
+    if (tid == 0 && t == 0) rec->ticket = 0;  // of the scan to come
     return;
   }
   const int64_t o = off[t];
@@ -210,18 +211,15 @@ static int prune_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, double t
   int32_t *tilec;
   int64_t *off, *partial;
   Sched *rec;
-  TSPG_TRY(sc.get(&tilec, ntiles));
-  TSPG_TRY(sc.get(&off, ntiles + 1));
-  TSPG_TRY(sc.get(&partial, (ntiles + kScanTile - 1) / kScanTile + 1));
-  TSPG_TRY(sc.get(&rec, 1));
-  TSPG_CUDA(ctx, cudaMemsetAsync(rec, 0, sizeof(Sched), s));
+  TSPG_TRY(sc.get_all(part(&tilec, ntiles), part(&off, ntiles + 1),
+                      part(&partial, (ntiles + kScanTile - 1) / kScanTile + 1), part(&rec, 1)));
   k_prune_tiles<false, PT, VT><<<unsigned(ntiles), 256, 0, s>>>(
-      (const PT *)M->rowptr, nullptr, (const VT *)M->val, m, M->nnz, VT(tol), ntiles, tilec, nullptr,
-      nullptr, 0, nullptr, nullptr);
+      (const PT *)M->rowptr, nullptr, (const VT *)M->val, m, M->nnz, VT(tol), ntiles, tilec, rec,
+      nullptr, nullptr, 0, nullptr, nullptr);
   ctx->launches += 1;
-  launch_scan(ctx, s, tilec, ntiles, partial, off, rec, nullptr);
   int64_t *h = ctx->h_words;
-  TSPG_CUDA(ctx, cudaMemcpyAsync(h, off + ntiles, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  launch_scan(ctx, s, tilec, ntiles, partial, off, rec, nullptr, HostWords(), h);
+  TSPG_CUDA(ctx, cudaGetLastError());
   TSPG_CUDA(ctx, cudaStreamSynchronize(s));
   const int64_t nnz = h[0];
   out->nnz = nnz;
@@ -236,7 +234,7 @@ static int prune_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, double t
     out->capacity = nnz;
   }
   k_prune_tiles<true, PT, VT><<<unsigned(ntiles), 256, 0, s>>>(
-      (const PT *)M->rowptr, M->col, (const VT *)M->val, m, M->nnz, VT(tol), ntiles, nullptr, off,
+      (const PT *)M->rowptr, M->col, (const VT *)M->val, m, M->nnz, VT(tol), ntiles, nullptr, nullptr, off,
       out->rowptr, out->rowptr_bits, out->col, (VT *)out->val);
   ctx->launches += 1;
   TSPG_CUDA(ctx, cudaGetLastError());

@@ -11,8 +11,9 @@ namespace tspg {
 // Masked segment lengths (select_ptrs' MaskedTransform, spacomm.cuh:539-553).
 template <typename PT>
 __global__ void k_pack_counts(const PT *ptr, int64_t len, const uint8_t *mask,
-                              int32_t *cnt) {
+                              int32_t *cnt, uint32_t *ticket = nullptr) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (ticket && i == 0) *ticket = 0;  // of the scan to come
   if (i < len) {
     const bool keep = (mask[i >> 3] >> (i & 7)) & 1;
     cnt[i] = keep ? int32_t(int64_t(ptr[i + 1]) - int64_t(ptr[i])) : 0;

@@ -322,17 +322,16 @@ inline int part_passes(int64_t n) { return (key_bits(n) + kPartBits - 1) / kPart
 
 struct PartScratch {
   uint32_t *table = nullptr, *dtotal = nullptr;
-  int64_t ntiles = 0;
+  int64_t ntiles = 0, table_len = 0;
   bool big = false;
 };
 
-inline int part_scratch(Scratch &sc, int64_t count, PartScratch *P) {
+inline void part_sizes(int64_t count, PartScratch *P) {
   const int64_t T16 = kPartThreads * 16, T4 = kPartThreads * 4;
   P->big = count >= kPartBigTiles * T16 / 4;
   const int64_t T = P->big ? T16 : T4;
   P->ntiles = (count + T - 1) / T;
-  TSPG_TRY(sc.get(&P->table, size_t(P->ntiles) << kPartBits));
-  return sc.get(&P->dtotal, size_t(1) << kPartBits);
+  P->table_len = P->ntiles << kPartBits;
 }
 
 template <int ITEMS, typename VT>

@@ -38,8 +38,9 @@ template <typename PTA, typename PTB>
 __global__ void __launch_bounds__(128)
     k_merge_cuts(int64_t m, const PTA *__restrict__ Ap, const int32_t *__restrict__ Aj,
                  const PTB *__restrict__ Bp, const int32_t *__restrict__ Bj, int64_t ntiles,
-                 MergeCut *cuts) {
+                 MergeCut *cuts, Sched *rec) {
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t == 0) rec->ticket = 0;  // of the scan to come
   if (t > ntiles) return;
   const int64_t ab = int64_t(Ap[0]), bb = int64_t(Bp[0]);
   auto start = [&](int64_t r) { return int64_t(__ldg(Ap + r)) - ab + int64_t(__ldg(Bp + r)) - bb; };
@@ -285,24 +286,19 @@ static int spadd_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
   int32_t *tilec;
   int64_t *off, *partial;
   Sched *rec;
-  TSPG_TRY(sc.get(&cuts, ntiles + 1));
-  TSPG_TRY(sc.get(&tilec, ntiles));
-  TSPG_TRY(sc.get(&off, ntiles + 1));
-  TSPG_TRY(sc.get(&partial, nb + 1));
-  TSPG_TRY(sc.get(&rec, 1));
-  TSPG_CUDA(ctx, cudaMemsetAsync(rec, 0, sizeof(Sched), s));
+  TSPG_TRY(sc.get_all(part(&cuts, ntiles + 1), part(&tilec, ntiles), part(&off, ntiles + 1),
+                      part(&partial, nb + 1), part(&rec, 1)));
   const PTA *Ap = (const PTA *)A->rowptr;
   const PTB *Bp = (const PTB *)B->rowptr;
   k_merge_cuts<PTA, PTB><<<unsigned((ntiles + 128) / 128), 128, 0, s>>>(m, Ap, A->col, Bp, B->col,
-                                                                       ntiles, cuts);
+                                                                       ntiles, cuts, rec);
   k_merge_tiles<false, PTA, PTB, VT><<<unsigned(ntiles), kMergeThreads, 0, s>>>(
       m, Ap, A->col, nullptr, Bp, B->col, nullptr, ntiles, cuts, tilec, nullptr, nullptr, 0, nullptr,
       nullptr);
   ctx->launches += 2;
-  launch_scan(ctx, s, tilec, ntiles, partial, off, rec, nullptr);
-  TSPG_CUDA(ctx, cudaGetLastError());
   int64_t *h = ctx->h_words;
-  TSPG_CUDA(ctx, cudaMemcpyAsync(h, off + ntiles, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  launch_scan(ctx, s, tilec, ntiles, partial, off, rec, nullptr, HostWords(), h);
+  TSPG_CUDA(ctx, cudaGetLastError());
   TSPG_CUDA(ctx, cudaStreamSynchronize(s));
   const int64_t nnz = h[0];
   if (C->rowptr_bits == 32 && nnz > INT32_MAX) return TSPG_EOVERFLOW;

@@ -612,8 +612,10 @@ __global__ void __launch_bounds__(256)
 }
 
 // Totals of the row products: mults and sum of min(products, n).
+// (host: mapped memory, written by the last block)
 __global__ void __launch_bounds__(256)
-    k_count_totals(const unsigned long long *rowf, int64_t m, int64_t n, unsigned long long *tot) {
+    k_count_totals(const unsigned long long *rowf, int64_t m, int64_t n, unsigned long long *tot,
+                   uint32_t *ticket, int64_t *host) {
   unsigned long long wm = 0, wu = 0;
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
   for (int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < m; r += stride) {
@@ -626,6 +628,12 @@ __global__ void __launch_bounds__(256)
   if ((threadIdx.x & 31) == 0 && (wm | wu)) {
     atomicAdd(tot, wm);
     atomicAdd(tot + 1, wu);
+  }
+  if (last_block(ticket) && threadIdx.x == 0) {
+    volatile int64_t *h = host;
+    h[0] = *(volatile int64_t *)tot;
+    h[1] = *(volatile int64_t *)(tot + 1);
+    __threadfence_system();
   }
 }
 
@@ -641,8 +649,8 @@ static void launch_count_mask(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A, 
   if (A->nnz > 0)
     k_count_mask<APT, BPT><<<unsigned((A->nnz + 8 * kMaskRun - 1) / (8 * kMaskRun)), 256, 0, s>>>(
         (const APT *)A->rowptr, A->col, (const BPT *)B->rowptr, A->nrows, words, rowf);
-  k_count_totals<<<grid_for(A->nrows, 256, ctx->num_sms * 4), 256, 0, s>>>(rowf, A->nrows, B->ncols,
-                                                                          tot);
+  k_count_totals<<<grid_for(A->nrows, 256, ctx->num_sms * 4), 256, 0, s>>>(
+      rowf, A->nrows, B->ncols, tot, (uint32_t *)(tot + 2), ctx->h_words);
   ctx->launches += 1 + (A->nnz > 0);
 }
 
@@ -660,9 +668,11 @@ extern "C" int tspg_spgemm_count_mask(tspg_ctx *ctx, void *stream, const tspg_cs
   Scratch sc(ctx, s);
   uint32_t *words;  // the mask words, then (8-byte aligned) two totals and the row products
   const int64_t nw = ((kdim + 31) / 32 + 1) & ~int64_t(1);
-  TSPG_TRY(sc.get(&words, nw + 2 * (A->nrows + 2)));
-  unsigned long long *tot = (unsigned long long *)(words + nw), *rowf = tot + 2;
-  TSPG_CUDA(ctx, cudaMemsetAsync(words, 0, sizeof(uint32_t) * (nw + 2 * (A->nrows + 2)), s));
+  TSPG_TRY(sc.get(&words, nw + 2 * (A->nrows + 3)));
+  unsigned long long *tot = (unsigned long long *)(words + nw), *rowf = tot + 3;  // ticket between
+  const int64_t zero = nw / 2 + A->nrows + 3;
+  k_zero<<<grid_for(zero, 256, ctx->num_sms * 8), 256, 0, s>>>((uint64_t *)words, zero);
+  ctx->launches += 1;
   if (A->nrows > 0) {
     if (A->rowptr_bits == 32 && B->rowptr_bits == 32) launch_count_mask<int32_t, int32_t>(ctx, s, A, B, words, rowf, tot);
     else if (A->rowptr_bits == 32) launch_count_mask<int32_t, int64_t>(ctx, s, A, B, words, rowf, tot);
@@ -675,7 +685,7 @@ extern "C" int tspg_spgemm_count_mask(tspg_ctx *ctx, void *stream, const tspg_cs
   }
   TSPG_CUDA(ctx, cudaGetLastError());
   int64_t *h = ctx->h_words;
-  TSPG_CUDA(ctx, cudaMemcpyAsync(h, tot, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  if (A->nrows == 0) h[0] = h[1] = 0;
   TSPG_CUDA(ctx, cudaStreamSynchronize(s));
   if (mults) *mults = h[0];
   if (c_nnz_upper) *c_nnz_upper = h[1];

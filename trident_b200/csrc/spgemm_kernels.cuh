@@ -89,12 +89,21 @@ constexpr int kHeavyPeriod = 64;
 __host__ __device__ inline int dense_sub(int64_t f) {
   return f >= (int64_t(1) << 20) ? CLS_DENSE0 : f >= (int64_t(1) << 17) ? CLS_DENSE1 : CLS_DENSE2;
 }
+// A group row by its products: many products on few columns (hub rows of a
+// small matrix) take more threads than their table asks for.  R-MAT of order
+// 1318 (FP32): 128-thread rows of 10^4 products were the call (0.17 ms).
+__host__ __device__ inline int wide_class(int c, int64_t f) {
+  if (c == CLS_G32 && f > 2048) c = CLS_G128;
+  if (c == CLS_G128 && f > 8192) c = CLS_G256;
+  if (c == CLS_G256 && f > 32768) c = CLS_G1024;
+  return c;
+}
 __host__ __device__ inline int sym_class(int64_t f, int64_t n, const Tune &t) {
   const int64_t fe = f < n ? f : n;
   if (f == 0) return -1;
-  if (fe <= t.sym[0]) return CLS_G32;
-  if (fe <= t.sym[1]) return CLS_G128;
-  if (fe <= t.sym[2]) return CLS_G256;
+  if (fe <= t.sym[0]) return wide_class(CLS_G32, f);
+  if (fe <= t.sym[1]) return wide_class(CLS_G128, f);
+  if (fe <= t.sym[2]) return wide_class(CLS_G256, f);
   if (fe <= t.sym[3]) return CLS_G1024;
   return dense_sub(f);
 }
@@ -123,9 +132,9 @@ __host__ __device__ inline int64_t onepass_bound(int64_t f, int64_t n, const Tun
 }
 __host__ __device__ inline int num_class(int64_t c, int64_t f, const Tune &t) {
   if (c == 0 || f < 0) return -1;  // f < 0: a one-pass row, already computed
-  if (c <= t.num[0]) return CLS_G32;
-  if (c <= t.num[1]) return CLS_G128;
-  if (c <= t.num[2]) return CLS_G256;
+  if (c <= t.num[0]) return wide_class(CLS_G32, f);
+  if (c <= t.num[1]) return wide_class(CLS_G128, f);
+  if (c <= t.num[2]) return wide_class(CLS_G256, f);
   if (c <= t.num[3]) return CLS_G1024;
   return dense_sub(f);
 }
@@ -252,6 +261,13 @@ __global__ void __launch_bounds__(128) k_setup(ProdDev<PT, VT> *dst, ProdDev<PT,
     base[0] = 0;
     base[1] = v.m;
   }
+}
+
+// Zero words (a launch costs a third of a small memset's call).
+static __global__ void __launch_bounds__(256) k_zero(uint64_t *p, int64_t n) {
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+       i += int64_t(gridDim.x) * blockDim.x)
+    p[i] = 0;
 }
 
 // True in every thread of the grid's last block to get here (the others'
@@ -855,7 +871,7 @@ static __global__ void k_finish_symbolic(Sched *Snum, const int64_t *total, Host
 static __global__ void __launch_bounds__(kScanThreads)
     k_scan_final(const int32_t *in, int64_t R, const int64_t *partial,
                  int64_t nb, int64_t *out, Sched *Snum, const int64_t *rowf,
-                 HostWords host = HostWords()) {
+                 HostWords host = HostWords(), int64_t *host_total = nullptr) {
   __shared__ int64_t tmp[kScanThreads / 32 + 1];
   __shared__ unsigned long long s_cnt[NCLS];
   if (threadIdx.x < NCLS) s_cnt[threadIdx.x] = 0;
@@ -894,7 +910,13 @@ static __global__ void __launch_bounds__(kScanThreads)
     ex += v[i];
   }
   const int64_t total = partial ? partial[nb] : tot;
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[R] = total;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    out[R] = total;
+    if (host_total) {
+      *(volatile int64_t *)host_total = total;
+      __threadfence_system();
+    }
+  }
   __syncthreads();
   if (threadIdx.x < NCLS && s_cnt[threadIdx.x])
     atomicAdd((unsigned long long *)&Snum->cnt[threadIdx.x], s_cnt[threadIdx.x]);
@@ -912,7 +934,7 @@ constexpr int64_t kFuseRows = 1 << 16;
 // ticket is used).
 static inline void launch_scan(tspg_ctx *ctx, cudaStream_t s, const int32_t *in, int64_t R,
                                int64_t *partial, int64_t *out, Sched *S, const int64_t *rowf,
-                               HostWords host = HostWords()) {
+                               HostWords host = HostWords(), int64_t *host_total = nullptr) {
   const int64_t nb = (R + kScanTile - 1) / kScanTile;
   const bool fuse = R < kFuseRows;
   if (nb > 1) {
@@ -921,7 +943,7 @@ static inline void launch_scan(tspg_ctx *ctx, cudaStream_t s, const int32_t *in,
     ctx->launches += fuse ? 1 : 2;
   }
   k_scan_final<<<(unsigned)nb, kScanThreads, 0, s>>>(in, R, nb > 1 ? partial : nullptr, nb, out, S,
-                                                     rowf, fuse ? host : HostWords());
+                                                     rowf, fuse ? host : HostWords(), host_total);
   ctx->launches += 1;
   if (host.words && !fuse) {
     k_finish_symbolic<<<1, 32, 0, s>>>(S, out + R, host);

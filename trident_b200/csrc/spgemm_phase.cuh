@@ -2193,7 +2193,6 @@ __device__ void onepass_lanes(const ProdDev<PT, VT> &P, const PhaseArgs &A, cons
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (c[u] >= 0) {
-          const VT v = av * x[u];
           uint32_t h = hash_slot(c[u], kLaneLog);
           int k = keys[h * 32];
           for (int it = 1; k != c[u] && k != -1 && it < kLaneSlots; ++it) {
@@ -2201,10 +2200,10 @@ __device__ void onepass_lanes(const ProdDev<PT, VT> &P, const PhaseArgs &A, cons
             k = keys[h * 32];
           }
           if (k == c[u]) {
-            vals[h * 32] += v;
+            vals[h * 32] = fma(av, x[u], vals[h * 32]);
           } else if (k == -1) {
             keys[h * 32] = c[u];
-            vals[h * 32] = v;
+            vals[h * 32] = av * x[u];
             ++n;
           } else {
             refused = true;

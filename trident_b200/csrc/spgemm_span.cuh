@@ -541,14 +541,15 @@ inline bool needs_sorted(const Tune &t, int64_t ncols) { return ncols > kRankMax
 // The row binning of a run.  While the bitmap of 128-thread span rows stays
 // small (8 CTAs per SM), numeric rows of more than kSpanWarpRow outputs leave
 // the warps for them.  Uniform rows of order 1024 with ~250 outputs: numeric
-// 49 -> 15 us; Poisson(15) of order 100k 0.55 -> 0.48 ms, of order 200k (5
-// CTAs per SM) 1.16 -> 1.23 ms.  And where 512-thread span rows with the full
+// 49 -> 15 us; Poisson(15) of order 100k (~225 outputs) 0.55 -> 0.48 ms, of
+// order 200k (5 CTAs per SM) 1.16 -> 1.23 ms; ~144 outputs, order 120k 0.56 ->
+// 0.60 ms.  And where 512-thread span rows with the full
 // bound's slots would have an SM to themselves, the bound drops to
 // kSpanHalfRow, at which two fit, the longer rows going to the DENSE kernel:
 // R-MAT of order 65k 1.39 -> 1.21 ms, 131k 2.05 -> 1.90 ms (a whole call); of
 // order 30k, where two fit anyway, 0.78 -> 0.83 ms.
 constexpr int64_t kSpanWarpCols = 131072;
-constexpr int32_t kSpanWarpRow = 128;
+constexpr int32_t kSpanWarpRow = 192;
 constexpr int32_t kSpanHalfRow = 4096;
 template <typename PT, typename VT>
 inline Tune span_tune(Tune t, int64_t ncols) {

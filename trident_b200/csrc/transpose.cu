@@ -238,9 +238,10 @@ static int transpose_passes(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, ts
   PartScratch P;
   int32_t *rows, *key, *idx = nullptr;
   VT *val = nullptr;
-  if (sc.get(&rows, nnz) != TSPG_OK || sc.get(&key, nnz) != TSPG_OK ||
-      part_scratch(sc, nnz, &P) != TSPG_OK ||
-      (passes > 1 && (sc.get(&idx, nnz) != TSPG_OK || sc.get(&val, nnz) != TSPG_OK)))
+  const int64_t more = passes > 1 ? nnz : 0;
+  part_sizes(nnz, &P);
+  if (sc.get_all(part(&rows, nnz), part(&key, nnz), part(&P.table, P.table_len),
+                 part(&P.dtotal, 1 << kPartBits), part(&idx, more), part(&val, more)) != TSPG_OK)
     return TSPG_OK;
   *done = true;
   TSPG_TRY(ensure_entries<VT>(T, nnz, s));
@@ -419,9 +420,9 @@ static int coo_passes(tspg_ctx *ctx, cudaStream_t s, int64_t nmaj, int64_t nmin,
   PartScratch P;
   int32_t *k1, *k2, *idx;
   VT *vals;
-  if (part_scratch(sc, nnz, &P) != TSPG_OK || sc.get(&k1, nnz) != TSPG_OK ||
-      sc.get(&k2, nnz) != TSPG_OK || sc.get(&idx, nnz) != TSPG_OK ||
-      sc.get(&vals, nnz) != TSPG_OK)
+  part_sizes(nnz, &P);
+  if (sc.get_all(part(&k1, nnz), part(&k2, nnz), part(&P.table, P.table_len),
+                 part(&P.dtotal, 1 << kPartBits), part(&idx, nnz), part(&vals, nnz)) != TSPG_OK)
     return TSPG_OK;
   *done = true;
   PartSpan S;

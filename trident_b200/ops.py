@@ -427,21 +427,21 @@ def _alias_csr(v: TspgCsr) -> DeviceCSR:
     return DeviceCSR(int(v.nrows), int(v.ncols), rp, col, val, nnz=nnz)
 
 
+_TYPESTR = {torch.int32: "<i4", torch.int64: "<i8", torch.float64: "<f8", torch.float32: "<f4"}
+
+
+class _DeviceArray:
+    __slots__ = ("__cuda_array_interface__",)
+
+    def __init__(self, ptr: int, count: int, dtype):
+        self.__cuda_array_interface__ = {"shape": (count,), "typestr": _TYPESTR[dtype], "data": (int(ptr), False),
+                                         "version": 3}
+
+
 def _device_view(ptr: int, count: int, dtype) -> torch.Tensor:
     """A torch tensor over `count` elements of library-owned device memory."""
-    itemsize = torch.empty(0, dtype=dtype).element_size()
-
-    class _Arr:
-        __cuda_array_interface__ = {
-            "shape": (count,),
-            "typestr": {torch.int32: "<i4", torch.int64: "<i8", torch.float64: "<f8",
-                        torch.float32: "<f4"}[dtype],
-            "data": (int(ptr), False),
-            "version": 3,
-        }
-
-    t = torch.as_tensor(_Arr(), device="cuda")
-    assert t.element_size() == itemsize
+    t = torch.as_tensor(_DeviceArray(ptr, count, dtype), device="cuda")
+    assert t.dtype == dtype
     return t
 
 
