@@ -115,3 +115,34 @@ def test_overlapped_kernels_of_a_large_batch_and_product(ctx):
     for i in range(2):
         check_product(b.result(i), A, B)
     b.close()
+
+
+@pytest.mark.parametrize("val_bits", [64, 32])
+def test_lane_rows(val_bits):
+    # numeric rows of 1 ... 32 outputs, 32 to a warp (even rows of 30 products
+    # first, then uneven ones that a warp takes one by one), 33 past the slots;
+    # a plan run twice, and a batch whose rows alternate between two products
+    rng = np.random.default_rng(5)
+    B = _rows(np.concatenate([np.full(400, 5), rng.choice([0, 1, 3, 33, 200], size=400)]), 50000, rng)
+    even = [np.sort(rng.choice(400, size=6, replace=False)) for _ in range(40000)]
+    mixed = [np.sort(rng.choice(800, size=k, replace=False)) for k in rng.choice([1, 2, 6, 7], size=20000)]
+    rp = np.concatenate([[0], np.cumsum([len(r) for r in even + mixed])]).astype(np.int64)
+    A = HostCSR(60000, 800, rp, np.concatenate(even + mixed).astype(np.int32), rng.uniform(-1, 1, rp[-1]))
+    tol = TOL64 if val_bits == 64 else TOL32
+    if val_bits == 32:
+        A, B = (HostCSR(M.nrows, M.ncols, M.rowptr, M.col, M.val.astype(np.float32).astype(np.float64))
+                for M in (A, B))
+    c = ops.Context(0)
+    dA, dB = A.to_device(val_bits=val_bits), B.to_device(val_bits=val_bits)
+    plan = ops.Plan(c, dA, dB)
+    for _ in range(2):
+        check_product(plan.numeric(dA, dB), A, B, tol=tol)
+    plan.close()
+    b = ops.Batch(c)
+    b.add(dA, dB)
+    b.add(dA, dB)
+    b.run()
+    for i in range(2):
+        check_product(b.result(i), A, B, tol=tol)
+    b.close()
+    c.close()

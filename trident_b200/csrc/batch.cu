@@ -326,7 +326,7 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
     cudaGraph_t g;
     TSPG_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(b->sched, 0, 2 * sizeof(Sched), s);
-    const Tune tune = span_tune<PT, VT>(ctx->tune, ncols);
+    const Tune tune = span_tune<PT, VT>(ctx->tune, ncols, false);
     const bool check = !(flags & TSPG_F_B_SORTED) && b->RB > 0 && needs_sorted(tune, ncols);
     k_set_tune<<<1, 32, 0, s>>>(b->sched, 2, tune);
     cudaMemsetAsync(b->cp, 0, sizeof(int64_t), s);

@@ -32,6 +32,7 @@ struct Tune {
   int32_t win;   // log2 of the products from which DENSE numeric rows take the window form; 0 = never
   int32_t fill;  // ... when their output also fills >= 1 / 2^fill of the columns
   int32_t cluster;  // CTAs per thread-block cluster working on one such row (0 = one CTA)
+  int32_t lane;     // numeric rows of at most this many outputs are lane rows (set per run)
 };
 constexpr int32_t kDefaultWinLog2 = 0, kDefaultWinFillLog2 = 4;  // window form off by default (measured slower)
 

@@ -123,7 +123,7 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
                          const tspg_csr *B, int flags, tspg_plan *P) {
   TSPG_TRY(set_smem_attr<PT, VT>(ctx->device));
   const int64_t m = A->nrows, n = B->ncols, k = A->ncols;
-  const Tune tune = span_tune<PT, VT>(ctx->tune, n);
+  const Tune tune = span_tune<PT, VT>(ctx->tune, n, P->E.col && P->E.nnz > 0);
   P->m = m;
   P->n = n;
   P->k = k;
@@ -228,7 +228,7 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
   phase_mark(ctx, 0, 0, s);
   TSPG_TRY((launch_symbolic_rows<PT, VT>(ctx, s, prods, pa, n, true)));
   if (onepass) {
-    k_onepass<PT, VT><<<ctx->num_sms, kOnepassThreads, kOnepassSmem, s>>>(prods, pa);
+    k_lanes<false, PT, VT><<<ctx->num_sms, kOnepassThreads, kOnepassSmem, s>>>(prods, pa);
     // the rows sent back (too many columns for their 64-slot attempt and
     // too large for a warp's full table): their symbolic count, as
     // 256-thread rows of their own record

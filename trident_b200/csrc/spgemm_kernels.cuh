@@ -64,7 +64,8 @@ enum {
   CLS_G256 = 4,
   CLS_G128 = 5,
   CLS_G32 = 6,
-  CLS_ONEPASS = 7  // symbolic only: warp rows computed whole in the symbolic launch
+  CLS_ONEPASS = 7,  // symbolic: rows computed whole in the symbolic launch
+  CLS_LANE = 7      // numeric: short rows, 32 of them by one warp, a lane each
 };
 constexpr int kCtaClasses = 4;  // classes [0, 4) are CTA-level
 __host__ __device__ constexpr bool cls_dense(int c) { return c <= CLS_DENSE2; }
@@ -132,6 +133,7 @@ __host__ __device__ inline int64_t onepass_bound(int64_t f, int64_t n, const Tun
 }
 __host__ __device__ inline int num_class(int64_t c, int64_t f, const Tune &t) {
   if (c == 0 || f < 0) return -1;  // f < 0: a one-pass row, already computed
+  if (c <= t.lane) return CLS_LANE;
   if (c <= t.num[0]) return wide_class(CLS_G32, f);
   if (c <= t.num[1]) return wide_class(CLS_G128, f);
   if (c <= t.num[2]) return wide_class(CLS_G256, f);

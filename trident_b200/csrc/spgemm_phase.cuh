@@ -2112,10 +2112,11 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
   phase_end();
 }
 
-// One-pass rows of a plain product (the symbolic record's CLS_ONEPASS list),
-// after k_groups in the symbolic launch: each row is multiplied in full into
-// the scratch, so no symbolic pass counts it (Galerkin A·P paid 1.8 ms of
-// symbolic and 3.5 ms of numeric launches for it).
+// Short rows, a lane each (k_lanes).  Symbolic launch (FINAL = false): the
+// one-pass rows of a plain product, after k_groups; each is multiplied in full
+// into the scratch, so no symbolic pass counts it (Galerkin A·P paid 1.8 ms of
+// symbolic and 3.5 ms of numeric launches for it).  Numeric launch (FINAL =
+// true): the rows of at most kLaneSlots outputs, into C.
 constexpr int kOnepassThreads = 512;
 constexpr int kLaneSlots = kCappedCols;            // columns a lane's row may hold
 constexpr int kLaneLog = 5;
@@ -2128,8 +2129,8 @@ static_assert(kNumT32 * 12 <= kOnepassSlice, "the warp form's table");
 // with the others (the next entry's B row bounds and the one after's column
 // in flight) and adds every product into its own kLaneSlots-slot hash table in
 // shared memory, [slot][lane]: no atomics, no bank conflicts.  The occupied
-// slots are sorted by insertion as they are gathered, and written to the
-// scratch.  A row with more than kLaneSlots columns goes back to the two-pass
+// slots are sorted by insertion as they are gathered, and written out.  A
+// one-pass row with more than kLaneSlots columns goes back to the two-pass
 // path.  (A list searched from the last hit on instead of the table: 105-148
 // instructions a product, Galerkin A·P 3.0 ms.)
 //
@@ -2137,9 +2138,9 @@ static_assert(kNumT32 * 12 <= kOnepassSlice, "the warp form's table");
 // per row: ~1040 warp instructions for the 119 products of a Galerkin A·P
 // row); lanes of neighbouring rows also read neighbouring B rows, so their
 // loads coalesce.
-template <typename PT, typename VT>
-__device__ void onepass_lanes(const ProdDev<PT, VT> &P, const PhaseArgs &A, const RowMeta &m,
-                              bool have, unsigned char *slice, int lane) {
+template <bool FINAL, typename PT, typename VT>
+__device__ void lane_rows(const ProdDev<PT, VT> &P, const PhaseArgs &A, const RowMeta &m,
+                          bool have, unsigned char *slice, int lane) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int U = 4;
   int *keys = (int *)slice + lane;
@@ -2192,7 +2193,7 @@ __device__ void onepass_lanes(const ProdDev<PT, VT> &P, const PhaseArgs &A, cons
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        if (c[u] >= 0) {
+        if (c[u] >= 0 && !refused) {
           uint32_t h = hash_slot(c[u], kLaneLog);
           int k = keys[h * 32];
           for (int it = 1; k != c[u] && k != -1 && it < kLaneSlots; ++it) {
@@ -2211,9 +2212,10 @@ __device__ void onepass_lanes(const ProdDev<PT, VT> &P, const PhaseArgs &A, cons
         }
       }
     }
+    if (__all_sync(FULL, refused || t + 1 >= na)) break;
     av = an;
     b0 = n0;
-    b1 = n1;
+    b1 = refused ? n0 : n1;
     kn = k2;
     an = a2;
   }
@@ -2235,6 +2237,20 @@ __device__ void onepass_lanes(const ProdDev<PT, VT> &P, const PhaseArgs &A, cons
     }
   }
   __syncwarp();
+  if constexpr (FINAL) {
+    if (have && (refused || n != m.c)) {  // only if the pattern changed
+      set_error(A.err, 112);
+      n = 0;
+    }
+    int32_t *const oj = P.Cj + m.off;
+    VT *const ox = P.Cx + m.off;
+    for (int i = 0; i < n; ++i) {
+      oj[i] = keys[i * 32];
+      ox[i] = vals[i * 32];
+    }
+    __syncwarp();
+    return;
+  }
   if (have && !refused) {
     int32_t *const oj = A.oj + m.off;
     VT *const ox = (VT *)A.ox + m.off;
@@ -2256,12 +2272,14 @@ __device__ void onepass_lanes(const ProdDev<PT, VT> &P, const PhaseArgs &A, cons
   __syncwarp();
 }
 
-template <typename PT, typename VT>
+template <bool FINAL, typename PT, typename VT>
 __global__ void __launch_bounds__(kOnepassThreads, 1)
-    k_onepass(const ProdDev<PT, VT> *prods, PhaseArgs A) {
+    k_lanes(const ProdDev<PT, VT> *prods, PhaseArgs A) {
+  static_assert(CLS_ONEPASS == CLS_LANE, "one list");
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int lst[kOnepassThreads];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  phase_begin();
   const int64_t count = A.S->cnt[CLS_ONEPASS], base = A.S->off[CLS_ONEPASS];
   const int64_t warps = int64_t(gridDim.x) * (kOnepassThreads / 32);
   unsigned char *slice = smem + w * kOnepassSlice;
@@ -2285,25 +2303,38 @@ __global__ void __launch_bounds__(kOnepassThreads, 1)
     const long long t0 = clock64();
     RowMeta mine{};
     if (have) {
-      mine = load_meta<false>(prods, A, base + i + lane);
-      mine.off = A.cp[mine.g];  // the row's scratch offset
+      mine = load_meta<FINAL>(prods, A, base + i + lane);
+      if (!FINAL) mine.off = A.cp[mine.g];  // the row's scratch offset
     }
     // lanes in step take as long as the longest row (~40 instructions a
     // product); a warp per row ~350 and 6 a product
     const int f = int(mine.f);
     const int fmax = __reduce_max_sync(0xffffffffu, f);
     const int fsum = __reduce_add_sync(0xffffffffu, f);
-    if (40 * int64_t(fmax) <= 350 * int64_t(rows) + 6 * int64_t(fsum)) {
-      onepass_lanes<PT, VT>(prods[0], A, mine, have, slice, lane);
+    const int p0 = __shfl_sync(0xffffffffu, mine.p, 0);
+    const bool lanes = 40 * int64_t(fmax) <= 350 * int64_t(rows) + 6 * int64_t(fsum) &&
+                       __all_sync(0xffffffffu, !have || mine.p == p0);
+    if (lanes) {
+      lane_rows<FINAL, PT, VT>(prods[p0], A, mine, have, slice, lane);
     } else {
-      for (int t = 0; t < rows; ++t)
-        num_hash_row<32, kNumT32, PT, VT, true>(prods, A, shfl_meta(mine, t), slice, gm, w, lane);
+      for (int t = 0; t < rows; ++t) {
+        const RowMeta m = shfl_meta(mine, t);
+        if constexpr (FINAL) {  // at most 32 outputs: sorted in registers
+          if (m.f <= 32)
+            num_esc_row<32, kNumT32, PT, VT>(prods, A, m, slice, gm, w, lane);
+          else
+            num_hash_row<32, kNumT32, PT, VT>(prods, A, m, slice, gm, w, lane);
+        } else {
+          num_hash_row<32, kNumT32, PT, VT, true>(prods, A, m, slice, gm, w, lane);
+        }
+      }
     }
     if (A.prof && lane == 0) {
       atomicAdd(A.prof + CLS_ONEPASS, (unsigned long long)(clock64() - t0));
       atomicAdd(A.prof + NCLS + CLS_ONEPASS, (unsigned long long)rows);
     }
   }
+  phase_end();
 }
 
 // Numeric launch: the one-pass rows (rowf < 0) go from the scratch into C.  A

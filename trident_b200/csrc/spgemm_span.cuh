@@ -552,7 +552,8 @@ constexpr int64_t kSpanWarpCols = 131072;
 constexpr int32_t kSpanWarpRow = 192;
 constexpr int32_t kSpanHalfRow = 4096;
 template <typename PT, typename VT>
-inline Tune span_tune(Tune t, int64_t ncols) {
+inline Tune span_tune(Tune t, int64_t ncols, bool addend) {
+  t.lane = addend ? 0 : kLaneSlots;  // lane rows take no addend
   if (ncols <= kSpanWarpCols && t.num[0] > kSpanWarpRow && t.num[1] >= t.num[0])
     t.num[0] = kSpanWarpRow;
   if (t.num[3] > kSpanHalfRow && t.num[2] <= kSpanHalfRow && ncols <= kRankMaxCols &&
@@ -624,7 +625,7 @@ inline int launch_numeric_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, 
                                PhaseArgs pa, int64_t ncols, const int64_t *cnt,
                                bool skip_empty, bool may_overlap) {
   TSPG_CUDA(ctx, launch_dense_cluster<PT, VT>(ctx, s, prods, pa));
-  const Tune tn = span_tune<PT, VT>(ctx->tune, ncols);
+  const Tune tn = span_tune<PT, VT>(ctx->tune, ncols, false);  // bounds only
   auto rows = [&](int c) { return cnt ? cnt[c] : int64_t(-1); };
   auto some = [&](int c) { return !skip_empty || rows(c) != 0; };
   const int64_t dense = cnt ? cnt[CLS_DENSE0] + cnt[CLS_DENSE1] + cnt[CLS_DENSE2] : -1;
@@ -673,6 +674,12 @@ inline int launch_numeric_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, 
     ctx->launches += 1;
     overlap = false;
   }
+  if (some(CLS_LANE)) {
+    TSPG_CUDA(ctx, launch_phase(overlap, ctx->num_sms, kOnepassThreads, kOnepassSmem, s,
+                                k_lanes<true, PT, VT>, prods, pa));
+    ctx->launches += 1;
+    overlap = may_overlap;
+  }
   if (some(CLS_G32) || (!(pa.skip >> CLS_G256 & 1u) && some(CLS_G256)) ||
       (!(pa.skip >> CLS_G128 & 1u) && some(CLS_G128))) {
     TSPG_CUDA(ctx, launch_phase(overlap, ctx->num_sms, kGroupThreads, kGroupDynSmem, s,
@@ -696,7 +703,8 @@ inline int set_smem_attr(int device) {
   };
   if (!raise(k_phase<PT, VT, false>, kDynSmem) || !raise(k_phase<PT, VT, true>, kDynSmem) ||
       !raise(k_groups<PT, VT, false>, kGroupDynSmem) ||
-      !raise(k_groups<PT, VT, true>, kGroupDynSmem) || !raise(k_onepass<PT, VT>, kOnepassSmem) ||
+      !raise(k_groups<PT, VT, true>, kGroupDynSmem) || !raise(k_lanes<false, PT, VT>, kOnepassSmem) ||
+      !raise(k_lanes<true, PT, VT>, kOnepassSmem) ||
       !raise(k_dense_rank<kRankThreads, 1, PT, VT>, kDynSmem) || !raise(k_dense_rank<512, 2, PT, VT>, kRank2Smem) ||
       !raise(k_span<128, false, PT, VT>, kSpanSmemMax) || !raise(k_span<256, false, PT, VT>, kSpanSmemMax) || !raise(k_span<512, false, PT, VT>, kSpanSmemMax) || !raise(k_span<128, true, PT, VT>, kSpanSmemMax) ||
       !raise(k_span<256, true, PT, VT>, kSpanSmemMax) ||
