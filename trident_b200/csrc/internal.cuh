@@ -340,10 +340,11 @@ __device__ __forceinline__ int64_t first_row(const PT *__restrict__ rp, int64_t 
   return lo;
 }
 
-// Rows of a window of 32 consecutive entries, one per lane (e ascending over
-// the lanes), r being the last row that starts at or before the window.  Lanes
-// search the next 32 row starts by shuffles; past those (runs of empty rows)
-// the next ones, then the offsets themselves.  r becomes lane 31's row.
+// Rows of a window of 32 consecutive entries, one per lane (lane l's entry e is
+// lane 0's + l), r being the last row that starts at or before the window.
+// Lanes search the next 32 row starts (relative to the window: 32 bits) by
+// shuffles; past those (runs of empty rows) the next ones, then the offsets
+// themselves.  r becomes lane 31's row.
 template <typename PT>
 __device__ __forceinline__ int64_t window_row(const PT *__restrict__ rp, int64_t m, int64_t base,
                                               int64_t &r, int64_t e, int lane) {
@@ -351,12 +352,13 @@ __device__ __forceinline__ int64_t window_row(const PT *__restrict__ rp, int64_t
   int64_t mine = r;
   bool open = true;  // this lane's row may lie past the starts seen so far
   for (int t = 0; t < 4; ++t) {
-    const int64_t nx = r + 1 + lane < m ? int64_t(__ldg(rp + r + 1 + lane)) - base : INT64_MAX;
+    const int64_t nx = r + 1 + lane < m ? int64_t(__ldg(rp + r + 1 + lane)) - base - (e - lane) : 32;
+    const int rel = nx < 32 ? (nx > 0 ? int(nx) : 0) : 32;  // starts at or before lane `rel`'s entry
     int j = 0;
 #pragma unroll
     for (int st = 16; st > 0; st >>= 1)
-      if (__shfl_sync(FULL, nx, j + st - 1) <= e) j += st;
-    if (__shfl_sync(FULL, nx, 31) <= e) j = 32;
+      if (__shfl_sync(FULL, rel, j + st - 1) <= lane) j += st;
+    if (__shfl_sync(FULL, rel, 31) <= lane) j = 32;
     if (open) mine = r + j;
     open = open && j == 32;
     if (!__any_sync(FULL, open)) break;
