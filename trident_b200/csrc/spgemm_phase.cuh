@@ -2171,6 +2171,17 @@ __device__ void lane_rows(const ProdDev<PT, VT> &P, const PhaseArgs &A, const Ro
     kn = __ldg(Aj + a0 + 1);
     an = __ldg(Ax + a0 + 1);
   }
+  int32_t c[U];
+  VT x[U];
+  auto fetch = [&](int64_t q, int64_t end, int32_t (&cc)[U], VT (&xx)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = q + u < end && !refused;
+      cc[u] = in ? __ldg(Bj + q + u) : -1;
+      xx[u] = in ? __ldg(Bx + q + u) : VT(0);
+    }
+  };
+  fetch(b0, b1, c, x);
   for (int t = 0; t < steps; ++t) {
     int64_t n0 = 0, n1 = 0;
     if (t + 1 < na) {
@@ -2183,14 +2194,13 @@ __device__ void lane_rows(const ProdDev<PT, VT> &P, const PhaseArgs &A, const Ro
       k2 = __ldg(Aj + a0 + t + 2);
       a2 = __ldg(Ax + a0 + t + 2);
     }
-    for (int64_t q = b0; __any_sync(FULL, q < b1); q += U) {
-      int32_t c[U];
-      VT x[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        c[u] = q + u < b1 ? __ldg(Bj + q + u) : -1;
-        x[u] = q + u < b1 ? __ldg(Bx + q + u) : VT(0);
-      }
+    for (int64_t q = b0;; q += U) {
+      // the next U entries' loads, of this B row or of the next one, go out
+      // before this step's products are added up
+      const bool more = __any_sync(FULL, q + U < b1);
+      int32_t cn[U];
+      VT xn[U];
+      fetch(more ? q + U : n0, more ? b1 : n1, cn, xn);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (c[u] >= 0 && !refused) {
@@ -2211,11 +2221,17 @@ __device__ void lane_rows(const ProdDev<PT, VT> &P, const PhaseArgs &A, const Ro
           }
         }
       }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        c[u] = cn[u];
+        x[u] = xn[u];
+      }
+      if (!more) break;
     }
     if (__all_sync(FULL, refused || t + 1 >= na)) break;
     av = an;
     b0 = n0;
-    b1 = refused ? n0 : n1;
+    b1 = n1;
     kn = k2;
     an = a2;
   }
