@@ -80,6 +80,20 @@ struct tspg_plan {
     }
     return TSPG_OK;
   }
+  // Give up the kept bitmaps (the numeric phase then walks those rows twice).
+  void drop_bits() {
+    for (void *p : {(void *)bits, (void *)slot}) {
+      for (int i = 0; i < nblocks; ++i) {
+        if (blocks[i] != p) continue;
+        ws_free(ctx, p, stream);
+        blocks[i] = blocks[--nblocks];
+        break;
+      }
+    }
+    bits = nullptr;
+    slot = nullptr;
+    nslots = 0;
+  }
   ~tspg_plan() {
     for (int i = nblocks - 1; i >= 0; --i) ws_free(ctx, blocks[i], stream);
   }
@@ -486,6 +500,13 @@ extern "C" int tspg_spgemm(tspg_ctx *ctx, void *stream, const tspg_csr *A,
   int st = TSPG_OK;
   if (C->rowptr_bits == 32 && nnz > INT32_MAX) st = TSPG_EOVERFLOW;
   if (st == TSPG_OK) st = ensure_out(C, nnz, A->val_bits / 8, (cudaStream_t)stream);
+  if (st == TSPG_ENOMEM && C->alloc && plan->nslots) {
+    // the output comes first: hand the kept bitmaps back to the device
+    plan->drop_bits();
+    cudaStreamSynchronize((cudaStream_t)stream);
+    cudaMemPoolTrimTo(ctx->pool, ctx->in_use);
+    st = ensure_out(C, nnz, A->val_bits / 8, (cudaStream_t)stream);
+  }
   if (st == TSPG_OK) {
     st = dispatch(plan->pt_bits, plan->vt_bits, [&](auto pt, auto vt) {
       using PT = std::remove_pointer_t<decltype(pt)>;

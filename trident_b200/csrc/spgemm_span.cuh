@@ -162,6 +162,19 @@ __device__ __forceinline__ void span_tile(const uint32_t *pre, const IX *bq, con
     cur = blk + __popc(__ballot_sync(FULL, lane < step && i2 < ne && pre[i2] <= t0)) - 1;
   }
   uint32_t nx = cur + 1 + lane < ne ? pre[cur + 1 + lane] : UINT32_MAX;
+  if (__shfl_sync(FULL, nx, 0) >= t0 + 128u) {  // one B row covers the tile
+    const IX q0 = bq[cur] + IX(t0 + lane);
+    const int32_t *__restrict__ bj = Bj + q0;
+    VT a = VT(0);
+    if constexpr (NUM) a = av[cur];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool in = t0 + 32u * u + lane < tot;
+      cc[u] = in ? __ldg(bj + 32 * u) : -1;
+      if constexpr (NUM) vv[u] = in ? a * __ldg(Bx + q0 + 32 * u) : VT(0);
+    }
+    return;
+  }
   // more than 32 entries start in the tile: reload them per window
   const bool again = __shfl_sync(FULL, nx, 31) <= t0 + 128u;
   VT xv[4];
@@ -213,6 +226,9 @@ __device__ __forceinline__ void span_row(const ProdDev<PT, VT> &P, const PhaseAr
   const int32_t *__restrict__ Bj = P.Bj;
   const VT *__restrict__ Bx = P.Bx;
   const bool reg = na <= NT && m.f <= int64_t(TILES) * TP * NW && !P.Ej;
+  // entries staged at a time: product numbers inside a stage are 32-bit, so a
+  // row of 2^31 products or more (B rows with repeated columns) takes one
+  const int64_t step = m.f < (int64_t(1) << 31) ? NT : 1;
   if (WIPE) {
     uint4 *b4 = (uint4 *)smem;
     for (int i = tid; i < nu8 * 8; i += NT) b4[i] = make_uint4(0, 0, 0, 0);
@@ -260,9 +276,8 @@ __device__ __forceinline__ void span_row(const ProdDev<PT, VT> &P, const PhaseAr
       for (int u = 0; u < 4; ++u)
         if (cc[t][u] >= 0 && mark(cc[t][u])) first |= 1u << (t * 4 + u);
   } else {
-    for (int64_t c0 = 0; c0 < na; c0 += NT) {
-      span_stage<NT, NUM, PT, VT>(P, a0 + c0, int(min(int64_t(NT), na - c0)), smem, L, sh, &ne,
-                                  &tot);
+    for (int64_t c0 = 0; c0 < na; c0 += step) {
+      span_stage<NT, NUM, PT, VT>(P, a0 + c0, int(min(step, na - c0)), smem, L, sh, &ne, &tot);
       for (uint32_t t0 = uint32_t(w) * TP; t0 < tot; t0 += uint32_t(NW * TILES) * TP) {
         tiles(std::false_type{}, t0);
 #pragma unroll
@@ -362,10 +377,9 @@ __device__ __forceinline__ void span_row(const ProdDev<PT, VT> &P, const PhaseAr
         keys[r] = col;
         atomicAdd(vals + r, v);
       };
-      for (int64_t c0 = 0; c0 < na; c0 += NT) {
-        if (na > NT)
-          span_stage<NT, NUM, PT, VT>(P, a0 + c0, int(min(int64_t(NT), na - c0)), smem, L, sh,
-                                      &ne, &tot);
+      for (int64_t c0 = 0; c0 < na; c0 += step) {
+        if (na > step)
+          span_stage<NT, NUM, PT, VT>(P, a0 + c0, int(min(step, na - c0)), smem, L, sh, &ne, &tot);
         for (uint32_t t0 = uint32_t(w) * TP; t0 < tot; t0 += uint32_t(NW * TILES) * TP) {
           tiles(std::bool_constant<NUM>{}, t0);
 #pragma unroll
