@@ -349,8 +349,8 @@ def run_ours(args, rank, world):
     bytes_c = csr_bytes(pm, nnz_c, rp_bits // 8)
     algo = bytes_p + bytes_a + bytes_c
     sym, num = statistics.mean(sym_ms), statistics.mean(num_ms)
-    dom_ms, dom_name = ((num, "numeric phase (k_dense_rank + k_phase + k_groups)") if num >= sym
-                        else (sym, "symbolic phase (k_phase + k_groups)"))
+    dom_ms, dom_name = ((num, "numeric phase (k_dense_rank + k_span + k_phase + k_groups)") if num >= sym
+                        else (sym, "symbolic phase (k_span + k_phase + k_groups)"))
     try:
         peak, peak_src = float(json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["hbm_gbs"]), "measured"
     except Exception:
@@ -731,7 +731,7 @@ def run_rap(args):
     try:
         prof = json.load(open(os.path.join(ROOT, "profiles", "traffic.json")))
         ent = prof.get(f"rap27pt_{n}^3", {}).get(
-            "A·P, both launches (k_groups + k_onepass, then the copy of the one-pass rows)")
+            "A·P, both launches (k_groups + k_lanes, then the copy of the one-pass rows)")
         if ent:
             ap_traffic = (int(ent["dram_bytes_per_launch"]), ent.get("source"))
     except Exception:
@@ -765,7 +765,7 @@ def run_rap(args):
         "RAP": {"ms": round(ms - ap_ms, 3), "symbolic_ms": round(rap_sym, 3), "numeric_ms": round(rap_num, 3),
                 "hbm_frac": round(brap / ((ms - ap_ms) * 1e-3) / 1e9 / peak, 4)},
         "roofline": {"bound": "hbm",
-                     "kernel": "A·P, both launches (k_groups + k_onepass, then the copy of the one-pass rows)",
+                     "kernel": "A·P, both launches (k_groups + k_lanes, then the copy of the one-pass rows)",
                      "achieved": round(bap / (ap_phases * 1e-3) / 1e9, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(bap / (ap_phases * 1e-3) / 1e9 / peak, 4), "traffic": ap_traffic[0],
                      "traffic_source": ap_traffic[1],

@@ -10,8 +10,10 @@
 //   cp[g]    int64  exclusive prefix of rowc over the flat row space
 //   list[]   uint64 rows binned by class, entry = (p << 40) | r
 //
-// Row classes (the same five for both phases, heaviest first so that the
-// persistent grid starts on the long rows):
+// Row classes (shared by both phases, heaviest first so that the persistent
+// grid starts on the long rows).  Where a bitmap of the column range leaves
+// room for two CTAs per SM, rows of every class but the shortest take the span
+// form instead of the one named here (spgemm_span.cuh):
 //   DENSE  (three sub-classes by product count, heaviest first) one CTA per
 //          row.  Symbolic: a bitmap of the whole column range in shared
 //          memory.  Numeric: the same bitmap, then a CTA scan that writes the
@@ -23,6 +25,8 @@
 //   G256   256-thread groups, named barriers.
 //   G128   128-thread groups.
 //   G32    one warp per row.
+//   LANE   one lane per row, 32 rows by a warp: numeric rows of at most 32
+//          outputs, and the one-pass rows of the symbolic launch.
 // Hash rows are sorted after accumulation by an in-place compaction into the
 // first half of the table and a stable LSD radix sort (bitonic below 65).
 #pragma once
@@ -109,13 +113,13 @@ __host__ __device__ inline int sym_class(int64_t f, int64_t n, const Tune &t) {
   return dense_sub(f);
 }
 // One-pass rows (plain products only, Sched::onepass set): rows of the
-// symbolic warp, 128- and 256-thread classes are multiplied whole by a warp
-// in the symbolic launch; their output waits in a scratch buffer for the
-// numeric launch, which copies it into C.  A row whose output bound
-// min(f, n) fits a 64-slot table is always finished there; a larger one is
-// finished only when it has fewer than kCappedCols columns (its 64-slot
-// attempt), else it is deferred to the two-pass path — so no row writes
-// more than kCappedCols scratch entries, and the scratch stays dense.
+// symbolic warp, 128- and 256-thread classes are multiplied whole in the
+// symbolic launch (k_lanes: a lane per row, or a warp per row where the 32
+// rows of a warp are uneven); their output waits in a scratch buffer for the
+// numeric launch, which copies it into C.  A row that turns out to hold more
+// columns than the form's table takes is deferred to the two-pass path — so
+// no row writes more than kCappedCols scratch entries, and the scratch stays
+// dense.
 constexpr int kCappedCols = 32;
 __host__ __device__ inline bool onepass_row(int64_t f, int64_t n, const Tune &t) {
   const int64_t fe = f < n ? f : n;
