@@ -54,6 +54,22 @@ def test_span_rows_fp32_wide_offsets(ctx, n):
                   A, B, tol=TOL32)
 
 
+@pytest.mark.parametrize("n", [64, 65, 16384, 16385, 32704, 32767, 32768, 32769])
+def test_warp_rows_over_the_whole_span(ctx, n):
+    # rows of 65 ... 190 products; first and last column, and columns on both
+    # sides of every unit boundary up to the slice's last unit
+    rng = np.random.default_rng(n)
+    edges = np.unique(np.clip(np.concatenate([np.arange(64, n + 1, 64), np.arange(63, n + 1, 64), [0, n - 1]]), 0, n - 1))
+    lens = np.minimum(rng.integers(4, 24, size=600), edges.size)
+    rp = np.zeros(601, np.int64)
+    rp[1:] = np.cumsum(lens)
+    col = np.concatenate([np.sort(rng.choice(edges, size=k, replace=False)) for k in lens]).astype(np.int32)
+    B = HostCSR(600, n, rp, col, rng.uniform(-1, 1, col.size))
+    A = _rows(rng.integers(4, 9, size=3000), 600, rng)
+    dA, dB = A.to_device(rowptr_bits=32), B.to_device(rowptr_bits=32)
+    check_product(ops.spgemm(ctx, dA, dB), A, B, tol=TOL64)
+
+
 def test_span_rows_with_an_addend(ctx):
     A, B = _pair(4097, False, seed=11)
     E = _rows(np.tile([0, 300, 1500], 21), 4097, np.random.default_rng(3))

@@ -1183,19 +1183,30 @@ __device__ void num_esc_row(const ProdDev<PT, VT> *prods, const PhaseArgs &A, co
   prof_sub_g(A, 13, tp, lane == 0);
 }
 
-// Column bitmap with a uint16 counter per 128 columns (span rows): o is a
-// column less the bitmap's first.  span_mark sets the column's bit and, the
+// Column bitmap with a uint16 counter per unit of 2^U columns (span rows): o is
+// a column less the bitmap's first.  span_mark sets the column's bit and, the
 // first time, counts it in its unit (true then); once the counters hold the
-// units' rank bases, span_rank is the column's rank.
+// units' rank bases, span_rank is the column's rank.  Units of 128 columns where
+// the room of a CTA bounds the rows in flight; 64 in a warp's slice, which has
+// room for the counters, and where the rank's instructions are the row's time
+// (27-point stencil on 63^3 squared: 1.70 -> 1.66 ms).
+template <int U = 7>
 __device__ __forceinline__ bool span_mark(uint32_t *bm, uint32_t *uc, uint32_t o) {
   uint32_t *x = bm + (o >> 5);
   const uint32_t bit = 1u << (o & 31);
   if (*(volatile uint32_t *)x & bit) return false;
   if (atomicOr(x, bit) & bit) return false;
-  atomicAdd(uc + (o >> 8), 1u << ((o >> 3) & 16));
+  atomicAdd(uc + (o >> (U + 1)), 1u << ((o >> (U - 4)) & 16));
   return true;
 }
+template <int U = 7>
 __device__ __forceinline__ int span_rank(const uint32_t *bm, const uint32_t *uc, uint32_t o) {
+  if constexpr (U == 6) {
+    const uint2 x = ((const uint2 *)bm)[o >> 6];
+    const uint32_t below = (1u << (o & 31)) - 1u;
+    return ((const uint16_t *)uc)[o >> 6] + __popc(o & 32 ? x.x : x.x & below) +
+           __popc(o & 32 ? x.y & below : 0u);
+  }
   const uint4 x = ((const uint4 *)bm)[o >> 7];
   const uint32_t below = (1u << (o & 31)) - 1u;
   const int wi = (o >> 5) & 3;
@@ -1218,7 +1229,7 @@ __device__ __forceinline__ int span_rank(const uint32_t *bm, const uint32_t *uc,
 constexpr int kSpanWarpBits = 32768;
 constexpr int64_t kSpanWarpMin = 64;  // products; shorter rows sort in registers
 constexpr int64_t kSeqRow = 16;  // half of a warp's lanes busy in a B row
-constexpr int kSpanWarpBytes = kSpanWarpBits / 8 + kSpanWarpBits / 64 + int(kNumLim32) * 12;
+constexpr int kSpanWarpBytes = kSpanWarpBits / 8 + kSpanWarpBits / 32 + int(kNumLim32) * 12;
 static_assert(kSpanWarpBytes <= kTableSmem / (kGroupThreads / 32), "warp slice");
 
 // False (nothing done) when the row's span does not fit.
@@ -1247,37 +1258,38 @@ __device__ bool num_span_warp_row(const ProdDev<PT, VT> *prods, const PhaseArgs 
   }
   long long tp = clock64();
   uint32_t *bm = (uint32_t *)slice, *uc = bm + kSpanWarpBits / 32;
-  VT *vals = (VT *)(uc + kSpanWarpBits / 256);
+  VT *vals = (VT *)(uc + kSpanWarpBits / 128);
   int32_t *keys = (int32_t *)(vals + kNumLim32);
-  const int units = int((width + 127) >> 7), nu8 = (units + 7) >> 3;
-  for (int i = lane; i < nu8 * 8; i += 32) ((uint4 *)bm)[i] = make_uint4(0, 0, 0, 0);
+  const int units = int((width + 63) >> 6), nu8 = (units + 7) >> 3;
+  for (int i = lane; i < nu8 * 4; i += 32) ((uint4 *)bm)[i] = make_uint4(0, 0, 0, 0);
   for (int i = lane; i < nu8; i += 32) ((uint4 *)uc)[i] = make_uint4(0, 0, 0, 0);
   for (int64_t e = lane; e < m.c; e += 32) vals[e] = VT(0);
   __syncwarp();
   prof_sub_g(A, 9, tp, lane == 0);
   const bool seq = P.b_strict && m.f >= kSeqRow * na;
-  auto mark = [&](int32_t col, VT) { span_mark(bm, uc, uint32_t(col) - base); };
+  auto mark = [&](int32_t col, VT) { span_mark<6>(bm, uc, uint32_t(col) - base); };
   if (seq) for_products_rows<false, PT, VT>(P.Aj, P.Ax, P.Bp, P.Bj, P.Bx, m.a0, m.a1, lane, mark);
   else
     for_products_flat<32, false, PT, VT>(P.Aj, P.Ax, P.Bp, P.Bj, P.Bx, m.a0, m.a1, lane, 0, nullptr,
                                          nullptr, mark);
   __syncwarp();
   prof_sub_g(A, 10, tp, lane == 0);
-  int total;
-  {  // unit counts to unit bases: lane l owns units 8l ... 8l + 7
-    uint4 x = lane < nu8 ? ((uint4 *)uc)[lane] : make_uint4(0, 0, 0, 0);
+  int total = 0;
+  for (int g = lane; g < ((nu8 + 31) & ~31); g += 32) {
+    // unit counts to unit bases: lane l owns units 8l ... 8l + 7 of each 256
+    uint4 x = g < nu8 ? ((uint4 *)uc)[g] : make_uint4(0, 0, 0, 0);
     uint32_t *h = (uint32_t *)&x;
     const uint32_t y = x.x + x.y + x.z + x.w;
     const int s = int((y & 0xffffu) + (y >> 16)), inc = warp_scan_incl(s);
-    total = __shfl_sync(FULL, inc, 31);
-    uint32_t run = uint32_t(inc - s);
+    uint32_t run = uint32_t(total + inc - s);
+    total += __shfl_sync(FULL, inc, 31);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const uint32_t lo = h[k] & 0xffffu, hi = h[k] >> 16;
       h[k] = run | ((run + lo) << 16);
       run += lo + hi;
     }
-    if (lane < nu8) ((uint4 *)uc)[lane] = x;
+    if (g < nu8) ((uint4 *)uc)[g] = x;
   }
   __syncwarp();
   prof_sub_g(A, 11, tp, lane == 0);
@@ -1289,14 +1301,14 @@ __device__ bool num_span_warp_row(const ProdDev<PT, VT> *prods, const PhaseArgs 
   if (seq) {
     for_products_rows<true, PT, VT>(P.Aj, P.Ax, P.Bp, P.Bj, P.Bx, m.a0, m.a1, lane,
                                     [&](int32_t col, VT v) {
-                                      const int r = span_rank(bm, uc, uint32_t(col) - base);
+                                      const int r = span_rank<6>(bm, uc, uint32_t(col) - base);
                                       keys[r] = col;
                                       vals[r] += v;
                                     });
   } else {
     for_products_flat<32, true, PT, VT>(P.Aj, P.Ax, P.Bp, P.Bj, P.Bx, m.a0, m.a1, lane, 0, nullptr,
                                         nullptr, [&](int32_t col, VT v) {
-                                          const int r = span_rank(bm, uc, uint32_t(col) - base);
+                                          const int r = span_rank<6>(bm, uc, uint32_t(col) - base);
                                           keys[r] = col;
                                           atomicAdd(vals + r, v);
                                         });
