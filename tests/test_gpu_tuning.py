@@ -95,3 +95,56 @@ def test_plan_numeric_with_dense_rows(tctx):
         check_product(plan.numeric(dR2, dR2), R, R)
     finally:
         plan.close()
+
+
+def _poisoned_numeric(plan, A, B):
+    """The numeric call of a plan into arrays filled with values no result has."""
+    import ctypes as C
+
+    import torch
+
+    from trident_b200._lib import TspgCsrOut, check, lib
+    from trident_b200.csr import DeviceCSR
+    m, n = plan.shape
+    rp = torch.full((m + 1,), -3, dtype=torch.int64, device="cuda")
+    col = torch.full((plan.c_nnz,), -7, dtype=torch.int32, device="cuda")
+    val = torch.full((plan.c_nnz,), float("nan"), dtype=torch.float64, device="cuda")
+    o = TspgCsrOut()
+    o.nrows, o.ncols, o.rowptr, o.rowptr_bits, o.val_bits = m, n, rp.data_ptr(), 64, 64
+    o.col, o.val, o.capacity = col.data_ptr(), val.data_ptr(), plan.c_nnz
+    a, b = A.abi(), B.abi()
+    check(lib.tspg_spgemm_numeric(plan.ctx.h, torch.cuda.current_stream().cuda_stream, plan.h, C.byref(a),
+                                  C.byref(b), C.byref(o)), "tspg_spgemm_numeric")
+    return DeviceCSR(m, n, rp, col, val, nnz=plan.c_nnz)
+
+
+NARROW = {"num_lim": [64, 256, 512, 2048]}
+WINDOW = {"num_lim": [64, 256, 512, 2048], "dense_win_log2": 10, "dense_win_fill_log2": 12}
+PAIRS = [({}, NARROW), (NARROW, {}), ({}, WINDOW), (WINDOW, {}), (WINDOW, dict(WINDOW, dense_win_cluster=2)),
+         (dict(WINDOW, dense_win_cluster=2), {})]
+
+
+@pytest.mark.parametrize("made,now", PAIRS)
+def test_plan_keeps_the_tuning_it_was_made_with(tctx, made, now):
+    # rows of every class; a tuning set after the symbolic call holds for later
+    # calls, the plan's rows were classed with the one before it
+    import numpy as np
+
+    from trident_b200.csr import HostCSR
+    rng = np.random.default_rng(31)
+
+    def rows(lens, n):
+        rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+        col = np.concatenate([np.sort(rng.choice(n, size=k, replace=False)) for k in lens]).astype(np.int32)
+        return HostCSR(len(lens), n, rp, col, rng.uniform(-1, 1, col.size))
+
+    B = rows(np.full(200, 400), 30000)
+    A = rows(rng.choice([1, 2, 4, 8, 12, 20, 60], size=300), 200)
+    dA, dB = A.to_device(), B.to_device()
+    tctx.set_tuning(dict(tune.default_tuning(), **made))
+    plan = ops.Plan(tctx, dA, dB)
+    tctx.set_tuning(dict(tune.default_tuning(), **now))
+    for _ in range(2):
+        check_product(_poisoned_numeric(plan, dA, dB), A, B)
+    plan.close()
+    check_product(ops.spgemm(tctx, dA, dB), A, B)

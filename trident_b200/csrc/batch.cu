@@ -319,6 +319,7 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
 
   int64_t ncols = 0;
   for (int p = 0; p < nprod; ++p) ncols = std::max(ncols, b->B[p].ncols);
+  const Tune tune = span_tune<PT, VT>(b->tune, ncols, false);
 
   // ---- graph 1: symbolic
   if (rebuild) {
@@ -326,7 +327,6 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
     cudaGraph_t g;
     TSPG_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(b->sched, 0, 2 * sizeof(Sched), s);
-    const Tune tune = span_tune<PT, VT>(ctx->tune, ncols, false);
     const bool check = !(flags & TSPG_F_B_SORTED) && b->RB > 0 && needs_sorted(tune, ncols);
     k_set_tune<<<1, 32, 0, s>>>(b->sched, 2, tune);
     cudaMemsetAsync(b->cp, 0, sizeof(int64_t), s);
@@ -429,7 +429,8 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
                    b->curbuf, b->cur_stride, errw, ctx->d_prof ? ctx->d_prof + kProfPerPhase : nullptr};
       phase_mark(ctx, 1, 0, s);
       const int64_t before = ctx->launches;
-      const int st = launch_numeric_rows<PT, VT>(ctx, s, prods, pa, ncols, nullptr, false, R < kFuseRows);
+      const int st = launch_numeric_rows<PT, VT>(ctx, s, prods, pa, ncols, tune, nullptr, false,
+                                                     R < kFuseRows);
       row_kernels = int(ctx->launches - before);
       ctx->launches = before;  // counted at each replay
       if (st != TSPG_OK) {

@@ -32,6 +32,7 @@ struct tspg_plan {
   int64_t mults = 0;
   int64_t max_a_row = 0;
   int64_t ncnt[NCLS] = {};  // numeric rows per class
+  Tune tune{};                  // row binning of the symbolic call
   bool strict_checked = false;  // ProdDev::b_strict is known
   void *prods = nullptr;
   int64_t *base = nullptr;
@@ -137,7 +138,7 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
                          const tspg_csr *B, int flags, tspg_plan *P) {
   TSPG_TRY(set_smem_attr<PT, VT>(ctx->device));
   const int64_t m = A->nrows, n = B->ncols, k = A->ncols;
-  const Tune tune = span_tune<PT, VT>(ctx->tune, n, P->E.col && P->E.nnz > 0);
+  const Tune tune = P->tune = span_tune<PT, VT>(ctx->tune, n, P->E.col && P->E.nnz > 0);
   P->m = m;
   P->n = n;
   P->k = k;
@@ -323,7 +324,8 @@ static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P, const tspg_
     pa.slot_words = P->slot_words;
   }
   phase_mark(ctx, 1, 0, s);
-  TSPG_TRY((launch_numeric_rows<PT, VT>(ctx, s, prods, pa, P->n, P->ncnt, m < kFuseRows, true)));
+  TSPG_TRY((launch_numeric_rows<PT, VT>(ctx, s, prods, pa, P->n, P->tune, P->ncnt, m < kFuseRows,
+                                        true)));
   if (P->onepass)
     k_onepass_copy<PT, VT><<<grid_for(m * 32, 256, ctx->num_sms * 16), 256, 0, s>>>(
         prods, P->rowf, P->rowc, P->cp, P->oj, (const VT *)P->ox, m);

@@ -328,11 +328,11 @@ int cluster_slots(int device, int K) {
 
 // Launch the cluster kernel over the column-window rows of a numeric phase
 // (before k_phase, which then leaves those rows alone).  Returns the CUDA
-// status of the launch; does nothing when the tuning asks for no cluster.
+// status of the launch; does nothing when the run's tuning (K CTAs) asks for
+// no cluster.
 template <typename PT, typename VT>
 cudaError_t launch_dense_cluster(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, VT> *prods,
-                                 const PhaseArgs &pa) {
-  const int K = ctx->tune.cluster;
+                                 const PhaseArgs &pa, int K) {
   if (K == 0) return cudaSuccess;
   const int slots = cluster_slots<PT, VT>(ctx->device, K);
   if (slots <= 0) return cudaErrorInvalidConfiguration;

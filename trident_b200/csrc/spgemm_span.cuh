@@ -631,15 +631,17 @@ inline cudaError_t launch_span_class(tspg_ctx *ctx, cudaStream_t s,
 }
 
 // The persistent kernels of a numeric phase whose products have at most
-// `ncols` columns; cnt: rows per class when the host knows them (else null).
+// `ncols` columns; tn: the run's row binning (span_tune), the one in its Sched
+// records, by which the rows were classed: a kept plan runs with the tuning of
+// its symbolic call, whatever the context's is by now.  cnt: rows per class
+// when the host knows them (else null).
 // skip_empty: no kernel is launched for an empty class (small products, where
 // a launch counts).
 template <typename PT, typename VT>
 inline int launch_numeric_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, VT> *prods,
-                               PhaseArgs pa, int64_t ncols, const int64_t *cnt,
+                               PhaseArgs pa, int64_t ncols, const Tune &tn, const int64_t *cnt,
                                bool skip_empty, bool may_overlap) {
-  TSPG_CUDA(ctx, launch_dense_cluster<PT, VT>(ctx, s, prods, pa));
-  const Tune tn = span_tune<PT, VT>(ctx->tune, ncols, false);  // bounds only
+  TSPG_CUDA(ctx, launch_dense_cluster<PT, VT>(ctx, s, prods, pa, tn.cluster));
   auto rows = [&](int c) { return cnt ? cnt[c] : int64_t(-1); };
   auto some = [&](int c) { return !skip_empty || rows(c) != 0; };
   const int64_t dense = cnt ? cnt[CLS_DENSE0] + cnt[CLS_DENSE1] + cnt[CLS_DENSE2] : -1;
