@@ -254,7 +254,9 @@ int tspg_plan_destroy(tspg_plan *plan);
  * "first product" case, KokkosWrap.hpp:334-338); then C_out = A·B.  Either
  * one SpGEMM in which C_in's entries join their rows as products with
  * coefficient 1, or the product followed by tspg_spadd (flags
- * TSPG_F_ACC_FUSE / TSPG_F_ACC_SPLIT; by default by size).  C_out's arrays
+ * TSPG_F_ACC_FUSE / TSPG_F_ACC_SPLIT; by default by size; the first in any
+ * case when a row of C_in is unsorted or repeats a column, which the merge
+ * finds while it counts).  C_out's arrays
  * must not overlap C_in's. */
 int tspg_spgemm_acc(tspg_ctx *ctx, void *stream, const tspg_csr *A,
                     const tspg_csr *B, const tspg_csr *C_in,
@@ -292,7 +294,8 @@ int tspg_coo_to_csx(tspg_ctx *ctx, void *stream, int64_t nrows, int64_t ncols,
  * tspg_spadd — C = A + B, union pattern, alpha = beta = 1.  Replaces
  * cusparse_spgeam (include/cusparse_helpers.cuh:799-905) and
  * LocalMatrix::spadd (include/KokkosWrap.hpp:394-439).  Rows of A and B must
- * be sorted and duplicate-free.  Synchronises `stream` once. */
+ * be sorted and duplicate-free: TSPG_EUNSORTED, with nothing written, when a
+ * row's columns descend.  Synchronises `stream` once. */
 int tspg_spadd(tspg_ctx *ctx, void *stream, const tspg_csr *A,
                const tspg_csr *B, tspg_csr_out *C);
 

@@ -9,7 +9,8 @@ import torch
 import oracle
 from helpers import check_product, check_sum, random_csr
 from trident_b200 import ops, workloads
-from trident_b200._lib import TSPG_COLS, TSPG_F_ACC_FUSE, TSPG_F_ACC_SPLIT, TSPG_ROWS
+from trident_b200._lib import (TSPG_COLS, TSPG_EUNSORTED, TSPG_F_ACC_FUSE, TSPG_F_ACC_SPLIT, TSPG_ROWS,
+                               TspgError)
 from trident_b200.csr import HostCSR
 
 pytestmark = pytest.mark.gpu
@@ -255,3 +256,57 @@ def test_spadd_tile_edges(ctx, la, lb, n):
     check_sum(ops.spadd(ctx, A.to_device(), Z.to_device()), A, Z)
     check_sum(ops.spadd(ctx, Z.to_device(), A.to_device()), Z, A)
     check_sum(ops.spadd(ctx, A.to_device(), A.to_device()), A, A)
+
+
+def _canonical(M):
+    """Rows sorted, repeated columns summed."""
+    d = np.zeros((M.nrows, M.ncols))
+    s = np.zeros((M.nrows, M.ncols), bool)
+    r = np.repeat(np.arange(M.nrows), np.diff(M.rowptr))
+    np.add.at(d, (r, M.col), M.val)
+    s[r, M.col] = True
+    rp = np.concatenate([[0], np.cumsum(s.sum(1))]).astype(np.int64)
+    rr, cc = np.nonzero(s)
+    return HostCSR(M.nrows, M.ncols, rp, cc.astype(np.int32), d[rr, cc])
+
+
+@pytest.mark.parametrize("la,lb", [([3000], [6000]), ([6000, 40, 0], [3000, 50, 20]), ([2, 900, 900], [900, 1, 900])])
+def test_spadd_refuses_rows_that_descend(ctx, la, lb):
+    # cuts of such rows need not be in order: no tile may follow one
+    n = 7000
+    A, B = _sorted_rows(la, n, 5), _sorted_rows(lb, n, 6)
+    rng = np.random.default_rng(8)
+    U = HostCSR(B.nrows, n, B.rowptr, B.col.copy(), B.val)
+    for r in range(U.nrows):
+        U.col[U.rowptr[r]:U.rowptr[r + 1]] = rng.permutation(U.col[U.rowptr[r]:U.rowptr[r + 1]])
+    for X, Y in ((A, U), (U, A), (U, U)):
+        with pytest.raises(TspgError) as e:
+            ops.spadd(ctx, X.to_device(), Y.to_device())
+        assert e.value.status == TSPG_EUNSORTED
+    # one swapped pair of neighbours anywhere, a tile's first and last entry among them
+    for at in [0, 1, 1790, 1791, 1792, 2998]:
+        if at + 1 < A.rowptr[1]:
+            V = HostCSR(A.nrows, n, A.rowptr, A.col.copy(), A.val)
+            V.col[[at, at + 1]] = V.col[[at + 1, at]]
+            Z = _sorted_rows([0] * len(la), n, 3)
+            for X, Y in ((V, B), (B, V), (V, Z), (Z, V)):
+                with pytest.raises(TspgError) as e:
+                    ops.spadd(ctx, X.to_device(), Y.to_device())
+                assert e.value.status == TSPG_EUNSORTED
+    check_sum(ops.spadd(ctx, A.to_device(), B.to_device()), A, B)
+
+
+@pytest.mark.parametrize("dup", [False, True])
+@pytest.mark.parametrize("flags", [0, TSPG_F_ACC_SPLIT])
+def test_accumulator_in_any_order(ctx, dup, flags):
+    # a C_in larger than A and B, which the merge would take, with unsorted rows
+    # or repeated columns
+    A = random_csr(200, 150, per_row=3, seed=1)
+    B = random_csr(150, 900, per_row=4, seed=2)
+    E = random_csr(200, 900, per_row=60, seed=3, sort=dup, dup=dup)
+    if dup:  # sorted rows that repeat columns
+        for r in range(E.nrows):
+            E.col[E.rowptr[r]:E.rowptr[r + 1]].sort()
+    C = ops.sp_mma(ctx, A.to_device(), B.to_device(), E.to_device(), flags=flags)
+    rp, cj, cx, _ = oracle.spgemm(A, B)
+    check_sum(C, HostCSR(A.nrows, B.ncols, rp, cj, cx), _canonical(E))

@@ -155,6 +155,10 @@ inline std::pair<T **, size_t> part(T **p, int64_t count) {
   return {p, size_t(count)};
 }
 
+// tspg_spadd (spadd.cu); strict: rows with repeated columns are refused, too.
+int spadd_entry(tspg_ctx *ctx, void *stream, const tspg_csr *A, const tspg_csr *B, tspg_csr_out *C,
+                bool strict);
+
 inline int check_csr(const tspg_csr *M) {
   if (!M) return TSPG_EINVAL;
   if (M->nrows < 0 || M->ncols < 0 || M->nnz < 0) return TSPG_EINVAL;

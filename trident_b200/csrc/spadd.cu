@@ -82,28 +82,45 @@ __global__ void __launch_bounds__(128)
   cuts[t] = c;
 }
 
-// One tile: WRITE = false leaves its number of output entries in rowc[tile];
-// WRITE = true writes them from off[tile] on, and the offsets of the rows that
-// start in the tile.  A column in both rows leaves with A's entry (the two
+// One tile: WRITE = false leaves its number of output entries in tilec[tile]
+// and checks the order of the rows; WRITE = true writes them from off[tile] on,
+// and the offsets of the rows that start in the tile.  A column in both rows leaves with A's entry (the two
 // values added); B's entry of the pair is a "dup" and leaves nothing, so entry
 // x of the tile goes to slot x - (dups before x).
+//
+// The order check (order[0] = 1: a row descends, order[1] = 1: a row holds a
+// column twice): a cut inside a row that is not sorted may lie before the cut
+// it follows, so a tile with a negative share of A or B is left alone.  With
+// both shares at or above 0 every index stays inside the tile, whatever the
+// columns: the cursors start inside their row and move by one entry a step.
+// Each entry is compared with the one before it in its row by the thread that
+// merges it; that no entry is passed over is checked by comparing every
+// thread's end with the next one's start (in sorted rows they agree).
 template <bool WRITE, typename PTA, typename PTB, typename VT>
 __global__ void __launch_bounds__(kMergeThreads)
     k_merge_tiles(int64_t m, const PTA *__restrict__ Ap, const int32_t *__restrict__ Aj,
                   const VT *__restrict__ Ax, const PTB *__restrict__ Bp,
                   const int32_t *__restrict__ Bj, const VT *__restrict__ Bx, int64_t ntiles,
-                  const MergeCut *__restrict__ cuts, int32_t *tilec, const int64_t *off, void *Cp,
-                  int cp_bits, int32_t *Cj, VT *Cx) {
+                  const MergeCut *__restrict__ cuts, int32_t *tilec, volatile int64_t *order,
+                  const int64_t *off, void *Cp, int cp_bits, int32_t *Cj, VT *Cx) {
   __shared__ VT sv[WRITE ? kMergeTile + 2 : 1];       // A's values, then B's, one more of B
   __shared__ int32_t sc[kMergeTile + 2];              // one column of A before, A's, B's, one of B
   __shared__ uint16_t sea[kMergeRows], seb[kMergeRows];  // row ends in the tile
-  __shared__ uint16_t sdup[kMergeThreads + 1];        // dups before a thread's entries
+  __shared__ uint16_t sdup[kMergeThreads + 1];        // dups before a thread's entries; counting: A's before them
   __shared__ uint8_t sbit[kMergeThreads + 1];         // a thread's dups, bit per entry
   __shared__ int wsum[kMergeThreads / 32];
+  __shared__ int32_t sb0;  // one column of B before
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int64_t ab = int64_t(Ap[0]), bb = int64_t(Bp[0]);
   const MergeCut c0 = cuts[blockIdx.x], c1 = cuts[blockIdx.x + 1];
   const int nA = int(c1.i - c0.i), nB = int(c1.j - c0.j), n = nA + nB;
+  if (!WRITE && (nA < 0 || nB < 0)) {  // uniform
+    if (tid == 0) {
+      tilec[blockIdx.x] = 0;
+      order[0] = 1;
+    }
+    return;
+  }
   const int32_t *__restrict__ aj = Aj + ab + c0.i;
   const int32_t *__restrict__ bj = Bj + bb + c0.j;
   const int64_t rl = c1.row < m ? c1.row : m - 1;  // the last row with entries here, or one after
@@ -136,6 +153,10 @@ __global__ void __launch_bounds__(kMergeThreads)
     // its first), B's entry after it (same row as its last)
     const int64_t a0 = int64_t(Ap[c0.row]) - ab;
     sc[0] = c0.row < m && c0.i > a0 ? __ldg(aj - 1) : -1;
+    if (!WRITE) {
+      const int64_t b0 = int64_t(Bp[c0.row]) - bb;
+      sb0 = c0.row < m && c0.j > b0 ? __ldg(bj - 1) : -1;
+    }
     int32_t after = -1;
     if (c1.row < m && int64_t(Ap[c1.row]) - ab + int64_t(Bp[c1.row]) - bb < c1.i + c1.j &&
         c1.j < int64_t(Bp[c1.row + 1]) - bb) {
@@ -165,6 +186,9 @@ __global__ void __launch_bounds__(kMergeThreads)
   int32_t col[kMergePer];
   VT val[kMergePer];
   unsigned dups = 0;
+  int i = nA;
+  bool down = false, twice = false;
+  if (!WRITE && x0 >= n) sdup[tid] = uint16_t(nA);
   if (x0 < n) {
     int64_t lo = 0, hi = R - 1;  // the first row that ends past x0
     while (lo < hi) {
@@ -180,11 +204,14 @@ __global__ void __launch_bounds__(kMergeThreads)
       const int mid = (x + y) >> 1;
       if (sa[as + mid] <= sb[bs + q - 1 - mid]) x = mid + 1; else y = mid;
     }
-    int i = as + x, j = bs + q - x;
+    i = as + x;
+    int j = bs + q - x;
+    if (!WRITE) sdup[tid] = uint16_t(i);
     // columns at the cursors (INT32_MAX past the row's end) and of the A entry
     // before i (-1 when that is not in this row)
     int32_t ca = i < ae ? sa[i] : INT32_MAX, cb = j < be ? sb[j] : INT32_MAX;
     int32_t pa = i > as ? sa[i - 1] : k == 0 && i == 0 ? sc[0] : -1;
+    int32_t pb = WRITE ? -1 : j > bs ? sb[j - 1] : k == 0 && j == 0 ? sb0 : -1;
 #pragma unroll
     for (int t = 0; t < kMergePer; ++t) {
       if (x0 + t < n) {
@@ -194,7 +221,7 @@ __global__ void __launch_bounds__(kMergeThreads)
           be = eb(k);
           ca = i < ae ? sa[i] : INT32_MAX;
           cb = j < be ? sb[j] : INT32_MAX;
-          pa = -1;
+          pa = pb = -1;
         }
         if (ca <= cb) {  // (an exhausted A row has ca = INT32_MAX > any column)
           col[t] = ca;
@@ -203,6 +230,9 @@ __global__ void __launch_bounds__(kMergeThreads)
             const bool pair = cb == ca || (j == nB && i == nA - 1 && sb[nB] == ca);
             val[t] = sv[i];
             if (pair) val[t] += sv[nA + j];
+          } else {
+            down |= pa > ca;
+            twice |= pa == ca;
           }
           pa = ca;
           ++i;
@@ -210,7 +240,13 @@ __global__ void __launch_bounds__(kMergeThreads)
         } else {
           col[t] = cb;
           if (cb == pa) dups |= 1u << t;
-          if (WRITE) val[t] = sv[nA + j];
+          if (WRITE) {
+            val[t] = sv[nA + j];
+          } else {
+            down |= pb > cb;
+            twice |= pb == cb;
+            pb = cb;
+          }
           ++j;
           cb = j < be ? sb[j] : INT32_MAX;
         }
@@ -221,7 +257,12 @@ __global__ void __launch_bounds__(kMergeThreads)
   const int mine = __popc(dups);
   const int inc = warp_scan_incl(mine);
   if (lane == 31) wsum[w] = inc;
+  if (!WRITE && tid == 0) sdup[kMergeThreads] = uint16_t(nA);
   __syncthreads();
+  if (!WRITE) {
+    if (down || i != sdup[tid + 1]) order[0] = 1;
+    if (twice) order[1] = 1;
+  }
   int before = inc - mine, all = 0;
 #pragma unroll
   for (int v = 0; v < kMergeThreads / 32; ++v) {
@@ -270,9 +311,10 @@ __global__ void __launch_bounds__(kMergeThreads)
   }
 }
 
+// strict: rows with repeated columns are refused, too.
 template <typename PTA, typename PTB, typename VT>
 static int spadd_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
-                      const tspg_csr *B, tspg_csr_out *C) {
+                      const tspg_csr *B, tspg_csr_out *C, bool strict) {
   const int64_t m = A->nrows, total = A->nnz + B->nnz;
   if (m == 0 || total == 0) {
     C->nnz = 0;
@@ -292,15 +334,17 @@ static int spadd_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
   const PTB *Bp = (const PTB *)B->rowptr;
   k_merge_cuts<PTA, PTB><<<unsigned((ntiles + 128) / 128), 128, 0, s>>>(m, Ap, A->col, Bp, B->col,
                                                                        ntiles, cuts, rec);
+  int64_t *h = ctx->h_words;  // [0] nnz(C), [1] and [2] the order check
+  h[1] = h[2] = 0;
   k_merge_tiles<false, PTA, PTB, VT><<<unsigned(ntiles), kMergeThreads, 0, s>>>(
-      m, Ap, A->col, nullptr, Bp, B->col, nullptr, ntiles, cuts, tilec, nullptr, nullptr, 0, nullptr,
-      nullptr);
+      m, Ap, A->col, nullptr, Bp, B->col, nullptr, ntiles, cuts, tilec, h + 1, nullptr, nullptr, 0,
+      nullptr, nullptr);
   ctx->launches += 2;
-  int64_t *h = ctx->h_words;
   launch_scan(ctx, s, tilec, ntiles, partial, off, rec, nullptr, HostWords(), h);
   TSPG_CUDA(ctx, cudaGetLastError());
   TSPG_CUDA(ctx, cudaStreamSynchronize(s));
   const int64_t nnz = h[0];
+  if (h[1] || (strict && h[2])) return TSPG_EUNSORTED;
   if (C->rowptr_bits == 32 && nnz > INT32_MAX) return TSPG_EOVERFLOW;
   C->nnz = nnz;
   if (C->capacity < nnz) {
@@ -313,19 +357,15 @@ static int spadd_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
     C->capacity = nnz;
   }
   k_merge_tiles<true, PTA, PTB, VT><<<unsigned(ntiles), kMergeThreads, 0, s>>>(
-      m, Ap, A->col, (const VT *)A->val, Bp, B->col, (const VT *)B->val, ntiles, cuts, nullptr, off,
+      m, Ap, A->col, (const VT *)A->val, Bp, B->col, (const VT *)B->val, ntiles, cuts, nullptr, nullptr, off,
       C->rowptr, C->rowptr_bits, C->col, (VT *)C->val);
   ctx->launches += 1;
   TSPG_CUDA(ctx, cudaGetLastError());
   return TSPG_OK;
 }
 
-}  // namespace tspg
-
-using namespace tspg;
-
-extern "C" int tspg_spadd(tspg_ctx *ctx, void *stream, const tspg_csr *A,
-                          const tspg_csr *B, tspg_csr_out *C) {
+int spadd_entry(tspg_ctx *ctx, void *stream, const tspg_csr *A, const tspg_csr *B, tspg_csr_out *C,
+                bool strict) {
   if (!ctx || !C) return TSPG_EINVAL;
   TSPG_TRY(check_csr(A));
   TSPG_TRY(check_csr(B));
@@ -338,14 +378,21 @@ extern "C" int tspg_spadd(tspg_ctx *ctx, void *stream, const tspg_csr *A,
   TSPG_CUDA(ctx, cudaSetDevice(ctx->device));
   const int a = A->rowptr_bits, b = B->rowptr_bits;
   if (A->val_bits == 64) {
-    if (a == 32 && b == 32) return spadd_impl<int32_t, int32_t, double>(ctx, s, A, B, C);
-    if (a == 32 && b == 64) return spadd_impl<int32_t, int64_t, double>(ctx, s, A, B, C);
-    if (a == 64 && b == 32) return spadd_impl<int64_t, int32_t, double>(ctx, s, A, B, C);
-    return spadd_impl<int64_t, int64_t, double>(ctx, s, A, B, C);
+    if (a == 32 && b == 32) return spadd_impl<int32_t, int32_t, double>(ctx, s, A, B, C, strict);
+    if (a == 32 && b == 64) return spadd_impl<int32_t, int64_t, double>(ctx, s, A, B, C, strict);
+    if (a == 64 && b == 32) return spadd_impl<int64_t, int32_t, double>(ctx, s, A, B, C, strict);
+    return spadd_impl<int64_t, int64_t, double>(ctx, s, A, B, C, strict);
   } else {
-    if (a == 32 && b == 32) return spadd_impl<int32_t, int32_t, float>(ctx, s, A, B, C);
-    if (a == 32 && b == 64) return spadd_impl<int32_t, int64_t, float>(ctx, s, A, B, C);
-    if (a == 64 && b == 32) return spadd_impl<int64_t, int32_t, float>(ctx, s, A, B, C);
-    return spadd_impl<int64_t, int64_t, float>(ctx, s, A, B, C);
+    if (a == 32 && b == 32) return spadd_impl<int32_t, int32_t, float>(ctx, s, A, B, C, strict);
+    if (a == 32 && b == 64) return spadd_impl<int32_t, int64_t, float>(ctx, s, A, B, C, strict);
+    if (a == 64 && b == 32) return spadd_impl<int64_t, int32_t, float>(ctx, s, A, B, C, strict);
+    return spadd_impl<int64_t, int64_t, float>(ctx, s, A, B, C, strict);
   }
+}
+
+}  // namespace tspg
+
+extern "C" int tspg_spadd(tspg_ctx *ctx, void *stream, const tspg_csr *A,
+                          const tspg_csr *B, tspg_csr_out *C) {
+  return tspg::spadd_entry(ctx, stream, A, B, C, false);
 }

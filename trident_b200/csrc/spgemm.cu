@@ -733,15 +733,16 @@ extern "C" int tspg_spgemm_acc(tspg_ctx *ctx, void *stream, const tspg_csr *A,
   TSPG_TRY(check_out(C_out, A->nrows, B->ncols, A->val_bits));
   const bool fuse = (flags & TSPG_F_ACC_FUSE) ||
                     (!(flags & TSPG_F_ACC_SPLIT) && C_in->nnz <= A->nnz + B->nnz);
-  if (fuse) {
-    // one SpGEMM in which C_in's entries join their rows as products with
-    // coefficient 1
+  // one SpGEMM in which C_in's entries join their rows as products with
+  // coefficient 1
+  auto fused = [&]() -> int {
     tspg_plan *plan = nullptr;
     TSPG_TRY(symbolic_entry(ctx, stream, A, B, C_in, pflags, &plan, nullptr));
     const int st = tspg_spgemm_numeric(ctx, stream, plan, A, B, C_out);
     tspg_plan_destroy(plan);
     return st;
-  }
+  };
+  if (fuse) return fused();
   // the product into workspace, then the merge into C_out
   cudaStream_t s = (cudaStream_t)stream;
   tspg_plan *plan = nullptr;
@@ -769,10 +770,11 @@ extern "C" int tspg_spgemm_acc(tspg_ctx *ctx, void *stream, const tspg_csr *A,
   if (st == TSPG_OK) {
     tspg_csr prod{T.nrows, T.ncols, T.nnz, T.rowptr, T.rowptr_bits, T.val_bits,
                   T.col, T.val};
-    st = tspg_spadd(ctx, stream, &prod, C_in, C_out);
+    st = spadd_entry(ctx, stream, &prod, C_in, C_out, true);
   }
   ws_free(ctx, cx, s);
   ws_free(ctx, cj, s);
   ws_free(ctx, rp, s);
-  return st;
+  // rows of C_in in no order, or with a column twice: the merge takes neither
+  return st == TSPG_EUNSORTED ? fused() : st;
 }
