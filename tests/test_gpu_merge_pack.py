@@ -310,3 +310,55 @@ def test_accumulator_in_any_order(ctx, dup, flags):
     C = ops.sp_mma(ctx, A.to_device(), B.to_device(), E.to_device(), flags=flags)
     rp, cj, cx, _ = oracle.spgemm(A, B)
     check_sum(C, HostCSR(A.nrows, B.ncols, rp, cj, cx), _canonical(E))
+
+
+@pytest.mark.parametrize("la,lb,n", [
+    ([1791], [0], 4000), ([1791], [1], 4000), ([1792], [0], 4000), ([1792], [1], 4000), ([1793], [1792], 4000),
+    ([896] * 4, [896] * 4, 896), ([896, 896, 0], [896, 897, 0], 1000), ([1792] + [0] * 50 + [5], [0] * 51 + [3], 2000),
+    ([900] + [0] * 4000 + [900, 892], [0] * 4001 + [892, 0], 1000)])
+def test_spadd_edges_of_1792_entry_tiles(ctx, la, lb, n):
+    # totals of k * 1792 and one more or less, equal pairs and row boundaries
+    # (with runs of empty rows) at the cuts
+    A, B = _sorted_rows(la, n, 11), _sorted_rows(lb, n, 12)
+    check_sum(ops.spadd(ctx, A.to_device(), B.to_device()), A, B)
+    check_sum(ops.spadd(ctx, B.to_device(), A.to_device()), B, A)
+    check_sum(ops.spadd(ctx, A.to_device(), A.to_device()), A, A)
+
+
+@pytest.mark.parametrize("shift", [-1, 0, 1])
+def test_spadd_pair_cut_by_a_tile(ctx, shift):
+    # A's entry of the one equal pair is entry 1791 + shift of the merge, B's the next
+    k = 1791 + shift
+    a = np.concatenate([np.arange(k), [k], np.arange(5000, 6000)]).astype(np.int32)
+    b = np.concatenate([[k], np.arange(6000, 7000)]).astype(np.int32)
+    A, B = (HostCSR(2, 8000, np.array([0, c.size, c.size], np.int64), c, np.arange(1.0, c.size + 1)) for c in (a, b))
+    check_sum(ops.spadd(ctx, A.to_device(), B.to_device()), A, B)
+
+
+@pytest.mark.parametrize("form", ["spread", "ends", "packed"])
+def test_spadd_of_far_more_rows_than_entries(ctx, form):
+    # tiles of more than 1024 and more than 4096 rows; the offsets then come
+    # from a pass of their own, or from the tiles where its workspace is refused
+    m, rng = 300_000, np.random.default_rng(4)
+    la, lb = np.zeros(m, np.int64), np.zeros(m, np.int64)
+    if form == "spread":
+        la[rng.choice(m, 500, replace=False)] = 2
+        lb[rng.choice(m, 500, replace=False)] = 1
+    elif form == "ends":
+        la[[0, 1, m - 1]] = [2000, 3, 1792]
+        lb[[0, m - 2, m - 1]] = [1584, 7, 5]
+    else:
+        la[5000:5100], lb[5050:5200] = 300, 200
+        la[280_000] = lb[290_000] = 1
+    A, B = _sorted_rows(la, 5000, 21), _sorted_rows(lb, 5000, 22)
+    dA, dB = A.to_device(rowptr_bits=32), B.to_device(rowptr_bits=64)
+    for bits in (32, 64):
+        check_sum(ops.spadd(ctx, dA, dB, rowptr_bits=bits), A, B)
+    c = ops.Context(0, 1 << 20)
+    check_sum(ops.spadd(c, dA, dB), A, B)
+    small = ops.Context(0, c.mem()[1] - 256)  # the largest of the workspace blocks no longer fits
+    try:
+        check_sum(ops.spadd(small, dA, dB), A, B)
+    finally:
+        small.close()
+        c.close()

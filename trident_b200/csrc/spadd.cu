@@ -15,7 +15,9 @@
 // R-MAT of order 2^18, 64 draws a row, A + B: 0.83 -> 0.43 ms against one warp
 // per row merging 32-column chunks ranked by shuffles (about 400 instructions
 // per 32 entries, hub rows in a kernel of their own); 0.49 ms with a tile's
-// loads in loops of unknown length instead of all in flight.
+// loads in loops of unknown length instead of all in flight.  Long runs of empty
+// rows: 1M rows holding 300 + 300 entries 0.10 ms (a thread stepping over them
+// row by row, and a CTA writing their offsets: 15 ms; a warp per row: 0.21 ms).
 #include "internal.cuh"
 #include "spgemm_kernels.cuh"
 
@@ -25,7 +27,9 @@ constexpr int kMergeThreads = 256;
 constexpr int kMergePer = 7;  // merged entries per thread: odd, so that threads stepping through
                                // shared memory in step hit different banks
 constexpr int kMergeTile = kMergeThreads * kMergePer;
-constexpr int kMergeRows = 1024;                      // row ends kept in shared memory
+// Row ends kept in shared memory.  A tile over more rows (runs of empty ones:
+// it holds kMergeTile entries at most) searches the offsets for each entry's row.
+constexpr int kMergeRows = 1024;
 
 // A cut of the merged sequence before entry d: the row whose entries it falls
 // into (the last one starting at or before d), the first row starting at or
@@ -84,7 +88,8 @@ __global__ void __launch_bounds__(128)
 
 // One tile: WRITE = false leaves its number of output entries in tilec[tile]
 // and checks the order of the rows; WRITE = true writes them from off[tile] on,
-// and the offsets of the rows that start in the tile.  A column in both rows leaves with A's entry (the two
+// and the offsets of the rows that start in the tile (pos given: their entries'
+// slots, for k_tile_offsets; order[2] = 1 asks for that).  A column in both rows leaves with A's entry (the two
 // values added); B's entry of the pair is a "dup" and leaves nothing, so entry
 // x of the tile goes to slot x - (dups before x).
 //
@@ -102,10 +107,12 @@ __global__ void __launch_bounds__(kMergeThreads)
                   const VT *__restrict__ Ax, const PTB *__restrict__ Bp,
                   const int32_t *__restrict__ Bj, const VT *__restrict__ Bx, int64_t ntiles,
                   const MergeCut *__restrict__ cuts, int32_t *tilec, volatile int64_t *order,
-                  const int64_t *off, void *Cp, int cp_bits, int32_t *Cj, VT *Cx) {
+                  const int64_t *off, uint16_t *pos, void *Cp, int cp_bits, int32_t *Cj, VT *Cx) {
   __shared__ VT sv[WRITE ? kMergeTile + 2 : 1];       // A's values, then B's, one more of B
   __shared__ int32_t sc[kMergeTile + 2];              // one column of A before, A's, B's, one of B
-  __shared__ uint16_t sea[kMergeRows], seb[kMergeRows];  // row ends in the tile
+  __shared__ uint32_t send[kMergeRows];               // row ends in the tile
+  __shared__ uint32_t sfrom[kMergeTile];              // ends of the row that starts at an entry, so that
+                                                      // nobody steps over empty rows
   __shared__ uint16_t sdup[kMergeThreads + 1];        // dups before a thread's entries; counting: A's before them
   __shared__ uint8_t sbit[kMergeThreads + 1];         // a thread's dups, bit per entry
   __shared__ int wsum[kMergeThreads / 32];
@@ -165,23 +172,37 @@ __global__ void __launch_bounds__(kMergeThreads)
     }
     sb[nB] = after;
   }
-  // ends of row c0.row + k, clipped to the tile
-  auto end_a = [&](int64_t k) {
-    const int64_t e = int64_t(__ldg(Ap + c0.row + k + 1)) - ab - c0.i;
-    return int(e < nA ? e : nA);
+  // ends of row c0.row + k, clipped to the tile: A's, B's << 16
+  auto row_end = [&](int64_t k) {
+    const int64_t a = int64_t(__ldg(Ap + c0.row + k + 1)) - ab - c0.i;
+    const int64_t b = int64_t(__ldg(Bp + c0.row + k + 1)) - bb - c0.j;
+    return uint32_t(a < nA ? a : nA) | uint32_t(b < nB ? b : nB) << 16;
   };
-  auto end_b = [&](int64_t k) {
-    const int64_t e = int64_t(__ldg(Bp + c0.row + k + 1)) - bb - c0.j;
-    return int(e < nB ? e : nB);
-  };
-  if (small)
-    for (int k = tid; k < int(R); k += kMergeThreads) {
-      sea[k] = uint16_t(end_a(k));
-      seb[k] = uint16_t(end_b(k));
+  auto both = [](uint32_t e) { return int((e & 0xffffu) + (e >> 16)); };
+  if (small) {
+    for (int k0 = w * 32; k0 < int(R); k0 += kMergeThreads) {
+      const int k = k0 + lane;
+      const uint32_t e = k < int(R) ? row_end(k) : 0u, b = lane == 0 && k > 0 ? row_end(k - 1) : 0u;
+      const uint32_t up = __shfl_up_sync(0xffffffffu, e, 1);
+      const int s = both(lane > 0 ? up : b);
+      if (k < int(R)) {
+        send[k] = e;
+        if (both(e) > s) sfrom[s] = e;
+      }
     }
+  } else {  // far more rows than entries: the row of every entry, by a search
+    for (int x = tid; x < n; x += kMergeThreads) {
+      const int64_t d = c0.i + c0.j + x + ab + bb;
+      int64_t lo = c0.row, hi = rl;
+      while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (int64_t(__ldg(Ap + mid + 1)) + int64_t(__ldg(Bp + mid + 1)) > d) hi = mid; else lo = mid + 1;
+      }
+      sfrom[x] = row_end(lo - c0.row);
+    }
+  }
   __syncthreads();
-  auto ea = [&](int64_t k) { return small ? int(sea[k]) : end_a(k); };
-  auto eb = [&](int64_t k) { return small ? int(seb[k]) : end_b(k); };
+  auto ends = [&](int64_t k) { return small ? send[k] : row_end(k); };
   const int x0 = tid * kMergePer;
   int32_t col[kMergePer];
   VT val[kMergePer];
@@ -193,10 +214,12 @@ __global__ void __launch_bounds__(kMergeThreads)
     int64_t lo = 0, hi = R - 1;  // the first row that ends past x0
     while (lo < hi) {
       const int64_t mid = (lo + hi) >> 1;
-      if (ea(mid) + eb(mid) > x0) hi = mid; else lo = mid + 1;
+      if (both(ends(mid)) > x0) hi = mid; else lo = mid + 1;
     }
-    int64_t k = lo;
-    int as = k > 0 ? ea(k - 1) : 0, bs = k > 0 ? eb(k - 1) : 0, ae = ea(k), be = eb(k);
+    const int64_t k = lo;
+    const uint32_t ks = k > 0 ? ends(k - 1) : 0u, ke = ends(k);
+    const int as = int(ks & 0xffffu), bs = int(ks >> 16);
+    int ae = int(ke & 0xffffu), be = int(ke >> 16);
     // the row's merge path at x0
     const int q = x0 - as - bs, la = ae - as, lb = be - bs;
     int x = q > lb ? q - lb : 0, y = q < la ? q : la;
@@ -215,10 +238,10 @@ __global__ void __launch_bounds__(kMergeThreads)
 #pragma unroll
     for (int t = 0; t < kMergePer; ++t) {
       if (x0 + t < n) {
-        while (i == ae && j == be) {  // the next row with entries
-          ++k;
-          ae = ea(k);
-          be = eb(k);
+        if (i == ae && j == be) {  // the next row with entries
+          const uint32_t e = sfrom[x0 + t];
+          ae = int(e & 0xffffu);
+          be = int(e >> 16);
           ca = i < ae ? sa[i] : INT32_MAX;
           cb = j < be ? sb[j] : INT32_MAX;
           pa = pb = -1;
@@ -270,18 +293,23 @@ __global__ void __launch_bounds__(kMergeThreads)
     if (v < w) before += c;
     all += c;
   }
+  // rows that start in this tile (the last tile: up to row m)
+  const int64_t last = blockIdx.x == ntiles - 1 ? m + 1 : c1.first;
   if (!WRITE) {
-    if (tid == 0) tilec[blockIdx.x] = n - all;
+    if (tid == 0) {
+      tilec[blockIdx.x] = n - all;
+      if (last - c0.first > kTileRows) order[2] = 1;
+    }
     return;
   }
   // the inputs are dead: their space takes the output in order
-  int pos = x0 - before;
+  int p = x0 - before;
 #pragma unroll
   for (int t = 0; t < kMergePer; ++t) {
     if (x0 + t < n && !((dups >> t) & 1u)) {
-      sc[pos] = col[t];
-      sv[pos] = val[t];
-      ++pos;
+      sc[p] = col[t];
+      sv[p] = val[t];
+      ++p;
     }
   }
   sdup[tid] = uint16_t(before);
@@ -300,12 +328,17 @@ __global__ void __launch_bounds__(kMergeThreads)
       Cx[o + x] = sv[x];
     }
   }
-  // rows that start in this tile (the last tile: up to row m)
-  const int64_t last = blockIdx.x == ntiles - 1 ? m + 1 : c1.first;
+  auto slot = [&](int x) {  // output entries before entry x of the tile
+    return x - sdup[x / kMergePer] -
+           __popc(sbit[x / kMergePer] & ((1u << (x % kMergePer)) - 1u));
+  };
+  if (pos) {
+    for (int x = tid; x < n; x += kMergeThreads)
+      pos[int64_t(blockIdx.x) * kMergeTile + x] = uint16_t(slot(x));
+    return;
+  }
   for (int64_t r = c0.first + tid; r < last; r += kMergeThreads) {
-    const int x = int(int64_t(Ap[r]) - ab - c0.i + int64_t(Bp[r]) - bb - c0.j);
-    const int64_t at = o + x - sdup[x / kMergePer] -
-                       __popc(sbit[x / kMergePer] & ((1u << (x % kMergePer)) - 1u));
+    const int64_t at = o + slot(int(int64_t(Ap[r]) - ab - c0.i + int64_t(Bp[r]) - bb - c0.j));
     if (cp_bits == 32) ((int32_t *)Cp)[r] = int32_t(at);
     else ((int64_t *)Cp)[r] = at;
   }
@@ -334,11 +367,11 @@ static int spadd_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
   const PTB *Bp = (const PTB *)B->rowptr;
   k_merge_cuts<PTA, PTB><<<unsigned((ntiles + 128) / 128), 128, 0, s>>>(m, Ap, A->col, Bp, B->col,
                                                                        ntiles, cuts, rec);
-  int64_t *h = ctx->h_words;  // [0] nnz(C), [1] and [2] the order check
-  h[1] = h[2] = 0;
+  int64_t *h = ctx->h_words;  // [0] nnz(C), [1] and [2] the order check, [3] a tile of many rows
+  h[1] = h[2] = h[3] = 0;
   k_merge_tiles<false, PTA, PTB, VT><<<unsigned(ntiles), kMergeThreads, 0, s>>>(
-      m, Ap, A->col, nullptr, Bp, B->col, nullptr, ntiles, cuts, tilec, h + 1, nullptr, nullptr, 0,
-      nullptr, nullptr);
+      m, Ap, A->col, nullptr, Bp, B->col, nullptr, ntiles, cuts, tilec, h + 1, nullptr, nullptr,
+      nullptr, 0, nullptr, nullptr);
   ctx->launches += 2;
   launch_scan(ctx, s, tilec, ntiles, partial, off, rec, nullptr, HostWords(), h);
   TSPG_CUDA(ctx, cudaGetLastError());
@@ -356,10 +389,18 @@ static int spadd_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
     C->val = cx;
     C->capacity = nnz;
   }
+  // (refused by the budget: the tiles' CTAs walk their rows)
+  uint16_t *pos = nullptr;
+  if (h[3] && sc.get(&pos, size_t(total)) != TSPG_OK) pos = nullptr;
   k_merge_tiles<true, PTA, PTB, VT><<<unsigned(ntiles), kMergeThreads, 0, s>>>(
       m, Ap, A->col, (const VT *)A->val, Bp, B->col, (const VT *)B->val, ntiles, cuts, nullptr, nullptr, off,
-      C->rowptr, C->rowptr_bits, C->col, (VT *)C->val);
+      pos, C->rowptr, C->rowptr_bits, C->col, (VT *)C->val);
   ctx->launches += 1;
+  if (pos) {
+    k_tile_offsets<kMergeTile, PTA, PTB><<<unsigned((m + 256) / 256), 256, 0, s>>>(
+        Ap, Bp, m, off, ntiles, pos, C->rowptr, C->rowptr_bits);
+    ctx->launches += 1;
+  }
   TSPG_CUDA(ctx, cudaGetLastError());
   return TSPG_OK;
 }

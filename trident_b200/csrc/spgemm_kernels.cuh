@@ -930,6 +930,32 @@ static __global__ void __launch_bounds__(kScanThreads)
     finish_symbolic(Snum, total, host);
 }
 
+// Row offsets of an output written in equal tiles of TILE source entries, whose
+// CTAs write the offsets of the rows that start in them — unless some tile
+// holds more than kTileRows rows (long runs of empty ones: a CTA would walk
+// them alone; 1M rows of 600 entries: 15 ms a merge).  Then the tiles leave
+// every source entry's output slot, counted from the tile's first, in pos, and
+// this grid-wide pass takes each row's from there.  off: the tiles' first
+// slots, off[ntiles] the total; a row starts at source entry Ap[r] (+ Bp[r]).
+constexpr int64_t kTileRows = 4096;
+template <int TILE, typename PTA, typename PTB>
+__global__ void __launch_bounds__(256)
+    k_tile_offsets(const PTA *__restrict__ Ap, const PTB *__restrict__ Bp, int64_t m,
+                   const int64_t *__restrict__ off, int64_t ntiles,
+                   const uint16_t *__restrict__ pos, void *Cp, int cp_bits) {
+  const int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (r > m) return;
+  auto start = [&](int64_t q) {
+    int64_t d = int64_t(__ldg(Ap + q)) - int64_t(__ldg(Ap));
+    if (Bp) d += int64_t(__ldg(Bp + q)) - int64_t(__ldg(Bp));
+    return d;
+  };
+  const int64_t d = start(r);
+  const int64_t at = d < start(m) ? off[d / TILE] + pos[d] : off[ntiles];
+  if (cp_bits == 32) ((int32_t *)Cp)[r] = int32_t(at);
+  else ((int64_t *)Cp)[r] = at;
+}
+
 // Rows from which a step's last block no longer does what a small launch of
 // its own can: every block then pays a fence and a ticket (2.1M rows: count
 // pass +14 us, final scan +6 us, against 2-3 us a launch).
