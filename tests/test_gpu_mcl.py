@@ -106,3 +106,35 @@ def test_row_and_tile_edges(ctx, lens):
         np.testing.assert_array_equal(P.rowptr, prp)
         np.testing.assert_array_equal(P.col, cj)
         np.testing.assert_array_equal(P.val, cx)
+
+
+@pytest.mark.parametrize("form", ["spread", "ends", "packed", "run"])
+def test_prune_of_far_more_rows_than_entries(ctx, form):
+    # tiles of more than 4096 rows: the offsets come from a pass of their own,
+    # or from the tiles where its workspace is refused
+    m, rng = 300_000, np.random.default_rng(6)
+    lens = np.zeros(m, np.int64)
+    if form == "spread":
+        lens[rng.choice(m, 700, replace=False)] = 3
+    elif form == "ends":
+        lens[[0, 1, m - 1]] = [2048, 2048, 1]
+    elif form == "packed":
+        lens[5000:5100] = 300
+        lens[280_000] = 1
+    else:  # a run of exactly 4096 empty rows inside a tile, and one row less
+        lens[[0, 4097, 8193, 12290]] = [100, 50, 20, 3000]
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    H = HostCSR(m, 5000, rp, rng.integers(0, 5000, rp[-1]).astype(np.int32), rng.uniform(0.1, 1, rp[-1]))
+    c = ops.Context(0, 1 << 20)
+    ops.mcl_prune(c, H.to_device(), 0.3)
+    small = ops.Context(0, c.mem()[1] - 256)
+    for tol in (0.0, 0.5, 2.0):
+        prp, cj, cx = oracle.mcl_prune(H.rowptr, H.col, H.val, tol)
+        for x in (ctx, small):
+            for bits in (32, 64):
+                P = ops.mcl_prune(x, H.to_device(rowptr_bits=bits), tol).to_host()
+                np.testing.assert_array_equal(P.rowptr, prp)
+                np.testing.assert_array_equal(P.col, cj)
+                np.testing.assert_array_equal(P.val, cx)
+    small.close()
+    c.close()

@@ -97,16 +97,17 @@ __global__ void __launch_bounds__(256)
 // Prune: the entries with |v| > tol, in their order.  Tiles of kPruneTile
 // entries whatever the rows' lengths (a warp per row took 0.23 + 0.38 ms for
 // 46M entries in rows of up to 25k); warp w of a tile owns 256 consecutive
-// ones.  FILL = false leaves the tile's number of kept entries in tilec;
+// ones.  FILL = false leaves the tile's number of kept entries in tilec, and
+// *many = 1 when two row starts kTileRows rows apart lie in one tile;
 // FILL = true writes them from off[tile] on, and the offsets of the rows that
-// start in the tile.
+// start in the tile (pos given: the entries' slots, for k_tile_offsets).
 constexpr int kPruneTile = 2048;
 template <bool FILL, typename PT, typename VT>
 __global__ void __launch_bounds__(256)
     k_prune_tiles(const PT *__restrict__ rp, const int32_t *__restrict__ col,
                   const VT *__restrict__ val, int64_t m, int64_t nnz, VT tol, int64_t ntiles,
-                  int32_t *tilec, Sched *rec, const int64_t *off, void *np, int np_bits, int32_t *ocol,
-                  VT *oval) {
+                  int32_t *tilec, Sched *rec, volatile int64_t *many, const int64_t *off,
+                  uint16_t *pos, void *np, int np_bits, int32_t *ocol, VT *oval) {
   constexpr int U = 8;
   __shared__ unsigned mask[64 + 1];
   __shared__ int before[64 + 1];
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(256)
     if (lane == 0) mask[w * U + u] = b[u];
     kept += __popc(b[u]);
   }
-  if (FILL && w < 2) {
+  if (FILL && w < 2 && !pos) {
     // the first row that starts at or after d0 (w = 0), and the one that ends
     // this tile's rows (the last tile: one past row m)
     const int64_t d = w == 0 ? d0 : d1;
@@ -164,6 +165,12 @@ __global__ void __launch_bounds__(256)
   if (!FILL) {
     if (tid == 0) tilec[t] = before[64];
     if (tid == 0 && t == 0) rec->ticket = 0;  // of the scan to come
+    auto tile = [&](int64_t r) {
+      const int64_t x = (int64_t(__ldg(rp + r)) - base) / kPruneTile;
+      return x < ntiles ? x : ntiles - 1;
+    };
+    for (int64_t r = (t * 256 + tid) * kTileRows; r + kTileRows <= m; r += ntiles * 256 * kTileRows)
+      if (tile(r) == tile(r + kTileRows)) *many = 1;
     return;
   }
   const int64_t o = off[t];
@@ -174,6 +181,14 @@ __global__ void __launch_bounds__(256)
       ocol[q] = c[u];
       oval[q] = v[u];
     }
+  }
+  if (pos) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t e = d0 + w * 256 + u * 32 + lane;
+      if (e < d1) pos[e] = uint16_t(before[w * U + u] + __popc(b[u] & ((1u << lane) - 1u)));
+    }
+    return;
   }
   for (int64_t r = row0[0] + tid; r < row0[1]; r += 256) {
     const int x = int(int64_t(__ldg(rp + r)) - base - d0);
@@ -213,11 +228,12 @@ static int prune_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, double t
   Sched *rec;
   TSPG_TRY(sc.get_all(part(&tilec, ntiles), part(&off, ntiles + 1),
                       part(&partial, (ntiles + kScanTile - 1) / kScanTile + 1), part(&rec, 1)));
+  int64_t *h = ctx->h_words;  // [0] kept entries, [1] a tile of many rows
+  h[1] = 0;
   k_prune_tiles<false, PT, VT><<<unsigned(ntiles), 256, 0, s>>>(
       (const PT *)M->rowptr, nullptr, (const VT *)M->val, m, M->nnz, VT(tol), ntiles, tilec, rec,
-      nullptr, nullptr, 0, nullptr, nullptr);
+      h + 1, nullptr, nullptr, nullptr, 0, nullptr, nullptr);
   ctx->launches += 1;
-  int64_t *h = ctx->h_words;
   launch_scan(ctx, s, tilec, ntiles, partial, off, rec, nullptr, HostWords(), h);
   TSPG_CUDA(ctx, cudaGetLastError());
   TSPG_CUDA(ctx, cudaStreamSynchronize(s));
@@ -233,10 +249,18 @@ static int prune_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, double t
     out->val = cx;
     out->capacity = nnz;
   }
+  // (refused by the budget: the tiles' CTAs walk their rows)
+  uint16_t *pos = nullptr;
+  if (h[1] && sc.get(&pos, size_t(M->nnz)) != TSPG_OK) pos = nullptr;
   k_prune_tiles<true, PT, VT><<<unsigned(ntiles), 256, 0, s>>>(
-      (const PT *)M->rowptr, M->col, (const VT *)M->val, m, M->nnz, VT(tol), ntiles, nullptr, nullptr, off,
-      out->rowptr, out->rowptr_bits, out->col, (VT *)out->val);
+      (const PT *)M->rowptr, M->col, (const VT *)M->val, m, M->nnz, VT(tol), ntiles, nullptr, nullptr,
+      nullptr, off, pos, out->rowptr, out->rowptr_bits, out->col, (VT *)out->val);
   ctx->launches += 1;
+  if (pos) {
+    k_tile_offsets<kPruneTile, PT, PT><<<unsigned((m + 256) / 256), 256, 0, s>>>(
+        (const PT *)M->rowptr, (const PT *)nullptr, m, off, ntiles, pos, out->rowptr, out->rowptr_bits);
+    ctx->launches += 1;
+  }
   TSPG_CUDA(ctx, cudaGetLastError());
   return TSPG_OK;
 }
