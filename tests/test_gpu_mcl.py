@@ -138,3 +138,19 @@ def test_prune_of_far_more_rows_than_entries(ctx, form):
                 np.testing.assert_array_equal(P.val, cx)
     small.close()
     c.close()
+
+
+def test_inflate_many_short_rows_among_long_ones(ctx):
+    # more rows than one turn of every CTA (32 rows a warp), long rows in several turns
+    rng = np.random.default_rng(12)
+    lens = rng.choice([0, 1, 4, 33], size=400_000, p=[0.5, 0.2, 0.2, 0.1])
+    lens[[0, 1, 9000, 199_999, 200_000, 399_999]] = [300, 257, 2049, 5000, 256, 2048]
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    H = HostCSR(lens.size, 50, rp, np.zeros(rp[-1], np.int32), rng.uniform(0.1, 1, rp[-1]))
+    for power in (2.0, 1.5):
+        got = ops.mcl_inflate(ctx, H.to_device(), power).val.cpu().numpy()
+        want = oracle.mcl_inflate(H.rowptr, H.val, power)
+        assert np.all(np.abs(got - want) <= 1e-12 * np.abs(want))
+    got = ops.mcl_normalize(ctx, H.to_device()).val.cpu().numpy()
+    want = oracle.mcl_inflate(H.rowptr, H.val, 1.0)
+    assert np.all(np.abs(got - want) <= 1e-12 * np.abs(want))

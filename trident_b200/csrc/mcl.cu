@@ -19,11 +19,33 @@ namespace tspg {
 // and one write of the values.  Longer ones are powered and summed, then read
 // back.  The 8 rows of a CTA lie ngroups apart, so the neighbouring hub rows of
 // a graph go to different CTAs (a warp per row, hub rows of 25k entries: 0.61
-// ms for 46M entries).  power 2 is one multiplication (pow costs ~150
-// instructions an entry).
+// ms for 46M entries).  A warp takes 32 rows, marking the long ones, before the
+// CTA takes those together: meeting after every row cost matrices of short rows
+// more than the reads (1M rows of 4 entries 590 -> 240 us; a warp per row 416).
+// power 2 is one multiplication (pow costs ~150 instructions an entry).
 template <typename VT>
 __device__ __forceinline__ VT mcl_pow(VT v, VT power, int do_pow) {
   return do_pow == 2 ? v * v : do_pow ? VT(pow(v, power)) : v;
+}
+
+// One row of at most 32 U entries by one warp.
+template <int U, typename VT>
+__device__ __forceinline__ void mcl_warp_row(const VT *val, VT *out, int len, int lane, VT power,
+                                             int do_pow) {
+  VT v[U], sum = VT(0);
+#pragma unroll
+  for (int u = 0; u < U; ++u) v[u] = u * 32 + lane < len ? val[u * 32 + lane] : VT(0);
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (u * 32 + lane < len) {
+      v[u] = mcl_pow(v[u], power, do_pow);
+      sum += v[u];
+    }
+  sum = warp_sum(sum);
+  const bool keep = sum > VT(1e-20);
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (u * 32 + lane < len) out[u * 32 + lane] = keep ? v[u] / sum : VT(0);
 }
 
 template <typename PT, typename VT>
@@ -32,65 +54,64 @@ __global__ void __launch_bounds__(256)
                VT *out) {
   constexpr int U = 8;
   __shared__ VT part[8];
+  __shared__ unsigned longs[8];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  for (int64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
-    const int64_t r = w * ngroups + g;
-    const int64_t a0 = r < m ? int64_t(rp[r]) : 0, len = r < m ? int64_t(rp[r + 1]) - a0 : 0;
-    if (len > 0 && len <= 32 * U) {
-      VT v[U], sum = VT(0);
-#pragma unroll
-      for (int u = 0; u < U; ++u) v[u] = u * 32 + lane < len ? val[a0 + u * 32 + lane] : VT(0);
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (u * 32 + lane < len) {
-          v[u] = mcl_pow(v[u], power, do_pow);
-          sum += v[u];
-        }
-      sum = warp_sum(sum);
-      const bool keep = sum > VT(1e-20);
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (u * 32 + lane < len) out[a0 + u * 32 + lane] = keep ? v[u] / sum : VT(0);
+  const int64_t step = gridDim.x;
+  for (int64_t g0 = blockIdx.x; g0 < ngroups; g0 += 32 * step) {
+    unsigned mine = 0;
+    // lane l holds the bounds of the warp's l-th row of the 32
+    const int64_t gl = g0 + lane * step, rl = w * ngroups + gl;
+    const bool have = gl < ngroups && rl < m;
+    const int64_t s0 = have ? int64_t(rp[rl]) : 0;
+    const int64_t n0 = have ? int64_t(rp[rl + 1]) - s0 : 0;
+    for (unsigned todo = __ballot_sync(0xffffffffu, n0 > 0); todo; todo &= todo - 1) {
+      const int t = __ffs(todo) - 1;
+      const int64_t a0 = __shfl_sync(0xffffffffu, s0, t), len = __shfl_sync(0xffffffffu, n0, t);
+      if (len <= 32) mcl_warp_row<1>(val + a0, out + a0, int(len), lane, power, do_pow);
+      else if (len <= 32 * U) mcl_warp_row<U>(val + a0, out + a0, int(len), lane, power, do_pow);
+      else mine |= 1u << t;
     }
-    // the longer ones of the 8 rows, a CTA each (uniform over the CTA)
-    if (!__syncthreads_or(len > 32 * U)) continue;
+    if (lane == 0) longs[w] = mine;
+    // the longer ones, a CTA each (uniform over the CTA)
+    if (!__syncthreads_or(mine != 0)) continue;
     for (int q = 0; q < 8; ++q) {
-      const int64_t row = q * ngroups + g;
-      if (row >= m) break;
-      const int64_t b0 = int64_t(rp[row]), n = int64_t(rp[row + 1]) - b0;
-      if (n <= 32 * U) continue;
-      const bool held = n <= 256 * U;
-      VT v[U], sum = VT(0);
-      for (int64_t c = 0; c < n; c += 256 * U) {
+      for (unsigned todo = longs[q]; todo; todo &= todo - 1) {
+        const int64_t row = q * ngroups + g0 + (__ffs(todo) - 1) * step;
+        const int64_t b0 = int64_t(rp[row]), n = int64_t(rp[row + 1]) - b0;
+        const bool held = n <= 256 * U;
+        VT v[U], sum = VT(0);
+        for (int64_t c = 0; c < n; c += 256 * U) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) v[u] = c + u * 256 + tid < n ? val[b0 + c + u * 256 + tid] : VT(0);
+          for (int u = 0; u < U; ++u) v[u] = c + u * 256 + tid < n ? val[b0 + c + u * 256 + tid] : VT(0);
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (c + u * 256 + tid < n) {
-            v[u] = mcl_pow(v[u], power, do_pow);
-            sum += v[u];
-            if (!held && do_pow) out[b0 + c + u * 256 + tid] = v[u];
-          }
-      }
-      sum = warp_sum(sum);
-      if (lane == 0) part[w] = sum;
-      __syncthreads();
-      sum = VT(0);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) sum += part[k];
-      const bool keep = sum > VT(1e-20);
-      const VT *src = do_pow ? out : val;  // the thread's own writes, if powered
-      for (int64_t c = 0; c < n; c += 256 * U) {
-        if (!held) {
-#pragma unroll
-          for (int u = 0; u < U; ++u) v[u] = c + u * 256 + tid < n ? src[b0 + c + u * 256 + tid] : VT(0);
+          for (int u = 0; u < U; ++u)
+            if (c + u * 256 + tid < n) {
+              v[u] = mcl_pow(v[u], power, do_pow);
+              sum += v[u];
+              if (!held && do_pow) out[b0 + c + u * 256 + tid] = v[u];
+            }
         }
+        sum = warp_sum(sum);
+        if (lane == 0) part[w] = sum;
+        __syncthreads();
+        sum = VT(0);
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (c + u * 256 + tid < n) out[b0 + c + u * 256 + tid] = keep ? v[u] / sum : VT(0);
+        for (int k = 0; k < 8; ++k) sum += part[k];
+        const bool keep = sum > VT(1e-20);
+        const VT *src = do_pow ? out : val;  // the thread's own writes, if powered
+        for (int64_t c = 0; c < n; c += 256 * U) {
+          if (!held) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = c + u * 256 + tid < n ? src[b0 + c + u * 256 + tid] : VT(0);
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (c + u * 256 + tid < n) out[b0 + c + u * 256 + tid] = keep ? v[u] / sum : VT(0);
+        }
+        __syncthreads();  // part is free again
       }
-      __syncthreads();  // part is free again
     }
+    __syncthreads();  // longs is free again
   }
 }
 
