@@ -162,3 +162,29 @@ def test_lane_rows(val_bits):
         check_product(b.result(i), A, B, tol=tol)
     b.close()
     c.close()
+
+
+@pytest.mark.parametrize("m", [3000, 66000])
+def test_short_rows_of_many_a_entries(ctx, m):
+    # A rows of 1 ... 700 entries whose B rows are mostly empty: few products,
+    # by lanes where the rows of a warp are alike, else one by one
+    rng = np.random.default_rng(m)
+    bl = np.zeros(2000, np.int64)
+    bl[rng.choice(2000, size=60, replace=False)] = rng.choice([1, 2, 3], size=60)
+    B = _rows(bl, 9000, rng)
+    lens = np.full(m, 4)
+    lens[: m // 3] = rng.choice([1, 31, 32, 33, 64], size=m // 3)
+    at = rng.choice(m, size=200, replace=False)
+    lens[at] = rng.choice([255, 256, 257, 300, 700], size=200)
+    lens[m // 2: m // 2 + 64] = 700  # whole warps of them
+    A = _rows(lens, 2000, rng)
+    dA, dB = A.to_device(), B.to_device()
+    check_product(ops.spgemm(ctx, dA, dB), A, B)
+    plan = ops.Plan(ctx, dA, dB)
+    check_product(plan.numeric(dA, dB), A, B)
+    plan.close()
+    b = ops.Batch(ctx)
+    b.add(dA, dB)
+    b.run()
+    check_product(b.result(0), A, B)
+    b.close()

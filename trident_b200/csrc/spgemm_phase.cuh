@@ -158,6 +158,7 @@ __device__ __forceinline__ uint32_t warp_chunk(const int32_t *__restrict__ Bj,
   }
   uint32_t n = uint32_t(len);
   const unsigned nz = __ballot_sync(FULL, n > 0);
+  if (nz == 0) return 0;
   const int ne = __popc(nz);
   if (nz & (nz + 1u)) {  // a gap: lane i takes the i-th entry that has products
     const int src = lane < ne ? nth_bit(nz, lane) : 0;
@@ -221,17 +222,19 @@ __device__ __forceinline__ void for_products_flat(
   // positions fit 32 bits when B's row offsets do (nnz(B) < 2^31): the warp
   // form then shuffles half the words
   using IX = std::conditional_t<G == 32 && sizeof(PT) == 4, int32_t, int64_t>;
+  int32_t knext = G == 32 && a0 + lane < a1 ? __ldg(Aj + a0 + lane) : 0;  // the next chunk's entry
   for (int64_t c0 = a0; c0 < a1; c0 += G) {
     const int nc = int(min(int64_t(G), a1 - c0));
     IX len = 0, b0 = 0;
     VT a = VT(0);
     if (lane < nc) {
-      const int64_t k = __ldg(Aj + c0 + lane);
+      const int64_t k = G == 32 ? knext : __ldg(Aj + c0 + lane);
       if constexpr (NUM) a = __ldg(Ax + c0 + lane);
       b0 = IX(__ldg(Bp + k));
       len = IX(__ldg(Bp + k + 1)) - b0;
     }
     if constexpr (G == 32) {
+      if (c0 + 32 + lane < a1) knext = __ldg(Aj + c0 + 32 + lane);
       warp_chunk<NUM, IX, VT>(Bj, Bx, b0, len, a, lane,
                               [&](uint32_t, int32_t c, VT v) { fn(c, v); });
       continue;  // no staging to guard
@@ -1025,17 +1028,19 @@ __device__ void num_esc_row(const ProdDev<PT, VT> *prods, const PhaseArgs &A, co
   prof_sub_g(A, 9, tp, lane == 0);
   // expand: every product at its flat index
   int fb = 0;
+  int32_t knext = G == 32 && a0 + lane < a1 ? __ldg(P.Aj + a0 + lane) : 0;
   for (int64_t c0 = a0; c0 < a1; c0 += G) {
     const int nc = int(min(int64_t(G), a1 - c0));
     int64_t len = 0, b0 = 0;
     VT a = VT(0);
     if (lane < nc) {
-      const int64_t k = __ldg(P.Aj + c0 + lane);
+      const int64_t k = G == 32 ? knext : __ldg(P.Aj + c0 + lane);
       a = __ldg(P.Ax + c0 + lane);
       b0 = int64_t(__ldg(P.Bp + k));
       len = int64_t(__ldg(P.Bp + k + 1)) - b0;
     }
     if constexpr (G == 32) {
+      if (c0 + 32 + lane < a1) knext = __ldg(P.Aj + c0 + 32 + lane);
       fb += int(warp_chunk<true, int64_t, VT>(P.Bj, P.Bx, b0, len, a, lane,
                                               [&](uint32_t p, int32_t col, VT v) {
                                                 const uint32_t at = uint32_t(fb) + p;
@@ -2334,13 +2339,19 @@ __global__ void __launch_bounds__(kOnepassThreads, 1)
       mine = load_meta<FINAL>(prods, A, base + i + lane);
       if (!FINAL) mine.off = A.cp[mine.g];  // the row's scratch offset
     }
-    // lanes in step take as long as the longest row (~40 instructions a
-    // product); a warp per row ~350 and 6 a product
-    const int f = int(mine.f);
-    const int fmax = __reduce_max_sync(0xffffffffu, f);
-    const int fsum = __reduce_add_sync(0xffffffffu, f);
+    // lanes in step take as long as the longest row: ~40 instructions a
+    // product and ~36 an A entry, its B row empty or not (and the loads of
+    // each lane's entry); a warp per row ~350, 6 a product and next to nothing
+    // an entry.  70,000 rows of 2 to 16 products: 128 A entries each 183 us by
+    // lanes, 232 by warps; 256 each 352 and 286; 512 in one row of 32 257 and
+    // 215; 1024 444 and 222 (numeric phase).
+    constexpr int64_t kFar = 1 << 24;  // the 32 in one int
+    const int f = int(min(mine.f, kFar)), na = int(min(mine.a1 - mine.a0, kFar));
+    const int fmax = __reduce_max_sync(0xffffffffu, f), namax = __reduce_max_sync(0xffffffffu, na);
+    const int fsum = __reduce_add_sync(0xffffffffu, f), nasum = __reduce_add_sync(0xffffffffu, na);
     const int p0 = __shfl_sync(0xffffffffu, mine.p, 0);
-    const bool lanes = 40 * int64_t(fmax) <= 350 * int64_t(rows) + 6 * int64_t(fsum) &&
+    const bool lanes = 40 * int64_t(fmax) + 36 * int64_t(namax) + nasum / 2 <=
+                           350 * int64_t(rows) + 6 * int64_t(fsum) &&
                        __all_sync(0xffffffffu, !have || mine.p == p0);
     if (lanes) {
       lane_rows<FINAL, PT, VT>(prods[p0], A, mine, have, slice, lane);
