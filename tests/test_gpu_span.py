@@ -188,3 +188,72 @@ def test_short_rows_of_many_a_entries(ctx, m):
     b.run()
     check_product(b.result(0), A, B)
     b.close()
+
+
+def _common_columns(m, groups, na, cols, val_bits, rng):
+    """A (m rows of `na` entries) and B such that row i's products meet `na`
+    times in each of `cols` columns, and the exact values (m, cols)."""
+    B = HostCSR(groups * na, groups * cols, np.arange(groups * na + 1, dtype=np.int64) * cols,
+                (np.repeat(np.arange(groups), na * cols) * cols + np.tile(np.arange(cols), groups * na)).astype(np.int32),
+                rng.uniform(0.1, 1, groups * na * cols))
+    g = np.arange(m) % groups
+    A = HostCSR(m, groups * na, np.arange(m + 1, dtype=np.int64) * na,
+                (g[:, None] * na + np.arange(na)).ravel().astype(np.int32), rng.uniform(-1, 1, m * na))
+    if val_bits == 32:
+        for M in (A, B):
+            M.val = M.val.astype(np.float32).astype(np.float64)
+    a = A.val.reshape(m, na).astype(np.longdouble)
+    b = B.val.reshape(groups, na, cols).astype(np.longdouble)
+    exact = np.zeros((m, cols), np.longdouble)
+    for t in range(na):
+        exact += a[:, t, None] * b[g, t, :]
+    return A, B, exact
+
+
+@pytest.mark.parametrize("val_bits", [64, 32])
+@pytest.mark.parametrize("m,cols", [(66000, 12), (66000, 27)])
+def test_lane_rows_lose_nothing_to_their_order(val_bits, m, cols):
+    # 100 products an output by one lane.  Rounding each result alone, correctly,
+    # is an error of at most u in the norm; a running sum of these is 4 u off.
+    A, B, exact = _common_columns(m, 50, 100, cols, val_bits, np.random.default_rng(cols))
+    c = ops.Context(0)
+    dA, dB = A.to_device(val_bits=val_bits), B.to_device(val_bits=val_bits)
+    u = 2.0 ** -53 if val_bits == 64 else 2.0 ** -24
+    plan = ops.Plan(c, dA, dB)
+    for C in (ops.spgemm(c, dA, dB), plan.numeric(dA, dB)):
+        H = C.to_host()
+        np.testing.assert_array_equal(H.rowptr, np.arange(m + 1) * cols)
+        d = H.val.reshape(m, cols).astype(np.longdouble) - exact
+        assert float(np.sqrt((d * d).sum() / (exact * exact).sum())) <= u
+    plan.close()
+    c.close()
+
+
+def test_lane_rows_at_the_ends_of_the_number_range():
+    # sums that overflow, infinite and NaN operands, values whose rounding
+    # errors lie below the smallest number: as plain sums give them
+    m, na = 5000, 4
+    A, B, _ = _common_columns(m, 50, na, 6, 64, np.random.default_rng(1))
+    a, b = A.val.reshape(m, na), B.val.reshape(50, na, 6)
+    b[:] = 1.0
+    a[0::8] = 1e308
+    a[1::8] = [np.inf, 1, 2, 3]
+    a[2::8] = [1, np.inf, -np.inf, 1]
+    a[3::8] = [1, np.nan, 2, 3]
+    a[4::8] = 1e-310
+    a[5::8] = [1e300, 1.0, -1e300, 1.0]
+    a[6::8] = -0.0
+    a[7::8] = [1e308, 1e308, -1e308, -1e308]
+    A.val, B.val = a.ravel(), b.ravel()
+    c = ops.Context(0)
+    dA, dB = A.to_device(), B.to_device()
+    plan = ops.Plan(c, dA, dB)
+    got = plan.numeric(dA, dB).to_host().val.reshape(m, 6)
+    assert np.all(got[0::8] == np.inf) and np.all(got[1::8] == np.inf)
+    assert np.all(np.isnan(got[2::8])) and np.all(np.isnan(got[3::8]))
+    assert np.all(got[4::8] == 4e-310)
+    assert np.all(np.isin(got[5::8], [0.0, 1.0, 2.0]))
+    assert np.all(got[6::8] == 0.0)
+    assert not np.any(np.isfinite(got[7::8]) & (got[7::8] != 0.0))
+    plan.close()
+    c.close()

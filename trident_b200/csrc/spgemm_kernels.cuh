@@ -25,7 +25,7 @@
 //   G256   256-thread groups, named barriers.
 //   G128   128-thread groups.
 //   G32    one warp per row.
-//   LANE   one lane per row, 32 rows by a warp: numeric rows of at most 32
+//   LANE   one lane per row, 32 rows by a warp: numeric rows of at most 27
 //          outputs, and the one-pass rows of the symbolic launch.
 // Hash rows are sorted after accumulation by an in-place compaction into the
 // first half of the table and a stable LSD radix sort (bitonic below 65).
@@ -115,11 +115,11 @@ __host__ __device__ inline int sym_class(int64_t f, int64_t n, const Tune &t) {
 // One-pass rows (plain products only, Sched::onepass set): rows of the
 // symbolic warp, 128- and 256-thread classes are multiplied whole in the
 // symbolic launch (k_lanes: a lane per row, or a warp per row where the 32
-// rows of a warp are uneven); their output waits in a scratch buffer for the
-// numeric launch, which copies it into C.  A row that turns out to hold more
-// columns than the form's table takes is deferred to the two-pass path — so
-// no row writes more than kCappedCols scratch entries, and the scratch stays
-// dense.
+// rows of a warp are uneven or the row holds more columns than a lane's table);
+// their output waits in a scratch buffer for the numeric launch, which copies
+// it into C.  A row that turns out to hold more columns than the warp's table
+// takes is deferred to the two-pass path — so no row writes more than
+// kCappedCols scratch entries, and the scratch stays dense.
 constexpr int kCappedCols = 32;
 __host__ __device__ inline bool onepass_row(int64_t f, int64_t n, const Tune &t) {
   const int64_t fe = f < n ? f : n;

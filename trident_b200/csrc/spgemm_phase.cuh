@@ -2135,20 +2135,53 @@ __global__ void __launch_bounds__(kGroupThreads, 1)
 // symbolic and 3.5 ms of numeric launches for it).  Numeric launch (FINAL =
 // true): the rows of at most kLaneSlots outputs, into C.
 constexpr int kOnepassThreads = 512;
-constexpr int kLaneSlots = kCappedCols;            // columns a lane's row may hold
-constexpr int kLaneLog = 5;
-static_assert(kLaneSlots == 1 << kLaneLog, "hash table per lane");
-constexpr int kOnepassSlice = kLaneSlots * 32 * 12;  // per warp: 32 x 32 columns and values
+// Columns a lane's row may hold.  27 slots of 14 bytes for 16 warps leave a 196
+// KB share of the SM to shared memory and 60 KB to the L1, which neighbouring
+// rows' B rows are read through: Galerkin R·A·P 3.64 ms; 32 slots 4.61 ms with
+// 16 warps (28 KB of L1), 4.08 ms with 13, 31 slots with 14 warps 3.84 ms.
+constexpr int kLaneSlots = 27;
+// per warp: columns, values and what the sums' rounding left over
+constexpr int kOnepassSlice = kLaneSlots * 32 * 14;
 constexpr int kOnepassSmem = (kOnepassThreads / 32) * kOnepassSlice;
+static_assert(kOnepassSmem + kOnepassThreads * 4 <= 195 * 1024, "the L1's share");
 static_assert(kNumT32 * 12 <= kOnepassSlice, "the warp form's table");
+
+// A lane's running sums keep what their roundings left over (the fast two-sum,
+// on the unrounded product): one lane adds a whole row in order, where a warp's
+// lanes spread a row's products over four partial sums, and the error grew with
+// it (Galerkin R·AP, 48 products an output: 1.8e-16 to 2.8e-16 of the norm; with
+// the rest 0.6e-16).  The rest is kept as the upper 16 bits of its value: 5
+// significant bits in FP64, which leaves a thirtieth of it, 8 in FP32.
+template <typename VT>
+__device__ __forceinline__ VT rest_value(uint16_t r) {
+  if constexpr (sizeof(VT) == 8) return __hiloint2double(int(uint32_t(r) << 16), 0);
+  else return __uint_as_float(uint32_t(r) << 16);
+}
+template <typename VT>
+__device__ __forceinline__ uint16_t rest_bits(VT c) {  // rounded to nearest
+  if constexpr (sizeof(VT) == 8) return uint16_t((uint32_t(__double2hiint(c)) + 0x8000u) >> 16);
+  else return uint16_t((__float_as_uint(c) + 0x8000u) >> 16);
+}
+// sum + a x, its rounding error added to the rest
+template <typename VT>
+__device__ __forceinline__ VT add_rest(VT sum, VT a, VT x, uint16_t *rest) {
+  const VT s = fma(a, x, sum);
+  *rest = rest_bits<VT>(rest_value<VT>(*rest) + fma(a, x, sum - s));
+  return s;
+}
+// The value of a sum and its rest (which is NaN once the sum is not finite).
+template <typename VT>
+__device__ __forceinline__ VT with_rest(VT sum, uint16_t rest) {
+  const VT c = rest_value<VT>(rest);
+  return c - c == VT(0) ? sum + c : sum;
+}
 
 // 32 rows by one warp, a lane each: lane l walks row l's A entries in step
 // with the others (the next entry's B row bounds and the one after's column
 // in flight) and adds every product into its own kLaneSlots-slot hash table in
 // shared memory, [slot][lane]: no atomics, no bank conflicts.  The occupied
-// slots are sorted by insertion as they are gathered, and written out.  A
-// one-pass row with more than kLaneSlots columns goes back to the two-pass
-// path.  (A list searched from the last hit on instead of the table: 105-148
+// slots are sorted by insertion as they are gathered, and written out.  Returns
+// the lanes whose one-pass row has more than kLaneSlots columns.  (A list searched from the last hit on instead of the table: 105-148
 // instructions a product, Galerkin A·P 3.0 ms.)
 //
 // Rows this short spend a warp's time on what surrounds the products (a warp
@@ -2156,12 +2189,13 @@ static_assert(kNumT32 * 12 <= kOnepassSlice, "the warp form's table");
 // row); lanes of neighbouring rows also read neighbouring B rows, so their
 // loads coalesce.
 template <bool FINAL, typename PT, typename VT>
-__device__ void lane_rows(const ProdDev<PT, VT> &P, const PhaseArgs &A, const RowMeta &m,
+__device__ unsigned lane_rows(const ProdDev<PT, VT> &P, const PhaseArgs &A, const RowMeta &m,
                           bool have, unsigned char *slice, int lane) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int U = 4;
   int *keys = (int *)slice + lane;
   VT *vals = (VT *)(slice + kLaneSlots * 32 * 4) + lane;
+  uint16_t *rest = (uint16_t *)(slice + kLaneSlots * 32 * 12) + lane;
   const int32_t *__restrict__ Aj = P.Aj;
   const VT *__restrict__ Ax = P.Ax;
   const PT *__restrict__ Bp = P.Bp;
@@ -2221,17 +2255,18 @@ __device__ void lane_rows(const ProdDev<PT, VT> &P, const PhaseArgs &A, const Ro
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (c[u] >= 0 && !refused) {
-          uint32_t h = hash_slot(c[u], kLaneLog);
+          uint32_t h = __umulhi(uint32_t(c[u]) * 2654435761u, uint32_t(kLaneSlots));
           int k = keys[h * 32];
           for (int it = 1; k != c[u] && k != -1 && it < kLaneSlots; ++it) {
-            h = (h + 1) & (kLaneSlots - 1);
+            h = h + 1 < kLaneSlots ? h + 1 : 0;
             k = keys[h * 32];
           }
           if (k == c[u]) {
-            vals[h * 32] = fma(av, x[u], vals[h * 32]);
+            vals[h * 32] = add_rest<VT>(vals[h * 32], av, x[u], rest + h * 32);
           } else if (k == -1) {
             keys[h * 32] = c[u];
             vals[h * 32] = av * x[u];
+            rest[h * 32] = 0;
             ++n;
           } else {
             refused = true;
@@ -2257,7 +2292,7 @@ __device__ void lane_rows(const ProdDev<PT, VT> &P, const PhaseArgs &A, const Ro
   for (int i = 0; i < kLaneSlots; ++i) {
     const int k = keys[i * 32];
     if (k != -1) {
-      const VT v = vals[i * 32];
+      const VT v = with_rest<VT>(vals[i * 32], rest[i * 32]);
       int j = n++;
       for (; j > 0; --j) {
         const int kp = keys[(j - 1) * 32];
@@ -2282,7 +2317,7 @@ __device__ void lane_rows(const ProdDev<PT, VT> &P, const PhaseArgs &A, const Ro
       ox[i] = vals[i * 32];
     }
     __syncwarp();
-    return;
+    return 0;
   }
   if (have && !refused) {
     int32_t *const oj = A.oj + m.off;
@@ -2294,15 +2329,8 @@ __device__ void lane_rows(const ProdDev<PT, VT> &P, const PhaseArgs &A, const Ro
     A.rowc[m.g] = n;
     A.rowf[m.g] = -1 - m.off;
   }
-  const unsigned back = __ballot_sync(FULL, have && refused);
-  if (back) {
-    unsigned long long at = 0;
-    if (lane == 0) at = atomicAdd(&A.S->ndefer, (unsigned long long)__popc(back));
-    at = __shfl_sync(FULL, at, 0);
-    if (have && refused)
-      A.defer[at + __popc(back & ((1u << lane) - 1u))] = (uint64_t(m.p) << 40) | uint64_t(m.r);
-  }
   __syncwarp();
+  return __ballot_sync(FULL, have && refused);
 }
 
 template <bool FINAL, typename PT, typename VT>
@@ -2353,19 +2381,17 @@ __global__ void __launch_bounds__(kOnepassThreads, 1)
     const bool lanes = 40 * int64_t(fmax) + 36 * int64_t(namax) + nasum / 2 <=
                            350 * int64_t(rows) + 6 * int64_t(fsum) &&
                        __all_sync(0xffffffffu, !have || mine.p == p0);
-    if (lanes) {
-      lane_rows<FINAL, PT, VT>(prods[p0], A, mine, have, slice, lane);
-    } else {
-      for (int t = 0; t < rows; ++t) {
-        const RowMeta m = shfl_meta(mine, t);
-        if constexpr (FINAL) {  // at most 32 outputs: sorted in registers
-          if (m.f <= 32)
-            num_esc_row<32, kNumT32, PT, VT>(prods, A, m, slice, gm, w, lane);
-          else
-            num_hash_row<32, kNumT32, PT, VT>(prods, A, m, slice, gm, w, lane);
-        } else {
-          num_hash_row<32, kNumT32, PT, VT, true>(prods, A, m, slice, gm, w, lane);
-        }
+    unsigned todo = __ballot_sync(0xffffffffu, have);
+    if (lanes) todo = lane_rows<FINAL, PT, VT>(prods[p0], A, mine, have, slice, lane);
+    for (; todo; todo &= todo - 1) {  // by the warp
+      const RowMeta m = shfl_meta(mine, __ffs(todo) - 1);
+      if constexpr (FINAL) {  // at most kLaneSlots outputs: sorted in registers
+        if (m.f <= 32)
+          num_esc_row<32, kNumT32, PT, VT>(prods, A, m, slice, gm, w, lane);
+        else
+          num_hash_row<32, kNumT32, PT, VT>(prods, A, m, slice, gm, w, lane);
+      } else {
+        num_hash_row<32, kNumT32, PT, VT, true>(prods, A, m, slice, gm, w, lane);
       }
     }
     if (A.prof && lane == 0) {
