@@ -257,3 +257,23 @@ def test_lane_rows_at_the_ends_of_the_number_range():
     assert not np.any(np.isfinite(got[7::8]) & (got[7::8] != 0.0))
     plan.close()
     c.close()
+
+
+def test_plan_whose_b_rows_change_their_order(ctx):
+    # the same pattern, B's rows in another order at each call: a form that takes
+    # a row's span from the ends of its B rows must not be kept from a call before
+    n, rng = 40000, np.random.default_rng(17)
+    col = np.sort(np.clip(np.arange(n), 24, n - 25)[:, None] + np.arange(-8, 9) * 3, axis=1)
+    rp = np.arange(n + 1, dtype=np.int64) * 17
+    A = HostCSR(n, n, rp, col.ravel().astype(np.int32), rng.uniform(-1, 1, col.size))
+    dA = A.to_device()
+    plan = ops.Plan(ctx, dA, dA)
+    check_product(plan.numeric(dA, dA), A, A)
+    for _ in range(2):
+        o = np.argsort(rng.random(col.shape), axis=1)
+        U = HostCSR(n, n, rp, np.take_along_axis(col, o, 1).ravel().astype(np.int32),
+                    np.take_along_axis(A.val.reshape(n, 17), o, 1).ravel())
+        check_product(plan.numeric(dA, U.to_device()), A, A)
+        check_product(plan.numeric(U.to_device(), dA), A, A)
+        check_product(plan.numeric(dA, dA), A, A)
+    plan.close()

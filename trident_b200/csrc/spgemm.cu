@@ -33,7 +33,6 @@ struct tspg_plan {
   int64_t max_a_row = 0;
   int64_t ncnt[NCLS] = {};  // numeric rows per class
   Tune tune{};                  // row binning of the symbolic call
-  bool strict_checked = false;  // ProdDev::b_strict is known
   void *prods = nullptr;
   int64_t *base = nullptr;
   int64_t *rowf = nullptr;
@@ -280,16 +279,6 @@ static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P, const tspg_
                         tspg_csr_out *C) {
   const int64_t m = P->m;
   ProdDev<PT, VT> *prods = (ProdDev<PT, VT> *)P->prods;
-  // warp rows over long B rows add without atomics when no B row holds a
-  // column twice: worth a pass over B's columns where they are many (the
-  // answer belongs to the pattern, which a plan keeps)
-  if (!P->strict_checked && !P->onepass && P->ncnt[CLS_G32] >= kStrictRows &&
-      B->nnz >= kSeqRow * B->nrows && P->mults >= 8 * B->nnz) {
-    k_check_strict<PT, VT><<<grid_for(B->nnz, 1024, ctx->num_sms * 8), 256, 0, s>>>(
-        (const PT *)B->rowptr, B->col, B->nrows, P->sched + 2, prods);
-    ctx->launches += 1;
-    P->strict_checked = true;
-  }
   if (m == 0) {
     k_set_out<PT, VT><<<1, 1, 0, s>>>(prods, C->col, (VT *)C->val, C->rowptr,
                                       C->rowptr_bits);
@@ -313,8 +302,21 @@ static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P, const tspg_
     k_sched_offsets<<<1, 32, 0, s>>>(P->sched + 1);
     ctx->launches += 1;
   }
-  k_scatter<PT, VT, 1><<<grid_for(m, 256, INT32_MAX), 256, 0, s>>>(
-      prods, P->base, 1, m, P->rowf, P->rowc, P->cp, P->sched + 1, P->list, out);
+  // warp rows over long B rows take their span from the rows' ends, and add
+  // without atomics, when B's rows are sorted and hold no column twice: worth a
+  // pass over B's columns where they are many (in every call: a plan's operands
+  // have one pattern, but the order inside their rows is the call's; 27-point
+  // stencil on 63^3, 6.6M columns: beside the scatter, nothing of 1.64 ms)
+  const bool check = !P->onepass && P->ncnt[CLS_G32] >= kStrictRows &&
+                     B->nnz >= kSeqRow * B->nrows && P->mults >= 8 * B->nnz;
+  if (check) {
+    k_check_strict<PT, VT><<<grid_for(B->nnz, 2048, ctx->num_sms * 8), 256, 0, s>>>(
+        (const PT *)B->rowptr, B->col, B->nrows, P->sched + 2, prods);
+    ctx->launches += 1;
+  }
+  TSPG_CUDA(ctx, launch_phase(check, grid_for(m, 256, INT32_MAX), 256, 0, s, k_scatter<PT, VT, 1>,
+                              prods, P->base, 1, m, P->rowf, P->rowc, P->cp, P->sched + 1, P->list,
+                              out));
   PhaseArgs pa{P->base, P->sched + 1, P->list, P->rowf, P->rowc, P->cp,
                P->curbuf, P->cur_stride, ctx->d_words + kErrWord,
                ctx->d_prof ? ctx->d_prof + kProfPerPhase : nullptr};

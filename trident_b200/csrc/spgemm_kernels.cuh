@@ -360,20 +360,30 @@ __global__ void k_check_sorted_rows(const PT *Bp, const int32_t *Bj,
 
 // Are all of B's rows strictly increasing?  One streaming pass: the places
 // where a column is not above the one before it, less those between two rows,
-// are none.  rec: a zeroed record (its total and ticket are used).
+// are none.  rec: a record of zero total and ticket, left so.
 template <typename PT, typename VT>
 __global__ void __launch_bounds__(256)
     k_check_strict(const PT *__restrict__ Bp, const int32_t *__restrict__ Bj, int64_t nb, Sched *rec,
                    ProdDev<PT, VT> *prod) {
+  constexpr int U = 8;
+  phase_begin();
   const int64_t stride = int64_t(gridDim.x) * blockDim.x;
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
   const int64_t first = int64_t(Bp[0]), end = int64_t(Bp[nb]);
   int64_t n = 0;
-  for (int64_t q = first + t; q + 1 < end; q += stride * 4) {
+  for (int64_t q = first + t - lane; q + 1 < end; q += stride * U) {  // a warp's 32, uniform
+    int32_t c[U], z[U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int64_t p = q + u * stride;
-      if (p + 1 < end) n += __ldg(Bj + p) >= __ldg(Bj + p + 1);
+    for (int u = 0; u < U; ++u) {
+      const int64_t p = q + u * stride + lane;
+      c[u] = p < end ? __ldg(Bj + p) : 0;
+      z[u] = lane == 31 && p + 1 < end ? __ldg(Bj + p + 1) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int32_t up = __shfl_down_sync(0xffffffffu, c[u], 1);
+      n += q + u * stride + lane + 1 < end && c[u] >= (lane < 31 ? up : z[u]);
     }
   }
   for (int64_t r = t; r < nb; r += stride) {
@@ -382,8 +392,10 @@ __global__ void __launch_bounds__(256)
   }
   n = warp_sum(n);
   if ((threadIdx.x & 31) == 0 && n != 0) atomicAdd((unsigned long long *)&rec->total, (unsigned long long)n);
-  if (last_block(&rec->ticket) && threadIdx.x == 0)
+  if (last_block(&rec->ticket) && threadIdx.x == 0) {
     prod->b_strict = *(volatile int64_t *)&rec->total == 0;
+    rec->total = 0;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -771,6 +783,7 @@ __global__ void __launch_bounds__(256) k_scatter(
   }
   __syncthreads();
   if (c >= 0) list[s_base[c] + my] = (uint64_t(p) << 40) | uint64_t(r);
+  phase_end();
   if (MODE == 1 && out.finish && last_block(&S->ticket) && threadIdx.x == 0) sched_offsets(S);
 }
 
