@@ -277,3 +277,55 @@ def test_plan_whose_b_rows_change_their_order(ctx):
         check_product(plan.numeric(U.to_device(), dA), A, A)
         check_product(plan.numeric(dA, dA), A, A)
     plan.close()
+
+
+def _heavy_product(rng):
+    """A product that keeps bitmaps: 66,000 rows, 1,500 of them DENSE."""
+    B = _rows(np.concatenate([np.full(600, 900), np.full(100, 3)]), 60000, rng)
+    lens = np.ones(66000, np.int64)
+    lens[rng.choice(66000, size=1500, replace=False)] = 40
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    col = np.concatenate([np.sort(rng.choice(600, size=k, replace=False)) if k > 1 else [600 + i % 100]
+                          for i, k in enumerate(lens)]).astype(np.int32)
+    return HostCSR(66000, 700, rp, col, rng.uniform(-1, 1, col.size)), B
+
+
+HEAVY = {"sym_lim": [512, 2048, 4096, 4096], "num_lim": [256, 1024, 2048, 2048]}
+
+
+@pytest.mark.parametrize("refuse", [0, 1])
+def test_output_refused_beside_kept_bitmaps(refuse):
+    # the allocator refuses its first or second request once: the bitmaps are
+    # given back and only what is missing is asked for again
+    import ctypes as C
+
+    import torch
+
+    from trident_b200._lib import ALLOC_FN, TspgCsrOut, check, lib
+    from trident_b200.csr import DeviceCSR
+    A, B = _heavy_product(np.random.default_rng(9))
+    dA, dB = A.to_device(rowptr_bits=64), B.to_device(rowptr_bits=64)
+    c = ops.Context(0)
+    c.set_tuning(HEAVY)
+    asked, blocks = [], {}
+
+    def alloc(user, nbytes, stream):
+        asked.append(nbytes)
+        if len(asked) == refuse + 1:
+            return None
+        t = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+        blocks[t.data_ptr()] = t
+        return t.data_ptr()
+
+    rp = torch.empty(A.nrows + 1, dtype=torch.int64, device="cuda")
+    o = TspgCsrOut()
+    o.nrows, o.ncols, o.rowptr, o.rowptr_bits, o.val_bits = A.nrows, B.ncols, rp.data_ptr(), 64, 64
+    o.alloc = ALLOC_FN(alloc)
+    a, b = dA.abi(), dB.abi()
+    check(lib.tspg_spgemm(c.h, torch.cuda.current_stream().cuda_stream, C.byref(a), C.byref(b), C.byref(o), 0),
+          "tspg_spgemm")
+    nnz = int(o.nnz)
+    assert asked == ([4 * nnz, 4 * nnz, 8 * nnz], [4 * nnz, 8 * nnz, 8 * nnz])[refuse]
+    check_product(DeviceCSR(A.nrows, B.ncols, rp, blocks[o.col].view(torch.int32), blocks[o.val].view(torch.float64),
+                            nnz=nnz), A, B)
+    c.close()
