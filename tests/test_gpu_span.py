@@ -329,3 +329,20 @@ def test_output_refused_beside_kept_bitmaps(refuse):
     check_product(DeviceCSR(A.nrows, B.ncols, rp, blocks[o.col].view(torch.int32), blocks[o.val].view(torch.float64),
                             nnz=nnz), A, B)
     c.close()
+
+
+@pytest.mark.parametrize("n,keeps", [(60_000, True), (1_000_000, False)])
+def test_bitmaps_are_kept_only_where_they_are_filled(n, keeps):
+    # at 1M columns the symbolic DENSE rows are no span rows: no room for bitmaps
+    # (125 KB a row) is taken.  1,500 rows' bitmaps are the larger part at 60,000.
+    A, B = _heavy_product(np.random.default_rng(9))
+    B = HostCSR(B.nrows, n, B.rowptr, (B.col.astype(np.int64) * (n // 60_000)).astype(np.int32), B.val)
+    c = ops.Context(0)
+    c.set_tuning(HEAVY)
+    C = ops.spgemm(c, A.to_device(rowptr_bits=64), B.to_device(rowptr_bits=64))
+    if n == 60_000:
+        check_product(C, A, B)
+    bits = 1500 * ((n + 1023) // 1024) * 128
+    rows = 66_000 * (28 + 4) + 12 * 32 * 66_000  # row arrays, slots, one-pass scratch
+    assert (c.mem()[1] >= bits) == keeps and c.mem()[1] < (bits if keeps else 0) + rows + (1 << 20)
+    c.close()

@@ -214,7 +214,7 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
     const int64_t dense = h[HW_CNT] + h[HW_CNT + 1] + h[HW_CNT + 2];
     const int64_t words = ((n + 1023) >> 10) * 32;
     const int64_t slots = std::min(dense, kKeepBytes / (words * 4));
-    if (slots >= kKeepRows && B->nnz <= kKeepNnz && n <= kRankMaxCols &&
+    if (slots >= kKeepRows && B->nnz <= kKeepNnz && n <= kRankMaxCols && sym_dense_span<PT, VT>(n) &&
         P->get(&P->slot, size_t(m)) == TSPG_OK && P->get(&P->bits, size_t(slots * words)) == TSPG_OK) {
       TSPG_CUDA(ctx, cudaMemsetAsync(P->slot, 0xff, size_t(m) * sizeof(int32_t), s));
       P->nslots = slots;

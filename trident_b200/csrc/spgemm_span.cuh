@@ -583,6 +583,13 @@ inline Tune span_tune(Tune t, int64_t ncols, bool addend) {
 // against 3.85 ms).  The numeric 512-thread rows replace rows that had an SM
 // to themselves, so one CTA is enough for them.
 //
+// The symbolic DENSE and G1024 rows are span rows (which can keep their bitmaps)
+// up to this width.
+template <typename PT, typename VT>
+inline bool sym_dense_span(int64_t ncols) {
+  return span_ctas<512>(span_layout<512, false, PT, VT>(ncols, 0)) >= 2;
+}
+
 // The persistent kernels of a symbolic phase (one-pass rows aside).
 template <typename PT, typename VT>
 inline int launch_symbolic_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, VT> *prods,
@@ -590,13 +597,13 @@ inline int launch_symbolic_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT,
   const SpanLay L1 = span_layout<128, false, PT, VT>(ncols, 0);
   const SpanLay L2 = span_layout<256, false, PT, VT>(ncols, 0);
   const SpanLay L3 = span_layout<512, false, PT, VT>(ncols, 0);
-  if (span_ctas<512>(L3) >= 2) {
+  if (sym_dense_span<PT, VT>(ncols)) {
     TSPG_CUDA(ctx, (launch_span<512, false, PT, VT>(ctx, s, prods, pa, L3, 0, CLS_G1024 + 1, false)));
   } else {
     k_phase<PT, VT, false><<<ctx->num_sms, kSymThreads, kDynSmem, s>>>(prods, pa);
     ctx->launches += 1;
   }
-  const bool overlap = may_overlap && span_ctas<512>(L3) >= 2;  // k_phase lets nothing start early
+  const bool overlap = may_overlap && sym_dense_span<PT, VT>(ncols);  // k_phase lets nothing start early
   if (span_ctas<256>(L2) >= 2) {
     TSPG_CUDA(ctx, (launch_span<256, false, PT, VT>(ctx, s, prods, pa, L2, CLS_G256, CLS_G256 + 1,
                                                     overlap)));
