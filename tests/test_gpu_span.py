@@ -346,3 +346,30 @@ def test_bitmaps_are_kept_only_where_they_are_filled(n, keeps):
     rows = 66_000 * (28 + 4) + 12 * 32 * 66_000  # row arrays, slots, one-pass scratch
     assert (c.mem()[1] >= bits) == keeps and c.mem()[1] < (bits if keeps else 0) + rows + (1 << 20)
     c.close()
+
+
+def test_budget_goes_to_the_cursors_before_the_kept_bitmaps():
+    # one A row longer than the cursors in shared memory: its buffer comes after
+    # the bitmaps were taken, and a budget that holds either must do
+    rng = np.random.default_rng(19)
+    A, B = _heavy_product(rng)
+    k = 8200
+    B = HostCSR(700 + k, 60000, np.concatenate([B.rowptr, np.full(k, B.rowptr[-1])]), B.col, B.val)
+    lens = np.diff(A.rowptr)
+    lens[-1] = k
+    A = HostCSR(66000, 700 + k, np.concatenate([[0], np.cumsum(lens)]).astype(np.int64),
+                np.concatenate([A.col[:A.rowptr[-2]], np.arange(700, 700 + k, dtype=np.int32)]),
+                rng.uniform(-1, 1, int(lens.sum())))
+    dA, dB = A.to_device(rowptr_bits=64), B.to_device(rowptr_bits=64)
+    c = ops.Context(0)
+    c.set_tuning(HEAVY)
+    check_product(ops.spgemm(c, dA, dB), A, B)
+    need, cursors = c.mem()[1], 2 * 148 * k * 4
+    bits, slots = 1500 * ((60000 + 1023) // 1024) * 128, -(-66000 * 4 // 256) * 256
+    assert need > bits + cursors
+    for budget in (need, need - 512, need - cursors, need - cursors - 512, need - bits - 256, need - bits - slots):
+        t = ops.Context(0, budget)
+        t.set_tuning(HEAVY)
+        check_product(ops.spgemm(t, dA, dB), A, B)
+        t.close()
+    c.close()

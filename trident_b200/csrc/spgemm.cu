@@ -83,7 +83,7 @@ struct tspg_plan {
   // Give up the kept bitmaps (the numeric phase then walks those rows twice).
   void drop_bits() {
     for (void *p : {(void *)bits, (void *)slot}) {
-      for (int i = 0; i < nblocks; ++i) {
+      for (int i = 0; p && i < nblocks; ++i) {
         if (blocks[i] != p) continue;
         ws_free(ctx, p, stream);
         blocks[i] = blocks[--nblocks];
@@ -214,11 +214,14 @@ static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
     const int64_t dense = h[HW_CNT] + h[HW_CNT + 1] + h[HW_CNT + 2];
     const int64_t words = ((n + 1023) >> 10) * 32;
     const int64_t slots = std::min(dense, kKeepBytes / (words * 4));
-    if (slots >= kKeepRows && B->nnz <= kKeepNnz && n <= kRankMaxCols && sym_dense_span<PT, VT>(n) &&
-        P->get(&P->slot, size_t(m)) == TSPG_OK && P->get(&P->bits, size_t(slots * words)) == TSPG_OK) {
-      TSPG_CUDA(ctx, cudaMemsetAsync(P->slot, 0xff, size_t(m) * sizeof(int32_t), s));
-      P->nslots = slots;
-      P->slot_words = words;
+    if (slots >= kKeepRows && B->nnz <= kKeepNnz && n <= kRankMaxCols && sym_dense_span<PT, VT>(n)) {
+      if (P->get(&P->slot, size_t(m)) == TSPG_OK && P->get(&P->bits, size_t(slots * words)) == TSPG_OK) {
+        TSPG_CUDA(ctx, cudaMemsetAsync(P->slot, 0xff, size_t(m) * sizeof(int32_t), s));
+        P->nslots = slots;
+        P->slot_words = words;
+      } else {
+        P->drop_bits();
+      }
     }
   }
   if (m >= kFuseRows) {
@@ -289,7 +292,13 @@ static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P, const tspg_
   }
   if (P->max_a_row > kDenseCurSmem && !P->curbuf) {
     P->cur_stride = P->max_a_row;
-    TSPG_TRY(P->get(&P->curbuf, 2 * size_t(ctx->num_sms) * P->cur_stride));
+    const size_t words = 2 * size_t(ctx->num_sms) * P->cur_stride;
+    int st = P->get(&P->curbuf, words);
+    if (st == TSPG_ENOMEM && P->nslots) {  // what the phase needs comes before the kept bitmaps
+      P->drop_bits();
+      st = P->get(&P->curbuf, words);
+    }
+    TSPG_TRY(st);
   }
   OutArgs out;
   out.Cj = C->col;
