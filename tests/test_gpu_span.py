@@ -293,10 +293,10 @@ def _heavy_product(rng):
 HEAVY = {"sym_lim": [512, 2048, 4096, 4096], "num_lim": [256, 1024, 2048, 2048]}
 
 
-@pytest.mark.parametrize("refuse", [0, 1])
+@pytest.mark.parametrize("refuse", [(0,), (1,), (1, 2)])
 def test_output_refused_beside_kept_bitmaps(refuse):
-    # the allocator refuses its first or second request once: the bitmaps are
-    # given back and only what is missing is asked for again
+    # the allocator refuses a request: the pool's free blocks, then the bitmaps
+    # are given back, and only what is missing is asked for again
     import ctypes as C
 
     import torch
@@ -311,7 +311,7 @@ def test_output_refused_beside_kept_bitmaps(refuse):
 
     def alloc(user, nbytes, stream):
         asked.append(nbytes)
-        if len(asked) == refuse + 1:
+        if len(asked) - 1 in refuse:
             return None
         t = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
         blocks[t.data_ptr()] = t
@@ -325,7 +325,7 @@ def test_output_refused_beside_kept_bitmaps(refuse):
     check(lib.tspg_spgemm(c.h, torch.cuda.current_stream().cuda_stream, C.byref(a), C.byref(b), C.byref(o), 0),
           "tspg_spgemm")
     nnz = int(o.nnz)
-    assert asked == ([4 * nnz, 4 * nnz, 8 * nnz], [4 * nnz, 8 * nnz, 8 * nnz])[refuse]
+    assert asked == [k * nnz for k in {(0,): [4, 4, 8], (1,): [4, 8, 8], (1, 2): [4, 8, 8, 8]}[refuse]]
     check_product(DeviceCSR(A.nrows, B.ncols, rp, blocks[o.col].view(torch.int32), blocks[o.val].view(torch.float64),
                             nnz=nnz), A, B)
     c.close()

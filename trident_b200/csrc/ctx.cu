@@ -41,6 +41,28 @@ void ws_free(tspg_ctx *ctx, void *p, cudaStream_t s) {
   cudaFreeAsync(p, s);
 }
 
+int ensure_out(tspg_ctx *ctx, tspg_csr_out *C, int64_t nnz, int vbytes, cudaStream_t s,
+               OutBlocks *got) {
+  C->nnz = nnz;
+  if (C->capacity >= nnz) return TSPG_OK;
+  if (!C->alloc) return TSPG_ENOMEM;
+  OutBlocks one;
+  if (!got) got = &one;
+  for (int again = 0; again < 2 && !got->val; ++again) {
+    if (again) {
+      cudaStreamSynchronize(s);
+      cudaMemPoolTrimTo(ctx->pool, 0);  // blocks in use stay
+    }
+    if (!got->col) got->col = C->alloc(C->alloc_user, size_t(nnz) * 4, s);
+    if (got->col) got->val = C->alloc(C->alloc_user, size_t(nnz) * vbytes, s);
+  }
+  if (!got->val) return TSPG_ENOMEM;
+  C->col = (int32_t *)got->col;
+  C->val = got->val;
+  C->capacity = nnz;
+  return TSPG_OK;
+}
+
 }  // namespace tspg
 
 using namespace tspg;

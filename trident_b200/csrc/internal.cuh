@@ -119,6 +119,19 @@ inline void phase_mark(tspg_ctx *ctx, int k, int edge, cudaStream_t s) {
 int ws_alloc(tspg_ctx *ctx, void **p, size_t bytes, cudaStream_t s);
 void ws_free(tspg_ctx *ctx, void *p, cudaStream_t s);
 
+// Output capacity: use the caller's buffers, grow through its allocator, or
+// report the needed size (CsxBuffers::ensure_async semantics).  When the
+// allocator refuses, the pool's free blocks go back to the device (it keeps
+// what earlier calls used, 4 GB of bitmaps among it) and it is asked once more
+// for what is missing.  got: what an attempt that failed was given, for the
+// next one (an allocator frees nothing: a block asked for twice is held twice).
+// The columns come first, the values only after them.
+struct OutBlocks {
+  void *col = nullptr, *val = nullptr;
+};
+int ensure_out(tspg_ctx *ctx, tspg_csr_out *C, int64_t nnz, int vbytes, cudaStream_t s,
+               OutBlocks *got = nullptr);
+
 // RAII list of workspace blocks released at scope exit on one stream.
 struct Scratch {
   tspg_ctx *ctx;

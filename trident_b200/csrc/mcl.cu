@@ -261,15 +261,7 @@ static int prune_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, double t
   const int64_t nnz = h[0];
   out->nnz = nnz;
   if (out->rowptr_bits == 32 && nnz > INT32_MAX) return TSPG_EOVERFLOW;
-  if (out->capacity < nnz) {
-    if (!out->alloc) return TSPG_ENOMEM;
-    void *cj = out->alloc(out->alloc_user, size_t(nnz) * 4, s);
-    void *cx = out->alloc(out->alloc_user, size_t(nnz) * sizeof(VT), s);
-    if (!cj || !cx) return TSPG_ENOMEM;
-    out->col = (int32_t *)cj;
-    out->val = cx;
-    out->capacity = nnz;
-  }
+  TSPG_TRY(ensure_out(ctx, out, nnz, int(sizeof(VT)), s));
   // (refused by the budget: the tiles' CTAs walk their rows)
   uint16_t *pos = nullptr;
   if (h[1] && sc.get(&pos, size_t(M->nnz)) != TSPG_OK) pos = nullptr;

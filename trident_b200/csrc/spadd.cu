@@ -379,16 +379,7 @@ static int spadd_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
   const int64_t nnz = h[0];
   if (h[1] || (strict && h[2])) return TSPG_EUNSORTED;
   if (C->rowptr_bits == 32 && nnz > INT32_MAX) return TSPG_EOVERFLOW;
-  C->nnz = nnz;
-  if (C->capacity < nnz) {
-    if (!C->alloc) return TSPG_ENOMEM;
-    void *cj = C->alloc(C->alloc_user, size_t(nnz) * 4, s);
-    void *cx = C->alloc(C->alloc_user, size_t(nnz) * sizeof(VT), s);
-    if (!cj || !cx) return TSPG_ENOMEM;
-    C->col = (int32_t *)cj;
-    C->val = cx;
-    C->capacity = nnz;
-  }
+  TSPG_TRY(ensure_out(ctx, C, nnz, int(sizeof(VT)), s));
   // (refused by the budget: the tiles' CTAs walk their rows)
   uint16_t *pos = nullptr;
   if (h[3] && sc.get(&pos, size_t(total)) != TSPG_OK) pos = nullptr;

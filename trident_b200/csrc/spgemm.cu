@@ -346,29 +346,6 @@ static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P, const tspg_
   return TSPG_OK;
 }
 
-// Output capacity: use the caller's buffers, grow through its allocator, or
-// report the needed size (CsxBuffers::ensure_async semantics).  got: what the
-// allocator gave in an attempt that failed, for the next one (an allocator
-// frees nothing, so a block asked for twice is held twice).
-struct OutBlocks {
-  void *col = nullptr, *val = nullptr;
-};
-static int ensure_out(tspg_csr_out *C, int64_t nnz, int vbytes, cudaStream_t s,
-                      OutBlocks *got = nullptr) {
-  C->nnz = nnz;
-  if (C->capacity >= nnz) return TSPG_OK;
-  if (!C->alloc) return TSPG_ENOMEM;
-  OutBlocks one;
-  if (!got) got = &one;
-  if (!got->col) got->col = C->alloc(C->alloc_user, size_t(nnz) * 4, s);
-  if (got->col && !got->val) got->val = C->alloc(C->alloc_user, size_t(nnz) * vbytes, s);
-  if (!got->val) return TSPG_ENOMEM;
-  C->col = (int32_t *)got->col;
-  C->val = got->val;
-  C->capacity = nnz;
-  return TSPG_OK;
-}
-
 static int check_pair(const tspg_csr *A, const tspg_csr *B) {
   TSPG_TRY(check_csr(A));
   TSPG_TRY(check_csr(B));
@@ -486,7 +463,7 @@ extern "C" int tspg_spgemm_numeric(tspg_ctx *ctx, void *stream,
   if (C->rowptr_bits == 32 && plan->c_nnz > INT32_MAX) return TSPG_EOVERFLOW;
   cudaStream_t s = (cudaStream_t)stream;
   TSPG_CUDA(ctx, cudaSetDevice(ctx->device));
-  TSPG_TRY(ensure_out(C, plan->c_nnz, plan->vt_bits / 8, s));
+  TSPG_TRY(ensure_out(ctx, C, plan->c_nnz, plan->vt_bits / 8, s));
   // the plan's prods descriptor points at the symbolic call's operands; the
   // numeric call may pass new value arrays of the same pattern
   return dispatch(plan->pt_bits, plan->vt_bits, [&](auto pt, auto vt) {
@@ -521,13 +498,11 @@ extern "C" int tspg_spgemm(tspg_ctx *ctx, void *stream, const tspg_csr *A,
   int st = TSPG_OK;
   if (C->rowptr_bits == 32 && nnz > INT32_MAX) st = TSPG_EOVERFLOW;
   OutBlocks got;
-  if (st == TSPG_OK) st = ensure_out(C, nnz, A->val_bits / 8, (cudaStream_t)stream, &got);
+  if (st == TSPG_OK) st = ensure_out(ctx, C, nnz, A->val_bits / 8, (cudaStream_t)stream, &got);
   if (st == TSPG_ENOMEM && C->alloc && plan->nslots) {
-    // the output comes first: hand the kept bitmaps back to the device
+    // the output comes before the kept bitmaps
     plan->drop_bits();
-    cudaStreamSynchronize((cudaStream_t)stream);
-    cudaMemPoolTrimTo(ctx->pool, ctx->in_use);
-    st = ensure_out(C, nnz, A->val_bits / 8, (cudaStream_t)stream, &got);
+    st = ensure_out(ctx, C, nnz, A->val_bits / 8, (cudaStream_t)stream, &got);
   }
   if (st == TSPG_OK) {
     st = dispatch(plan->pt_bits, plan->vt_bits, [&](auto pt, auto vt) {

@@ -208,21 +208,6 @@ __global__ void k_copy_segs(const int64_t *tp, const int64_t *longseg, int64_t n
   }
 }
 
-// Room for `nnz` entries in T: the caller's buffers or its allocator.
-template <typename VT>
-static int ensure_entries(tspg_csr_out *T, int64_t nnz, cudaStream_t s) {
-  T->nnz = nnz;
-  if (T->capacity >= nnz) return TSPG_OK;
-  if (!T->alloc) return TSPG_ENOMEM;
-  void *cj = T->alloc(T->alloc_user, size_t(nnz) * 4, s);
-  void *cx = T->alloc(T->alloc_user, size_t(nnz) * sizeof(VT), s);
-  if (!cj || !cx) return TSPG_ENOMEM;
-  T->col = (int32_t *)cj;
-  T->val = cx;
-  T->capacity = nnz;
-  return TSPG_OK;
-}
-
 // Transpose by stable counting-sort passes over the column index.  *done =
 // false (nothing launched) when the matrix has no entries or too many for
 // 32-bit positions, or when the workspace is refused: the segment sort below
@@ -244,7 +229,7 @@ static int transpose_passes(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, ts
                  part(&P.dtotal, 1 << kPartBits), part(&idx, more), part(&val, more)) != TSPG_OK)
     return TSPG_OK;
   *done = true;
-  TSPG_TRY(ensure_entries<VT>(T, nnz, s));
+  TSPG_TRY(ensure_out(ctx, T, nnz, int(sizeof(VT)), s));
   PartSpan S;
   S.count = nnz;
   S.rp = M->rowptr;
@@ -307,7 +292,7 @@ static int transpose_segments(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, 
     k_scan_final<<<(unsigned)nb, kScanThreads, 0, s>>>(cnt, n, partial, nb, tp, dummy, nullptr);
   }
   ctx->launches += (m > 0 && nnz > 0) + (n > 0 ? 3 : 0);
-  TSPG_TRY(ensure_entries<VT>(T, nnz, s));
+  TSPG_TRY(ensure_out(ctx, T, nnz, int(sizeof(VT)), s));
   if (m > 0 && nnz > 0) {
     if (seq)
       k_seq_scatter<VT><<<ge, 256, 0, s>>>(M->col, (const VT *)M->val, nnz, tp, cursor, T->col,
@@ -446,7 +431,7 @@ static int coo_passes(tspg_ctx *ctx, cudaStream_t s, int64_t nmaj, int64_t nmin,
       TSPG_CUDA(ctx, cudaMemcpyAsync(h, bad, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
       TSPG_CUDA(ctx, cudaStreamSynchronize(s));
       if (h[0] != 0) return TSPG_EINVAL;
-      TSPG_TRY(ensure_entries<VT>(out, nnz, s));
+      TSPG_TRY(ensure_out(ctx, out, nnz, int(sizeof(VT)), s));
       x[1] = out->col;
       v[1] = (VT *)out->val;
       checked = true;
