@@ -88,3 +88,30 @@ def test_refused_once_and_asked_again(call, refuse):
         assert status == 0
         check(hook.result(o))
     ctx.close()
+
+
+def test_transpose_output_does_not_wait_for_the_workspace():
+    # an allocator with room for the output, but not beside 24 bytes an entry
+    ctx = ops.Context(0)
+    A = random_csr(500, 800, per_row=400, seed=4)
+    keep, calls = _calls(ctx, A, A)
+    m, n, run, check = calls["transpose"]
+
+    class Tight(Hook):
+        def _alloc(self, user, nbytes, stream):
+            if ctx.mem()[0] > 8 * A.nnz:
+                self.refuse = (len(self.asked),)
+            return super()._alloc(user, nbytes, stream)
+
+    hook = Tight(())
+    o = hook.out(m, n)
+    assert run(o) == 0
+    check(hook.result(o))
+    # and a budget that only the segment sort fits
+    ref = hook.result(o).to_host()
+    small = ops.Context(0, 12 * A.nnz)
+    got = ops.transpose(small, A.to_device()).to_host()
+    for x, y in ((got.rowptr, ref.rowptr), (got.col, ref.col), (got.val, ref.val)):
+        np.testing.assert_array_equal(x, y)
+    small.close()
+    ctx.close()

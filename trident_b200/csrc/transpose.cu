@@ -225,11 +225,13 @@ static int transpose_passes(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *M, ts
   VT *val = nullptr;
   const int64_t more = passes > 1 ? nnz : 0;
   part_sizes(nnz, &P);
+  // the output first: what room it leaves decides between the passes and the
+  // segment sort, not the other way round
+  TSPG_TRY(ensure_out(ctx, T, nnz, int(sizeof(VT)), s));
   if (sc.get_all(part(&rows, nnz), part(&key, nnz), part(&P.table, P.table_len),
                  part(&P.dtotal, 1 << kPartBits), part(&idx, more), part(&val, more)) != TSPG_OK)
     return TSPG_OK;
   *done = true;
-  TSPG_TRY(ensure_out(ctx, T, nnz, int(sizeof(VT)), s));
   PartSpan S;
   S.count = nnz;
   S.rp = M->rowptr;
