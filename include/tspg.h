@@ -147,7 +147,12 @@ int tspg_ctx_phase_ms(tspg_ctx *ctx, float *symbolic_ms, float *numeric_ms);
  * above the last bound are DENSE rows.  hash_load = hash-table slots per key
  * (2, 4 or 8).  Bounds must be positive, non-decreasing and at most the table
  * capacities sym <= {512, 2048, 4096, 24576}, num <= {256, 1024, 2048, 8192}
- * (the defaults); otherwise TSPG_EINVAL.  dense_win_log2: numeric DENSE
+ * (the defaults); otherwise TSPG_EINVAL.  num_lim[0] and num_lim[3] at their
+ * defaults leave these two bounds to the library, which lowers them to 192 and
+ * 4096 for the matrix widths at which that measured faster; any other value
+ * holds as given.  Numeric rows of at most 27 outputs go by single lanes, and
+ * rows of many products on few columns take a group wider than their bound
+ * asks for, whatever the bounds.  dense_win_log2: numeric DENSE
  * rows with at least 2^dense_win_log2 products, an output filling at least
  * 1/2^dense_win_fill_log2 of the columns and sorted B rows take the
  * column-window form (a shared-memory FP64 accumulator per window of

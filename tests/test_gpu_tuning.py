@@ -148,3 +148,31 @@ def test_plan_keeps_the_tuning_it_was_made_with(tctx, made, now):
         check_product(_poisoned_numeric(plan, dA, dB), A, B)
     plan.close()
     check_product(ops.spgemm(tctx, dA, dB), A, B)
+
+
+@pytest.mark.parametrize("bounds,cls", [([256, 1024, 2048, 8192], 5), ([255, 1024, 2048, 8192], 6),
+                                        ([200, 1024, 2048, 8192], 6), ([199, 1024, 2048, 8192], 5)])
+def test_bounds_of_the_caller_hold(tctx, bounds, cls):
+    # rows of 200 outputs: warp rows (class 6) up to the caller's bound; at the
+    # default the library picks 192 for this width (class 5, 128 threads)
+    import ctypes as C
+
+    import numpy as np
+
+    from trident_b200._lib import check, lib
+    from trident_b200.csr import HostCSR
+    rng = np.random.default_rng(2)
+    col = np.concatenate([np.sort(rng.choice(3000, size=100, replace=False)) for _ in range(40)]).astype(np.int32)
+    for i in range(0, 40, 2):  # rows 2i and 2i + 1 share no column
+        both = np.sort(rng.choice(3000, size=200, replace=False)).astype(np.int32)
+        col[i * 100:(i + 1) * 100], col[(i + 1) * 100:(i + 2) * 100] = both[::2], both[1::2]
+    B = HostCSR(40, 3000, np.arange(41, dtype=np.int64) * 100, col, rng.uniform(-1, 1, col.size))
+    acol = ((np.arange(2000) % 20)[:, None] * 2 + np.arange(2)).ravel().astype(np.int32)
+    A = HostCSR(2000, 40, np.arange(2001, dtype=np.int64) * 2, acol, rng.uniform(-1, 1, 4000))
+    tctx.set_tuning({"num_lim": bounds})
+    check(lib.tspg_ctx_class_profile(tctx.h, 1), "tspg_ctx_class_profile")
+    check_product(ops.spgemm(tctx, A.to_device(), B.to_device()), A, B)
+    out = (C.c_uint64 * 64)()
+    check(lib.tspg_ctx_class_cycles(tctx.h, out), "tspg_ctx_class_cycles")
+    check(lib.tspg_ctx_class_profile(tctx.h, 0), "tspg_ctx_class_profile")
+    assert [out[32 + 8 + c] for c in (5, 6)] == [2000 * (c == cls) for c in (5, 6)]

@@ -552,7 +552,8 @@ inline cudaError_t launch_span(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, 
 // rank form's bitmap, or taken by the window form of the tuning.
 inline bool needs_sorted(const Tune &t, int64_t ncols) { return ncols > kRankMaxCols || t.win != 0; }
 
-// The row binning of a run.  While the bitmap of 128-thread span rows stays
+// The row binning of a run: the caller's, where a bound at its default (the
+// table's capacity) leaves the choice to the width.  While the bitmap of 128-thread span rows stays
 // small (8 CTAs per SM), numeric rows of more than kSpanWarpRow outputs leave
 // the warps for them.  Uniform rows of order 1024 with ~250 outputs: numeric
 // 49 -> 15 us; Poisson(15) of order 100k (~225 outputs) 0.55 -> 0.48 ms, of
@@ -568,9 +569,9 @@ constexpr int32_t kSpanHalfRow = 4096;
 template <typename PT, typename VT>
 inline Tune span_tune(Tune t, int64_t ncols, bool addend) {
   t.lane = addend ? 0 : kLaneSlots;  // lane rows take no addend
-  if (ncols <= kSpanWarpCols && t.num[0] > kSpanWarpRow && t.num[1] >= t.num[0])
+  if (ncols <= kSpanWarpCols && t.num[0] == kNumLim32 && t.num[1] >= t.num[0])
     t.num[0] = kSpanWarpRow;
-  if (t.num[3] > kSpanHalfRow && t.num[2] <= kSpanHalfRow && ncols <= kRankMaxCols &&
+  if (t.num[3] == kNumLim1024 && t.num[2] <= kSpanHalfRow && ncols <= kRankMaxCols &&
       span_ctas<512>(span_layout<512, true, PT, VT>(ncols, uint32_t(t.num[3]))) < 2 &&
       span_ctas<512>(span_layout<512, true, PT, VT>(ncols, uint32_t(kSpanHalfRow))) >= 2)
     t.num[3] = kSpanHalfRow;

@@ -12,7 +12,8 @@ descent on a representative workload, timing every candidate with CUDA events
      "num_lim": [...], "hash_load": k}, "ms": best, "default_ms": ...,
      "trials": [[tuning, ms], ...]}
 
-`Context.load_tuning(path)` applies such a file; bench.py applies the
+num_lim[0] and num_lim[3] at their caps leave these two bounds to the library
+(it lowers them by the matrix width).  `Context.load_tuning(path)` applies such a file; bench.py applies the
 committed file of its workload.  Results do not depend on the tuning (the
 GPU tests check that); only the speed does.
 
