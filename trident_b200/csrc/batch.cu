@@ -217,7 +217,7 @@ template <typename PT, typename VT>
 static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
   tspg_ctx *ctx = b->ctx;
   const int nprod = (int)b->A.size();
-  TSPG_TRY((set_smem_attr<PT, VT>(ctx->device)));
+  TSPG_TRY((set_smem_attr<PT, VT>(ctx)));
   // the cluster form must be launchable before it is captured (k_phase leaves
   // its rows alone)
   if (ctx->tune.cluster && cluster_slots<PT, VT>(ctx->device, ctx->tune.cluster) <= 0)

@@ -65,6 +65,10 @@ struct tspg_ctx {
   int64_t *h_words = nullptr;
   // device words: error flag and small counters that live with the context
   int64_t *d_words = nullptr;
+  // kernels whose shared-memory limit this context has raised (set_smem_attr's
+  // four instantiations, then the counting-sort scatter's four); the device
+  // forgets them with its primary context, which a context does not outlive
+  uint32_t smem_raised = 0;
   std::unordered_map<void *, size_t> live;
   std::mutex live_mu;  // ws_alloc / ws_free may be called from a releasing thread
   // instrumentation

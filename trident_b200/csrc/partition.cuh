@@ -353,13 +353,11 @@ inline int part_pass_t(tspg_ctx *ctx, cudaStream_t s, const PartScratch &P, cons
                        bool source, int shift, int bits, const int32_t *key, const int32_t *idx, const VT *val,
                        int32_t *okey, int32_t *oidx, VT *oval) {
   constexpr uint32_t bytes = part_smem<ITEMS, VT>();
-  constexpr int kMaxDev = 64;
-  static bool done[kMaxDev] = {};  // per device and instantiation; benign if raced
-  const bool cached = ctx->device >= 0 && ctx->device < kMaxDev;
-  if (!cached || !done[ctx->device]) {
+  const uint32_t mine = 16u << ((ITEMS == 16 ? 2 : 0) + (sizeof(VT) == 8 ? 1 : 0));
+  if (!(ctx->smem_raised & mine)) {
     TSPG_CUDA(ctx, cudaFuncSetAttribute(k_part_scatter<ITEMS, VT>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    if (cached) done[ctx->device] = true;
+    ctx->smem_raised |= mine;
   }
   const unsigned g = unsigned(P.ntiles);
   k_part_count<ITEMS><<<g, kPartThreads, 0, s>>>(key, S, source, shift, bits, P.table);

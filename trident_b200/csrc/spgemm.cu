@@ -135,7 +135,7 @@ static inline unsigned grid_for(int64_t work, int per_block, int cap) {
 template <typename PT, typename VT>
 static int symbolic_impl(tspg_ctx *ctx, cudaStream_t s, const tspg_csr *A,
                          const tspg_csr *B, int flags, tspg_plan *P) {
-  TSPG_TRY(set_smem_attr<PT, VT>(ctx->device));
+  TSPG_TRY(set_smem_attr<PT, VT>(ctx));
   const int64_t m = A->nrows, n = B->ncols, k = A->ncols;
   const Tune tune = P->tune = span_tune<PT, VT>(ctx->tune, n, P->E.col && P->E.nnz > 0);
   P->m = m;

@@ -715,13 +715,12 @@ inline int launch_numeric_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, 
 }
 
 // Dynamic shared-memory limits of the persistent kernels (a per-device
-// attribute of each kernel; the caller has made ctx->device current).
+// attribute of each kernel; the caller has made ctx->device current), raised
+// once by each context.
 template <typename PT, typename VT>
-inline int set_smem_attr(int device) {
-  constexpr int kMaxDev = 64;
-  static bool done[kMaxDev] = {};  // per device and instantiation; benign if raced
-  const bool cached = device >= 0 && device < kMaxDev;
-  if (cached && done[device]) return TSPG_OK;
+inline int set_smem_attr(tspg_ctx *ctx) {
+  const uint32_t mine = 1u << ((sizeof(PT) == 8 ? 2 : 0) + (sizeof(VT) == 8 ? 1 : 0));
+  if (ctx->smem_raised & mine) return TSPG_OK;
   auto raise = [](auto *k, int bytes) {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
   };
@@ -734,7 +733,7 @@ inline int set_smem_attr(int device) {
       !raise(k_span<256, true, PT, VT>, kSpanSmemMax) ||
       !raise(k_span<512, true, PT, VT>, kSpanSmemMax))
     return TSPG_ECUDA;
-  if (cached) done[device] = true;
+  ctx->smem_raised |= mine;
   return TSPG_OK;
 }
 
