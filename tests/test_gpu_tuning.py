@@ -176,3 +176,42 @@ def test_bounds_of_the_caller_hold(tctx, bounds, cls):
     check(lib.tspg_ctx_class_cycles(tctx.h, out), "tspg_ctx_class_cycles")
     check(lib.tspg_ctx_class_profile(tctx.h, 0), "tspg_ctx_class_profile")
     assert [out[32 + 8 + c] for c in (5, 6)] == [2000 * (c == cls) for c in (5, 6)]
+
+
+def _class_rows(ctx, run):
+    """Numeric rows per class (DENSE0..2, G1024, G256, G128, G32, LANE) of a call."""
+    import ctypes as C
+
+    from trident_b200._lib import check, lib
+    check(lib.tspg_ctx_class_profile(ctx.h, 1), "tspg_ctx_class_profile")
+    run()
+    out = (C.c_uint64 * 64)()
+    check(lib.tspg_ctx_class_cycles(ctx.h, out), "tspg_ctx_class_cycles")
+    check(lib.tspg_ctx_class_profile(ctx.h, 0), "tspg_ctx_class_profile")
+    return [int(x) for x in out[40:48]]
+
+
+def _alike_rows(m, na, cols, groups=20):
+    """m rows of na * cols products on the same `cols` columns."""
+    import numpy as np
+
+    from trident_b200.csr import HostCSR
+    rng = np.random.default_rng(m + na)
+    base = np.sort(rng.choice(3 * cols, size=cols, replace=False))
+    col = (np.repeat(np.arange(groups), na * cols) * 3 * cols + np.tile(base, groups * na)).astype(np.int32)
+    B = HostCSR(groups * na, groups * 3 * cols, np.arange(groups * na + 1, dtype=np.int64) * cols, col,
+                rng.uniform(-1, 1, col.size))
+    g = np.arange(m) * groups // m
+    A = HostCSR(m, groups * na, np.arange(m + 1, dtype=np.int64) * na,
+                (g[:, None] * na + np.arange(na)).ravel().astype(np.int32), rng.uniform(-1, 1, m * na))
+    return A, B
+
+
+@pytest.mark.parametrize("m,na,cols,cls", [(3000, 24, 100, 5), (4000, 24, 100, 6), (1500, 25, 400, 4), (2000, 25, 400, 5),
+                                           (300, 21, 100, 5), (300, 20, 100, 6)])
+def test_wider_rows_only_where_the_others_do_not_cover_them(tctx, m, na, cols, cls):
+    # rows of 2,400 and 10,000 products on 100 and 400 columns: as many as the chip
+    # has warps (3,552) or 128-thread groups (1,776), or fewer
+    A, B = _alike_rows(m, na, cols)
+    rows = _class_rows(tctx, lambda: check_product(ops.spgemm(tctx, A.to_device(), B.to_device()), A, B))
+    assert rows[cls] == m and sum(rows) == m

@@ -94,14 +94,31 @@ constexpr int kHeavyPeriod = 64;
 __host__ __device__ inline int dense_sub(int64_t f) {
   return f >= (int64_t(1) << 20) ? CLS_DENSE0 : f >= (int64_t(1) << 17) ? CLS_DENSE1 : CLS_DENSE2;
 }
+// How a run's totals bear on a row's class (set with the list offsets).
+struct RowRule {
+  // products above which a warp, 128- or 256-thread row is worked by more threads
+  int64_t wide32 = 2048, wide128 = 8192, wide256 = 32768;
+};
 // A group row by its products: many products on few columns (hub rows of a
 // small matrix) take more threads than their table asks for.  R-MAT of order
 // 1318 (FP32): 128-thread rows of 10^4 products were the call (0.17 ms).
-__host__ __device__ inline int wide_class(int c, int64_t f) {
-  if (c == CLS_G32 && f > 2048) c = CLS_G128;
-  if (c == CLS_G128 && f > 8192) c = CLS_G256;
-  if (c == CLS_G256 && f > 32768) c = CLS_G1024;
+__host__ __device__ inline int wide_class(int c, int64_t f, const RowRule &r = RowRule()) {
+  if (c == CLS_G32 && f > r.wide32) c = CLS_G128;
+  if (c == CLS_G128 && f > r.wide128) c = CLS_G256;
+  if (c == CLS_G256 && f > r.wide256) c = CLS_G1024;
   return c;
+}
+// ... in the numeric phase only while the row is more than its share of the
+// run's products, so that the others do not cover it: 24, 12 and 6 such groups
+// per SM.  70,000 rows of 2,400 products and 150 outputs: warps 1.21 ms, 128
+// threads each 1.92; 5,000 rows of 6,080 and 190: 0.29 and 0.38 ms.
+__device__ inline RowRule row_rule(int64_t products) {
+  constexpr int64_t kSms = 148;
+  RowRule r;
+  r.wide32 = max(r.wide32, products / (kSms * 24));
+  r.wide128 = max(r.wide128, products / (kSms * 12));
+  r.wide256 = max(r.wide256, products / (kSms * 6));
+  return r;
 }
 __host__ __device__ inline int sym_class(int64_t f, int64_t n, const Tune &t) {
   const int64_t fe = f < n ? f : n;
@@ -135,12 +152,12 @@ __host__ __device__ inline int64_t onepass_bound(int64_t f, int64_t n, const Tun
   const int64_t fe = f < n ? f : n;
   return onepass_full(f, n, t) ? fe : kCappedCols;
 }
-__host__ __device__ inline int num_class(int64_t c, int64_t f, const Tune &t) {
+__host__ __device__ inline int num_class(int64_t c, int64_t f, const Tune &t, const RowRule &r) {
   if (c == 0 || f < 0) return -1;  // f < 0: a one-pass row, already computed
   if (c <= t.lane) return CLS_LANE;
-  if (c <= t.num[0]) return wide_class(CLS_G32, f);
-  if (c <= t.num[1]) return wide_class(CLS_G128, f);
-  if (c <= t.num[2]) return wide_class(CLS_G256, f);
+  if (c <= t.num[0]) return wide_class(CLS_G32, f, r);
+  if (c <= t.num[1]) return wide_class(CLS_G128, f, r);
+  if (c <= t.num[2]) return wide_class(CLS_G256, f, r);
   if (c <= t.num[3]) return CLS_G1024;
   return dense_sub(f);
 }
@@ -183,6 +200,7 @@ __device__ __forceinline__ void addend_row(const ProdDev<PT, VT> &P, int64_t r, 
 
 // Work schedule of one phase: rows per class, their list offsets and the
 // work-item prefix the persistent kernel decodes.
+// A run's numeric record follows its symbolic one in memory.
 struct Sched {
   Tune tune;  // row binning of this run, set by k_set_tune after the reset
   int64_t cnt[NCLS];
@@ -203,6 +221,7 @@ struct Sched {
   int32_t rank_left;            // DENSE rows that kernel left to k_phase (0 / 1)
   int32_t pad32b;
   unsigned long long nlong;     // A rows left to k_row_mults_long
+  RowRule rule;                 // symbolic record: for the numeric classes
 };
 
 __device__ __forceinline__ int find_prod(const int64_t *base, int nprod,
@@ -306,6 +325,7 @@ __device__ __forceinline__ void sched_offsets(Sched *S) {
   S->work2 = 0;
   S->work3 = 0;
   S->rank_left = 0;
+  S->rule = row_rule(*(volatile int64_t *)&S->total);
 }
 
 // int32 row offsets widened to int64 (operands of mixed offset widths).
@@ -742,7 +762,7 @@ __global__ void __launch_bounds__(256) k_scatter(
       c = sym_class(rowf[g], prods[p].n, S->tune);
       if (S->onepass && rowc[g] > 0) c = CLS_ONEPASS;  // the count pass's choice (bound > 0)
     } else {
-      c = num_class(rowc[g], rowf[g], S->tune);
+      c = num_class(rowc[g], rowf[g], S->tune, S[-1].rule);
       const int64_t off = cp[g] - cp[base[p]];
       void *const Cp = out.set ? out.Cp : prods[p].Cp;
       const bool narrow = (out.set ? out.cp_bits : prods[p].cp_bits) == 32;
@@ -907,7 +927,7 @@ static __global__ void __launch_bounds__(kScanThreads)
     v[i] = (j0 + i < R) ? in[j0 + i] : 0;
     s += v[i];
     if (rowf && v[i] > 0) {
-      const int c = num_class(v[i], rowf[j0 + i], Snum->tune);
+      const int c = num_class(v[i], rowf[j0 + i], Snum->tune, Snum[-1].rule);
       if (c >= 0) packed += 1u << (4 * c);
     }
   }
