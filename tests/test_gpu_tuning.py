@@ -215,3 +215,14 @@ def test_wider_rows_only_where_the_others_do_not_cover_them(tctx, m, na, cols, c
     A, B = _alike_rows(m, na, cols)
     rows = _class_rows(tctx, lambda: check_product(ops.spgemm(tctx, A.to_device(), B.to_device()), A, B))
     assert rows[cls] == m and sum(rows) == m
+
+
+@pytest.mark.parametrize("m,na,cls", [(4000, 1, 7), (4000, 2, 6), (19_000, 9, 7), (19_000, 10, 6), (38_000, 60, 7)])
+def test_lane_rows_want_warps_full_of_rows(tctx, m, na, cls):
+    # rows of 20 products and more on 20 columns: by lanes while the rows to a
+    # warp (of 2,368) make up for a lane's time a product
+    A, B = _alike_rows(m, na, 20, groups=10)
+    p = ops.Plan(tctx, A.to_device(), B.to_device())
+    rows = _class_rows(tctx, lambda: check_product(p.numeric(A.to_device(), B.to_device()), A, B))
+    p.close()
+    assert rows[cls] == m and sum(rows) == m

@@ -98,6 +98,7 @@ __host__ __device__ inline int dense_sub(int64_t f) {
 struct RowRule {
   // products above which a warp, 128- or 256-thread row is worked by more threads
   int64_t wide32 = 2048, wide128 = 8192, wide256 = 32768;
+  int64_t lane = INT64_MAX;  // ... up to which a row of few outputs is a lane row
 };
 // A group row by its products: many products on few columns (hub rows of a
 // small matrix) take more threads than their table asks for.  R-MAT of order
@@ -112,12 +113,18 @@ __host__ __device__ inline int wide_class(int c, int64_t f, const RowRule &r = R
 // run's products, so that the others do not cover it: 24, 12 and 6 such groups
 // per SM.  70,000 rows of 2,400 products and 150 outputs: warps 1.21 ms, 128
 // threads each 1.92; 5,000 rows of 6,080 and 190: 0.29 and 0.38 ms.
-__device__ inline RowRule row_rule(int64_t products) {
-  constexpr int64_t kSms = 148;
+//
+// Lane rows want 32 rows a warp to be worth it (k_lanes has 16 warps per SM):
+// with r rows to a warp they take ~130 issue slots a product of the longest
+// row, single warps ~1500 a row and 8 a product.  20,000 rows (8.4 to a warp):
+// 144 products 59 us by lanes and 80 by warps, 240 86 and 89, 810 283 and 142.
+__device__ inline RowRule row_rule(int64_t products, int64_t rows) {
+  constexpr int64_t kSms = 148, kLaneWarps = kSms * 16;
   RowRule r;
   r.wide32 = max(r.wide32, products / (kSms * 24));
   r.wide128 = max(r.wide128, products / (kSms * 12));
   r.wide256 = max(r.wide256, products / (kSms * 6));
+  r.lane = rows >= 16 * kLaneWarps ? INT64_MAX : 1500 * rows / (130 * kLaneWarps - 8 * rows);
   return r;
 }
 __host__ __device__ inline int sym_class(int64_t f, int64_t n, const Tune &t) {
@@ -154,7 +161,7 @@ __host__ __device__ inline int64_t onepass_bound(int64_t f, int64_t n, const Tun
 }
 __host__ __device__ inline int num_class(int64_t c, int64_t f, const Tune &t, const RowRule &r) {
   if (c == 0 || f < 0) return -1;  // f < 0: a one-pass row, already computed
-  if (c <= t.lane) return CLS_LANE;
+  if (c <= t.lane && f <= r.lane) return CLS_LANE;
   if (c <= t.num[0]) return wide_class(CLS_G32, f, r);
   if (c <= t.num[1]) return wide_class(CLS_G128, f, r);
   if (c <= t.num[2]) return wide_class(CLS_G256, f, r);
@@ -325,7 +332,7 @@ __device__ __forceinline__ void sched_offsets(Sched *S) {
   S->work2 = 0;
   S->work3 = 0;
   S->rank_left = 0;
-  S->rule = row_rule(*(volatile int64_t *)&S->total);
+  S->rule = row_rule(*(volatile int64_t *)&S->total, *(volatile int64_t *)&S->nonempty);
 }
 
 // int32 row offsets widened to int64 (operands of mixed offset widths).

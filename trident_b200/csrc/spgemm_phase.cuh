@@ -2367,19 +2367,20 @@ __global__ void __launch_bounds__(kOnepassThreads, 1)
       mine = load_meta<FINAL>(prods, A, base + i + lane);
       if (!FINAL) mine.off = A.cp[mine.g];  // the row's scratch offset
     }
-    // lanes in step take as long as the longest row: ~40 instructions a
-    // product and ~36 an A entry, its B row empty or not (and the loads of
-    // each lane's entry); a warp per row ~350, 6 a product and next to nothing
-    // an entry.  70,000 rows of 2 to 16 products: 128 A entries each 183 us by
-    // lanes, 232 by warps; 256 each 352 and 286; 512 in one row of 32 257 and
-    // 215; 1024 444 and 222 (numeric phase).
+    // Issue slots: lanes in step take as long as the longest row, ~130 a product
+    // and ~200 an A entry, its B row empty or not (with ~3 for the loads of
+    // each lane's entry); a warp per row ~1500 and 8 a product.  Numeric phase,
+    // 32 rows a warp (300,000 rows, 324 products): lanes 0.56 ms, warps 0.92; 9
+    // rows (20,000 rows): 144 products 59 and 80 us, 240 86 and 89, 810 283 and
+    // 142.  70,000 rows of 2 to 16 products: 128 A entries each 183 us by lanes,
+    // 232 by warps; 256 each 352 and 286; 1024 in one row of 32 444 and 222.
     constexpr int64_t kFar = 1 << 24;  // the 32 in one int
     const int f = int(min(mine.f, kFar)), na = int(min(mine.a1 - mine.a0, kFar));
     const int fmax = __reduce_max_sync(0xffffffffu, f), namax = __reduce_max_sync(0xffffffffu, na);
     const int fsum = __reduce_add_sync(0xffffffffu, f), nasum = __reduce_add_sync(0xffffffffu, na);
     const int p0 = __shfl_sync(0xffffffffu, mine.p, 0);
-    const bool lanes = 40 * int64_t(fmax) + 36 * int64_t(namax) + nasum / 2 <=
-                           350 * int64_t(rows) + 6 * int64_t(fsum) &&
+    const bool lanes = 130 * int64_t(fmax) + 200 * int64_t(namax) + 3 * int64_t(nasum) <=
+                           1500 * int64_t(rows) + 8 * int64_t(fsum) &&
                        __all_sync(0xffffffffu, !have || mine.p == p0);
     unsigned todo = __ballot_sync(0xffffffffu, have);
     if (lanes) todo = lane_rows<FINAL, PT, VT>(prods[p0], A, mine, have, slice, lane);
