@@ -373,3 +373,16 @@ def test_budget_goes_to_the_cursors_before_the_kept_bitmaps():
         check_product(ops.spgemm(t, dA, dB), A, B)
         t.close()
     c.close()
+
+
+@pytest.mark.parametrize("na", [23, 24])
+@pytest.mark.parametrize("cols", [28, 32, 33, 48, 50, 64, 98, 99, 128, 190])
+def test_warp_rows_of_many_products_an_output(na, cols):
+    # both sides of the rule between the hash and the span form of a warp row
+    from test_gpu_tuning import _alike_rows
+    A, B = _alike_rows(4500, na, cols)
+    c = ops.Context(0)
+    plan = ops.Plan(c, A.to_device(), B.to_device())
+    check_product(plan.numeric(A.to_device(), B.to_device()), A, B)
+    plan.close()
+    c.close()

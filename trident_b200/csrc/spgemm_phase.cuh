@@ -1237,6 +1237,17 @@ constexpr int64_t kSeqRow = 16;  // half of a warp's lanes busy in a B row
 constexpr int kSpanWarpBytes = kSpanWarpBits / 8 + kSpanWarpBits / 32 + int(kNumLim32) * 12;
 static_assert(kSpanWarpBytes <= kTableSmem / (kGroupThreads / 32), "warp slice");
 
+// ... where the hash form walks the products once and the span form twice: rows
+// of 24 products or more an output, whose table is lightly loaded (few probes)
+// or has the copies of the rows of at most 32 outputs.  70,000 rows of 32
+// products an output, hash and span: 40 outputs 0.73 and 0.88 ms, 64 (half the
+// slots taken) 1.75 and 0.95; 5,000 rows of 64: 40 outputs 0.15 and 0.19 ms,
+// 150 0.43 and 0.49.
+__device__ __forceinline__ bool hash_warp_row(const RowMeta &m, const Tune &t) {
+  if (m.f < 24 * m.c) return false;
+  return m.c <= 32 || 13 * m.c <= 5 * int64_t(pow2_at_least(t.load * m.c, 32));
+}
+
 // False (nothing done) when the row's span does not fit.
 template <typename PT, typename VT>
 __device__ bool num_span_warp_row(const ProdDev<PT, VT> *prods, const PhaseArgs &A,
@@ -1986,7 +1997,8 @@ __device__ void group_rows(const ProdDev<PT, VT> *prods, const PhaseArgs &A,
         const RowMeta m = shfl_meta(mine, t);
         if constexpr (NUM) {
           const ProdDev<PT, VT> &P = prods[m.p];
-          const bool span = !P.Ej && m.f > kSpanWarpMin && (P.b_strict || P.n <= kSpanWarpBits);
+          const bool span = !P.Ej && m.f > kSpanWarpMin && (P.b_strict || P.n <= kSpanWarpBits) &&
+                            !hash_warp_row(m, A.S->tune);
           if (span && num_span_warp_row<PT, VT>(prods, A, m, slice, lane)) {
           } else if (esc_fits(m, TMAXN / 2))
             num_esc_row<G, TMAXN, PT, VT>(prods, A, m, slice, gm, gid, lane);
