@@ -386,3 +386,28 @@ def test_warp_rows_of_many_products_an_output(na, cols):
     check_product(plan.numeric(A.to_device(), B.to_device()), A, B)
     plan.close()
     c.close()
+
+
+@pytest.mark.parametrize("cols", [26, 27, 28, 31, 32, 33, 200])
+@pytest.mark.parametrize("late", [False, True])
+def test_one_pass_rows_at_the_lanes_and_the_warps_bound(cols, late):
+    # one-pass rows that a lane, a warp or neither holds, their columns in every B
+    # row or spread over them; counted at once (table and products that fit) or
+    # later; every fourth stretch of rows is short, so warps change their mind
+    m, groups, na, rng = 66000, 40, 12, np.random.default_rng(cols)
+    width = 200
+    B_rows, per = [], -(-cols // na) + 3
+    for g in range(groups):
+        mine = np.sort(rng.choice(width, size=cols if g % 4 else 9, replace=False))
+        for t in range(na):
+            part = mine if not late or g % 4 == 0 else np.unique(np.r_[mine[:3], np.roll(mine, -t * (cols // na + 1))[:per]])
+            B_rows.append(g * width + np.sort(part))
+    rp = np.concatenate([[0], np.cumsum([len(r) for r in B_rows])]).astype(np.int64)
+    B = HostCSR(groups * na, groups * width, rp, np.concatenate(B_rows).astype(np.int32), rng.uniform(-1, 1, rp[-1]))
+    g = np.arange(m) * groups // m
+    A = HostCSR(m, groups * na, np.arange(m + 1, dtype=np.int64) * na,
+                (g[:, None] * na + np.arange(na)).ravel().astype(np.int32), rng.uniform(-1, 1, m * na))
+    c = ops.Context(0)
+    check_product(ops.spgemm(c, A.to_device(), B.to_device()), A, B)
+    c.close()
+

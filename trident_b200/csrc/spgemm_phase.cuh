@@ -209,12 +209,16 @@ __device__ __forceinline__ uint32_t warp_chunk(const int32_t *__restrict__ Bj,
 // flight), each finding its entry as the last one whose first product number
 // is <= its own.  G = 32 keeps the per-entry data in registers (warp_chunk);
 // larger groups stage it in `stage` (24 bytes per lane of shared memory).
-template <int G, bool NUM, typename PT, typename VT, typename F>
+// stop (G = 32): true, for the whole warp, ends the walk after a chunk.
+struct NeverStop {
+  __device__ __forceinline__ bool operator()() const { return false; }
+};
+template <int G, bool NUM, typename PT, typename VT, typename F, typename S = NeverStop>
 __device__ __forceinline__ void for_products_flat(
     const int32_t *__restrict__ Aj, const VT *__restrict__ Ax,
     const PT *__restrict__ Bp, const int32_t *__restrict__ Bj,
     const VT *__restrict__ Bx, int64_t a0, int64_t a1, int lane, int gid,
-    int64_t *tmp, unsigned char *stage, F &&fn) {
+    int64_t *tmp, unsigned char *stage, F &&fn, S &&stop = S()) {
   constexpr int U = 4;
   int64_t *spre = (int64_t *)stage;
   int64_t *sb0 = spre + G;
@@ -237,6 +241,7 @@ __device__ __forceinline__ void for_products_flat(
       if (c0 + 32 + lane < a1) knext = __ldg(Aj + c0 + 32 + lane);
       warp_chunk<NUM, IX, VT>(Bj, Bx, b0, len, a, lane,
                               [&](uint32_t, int32_t c, VT v) { fn(c, v); });
+      if (stop()) break;
       continue;  // no staging to guard
     } else {
       IX tot;
@@ -795,14 +800,20 @@ __device__ __forceinline__ int warp_lean_output(const PhaseArgs &A, int *keys, c
   return nt;
 }
 
+// A refused one-pass row of at most this table and these products is counted by
+// its warp there and then; larger ones wait for 256 threads each (500,000 rows
+// of 384 products on 32 columns: a call 2.6 ms, all of them waiting 7.0).
+constexpr int kRefusedT = 2048;
+constexpr int64_t kRefusedF = 16384;
+
 // ONEPASS (rows of a plain product taken by a warp in the symbolic launch):
 // m.off is the row's scratch offset; the row is written to the scratch
 // (A.oj / A.ox) with the count found here, which goes to rowc, and rowf
 // becomes -1 - offset (the numeric launch copies the row into C and skips it
 // otherwise).  A row whose bound min(products, ncols) needs more than 64
-// slots and which holds kCappedCols columns or more is instead listed in
-// A.defer for the two-pass path (its symbolic count follows in the same
-// launch sequence).
+// slots and which holds kCappedCols columns or more is a two-pass row instead:
+// counted here, or listed in A.defer (its symbolic count then follows in the
+// same launch sequence).
 template <int G, int TMAX, typename PT, typename VT, bool ONEPASS = false>
 __device__ void num_hash_row(const ProdDev<PT, VT> *prods, const PhaseArgs &A,
                              const RowMeta &m, unsigned char *slice, const GroupMem &gm,
@@ -862,7 +873,21 @@ __device__ void num_hash_row(const ProdDev<PT, VT> *prods, const PhaseArgs &A,
       }
       atomicAdd(myv + h, v);
     };
-    if constexpr (G <= 256) {
+    if constexpr (ONEPASS) {
+      bool wide = false;  // a B row that is too long by itself
+      if (capped) {
+        const int64_t k = a0 + lane < a1 ? __ldg(P.Aj + a0 + lane) : -1;
+        wide = k >= 0 && int64_t(__ldg(P.Bp + k + 1)) - int64_t(__ldg(P.Bp + k)) >= kCappedCols;
+        wide = __any_sync(0xffffffffu, wide);
+        if (wide && lane == 0) ocnt[1] = 1;
+      }
+      if (!wide)
+        for_products_flat<G, true, PT, VT>(P.Aj, P.Ax, P.Bp, P.Bj, P.Bx, a0, a1, lane, gid, gm.tmp,
+                                           gm.stage, ins, [&]() {
+                                             __syncwarp();
+                                             return capped && ((volatile int *)ocnt)[1] != 0;
+                                           });
+    } else if constexpr (G <= 256) {
       for_products_flat<G, true, PT, VT>(P.Aj, P.Ax, P.Bp, P.Bj, P.Bx, a0, a1, lane, gid,
                                          gm.tmp, gm.stage, ins);
     } else {
@@ -876,8 +901,10 @@ __device__ void num_hash_row(const ProdDev<PT, VT> *prods, const PhaseArgs &A,
     if (capped) {
       const bool refused = ((volatile int *)ocnt)[1] != 0;
       __syncwarp();
-      if (refused) {  // 32 columns or more: the two-pass path
-        if (lane == 0) {
+      if (refused) {  // 32 columns or more: the two-pass path, its count at once if the slice holds it
+        if (int64_t(A.S->tune.load) * c <= kRefusedT && m.f <= kRefusedF) {
+          sym_hash_row<32, kRefusedT, PT, VT>(prods, A, m, (int *)slice, gm, gid, lane);
+        } else if (lane == 0) {
           const unsigned long long i = atomicAdd(&A.S->ndefer, 1ull);
           A.defer[i] = (uint64_t(m.p) << 40) | uint64_t(m.r);
         }
@@ -2156,7 +2183,7 @@ constexpr int kLaneSlots = 27;
 constexpr int kOnepassSlice = kLaneSlots * 32 * 14;
 constexpr int kOnepassSmem = (kOnepassThreads / 32) * kOnepassSlice;
 static_assert(kOnepassSmem + kOnepassThreads * 4 <= 195 * 1024, "the L1's share");
-static_assert(kNumT32 * 12 <= kOnepassSlice, "the warp form's table");
+static_assert(kNumT32 * 12 <= kOnepassSlice && kRefusedT * 4 <= kOnepassSlice, "the warp forms' tables");
 
 // A lane's running sums keep what their roundings left over (the fast two-sum,
 // on the unrounded product): one lane adds a whole row in order, where a warp's
@@ -2358,6 +2385,9 @@ __global__ void __launch_bounds__(kOnepassThreads, 1)
   unsigned char *slice = smem + w * kOnepassSlice;
   GroupMem gm{};
   gm.lst = lst + w * 32;
+  // one-pass rows: the warp's last rows had more columns than a lane holds, so
+  // the next ones (neighbours, most often alike) go to the warp at once
+  bool shy = false;
   while (true) {
     unsigned long long v = 0;
     if (lane == 0) {
@@ -2393,9 +2423,12 @@ __global__ void __launch_bounds__(kOnepassThreads, 1)
     const int p0 = __shfl_sync(0xffffffffu, mine.p, 0);
     const bool lanes = 130 * int64_t(fmax) + 200 * int64_t(namax) + 3 * int64_t(nasum) <=
                            1500 * int64_t(rows) + 8 * int64_t(fsum) &&
-                       __all_sync(0xffffffffu, !have || mine.p == p0);
+                       !shy && __all_sync(0xffffffffu, !have || mine.p == p0);
     unsigned todo = __ballot_sync(0xffffffffu, have);
-    if (lanes) todo = lane_rows<FINAL, PT, VT>(prods[p0], A, mine, have, slice, lane);
+    if (lanes) {
+      todo = lane_rows<FINAL, PT, VT>(prods[p0], A, mine, have, slice, lane);
+      shy = !FINAL && 2 * __popc(todo) > rows;
+    }
     for (; todo; todo &= todo - 1) {  // by the warp
       const RowMeta m = shfl_meta(mine, __ffs(todo) - 1);
       if constexpr (FINAL) {  // at most kLaneSlots outputs: sorted in registers
@@ -2406,6 +2439,12 @@ __global__ void __launch_bounds__(kOnepassThreads, 1)
       } else {
         num_hash_row<32, kNumT32, PT, VT, true>(prods, A, m, slice, gm, w, lane);
       }
+    }
+    if (!FINAL && !lanes) {
+      __syncwarp();
+      const bool held = have && *(volatile int64_t *)(A.rowf + mine.g) < 0 &&
+                        *(volatile int32_t *)(A.rowc + mine.g) <= kLaneSlots;
+      shy = 2 * __popc(__ballot_sync(0xffffffffu, held)) < rows;
     }
     if (A.prof && lane == 0) {
       atomicAdd(A.prof + CLS_ONEPASS, (unsigned long long)(clock64() - t0));
