@@ -411,3 +411,18 @@ def test_one_pass_rows_at_the_lanes_and_the_warps_bound(cols, late):
     check_product(ops.spgemm(c, A.to_device(), B.to_device()), A, B)
     c.close()
 
+
+
+@pytest.mark.parametrize("na", [23, 24])
+@pytest.mark.parametrize("cols,rows", [(300, 888), (1200, 444), (3000, 148)])
+@pytest.mark.parametrize("less", [0, 1])
+def test_classes_of_many_products_an_output(na, cols, rows, less):
+    # 128-, 256- and 512-thread rows on both sides of the rule between the forms
+    from test_gpu_tuning import _alike_rows
+    A, B = _alike_rows(rows - less, na, cols, groups=10)
+    c = ops.Context(0)
+    plan = ops.Plan(c, A.to_device(), B.to_device())
+    for _ in range(2):
+        check_product(plan.numeric(A.to_device(), B.to_device()), A, B)
+    plan.close()
+    c.close()

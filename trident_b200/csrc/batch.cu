@@ -429,7 +429,7 @@ static int batch_run_impl(tspg_batch *b, cudaStream_t s, int flags) {
                    b->curbuf, b->cur_stride, errw, ctx->d_prof ? ctx->d_prof + kProfPerPhase : nullptr};
       phase_mark(ctx, 1, 0, s);
       const int64_t before = ctx->launches;
-      const int st = launch_numeric_rows<PT, VT>(ctx, s, prods, pa, ncols, tune, nullptr, false,
+      const int st = launch_numeric_rows<PT, VT>(ctx, s, prods, pa, ncols, tune, nullptr, 0, false,
                                                      R < kFuseRows);
       row_kernels = int(ctx->launches - before);
       ctx->launches = before;  // counted at each replay

@@ -335,8 +335,8 @@ static int numeric_impl(tspg_ctx *ctx, cudaStream_t s, tspg_plan *P, const tspg_
     pa.slot_words = P->slot_words;
   }
   phase_mark(ctx, 1, 0, s);
-  TSPG_TRY((launch_numeric_rows<PT, VT>(ctx, s, prods, pa, P->n, P->tune, P->ncnt, m < kFuseRows,
-                                        true)));
+  TSPG_TRY((launch_numeric_rows<PT, VT>(ctx, s, prods, pa, P->n, P->tune, P->ncnt,
+                                        P->c_nnz > 0 ? P->mults / P->c_nnz : 0, m < kFuseRows, true)));
   if (P->onepass)
     k_onepass_copy<PT, VT><<<grid_for(m * 32, 256, ctx->num_sms * 16), 256, 0, s>>>(
         prods, P->rowf, P->rowc, P->cp, P->oj, (const VT *)P->ox, m);

@@ -638,20 +638,32 @@ inline cudaError_t launch_span_class(tspg_ctx *ctx, cudaStream_t s,
                                        overlap);
 }
 
+// Products an output from which a class of many rows (a row or a few for every
+// SM) takes the hash form instead of the span form, which walks the products
+// twice.  Numeric phase, hash and span: 5,000 rows of 20,000 products on 400
+// columns 0.54 and 0.70 ms; 1,000 of 200,000 on 2,000 1.18 and 1.33; 300 of
+// 800,000 on 4,000 1.39 and 2.26; at 20 products an output (5,000 rows on 2,000
+// columns) 1.25 and 1.13.  Fewer rows than that end on the longest one, which
+// the wider span rows finish sooner (200 of 100,000 on 500: 0.42 and 0.23 ms).
+constexpr int64_t kHashPerOut = 24;
 // The persistent kernels of a numeric phase whose products have at most
 // `ncols` columns; tn: the run's row binning (span_tune), the one in its Sched
 // records, by which the rows were classed: a kept plan runs with the tuning of
 // its symbolic call, whatever the context's is by now.  cnt: rows per class
 // when the host knows them (else null).
-// skip_empty: no kernel is launched for an empty class (small products, where
-// a launch counts).
+// per_out: products an output of the run (0: not known).  skip_empty: no kernel
+// is launched for an empty class (small products, where a launch counts).
 template <typename PT, typename VT>
 inline int launch_numeric_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, VT> *prods,
                                PhaseArgs pa, int64_t ncols, const Tune &tn, const int64_t *cnt,
-                               bool skip_empty, bool may_overlap) {
+                               int64_t per_out, bool skip_empty, bool may_overlap) {
   TSPG_CUDA(ctx, launch_dense_cluster<PT, VT>(ctx, s, prods, pa, tn.cluster));
   auto rows = [&](int c) { return cnt ? cnt[c] : int64_t(-1); };
   auto some = [&](int c) { return !skip_empty || rows(c) != 0; };
+  // many rows of many products an output: the hash forms, which walk them once
+  auto hashed = [&](int c, int per_sm) {
+    return per_out >= kHashPerOut && rows(c) >= int64_t(per_sm) * ctx->num_sms;
+  };
   const int64_t dense = cnt ? cnt[CLS_DENSE0] + cnt[CLS_DENSE1] + cnt[CLS_DENSE2] : -1;
   const uint32_t nb = uint32_t((ncols + 1023) >> 10);
   bool overlap = false;  // the first kernel of the phase starts after the binning
@@ -666,7 +678,7 @@ inline int launch_numeric_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, 
     ctx->launches += 1;
     overlap = may_overlap;
   }
-  if (span_ctas<512>(span_layout<512, true, PT, VT>(ncols, uint32_t(tn.num[3]))) >= 1) {
+  if (!hashed(CLS_G1024, 1) && span_ctas<512>(span_layout<512, true, PT, VT>(ncols, uint32_t(tn.num[3]))) >= 1) {
     pa.skip |= 1u << CLS_G1024;
     if (some(CLS_G1024)) {
       TSPG_CUDA(ctx, (launch_span_class<512>(ctx, s, prods, pa, ncols, uint32_t(tn.num[3]),
@@ -674,7 +686,7 @@ inline int launch_numeric_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, 
       overlap = may_overlap;
     }
   }
-  if (span_ctas<256>(span_layout<256, true, PT, VT>(ncols, uint32_t(tn.num[2]))) >= 2) {
+  if (!hashed(CLS_G256, 3) && span_ctas<256>(span_layout<256, true, PT, VT>(ncols, uint32_t(tn.num[2]))) >= 2) {
     pa.skip |= 1u << CLS_G256;
     if (some(CLS_G256)) {
       TSPG_CUDA(ctx, (launch_span_class<256>(ctx, s, prods, pa, ncols, uint32_t(tn.num[2]),
@@ -682,7 +694,7 @@ inline int launch_numeric_rows(tspg_ctx *ctx, cudaStream_t s, const ProdDev<PT, 
       overlap = may_overlap;
     }
   }
-  if (span_ctas<128>(span_layout<128, true, PT, VT>(ncols, uint32_t(tn.num[1]))) >= 2) {
+  if (!hashed(CLS_G128, 6) && span_ctas<128>(span_layout<128, true, PT, VT>(ncols, uint32_t(tn.num[1]))) >= 2) {
     pa.skip |= 1u << CLS_G128;
     if (some(CLS_G128)) {
       TSPG_CUDA(ctx, (launch_span_class<128>(ctx, s, prods, pa, ncols, uint32_t(tn.num[1]),
