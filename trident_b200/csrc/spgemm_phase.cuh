@@ -2218,10 +2218,11 @@ __device__ __forceinline__ VT with_rest(VT sum, uint16_t rest) {
 // 32 rows by one warp, a lane each: lane l walks row l's A entries in step
 // with the others (the next entry's B row bounds and the one after's column
 // in flight) and adds every product into its own kLaneSlots-slot hash table in
-// shared memory, [slot][lane]: no atomics, no bank conflicts.  The occupied
-// slots are sorted by insertion as they are gathered, and written out.  Returns
-// the lanes whose one-pass row has more than kLaneSlots columns.  (A list searched from the last hit on instead of the table: 105-148
-// instructions a product, Galerkin A·P 3.0 ms.)
+// shared memory, [slot][lane]: no atomics, no bank conflicts (of the 16-bit
+// rests two lanes share a bank).  The occupied slots are sorted by insertion as
+// they are gathered, and written out.  Returns the lanes whose one-pass row has
+// more than kLaneSlots columns.  (A list searched from the last hit on instead
+// of the table: 105-148 instructions a product, Galerkin A·P 3.0 ms.)
 //
 // Rows this short spend a warp's time on what surrounds the products (a warp
 // per row: ~1040 warp instructions for the 119 products of a Galerkin A·P
